@@ -48,6 +48,13 @@ struct lcmc_ctx {
     double *d_cell_abs = nullptr;
     int *d_cell_fp64 = nullptr;
     int *d_p2c = nullptr, *d_resc_count = nullptr, *d_resc_list = nullptr;
+    // FP64 colour phases (allocated when a replica first needs them)
+    int *d_ex_p = nullptr;
+    long long *d_ex_r = nullptr;
+    unsigned char *d_ex_flag = nullptr;
+    double2 *d_ex_rows = nullptr;
+    long long ex_cap = 0, ex_alloc = 0;
+    int ex_act = 0, ex_nb = 1;
     int nphase = 8; // colour phases per sweep (LCMC_MAX_COLOURS with a fine-grid replica)
     // Replica groups of a batch: the colour phases of each group run on their
     // own stream (a branch of the sweep graph between the rebin and the
@@ -514,6 +521,13 @@ static DevView view(const lcmc_ctx *c, int parity)
     v.r_hi = c->R;
     v.ngroup = c->ngroup;
     v.resc_list = c->d_resc_list;
+    v.ex_p = c->d_ex_p;
+    v.ex_r = c->d_ex_r;
+    v.ex_flag = c->d_ex_flag;
+    v.ex_rows = c->d_ex_rows;
+    v.ex_cap = c->ex_cap;
+    v.ex_act = c->ex_act;
+    v.ex_nb = c->ex_nb;
     v.rec_dE = c->d_rec_dE;
     v.rec_lu = c->d_rec_lu;
     v.outcome = c->d_outcome;
@@ -561,7 +575,8 @@ static void free_ctx(lcmc_ctx *c)
                     c->d_perm, c->d_scid, c->d_cell_count, c->d_cell_start, c->d_block_sums, c->d_flag, c->d_cell_e0,
                     c->d_cell_e1, c->d_cell_n0, c->d_cell_n1, c->d_cell_pairs, c->d_cell_cands, c->d_outcome,
                     c->d_pe0, c->d_pe1, c->d_phard, c->d_red, c->d_red_part, c->d_cell_abs, c->d_cell_fp64,
-                    c->d_rec_dE, c->d_rec_lu, c->d_p2c, c->d_resc_count, c->d_resc_list};
+                    c->d_rec_dE, c->d_rec_lu, c->d_p2c, c->d_resc_count, c->d_resc_list, c->d_ex_p, c->d_ex_r, c->d_ex_flag,
+                    c->d_ex_rows};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (int k = 0; k < 8; k++)
@@ -994,6 +1009,7 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
     enqueue_rebin(c, parity);
     cudaEventRecordWithFlags(c->ev[1], c->stream, cudaEventRecordExternal);
     DevView v = view(c, parity ^ 1);
+    if (c->any_exact) launch_exact_offsets(v, c->stream);
     if (c->ngroup > 1) cudaEventRecord(c->ev_fork, c->stream);
     for (int g = 0; g < c->ngroup; g++) {
         // group g's phases: its replicas' cells, its own hand-over lists, its own stream
@@ -1002,6 +1018,7 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
         vg.r_hi = c->grp_hi[g];
         vg.resc_count = c->d_resc_count + (size_t)g * c->nphase;
         vg.resc_list = c->d_resc_list + (size_t)g * c->nphase * c->ctot;
+        if (c->d_ex_rows) vg.ex_rows = c->d_ex_rows + (size_t)g * c->ex_alloc * 32;
         cudaStream_t sg = g == 0 ? c->stream : c->side[g];
         if (g > 0) cudaStreamWaitEvent(sg, c->ev_fork, 0);
         for (int ci = 0; ci < c->nphase; ci++) {
@@ -1033,6 +1050,36 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
     launch_sweep_advance(v, c->stream);
     if (c->hist_cap > 0) launch_hist_record(v, c->stream);
     cudaEventRecordWithFlags(c->ev[4], c->stream, cudaEventRecordExternal);
+}
+
+// Scratch of the FP64 colour phases, one set of records per replica group.
+// Active cells of a phase: at most ceil(nc / 2) per axis (two or three colours).
+static int ensure_exact_scratch(lcmc_ctx *c)
+{
+    if (!c->any_exact || c->d_ex_rows) return LCMC_OK;
+    long long act = 0;
+    int most = 1; // particles of the largest replica group
+    for (int r = 0; r < c->R; r++) {
+        const long long h = (c->rep[r].nc_max + 1) / 2;
+        act += h * h * h;
+    }
+    for (int g = 0; g < c->ngroup; g++) {
+        int n = 0;
+        for (int r = c->grp_lo[g]; r < c->grp_hi[g]; r++) n += c->rep[r].n;
+        most = std::max(most, n);
+    }
+    long long cap, alloc;
+    exact_scratch_size(most, &cap, &alloc, &c->ex_nb);
+    const size_t np = (size_t)c->nphase;
+    if (!c->d_ex_p) CUDA_TRY(c, dalloc(&c->d_ex_p, np * (act + 1)));
+    if (!c->d_ex_r) CUDA_TRY(c, dalloc(&c->d_ex_r, np * (act + 1)));
+    if (!c->d_ex_flag) CUDA_TRY(c, dalloc(&c->d_ex_flag, np * act));
+    CUDA_TRY(c, dalloc(&c->d_ex_rows, (size_t)c->ngroup * alloc * 32));
+    c->ex_act = (int)act;
+    c->ex_cap = cap;
+    c->ex_alloc = alloc;
+    exact_init();
+    return LCMC_OK;
 }
 
 static int check_flags(lcmc_ctx *c)
@@ -1139,6 +1186,8 @@ extern "C" int lcmc_sweep(lcmc_ctx *ctx, int n_sweeps)
     for (int s = 0; s < n_sweeps; s++) {
         const int par = ctx->cur;
         if (!ctx->graph[par]) {
+            int rc = ensure_exact_scratch(ctx);
+            if (rc) return rc;
             cudaGraph_t g;
             CUDA_TRY(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
             enqueue_sweep(ctx, par);
@@ -1219,11 +1268,13 @@ extern "C" int lcmc_get_stream(lcmc_ctx *ctx, void **stream)
 extern "C" int lcmc_kernels_per_sweep(lcmc_ctx *ctx)
 {
     if (!ctx) return LCMC_EINVAL;
-    // rebin: setup, bin, 3 scan, scatter, sort, gather; phases, per replica group (FP32: with the FP64 hand-over
-    // kernel); statistics: chunk sums, sums; volume: propose,
+    // rebin: setup, bin, 3 scan, scatter, sort, gather; phases, per replica group (FP64: offsets, then terms and
+    // decisions per batch of cells; FP32: with the FP64 hand-over kernel); statistics: chunk sums, sums; volume: propose,
     // energy, chunk sums, accept, scale; surrogate: 2 feature kernels, 2 GEMMs + 3 small kernels, stage 1;
     // recording; history: chunk sums, rows; sweep counter
-    int n = 8 + ctx->ngroup * ctx->nphase * ((int)ctx->any_exact + 2 * (int)ctx->any_fast) + 5 * (int)ctx->any_npt + 3;
+    const int exact = ctx->any_exact ? 2 * ctx->ex_nb : 0;
+    int n = 8 + (int)ctx->any_exact + ctx->ngroup * ctx->nphase * (exact + 2 * (int)ctx->any_fast) +
+            5 * (int)ctx->any_npt + 3;
     if (ctx->any_npt && (ctx->any_da || ctx->rec_cap > 0)) n += 2;
     if (ctx->any_npt && ctx->any_da) n += 6;
     if (ctx->any_npt && ctx->any_screen) n += 3; // screen energies, chunk sums, stage 1

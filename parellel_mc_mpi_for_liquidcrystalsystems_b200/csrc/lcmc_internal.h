@@ -143,12 +143,21 @@ struct DevView {
                                // (per group: a group's view points at its own nphase counts and lists)
     int *resc_list;            // [nphase x ctot] their codes: cell * 4 + mode (1 large term, 2 capacity)
     int *cell_fp64;            // per cell: 0 FP32, 1 attempted in FP64 (large term), 2 (capacity)
+    // FP64 colour phases: per phase the particle and record-row prefixes over the
+    // active cells ([nphase][ex_act + 1]), cells attempted sequentially
+    // ([nphase][ex_act]), and the scratch of ex_cap rows of 32 double2 per batch
+    int *ex_p;
+    long long *ex_r;
+    unsigned char *ex_flag;
+    double2 *ex_rows;
+    long long ex_cap;
+    int ex_act, ex_nb;
     unsigned char *outcome;    // [ntot] by particle slot of id: 0/1/2
     double *rec_dE, *rec_lu;   // [ntot] by particle slot of id: dE and log u of the last sweep (null: off)
     double *scratch_d;         // [R * 8] small reductions
     double *red_part;          // [R x red_nchunk x LCMC_RED_K] per-chunk partial sums
     int red_nchunk;            // chunks of LCMC_RED_CHUNK particles per replica (largest replica)
-    // this sweep's trial moves, by sorted slot (FP32 kernel systems)
+    // this sweep's trial moves, by sorted slot (tdU and the displacement: FP32 kernel systems)
     double *tnx, *tny, *tnz;   // new position, wrapped
     double *tux, *tuy, *tuz;   // new orientation, normalised
     double *tdU;               // colloid-term change

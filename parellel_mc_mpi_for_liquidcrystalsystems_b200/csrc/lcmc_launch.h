@@ -14,6 +14,9 @@ void launch_sweep_stats(const DevView &v, cudaStream_t s);
 void launch_sweep_advance(const DevView &v, cudaStream_t s);
 
 // lcmc_sweep_exact.cu (FP64, bit-identical to the CPU oracle)
+void exact_init(); // before the first FP64 colour phase
+void exact_scratch_size(int ntot, long long *cap, long long *alloc, int *nb);
+void launch_exact_offsets(const DevView &v, cudaStream_t s); // after the rebin, before the colour phases
 void launch_phase_exact(const DevView &v, cudaStream_t s, int ci, int grid);
 void launch_energy_exact(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int scaled, int grid);
 int energy_exact_blocks_per_sm(); // resident blocks of 128 threads per SM

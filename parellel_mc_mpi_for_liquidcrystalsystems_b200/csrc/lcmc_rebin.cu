@@ -231,10 +231,10 @@ __global__ void k_sort_cells(DevView v)
     }
 }
 
-// Permute into the other buffer and, for systems on the FP32 kernel, build
-// this sweep's trial move of every particle (a particle is attempted once per
-// sweep from its sweep-start state, so the trial is known now): new state,
-// displacement, colloid-term change, log of the Metropolis draw, hard-core flag.
+// Permute into the other buffer and build this sweep's trial move of every
+// particle (a particle is attempted once per sweep from its sweep-start state,
+// so the trial is known now): new state, log of the Metropolis draw, trial code,
+// and for systems on the FP32 kernel the displacement and colloid-term change.
 __global__ void k_gather(DevView v)
 {
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < v.ntot; g += gridDim.x * blockDim.x) {
@@ -251,27 +251,27 @@ __global__ void k_gather(DevView v)
         v.qid[g] = id;
         v.scid[g] = v.cid[src];
         const Replica &p = v.rep[v.p2r[g]];
-        if (!p.use_fast) continue;
         double rn[3], en[3], dsp[3], u;
         const int ok = make_trial(p, (uint32_t)id, ro, eo, rn, en, dsp, &u);
         const int cl = v.cid[src] - p.cell_off;
         const int cx = cl % p.nc[0], cy = (cl / p.nc[0]) % p.nc[1], cz = cl / (p.nc[0] * p.nc[1]);
         // 0 trial to evaluate, 1 colloid hard-core reject, 3 leaves its cell (rejected)
         const unsigned char code = !ok ? 1 : (leaves_cell(p, cx, cy, cz, ro, dsp) ? 3 : 0);
-        double dU = 0.0;
-        if (code == 0 && p.k.coll_on) dU = colloid_rod(p.k, rn, en, p.L) - colloid_rod(p.k, ro, eo, p.L);
         v.tnx[g] = rn[0];
         v.tny[g] = rn[1];
         v.tnz[g] = rn[2];
         v.tux[g] = en[0];
         v.tuy[g] = en[1];
         v.tuz[g] = en[2];
+        v.tlu[g] = log_unit(u);
+        v.thard[g] = code;
+        if (!p.use_fast) continue;
+        double dU = 0.0;
+        if (code == 0 && p.k.coll_on) dU = colloid_rod(p.k, rn, en, p.L) - colloid_rod(p.k, ro, eo, p.L);
         v.tdx[g] = (float)dsp[0];
         v.tdy[g] = (float)dsp[1];
         v.tdz[g] = (float)dsp[2];
         v.tdU[g] = dU;
-        v.tlu[g] = log_unit(u);
-        v.thard[g] = code;
         // FP32 copy relative to the particle's own cell origin
         const double lx = fold_rel(ro[0], p.shift[0] + (double)cx * p.w[0], 0.5 * p.w[0], p.L[0], 1.0 / p.L[0]);
         const double ly = fold_rel(ro[1], p.shift[1] + (double)cy * p.w[1], 0.5 * p.w[1], p.L[1], 1.0 / p.L[1]);

@@ -5,12 +5,12 @@
 // (MCnptColloid.c:2607-2681, 1758-1854), so the accept/reject sequence equals
 // the oracle's canonical sweep.
 //
-// One warp per active cell.  The particles of the cell are attempted one after
-// another in ascending id (the reference picks a random particle per cycle,
-// MCnptColloid.c:2475; its MPI path loops over an active subcell's particles,
-// 683-700).  For each attempt the 32 lanes split the stencil slots q (q mod 32),
-// sum the old and new pair energies lane-locally in q order and combine them
-// with a xor butterfly: the canonical order the oracle reproduces.
+// The particles of a cell are attempted one after another in ascending id (the
+// reference picks a random particle per cycle, MCnptColloid.c:2475; its MPI path
+// loops over an active subcell's particles, 683-700).  For each attempt the 32
+// lanes of a warp split the stencil slots q (q mod 32), sum the old and new pair
+// energies lane-locally in q order and combine them with a xor butterfly: the
+// canonical order the oracle reproduces.
 #include <cuda_runtime.h>
 
 #include "lcmc_gb.cuh"
@@ -39,154 +39,634 @@ __device__ __forceinline__ double warp_sum_butterfly(double x)
     return x;
 }
 
-__global__ void __launch_bounds__(128) k_phase_exact(DevView v, int ci)
-{
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
-    __shared__ int s_cell[4][27];
-    __shared__ int s_base[4][28];
-    const int *off = v.act_off + ci * (v.R + 1);
-    const int total = off[v.r_hi]; // this launch's replicas: active cells [off[r_lo], off[r_hi])
-    for (int a = off[v.r_lo] + blockIdx.x * nw + wib; a < total; a += gridDim.x * nw) {
-        const int r = find_replica(off, v.R, a);
-        const Replica &p = v.rep[r];
-        if (p.use_fast) continue;
-        const int col = p.perm[ci];
-        const int bx = col % p.kc[0], by = (col / p.kc[0]) % p.kc[1], bz = col / (p.kc[0] * p.kc[1]);
-        const int nc0 = p.nc[0], nc1 = p.nc[1], nc2 = p.nc[2];
-        const int nax = axis_colour_count(nc0, p.kc[0], bx), nay = axis_colour_count(nc1, p.kc[1], by);
-        int loc = a - off[r];
-        const int cx = axis_colour_cell(nc0, p.kc[0], bx, loc % nax);
-        loc /= nax;
-        const int cy = axis_colour_cell(nc1, p.kc[1], by, loc % nay);
-        const int cz = axis_colour_cell(nc2, p.kc[2], bz, loc / nay);
-        const int cell = p.cell_off + (cz * nc1 + cy) * nc0 + cx;
+// An active cell and its stencil, as one warp holds it: kept cells and the
+// prefix of their counts in shared memory, canonical order (dz, dy, dx =
+// -1..1, duplicates of small grids dropped at their first occurrence).
+struct CellView {
+    int r, cell, cx, cy, cz;
+    int ncell; // kept stencil cells
+    int total; // particles in them (the cell's own included)
+    int own;   // kept slot of the cell itself
+    int cs, na; // first slot and count of its particles
+};
 
-        // canonical stencil: dz, dy, dx = -1..1, duplicates dropped at first occurrence
-        int c = -1;
-        if (lane < 27) {
-            int dz = lane / 9 - 1, dy = (lane / 3) % 3 - 1, dx = lane % 3 - 1;
-            int x = (cx + dx + nc0) % nc0, y = (cy + dy + nc1) % nc1, z = (cz + dz + nc2) % nc2;
-            c = p.cell_off + (z * nc1 + y) * nc0 + x;
+// Active cell a (of the colour-phase enumeration) -> replica and coordinates.
+__device__ __forceinline__ void active_cell(const DevView &v, const int *off, int ci, int a, CellView &c)
+{
+    c.r = find_replica(off, v.R, a);
+    const Replica &p = v.rep[c.r];
+    const int col = p.perm[ci];
+    const int bx = col % p.kc[0], by = (col / p.kc[0]) % p.kc[1], bz = col / (p.kc[0] * p.kc[1]);
+    const int nc0 = p.nc[0], nc1 = p.nc[1], nc2 = p.nc[2];
+    const int nax = axis_colour_count(nc0, p.kc[0], bx), nay = axis_colour_count(nc1, p.kc[1], by);
+    int loc = a - off[c.r];
+    c.cx = axis_colour_cell(nc0, p.kc[0], bx, loc % nax);
+    loc /= nax;
+    c.cy = axis_colour_cell(nc1, p.kc[1], by, loc % nay);
+    c.cz = axis_colour_cell(nc2, p.kc[2], bz, loc / nay);
+    c.cell = p.cell_off + (c.cz * nc1 + c.cy) * nc0 + c.cx;
+    c.cs = v.cell_start[c.cell];
+    c.na = v.cell_start[c.cell + 1] - c.cs;
+}
+
+// The stencil of c (every lane of the warp): s_first[k] = first particle slot
+// of kept cell k, s_base[k] = its prefix (s_base[ncell] = total).
+__device__ __forceinline__ void cell_stencil(const DevView &v, CellView &c, int lane, int *s_first, int *s_base)
+{
+    const Replica &p = v.rep[c.r];
+    const int nc0 = p.nc[0], nc1 = p.nc[1], nc2 = p.nc[2];
+    int cc = -1;
+    if (lane < 27) {
+        const int dz = lane / 9 - 1, dy = (lane / 3) % 3 - 1, dx = lane % 3 - 1;
+        const int x = (c.cx + dx + nc0) % nc0, y = (c.cy + dy + nc1) % nc1, z = (c.cz + dz + nc2) % nc2;
+        cc = p.cell_off + (z * nc1 + y) * nc0 + x;
+    }
+    const unsigned same = __match_any_sync(0xffffffffu, cc);
+    const bool keep = lane < 27 && (__ffs(same) - 1) == lane;
+    const unsigned kb = __ballot_sync(0xffffffffu, keep);
+    const unsigned ob = __ballot_sync(0xffffffffu, keep && cc == c.cell);
+    c.ncell = __popc(kb);
+    c.own = __popc(kb & ((ob & (0u - ob)) - 1u));
+    const int slot = __popc(kb & ((1u << lane) - 1u));
+    int first = 0, cnt = 0;
+    if (keep) {
+        first = v.cell_start[cc];
+        cnt = v.cell_start[cc + 1] - first;
+    }
+    int inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    __syncwarp();
+    if (keep) {
+        s_first[slot] = first;
+        s_base[slot] = inc - cnt;
+    }
+    c.total = __shfl_sync(0xffffffffu, inc, 31);
+    if (lane == 0) s_base[c.ncell] = c.total;
+    __syncwarp();
+}
+
+// ---------------------------------------------------------------------------
+// FP64 colour phase in two kernels.
+//
+// What bounds it: the attempts of a cell follow one another, so a warp that
+// walks the stencil for each attempt in turn spends its time in the latency of
+// FP64 distances, divisions and square roots with most of the GPU idle (one
+// warp per active cell: a 1000-rod box has one active cell in a phase).  But
+// only the choice between terms depends on the earlier attempts, not the terms:
+// particle k sees static cells, and each in-cell partner m in its old state or,
+// if m < k was accepted, in its trial state, which is known before the phase
+// (the gather drew every trial move).  So
+//   k_exact_terms   warp per active particle, all cells at once: distances to
+//                   every stencil slot, the in-cutoff terms of the old and the
+//                   trial state through a compacted list with all lanes busy,
+//                   then the lane sums of the canonical order as far as they do
+//                   not depend on a decision;
+//   k_exact_decide  warp per cell: for each attempt in ascending id, the lane
+//                   sums completed with the chosen in-cell terms and the static
+//                   terms after them, the xor butterfly, the Metropolis test.
+// The order of every FP64 addition is the canonical one (lane q mod 32 adds the
+// stencil slots q in increasing q; a term beyond the cutoff adds +0.0, which
+// changes no bit), so outcomes and energies equal the CPU oracle's bit for bit.
+//
+// Record of particle k, rows of 32 double2 (lane = q mod 32, x = old state of k,
+// y = its trial state):
+//   0            ExactHead
+//   1            sums over the static slots before the own cell
+//   2 .. 1+J     own-cell slots, partner in its old state (J chunks of 32 slots)
+//   2+J .. 1+2J  own-cell slots, partner in its trial state
+//   2+2J ..      the lane's static terms after the own cell, in order (nsuf rows)
+// The records of a phase lie in a scratch of ex_cap rows; a phase with more is
+// run in ex_nb batches of cells.  A cell above a capacity (particles, stencil,
+// in-cutoff terms, terms after the own cell in one lane) is attempted by
+// k_exact_decide the sequential way (exact_cell_sequential).
+// ---------------------------------------------------------------------------
+constexpr int EX_NA = 256;   // particles of a cell
+constexpr int EX_CH = 96;    // chunks of 32 stencil slots
+constexpr int EX_ENT = 640;  // in-cutoff terms of a particle
+constexpr int EX_SUF = 12;   // static terms after the own cell, per lane
+constexpr int EX_J = 10;     // most chunks an own cell touches
+constexpr int EX_PFS = 6;    // of the suffix rows, those fetched ahead
+
+__host__ __device__ __forceinline__ int ex_chunks(int na) { return (na + 62) / 32; }
+__host__ __device__ __forceinline__ int ex_rows_per_particle(int na) { return 2 + 2 * ex_chunks(na) + EX_SUF; }
+
+struct ExactHead {
+    double uo, un, lu;          // colloid term of the old and the trial state, log of the Metropolis draw
+    int code, nsuf, nstat, pad; // trial code (thard), suffix rows, in-cutoff static terms
+    unsigned mask[4][EX_J];     // in-cutoff own-cell slots per chunk: (old, old), (trial, old), (old, trial), (trial, trial)
+};
+static_assert(sizeof(ExactHead) <= 512, "one row");
+
+// Per phase: exclusive prefix of the particles and of the record rows over the
+// active cells of replicas on the FP64 kernel.  Block per phase.
+__global__ void __launch_bounds__(1024) k_exact_offsets(DevView v)
+{
+    const int ci = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int *off = v.act_off + ci * (v.R + 1);
+    const int total = off[v.R];
+    int *ep = v.ex_p + (size_t)ci * (v.ex_act + 1);
+    long long *er = v.ex_r + (size_t)ci * (v.ex_act + 1);
+    unsigned char *fl = v.ex_flag + (size_t)ci * v.ex_act;
+    __shared__ long long sp[32], sr[32];
+    long long bp = 0, br = 0;
+    for (int b = 0; b < total; b += 1024) {
+        const int a = b + t;
+        long long np = 0, nr = 0;
+        if (a < total) {
+            CellView c;
+            active_cell(v, off, ci, a, c);
+            const bool mine = !v.rep[c.r].use_fast;
+            const bool fits = c.na <= EX_NA;
+            if (mine && fits) {
+                np = c.na;
+                nr = (long long)c.na * ex_rows_per_particle(c.na);
+            }
+            fl[a] = mine && !fits;
         }
-        unsigned same = __match_any_sync(0xffffffffu, c);
-        bool keep = lane < 27 && (__ffs(same) - 1) == lane;
-        unsigned kb = __ballot_sync(0xffffffffu, keep);
-        int ncell = __popc(kb);
-        int slot = __popc(kb & ((1u << lane) - 1u));
-        if (keep) s_cell[wib][slot] = c;
-        // exclusive prefix of counts over kept cells in slot order
-        int cnt_slot = 0;
-        __syncwarp();
-        if (lane < ncell) cnt_slot = v.cell_start[s_cell[wib][lane] + 1] - v.cell_start[s_cell[wib][lane]];
-        int inc = cnt_slot;
+        long long ip = np, ir = nr;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += y;
+            const long long y = __shfl_up_sync(0xffffffffu, ip, o), z = __shfl_up_sync(0xffffffffu, ir, o);
+            if (lane >= o) {
+                ip += y;
+                ir += z;
+            }
         }
-        if (lane < ncell) s_base[wib][lane] = inc - cnt_slot;
-        if (lane == 31) s_base[wib][ncell] = inc;
-        __syncwarp();
+        if (lane == 31) {
+            sp[w] = ip;
+            sr[w] = ir;
+        }
+        __syncthreads();
+        long long op = bp, orr = br;
+        for (int q = 0; q < 32; q++) {
+            if (q < w) {
+                op += sp[q];
+                orr += sr[q];
+            }
+            bp += sp[q];
+            br += sr[q];
+        }
+        if (a < total) {
+            ep[a] = (int)(op + ip - np);
+            er[a] = orr + ir - nr;
+        }
+        __syncthreads();
+    }
+    if (t == 0) {
+        ep[total] = (int)bp;
+        er[total] = br;
+    }
+}
 
-        const int cs = v.cell_start[cell], ce = v.cell_start[cell + 1];
+// first a in [lo, hi) with x[a] >= key, else hi
+template <typename T, typename K>
+__device__ __forceinline__ int lower_bound_dev(const T *x, int lo, int hi, K key)
+{
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if ((K)x[mid] < key) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+struct ExactBatch {
+    int lo, hi;     // active cells of this batch
+    long long row0; // row prefix that is scratch row 0
+};
+
+__device__ __forceinline__ ExactBatch exact_batch(const DevView &v, const int *off, const long long *er, int b)
+{
+    ExactBatch e;
+    const int a0 = off[v.r_lo], a1 = off[v.r_hi];
+    const long long r0 = er[a0];
+    e.row0 = r0 + (long long)b * v.ex_cap;
+    e.lo = b == 0 ? a0 : lower_bound_dev(er, a0, a1, e.row0);
+    e.hi = lower_bound_dev(er, a0, a1, e.row0 + (long long)v.ex_cap);
+    return e;
+}
+
+__global__ void __launch_bounds__(128) k_exact_terms(DevView v, int ci, int b)
+{
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    __shared__ int s_first[4][27], s_base[4][28];
+    __shared__ unsigned s_mask[4][4][EX_CH];
+    __shared__ unsigned short s_off[4][EX_CH];
+    __shared__ int s_ent[4][EX_ENT];
+    __shared__ double s_val[4][EX_ENT];
+    const int *off = v.act_off + ci * (v.R + 1);
+    const int *ep = v.ex_p + (size_t)ci * (v.ex_act + 1);
+    const long long *er = v.ex_r + (size_t)ci * (v.ex_act + 1);
+    const ExactBatch eb = exact_batch(v, off, er, b);
+    const int p_hi = ep[eb.hi];
+    for (int idx = ep[eb.lo] + blockIdx.x * 4 + wib; idx < p_hi; idx += gridDim.x * 4) {
+        // the last active cell whose prefix is <= idx (cells without particles share their successor's prefix)
+        const int a = lower_bound_dev(ep, eb.lo, eb.hi, idx + 1) - 1;
+        CellView c;
+        active_cell(v, off, ci, a, c);
+        cell_stencil(v, c, lane, s_first[wib], s_base[wib]);
+        const Replica &p = v.rep[c.r];
+        const int k = idx - ep[a], g = c.cs + k;
+        double2 *rec = v.ex_rows + ((size_t)(er[a] - eb.row0) + (size_t)k * ex_rows_per_particle(c.na)) * 32;
+        ExactHead *hd = reinterpret_cast<ExactHead *>(rec);
+        const int code = v.thard[g];
+        if (lane == 0) {
+            hd->code = code;
+            hd->lu = v.tlu[g];
+        }
+        if (code) { // colloid hard core or out of its cell: never evaluated
+            __syncwarp();
+            continue;
+        }
+        const int nch = (c.total + 31) >> 5;
+        if (nch > EX_CH) {
+            if (lane == 0) v.ex_flag[(size_t)ci * v.ex_act + a] = 1;
+            __syncwarp();
+            continue;
+        }
+        const double ro[3] = {v.px[g], v.py[g], v.pz[g]};
+        const double rn[3] = {v.tnx[g], v.tny[g], v.tnz[g]};
+        const double rc2 = p.k.rc2;
+        const int q13 = s_base[wib][c.own];
+        // 1 distances: in-cutoff terms appended to the list, masks per chunk
+        int ne = 0, sc = 0, nstat = 0;
+        for (int h = 0; h < nch; h++) {
+            const int q = 32 * h + lane;
+            bool f0 = false, f1 = false, f2 = false, f3 = false;
+            int j = 0;
+            if (q < c.total) {
+                while (s_base[wib][sc + 1] <= q) sc++;
+                j = s_first[wib][sc] + (q - s_base[wib][sc]);
+                if (j != g) {
+                    double d[3];
+                    const double xj = v.px[j], yj = v.py[j], zj = v.pz[j];
+                    f0 = dist_fold(ro[0], ro[1], ro[2], xj, yj, zj, p.L, d) < rc2;
+                    f1 = dist_fold(rn[0], rn[1], rn[2], xj, yj, zj, p.L, d) < rc2;
+                    if (sc == c.own && j < g && v.thard[j] == 0) { // partner's trial state
+                        const double xt = v.tnx[j], yt = v.tny[j], zt = v.tnz[j];
+                        f2 = dist_fold(ro[0], ro[1], ro[2], xt, yt, zt, p.L, d) < rc2;
+                        f3 = dist_fold(rn[0], rn[1], rn[2], xt, yt, zt, p.L, d) < rc2;
+                    }
+                    if (sc != c.own) nstat += (int)f0 + (int)f1;
+                }
+            }
+            const unsigned b0 = __ballot_sync(0xffffffffu, f0), b1 = __ballot_sync(0xffffffffu, f1);
+            const unsigned b2 = __ballot_sync(0xffffffffu, f2), b3 = __ballot_sync(0xffffffffu, f3);
+            const int n0 = __popc(b0), n1 = __popc(b1), n2 = __popc(b2), n3 = __popc(b3);
+            const bool fits = ne + n0 + n1 + n2 + n3 <= EX_ENT;
+            if (fits) {
+                if (f0) s_ent[wib][ne + __popc(b0 & lt)] = j;
+                if (f1) s_ent[wib][ne + n0 + __popc(b1 & lt)] = j | (1 << 30);
+                if (f2) s_ent[wib][ne + n0 + n1 + __popc(b2 & lt)] = j | (int)(2u << 30);
+                if (f3) s_ent[wib][ne + n0 + n1 + n2 + __popc(b3 & lt)] = j | (int)(3u << 30);
+            }
+            if (lane == 0) {
+                s_mask[wib][0][h] = b0;
+                s_mask[wib][1][h] = b1;
+                s_mask[wib][2][h] = b2;
+                s_mask[wib][3][h] = b3;
+                s_off[wib][h] = (unsigned short)ne;
+            }
+            ne += n0 + n1 + n2 + n3;
+            if (!fits) ne = EX_ENT + 1; // stays above the capacity
+        }
+        if (ne > EX_ENT) {
+            if (lane == 0) v.ex_flag[(size_t)ci * v.ex_act + a] = 1;
+            __syncwarp();
+            continue;
+        }
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) nstat += __shfl_xor_sync(0xffffffffu, nstat, o);
+        __syncwarp();
+        // 2 the listed terms, two per lane and round (independent chains)
+        for (int e0 = 0; e0 < ne; e0 += 64) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int e = e0 + 32 * h + lane;
+                if (e < ne) {
+                    const unsigned u = (unsigned)s_ent[wib][e];
+                    const int j = (int)(u & 0x3fffffffu);
+                    const bool nk = u & (1u << 30), nj = u & (2u << 30);
+                    const double ri[3] = {nk ? rn[0] : ro[0], nk ? rn[1] : ro[1], nk ? rn[2] : ro[2]};
+                    const double ei[3] = {nk ? v.tux[g] : v.ox[g], nk ? v.tuy[g] : v.oy[g], nk ? v.tuz[g] : v.oz[g]};
+                    const double rj[3] = {nj ? v.tnx[j] : v.px[j], nj ? v.tny[j] : v.py[j], nj ? v.tnz[j] : v.pz[j]};
+                    const double ej[3] = {nj ? v.tux[j] : v.ox[j], nj ? v.tuy[j] : v.oy[j], nj ? v.tuz[j] : v.oz[j]};
+                    double d[3];
+                    const double r2 = dist_fold(ri[0], ri[1], ri[2], rj[0], rj[1], rj[2], p.L, d);
+                    s_val[wib][e] = pair_exact(p.k, r2, d, ei, ej);
+                }
+            }
+        }
+        // colloid terms: lane 0 the old state, lane 1 the trial state
+        if (lane < 2 && p.k.coll_on) {
+            const double r3[3] = {lane ? rn[0] : ro[0], lane ? rn[1] : ro[1], lane ? rn[2] : ro[2]};
+            const double e3[3] = {lane ? v.tux[g] : v.ox[g], lane ? v.tuy[g] : v.oy[g], lane ? v.tuz[g] : v.oz[g]};
+            const double u = colloid_rod(p.k, r3, e3, p.L);
+            if (lane == 0) hd->uo = u;
+            else hd->un = u;
+        }
+        __syncwarp();
+        // 3 the lane sums, in slot order
+        const int J = ex_chunks(c.na);
+        const int c0 = q13 >> 5, c1 = (q13 + c.na - 1) >> 5;
+        double po = 0.0, pn = 0.0;
+        int ns = 0;
+        double2 *suf = rec + (size_t)(2 + 2 * J) * 32;
+        for (int h = 0; h < nch; h++) {
+            const unsigned b0 = s_mask[wib][0][h], b1 = s_mask[wib][1][h];
+            const unsigned b2 = s_mask[wib][2][h], b3 = s_mask[wib][3][h];
+            const int o0 = s_off[wib][h], o1 = o0 + __popc(b0);
+            const double t0 = (b0 >> lane) & 1u ? s_val[wib][o0 + __popc(b0 & lt)] : 0.0;
+            const double t1 = (b1 >> lane) & 1u ? s_val[wib][o1 + __popc(b1 & lt)] : 0.0;
+            const int q = 32 * h + lane;
+            const bool mine = q >= q13 && q < q13 + c.na;
+            if (h >= c0 && h <= c1) { // (uniform) a chunk of the own cell: every lane writes both rows
+                const int o2 = o1 + __popc(b1), o3 = o2 + __popc(b2);
+                const double t2 = (b2 >> lane) & 1u ? s_val[wib][o2 + __popc(b2 & lt)] : 0.0;
+                const double t3 = (b3 >> lane) & 1u ? s_val[wib][o3 + __popc(b3 & lt)] : 0.0;
+                rec[(size_t)(2 + h - c0) * 32 + lane] = mine ? make_double2(t0, t1) : make_double2(0.0, 0.0);
+                rec[(size_t)(2 + J + h - c0) * 32 + lane] = mine ? make_double2(t2, t3) : make_double2(0.0, 0.0);
+                const unsigned own = __ballot_sync(0xffffffffu, mine);
+                if (lane == 0) {
+                    hd->mask[0][h - c0] = b0 & own;
+                    hd->mask[1][h - c0] = b1 & own;
+                    hd->mask[2][h - c0] = b2 & own;
+                    hd->mask[3][h - c0] = b3 & own;
+                }
+            }
+            if (q < q13) {
+                po += t0;
+                pn += t1;
+            } else if (!mine && (((b0 | b1) >> lane) & 1u)) {
+                if (ns < EX_SUF) suf[(size_t)ns * 32 + lane] = make_double2(t0, t1);
+                ns++;
+            }
+        }
+        rec[32 + lane] = make_double2(po, pn);
+        int nsuf = ns;
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) nsuf = max(nsuf, __shfl_xor_sync(0xffffffffu, nsuf, o));
+        if (nsuf > EX_SUF) {
+            if (lane == 0) v.ex_flag[(size_t)ci * v.ex_act + a] = 1;
+        } else {
+            for (int s = ns; s < nsuf; s++) suf[(size_t)s * 32 + lane] = make_double2(0.0, 0.0);
+            // chunks J covers beyond the last one the cell touches
+            for (int h = c1 - c0 + 1; h < J; h++) {
+                rec[(size_t)(2 + h) * 32 + lane] = make_double2(0.0, 0.0);
+                rec[(size_t)(2 + J + h) * 32 + lane] = make_double2(0.0, 0.0);
+                if (lane < 4) hd->mask[lane][h] = 0u;
+            }
+            if (lane == 0) {
+                hd->nsuf = nsuf;
+                hd->nstat = nstat;
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// One cell attempted by one warp, attempt after attempt: for every particle
+// the lanes split the stencil slots, evaluate the terms where they are found
+// and combine the lane sums (the canonical order again).  For cells above a
+// capacity of the two-kernel path.
+__device__ __noinline__ void exact_cell_sequential(const DevView *__restrict__ vp, const CellView &c, int lane,
+                                                   const int *s_first, const int *s_base)
+{
+    const DevView &v = *vp;
+    const Replica &p = v.rep[c.r];
+    const int cell = c.cell;
+    const int cs = c.cs, ce = c.cs + c.na;
+    double dE_sum = 0.0, dE_abs = 0.0;
+    int nacc = 0, nhard = 0;
+    unsigned long long npairs = 0ull;
+    const unsigned long long cands = (unsigned long long)(c.total - 1) * (unsigned long long)(ce - cs);
+    for (int g = cs; g < ce; g++) {
+        const uint32_t id = (uint32_t)v.id[g];
+        const int code = v.thard[g];
+        const double lu = v.tlu[g];
+        if (code) { // colloid hard core (1), out of its cell (3): rejected, no energy evaluation
+            if (lane == 0) {
+                v.outcome[p.p_off + id] = code == 1 ? 2 : 0;
+                if (v.rec_dE) {
+                    v.rec_dE[p.p_off + id] = 0.0;
+                    v.rec_lu[p.p_off + id] = lu;
+                }
+            }
+            nhard += code == 1;
+            continue;
+        }
+        const double ro[3] = {v.px[g], v.py[g], v.pz[g]}, eo[3] = {v.ox[g], v.oy[g], v.oz[g]};
+        const double rn[3] = {v.tnx[g], v.tny[g], v.tnz[g]}, en[3] = {v.tux[g], v.tuy[g], v.tuz[g]};
+        double po = 0.0, pn = 0.0;
+        int np = 0;
+        for (int s = 0; s < c.ncell; s++) {
+            const int B = s_base[s], n_s = s_base[s + 1] - B;
+            const int g0 = s_first[s];
+            for (int q = B + ((lane - B) & 31); q < B + n_s; q += 32) {
+                const int j = g0 + (q - B);
+                if (j == g) continue;
+                const double rj[3] = {v.px[j], v.py[j], v.pz[j]}, ej[3] = {v.ox[j], v.oy[j], v.oz[j]};
+                double d[3];
+                double r2 = dist_fold(ro[0], ro[1], ro[2], rj[0], rj[1], rj[2], p.L, d);
+                if (r2 < p.k.rc2) {
+                    po += pair_exact(p.k, r2, d, eo, ej);
+                    np++;
+                }
+                r2 = dist_fold(rn[0], rn[1], rn[2], rj[0], rj[1], rj[2], p.L, d);
+                if (r2 < p.k.rc2) {
+                    pn += pair_exact(p.k, r2, d, en, ej);
+                    np++;
+                }
+            }
+        }
+        double Eo = warp_sum_butterfly(po);
+        double En = warp_sum_butterfly(pn);
+        if (p.k.coll_on) {
+            Eo = Eo + colloid_rod(p.k, ro, eo, p.L);
+            En = En + colloid_rod(p.k, rn, en, p.L);
+        }
+        const double dE = En - Eo;
+        const bool acc = (dE <= 0.0) || (lu <= -p.k.beta * dE);
+        npairs += (unsigned long long)np;
+        if (acc) {
+            if (lane == 0) {
+                v.px[g] = rn[0];
+                v.py[g] = rn[1];
+                v.pz[g] = rn[2];
+                v.ox[g] = en[0];
+                v.oy[g] = en[1];
+                v.oz[g] = en[2];
+            }
+            dE_sum += dE;
+            dE_abs += fabs(dE);
+            nacc++;
+        }
+        if (lane == 0) {
+            v.outcome[p.p_off + id] = acc ? 1 : 0;
+            if (v.rec_dE) {
+                v.rec_dE[p.p_off + id] = dE;
+                v.rec_lu[p.p_off + id] = lu;
+            }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
+    if (lane == 0) {
+        v.cell_e0[cell] = dE_sum;
+        v.cell_abs[cell] = dE_abs;
+        v.cell_fp64[cell] = 0;
+        v.cell_n0[cell] = nacc;
+        v.cell_n1[cell] = nhard;
+        v.cell_pairs[cell] = npairs;
+        v.cell_cands[cell] = cands;
+    }
+    __syncwarp();
+}
+
+__device__ __forceinline__ void cp_row_async(void *dst, const void *src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+
+// Rows fetched ahead of an attempt, three attempts deep: the scratch rows come
+// from L2, and the chain of one attempt (a dozen additions, ten shuffles, the
+// test) is what remains.
+constexpr int EX_STAGES = 3;
+constexpr int EX_PF = 2 + 2 * EX_J + EX_PFS;
+
+__global__ void __launch_bounds__(32) k_exact_decide(const __grid_constant__ DevView v, int ci, int b)
+{
+    extern __shared__ double2 ex_buf[]; // [EX_STAGES][EX_PF][32]
+    __shared__ int s_first[27], s_base[28];
+    const int lane = threadIdx.x;
+    const int *off = v.act_off + ci * (v.R + 1);
+    const long long *er = v.ex_r + (size_t)ci * (v.ex_act + 1);
+    const ExactBatch eb = exact_batch(v, off, er, b);
+    const int a1 = b == v.ex_nb - 1 ? off[v.r_hi] : eb.hi; // the last batch takes the cells beyond the scratch
+    for (int a = eb.lo + blockIdx.x; a < a1; a += gridDim.x) {
+        CellView c;
+        active_cell(v, off, ci, a, c);
+        const Replica &p = v.rep[c.r];
+        if (p.use_fast) continue;
+        cell_stencil(v, c, lane, s_first, s_base);
+        if (a >= eb.hi || v.ex_flag[(size_t)ci * v.ex_act + a]) {
+            exact_cell_sequential(&v, c, lane, s_first, s_base);
+            continue;
+        }
+        const int na = c.na, J = ex_chunks(na), rpp = ex_rows_per_particle(na);
+        const int npf = 2 + 2 * J + EX_PFS;
+        const double2 *rows = v.ex_rows + (size_t)(er[a] - eb.row0) * 32 + lane;
+        const int q13 = s_base[c.own], c0 = q13 >> 5;
+        const double beta = p.k.beta;
+        const bool coll = p.k.coll_on;
+        auto fetch = [&](int k) {
+            if (k < na) {
+                const double2 *src = rows + (size_t)k * rpp * 32;
+                double2 *dst = ex_buf + (size_t)(k % EX_STAGES) * EX_PF * 32 + lane;
+                for (int i = 0; i < npf; i++) cp_row_async(dst + i * 32, src + (size_t)i * 32);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+#pragma unroll
+        for (int k = 0; k < EX_STAGES - 1; k++) fetch(k);
+        unsigned accm = 0u; // lane j: accepted particles at the slots of chunk c0 + j
         double dE_sum = 0.0, dE_abs = 0.0;
         int nacc = 0, nhard = 0;
         unsigned long long npairs = 0ull;
-        const unsigned long long cands = (unsigned long long)(s_base[wib][ncell] - 1) * (unsigned long long)(ce - cs);
-        for (int g = cs; g < ce; g++) {
-            const uint32_t id = (uint32_t)v.id[g];
-            double ro[3] = {v.px[g], v.py[g], v.pz[g]};
-            double eo[3] = {v.ox[g], v.oy[g], v.oz[g]};
-            double rn[3], en[3], dsp[3], uacc;
-            int ok = make_trial(p, id, ro, eo, rn, en, dsp, &uacc);
-            if (ok && leaves_cell(p, cx, cy, cz, ro, dsp)) { // out of its cell: rejected, no energy evaluation
-                if (lane == 0) {
-                    v.outcome[p.p_off + id] = 0;
-                    if (v.rec_dE) {
-                        v.rec_dE[p.p_off + id] = 0.0;
-                        v.rec_lu[p.p_off + id] = log_unit(uacc);
-                    }
+        for (int k = 0; k < na; k++) {
+            fetch(k + EX_STAGES - 1);
+            asm volatile("cp.async.wait_group %0;" ::"n"(EX_STAGES - 1) : "memory");
+            __syncwarp();
+            const double2 *rw = ex_buf + (size_t)(k % EX_STAGES) * EX_PF * 32 + lane;
+            const ExactHead *hd = reinterpret_cast<const ExactHead *>(rw - lane);
+            const int g = c.cs + k;
+            const int code = hd->code;
+            const double lu = hd->lu;
+            double dE = 0.0;
+            bool acc = false;
+            if (code) {
+                nhard += code == 1;
+            } else {
+                const int nsuf = hd->nsuf;
+                double po = rw[32].x, pn = rw[32].y;
+                for (int j = 0; j < J; j++) {
+                    const unsigned m = __shfl_sync(0xffffffffu, accm, j);
+                    const double2 x = rw[(2 + j + ((m >> lane) & 1u ? J : 0)) * 32];
+                    po += x.x;
+                    pn += x.y;
                 }
-                continue;
-            }
-            if (!ok) {
-                if (lane == 0) {
-                    v.outcome[p.p_off + id] = 2;
-                    if (v.rec_dE) {
-                        v.rec_dE[p.p_off + id] = 0.0;
-                        v.rec_lu[p.p_off + id] = log_unit(uacc);
-                    }
+                for (int s = 0; s < nsuf; s++) {
+                    const double2 x = s < EX_PFS ? rw[(2 + 2 * J + s) * 32]
+                                                 : rows[((size_t)k * rpp + 2 + 2 * J + s) * 32];
+                    po += x.x;
+                    pn += x.y;
                 }
-                nhard++;
-                continue;
-            }
-            double po = 0.0, pn = 0.0;
-            int np = 0;
-            for (int s = 0; s < ncell; s++) {
-                const int B = s_base[wib][s], n_s = s_base[wib][s + 1] - B;
-                const int g0 = v.cell_start[s_cell[wib][s]];
-                for (int q = B + ((lane - B) & 31); q < B + n_s; q += 32) {
-                    const int j = g0 + (q - B);
-                    if (j == g) continue;
-                    double rj[3] = {v.px[j], v.py[j], v.pz[j]};
-                    double ej[3] = {v.ox[j], v.oy[j], v.oz[j]};
-                    double d[3];
-                    double r2 = dist_fold(ro[0], ro[1], ro[2], rj[0], rj[1], rj[2], p.L, d);
-                    if (r2 < p.k.rc2) {
-                        po += pair_exact(p.k, r2, d, eo, ej);
-                        np++;
-                    }
-                    r2 = dist_fold(rn[0], rn[1], rn[2], rj[0], rj[1], rj[2], p.L, d);
-                    if (r2 < p.k.rc2) {
-                        pn += pair_exact(p.k, r2, d, en, ej);
-                        np++;
-                    }
+#pragma unroll
+                for (int o = 16; o >= 1; o >>= 1) {
+                    const double yo = __shfl_xor_sync(0xffffffffu, po, o), yn = __shfl_xor_sync(0xffffffffu, pn, o);
+                    po = po + yo;
+                    pn = pn + yn;
                 }
-            }
-            double Eo = warp_sum_butterfly(po);
-            double En = warp_sum_butterfly(pn);
-            if (p.k.coll_on) {
-                Eo = Eo + colloid_rod(p.k, ro, eo, p.L);
-                En = En + colloid_rod(p.k, rn, en, p.L);
-            }
-            const double dE = En - Eo;
-            const bool acc = (dE <= 0.0) || (log_unit(uacc) <= -p.k.beta * dE);
-            npairs += (unsigned long long)np;
-            if (acc) {
-                if (lane == 0) {
-                    v.px[g] = rn[0];
-                    v.py[g] = rn[1];
-                    v.pz[g] = rn[2];
-                    v.ox[g] = en[0];
-                    v.oy[g] = en[1];
-                    v.oz[g] = en[2];
+                if (coll) {
+                    po = po + hd->uo;
+                    pn = pn + hd->un;
                 }
-                dE_sum += dE;
-                dE_abs += fabs(dE);
-                nacc++;
+                dE = pn - po;
+                acc = (dE <= 0.0) || (lu <= -beta * dE);
+                if (lane < J)
+                    npairs += (unsigned long long)(__popc((hd->mask[0][lane] & ~accm) | (hd->mask[2][lane] & accm)) +
+                                                   __popc((hd->mask[1][lane] & ~accm) | (hd->mask[3][lane] & accm)));
+                if (lane == 0) npairs += (unsigned long long)hd->nstat;
+                if (acc) {
+                    const int q = q13 + k;
+                    if (lane == (q >> 5) - c0) accm |= 1u << (q & 31);
+                    dE_sum += dE;
+                    dE_abs += fabs(dE);
+                    nacc++;
+                }
             }
             if (lane == 0) {
-                v.outcome[p.p_off + id] = acc ? 1 : 0;
+                const int id = v.id[g];
+                v.outcome[p.p_off + id] = code ? (code == 1 ? 2 : 0) : (acc ? 1 : 0);
                 if (v.rec_dE) {
                     v.rec_dE[p.p_off + id] = dE;
-                    v.rec_lu[p.p_off + id] = log_unit(uacc);
+                    v.rec_lu[p.p_off + id] = lu;
                 }
             }
-            __syncwarp();
+            __syncwarp(); // the stage may be refilled
         }
-        // pair counter: sum over lanes
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        // accepted trial states to the master arrays
+        for (int k0 = 0; k0 < na; k0 += 32) {
+            const int k = k0 + lane, q = q13 + k;
+            const unsigned m = __shfl_sync(0xffffffffu, accm, k < na ? (q >> 5) - c0 : 0);
+            if (k < na && ((m >> (q & 31)) & 1u)) {
+                const int g = c.cs + k;
+                v.px[g] = v.tnx[g];
+                v.py[g] = v.tny[g];
+                v.pz[g] = v.tnz[g];
+                v.ox[g] = v.tux[g];
+                v.oy[g] = v.tuy[g];
+                v.oz[g] = v.tuz[g];
+            }
+        }
 #pragma unroll
         for (int o = 16; o >= 1; o >>= 1) npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
         if (lane == 0) {
-            v.cell_e0[cell] = dE_sum;
-            v.cell_abs[cell] = dE_abs;
-            v.cell_fp64[cell] = 0;
-            v.cell_n0[cell] = nacc;
-            v.cell_n1[cell] = nhard;
-            v.cell_pairs[cell] = npairs;
-            v.cell_cands[cell] = cands;
+            v.cell_e0[c.cell] = dE_sum;
+            v.cell_abs[c.cell] = dE_abs;
+            v.cell_fp64[c.cell] = 0;
+            v.cell_n0[c.cell] = nacc;
+            v.cell_n1[c.cell] = nhard;
+            v.cell_pairs[c.cell] = npairs;
+            v.cell_cands[c.cell] = (unsigned long long)(c.total - 1) * (unsigned long long)na;
         }
         __syncwarp();
     }
@@ -362,9 +842,37 @@ __global__ void __launch_bounds__(128, LCMC_ENERGY_MIN_BLOCKS) k_energy_exact(De
 
 namespace lcmc {
 
+// Scratch rows (of 512 bytes) for ntot particles on the FP64 kernel: *cap rows
+// per batch and *nb batches per phase.  Most systems run in one batch; the
+// bound of 256 MB keeps the rows near the L2.  Active particles of a phase are
+// about an eighth of the system (all of it in a one-cell box); cells that the
+// batches do not reach are attempted sequentially.
+void exact_scratch_size(int ntot, long long *cap, long long *alloc, int *nb)
+{
+    const long long most = 256ll << 20 >> 9;
+    const long long all = (long long)ntot * ex_rows_per_particle(EX_NA);
+    *cap = all < most ? all : most;
+    *alloc = *cap + (long long)EX_NA * ex_rows_per_particle(EX_NA);
+    const long long typical = (long long)ntot * ex_rows_per_particle(64) / 4;
+    *nb = all <= most ? 1 : (int)((typical + most - 1) / most) + 1;
+}
+
+void exact_init()
+{
+    cudaFuncSetAttribute(k_exact_decide, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         EX_STAGES * EX_PF * 32 * (int)sizeof(double2));
+}
+
+void launch_exact_offsets(const DevView &v, cudaStream_t s) { k_exact_offsets<<<v.nphase, 1024, 0, s>>>(v); }
+
 void launch_phase_exact(const DevView &v, cudaStream_t s, int ci, int grid)
 {
-    k_phase_exact<<<grid, 128, 0, s>>>(v, ci);
+    const int bytes = EX_STAGES * EX_PF * 32 * (int)sizeof(double2);
+    const int gt = min(grid, (v.ntot + 3) / 4), gd = min(grid, v.ex_act);
+    for (int b = 0; b < v.ex_nb; b++) {
+        k_exact_terms<<<gt, 128, 0, s>>>(v, ci, b);
+        k_exact_decide<<<gd, 32, bytes, s>>>(v, ci, b);
+    }
 }
 
 int energy_exact_blocks_per_sm()
