@@ -120,7 +120,7 @@ __device__ __forceinline__ void cell_stencil(const DevView &v, CellView &c, int 
 // particle k sees static cells, and each in-cell partner m in its old state or,
 // if m < k was accepted, in its trial state, which is known before the phase
 // (the gather drew every trial move).  So
-//   k_exact_terms   warp per active particle, all cells at once: distances to
+//   k_exact_terms   block per active particle, all cells at once: distances to
 //                   every stencil slot, the in-cutoff terms of the old and the
 //                   trial state through a compacted list with all lanes busy,
 //                   then the lane sums of the canonical order as far as they do
@@ -148,10 +148,12 @@ constexpr int EX_NA = 256;   // particles of a cell
 constexpr int EX_CH = 96;    // chunks of 32 stencil slots
 constexpr int EX_ENT = 640;  // in-cutoff terms of a particle
 constexpr int EX_SUF = 12;   // static terms after the own cell, per lane
-constexpr int EX_J = 10;     // most chunks an own cell touches
+constexpr int EX_J = 9;      // most chunks an own cell touches
 constexpr int EX_PFS = 6;    // of the suffix rows, those fetched ahead
 
-__host__ __device__ __forceinline__ int ex_chunks(int na) { return (na + 62) / 32; }
+// chunks of 32 slots that na consecutive slots can touch, rounded up to a class
+// (2, 3, 5, 9) the decisions are unrolled for (chunks beyond the cell's are empty)
+__host__ __device__ __forceinline__ int ex_chunks(int na) { return na <= 33 ? 2 : (na <= 65 ? 3 : (na <= 129 ? 5 : EX_J)); }
 __host__ __device__ __forceinline__ int ex_rows_per_particle(int na) { return 2 + 2 * ex_chunks(na) + EX_SUF; }
 
 struct ExactHead {
@@ -250,58 +252,66 @@ __device__ __forceinline__ ExactBatch exact_batch(const DevView &v, const int *o
     return e;
 }
 
-__global__ void __launch_bounds__(128) k_exact_terms(DevView v, int ci, int b)
+__global__ void __launch_bounds__(128) k_exact_terms(const __grid_constant__ DevView v, int ci, int b)
 {
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    __shared__ int s_first[4][27], s_base[4][28];
-    __shared__ unsigned s_mask[4][4][EX_CH];
-    __shared__ unsigned short s_off[4][EX_CH];
-    __shared__ int s_ent[4][EX_ENT];
-    __shared__ double s_val[4][EX_ENT];
+    __shared__ int s_first[27], s_base[28];
+    __shared__ unsigned s_mask[4][EX_CH];
+    __shared__ unsigned short s_off[EX_CH];
+    __shared__ int s_ent[EX_ENT];
+    __shared__ double s_val[EX_ENT];
+    __shared__ int s_ne, s_nstat;
+    __shared__ CellView s_c;
     const int *off = v.act_off + ci * (v.R + 1);
     const int *ep = v.ex_p + (size_t)ci * (v.ex_act + 1);
     const long long *er = v.ex_r + (size_t)ci * (v.ex_act + 1);
     const ExactBatch eb = exact_batch(v, off, er, b);
     const int p_hi = ep[eb.hi];
-    for (int idx = ep[eb.lo] + blockIdx.x * 4 + wib; idx < p_hi; idx += gridDim.x * 4) {
+    for (int idx = ep[eb.lo] + blockIdx.x; idx < p_hi; idx += gridDim.x) {
         // the last active cell whose prefix is <= idx (cells without particles share their successor's prefix)
         const int a = lower_bound_dev(ep, eb.lo, eb.hi, idx + 1) - 1;
-        CellView c;
-        active_cell(v, off, ci, a, c);
-        cell_stencil(v, c, lane, s_first[wib], s_base[wib]);
+        if (w == 0) {
+            CellView c;
+            active_cell(v, off, ci, a, c);
+            cell_stencil(v, c, lane, s_first, s_base);
+            if (lane == 0) {
+                s_c = c;
+                s_ne = 0;
+                s_nstat = 0;
+            }
+        }
+        __syncthreads();
+        const CellView c = s_c;
         const Replica &p = v.rep[c.r];
         const int k = idx - ep[a], g = c.cs + k;
         double2 *rec = v.ex_rows + ((size_t)(er[a] - eb.row0) + (size_t)k * ex_rows_per_particle(c.na)) * 32;
         ExactHead *hd = reinterpret_cast<ExactHead *>(rec);
         const int code = v.thard[g];
-        if (lane == 0) {
+        if (t == 0) {
             hd->code = code;
             hd->lu = v.tlu[g];
         }
-        if (code) { // colloid hard core or out of its cell: never evaluated
-            __syncwarp();
-            continue;
-        }
         const int nch = (c.total + 31) >> 5;
-        if (nch > EX_CH) {
-            if (lane == 0) v.ex_flag[(size_t)ci * v.ex_act + a] = 1;
-            __syncwarp();
+        // a trial in the colloid or out of its cell is never evaluated
+        if (code || nch > EX_CH) { // (uniform)
+            if (t == 0 && !code) v.ex_flag[(size_t)ci * v.ex_act + a] = 1;
+            __syncthreads();
             continue;
         }
         const double ro[3] = {v.px[g], v.py[g], v.pz[g]};
         const double rn[3] = {v.tnx[g], v.tny[g], v.tnz[g]};
         const double rc2 = p.k.rc2;
-        const int q13 = s_base[wib][c.own];
-        // 1 distances: in-cutoff terms appended to the list, masks per chunk
-        int ne = 0, sc = 0, nstat = 0;
-        for (int h = 0; h < nch; h++) {
+        const int q13 = s_base[c.own];
+        // 1 distances, a chunk of 32 slots per warp: in-cutoff terms appended to the list, masks per chunk
+        int sc = 0, nstat = 0;
+        for (int h = w; h < nch; h += 4) {
             const int q = 32 * h + lane;
             bool f0 = false, f1 = false, f2 = false, f3 = false;
             int j = 0;
             if (q < c.total) {
-                while (s_base[wib][sc + 1] <= q) sc++;
-                j = s_first[wib][sc] + (q - s_base[wib][sc]);
+                while (s_base[sc + 1] <= q) sc++;
+                j = s_first[sc] + (q - s_base[sc]);
                 if (j != g) {
                     double d[3];
                     const double xj = v.px[j], yj = v.py[j], zj = v.pz[j];
@@ -318,115 +328,117 @@ __global__ void __launch_bounds__(128) k_exact_terms(DevView v, int ci, int b)
             const unsigned b0 = __ballot_sync(0xffffffffu, f0), b1 = __ballot_sync(0xffffffffu, f1);
             const unsigned b2 = __ballot_sync(0xffffffffu, f2), b3 = __ballot_sync(0xffffffffu, f3);
             const int n0 = __popc(b0), n1 = __popc(b1), n2 = __popc(b2), n3 = __popc(b3);
-            const bool fits = ne + n0 + n1 + n2 + n3 <= EX_ENT;
-            if (fits) {
-                if (f0) s_ent[wib][ne + __popc(b0 & lt)] = j;
-                if (f1) s_ent[wib][ne + n0 + __popc(b1 & lt)] = j | (1 << 30);
-                if (f2) s_ent[wib][ne + n0 + n1 + __popc(b2 & lt)] = j | (int)(2u << 30);
-                if (f3) s_ent[wib][ne + n0 + n1 + n2 + __popc(b3 & lt)] = j | (int)(3u << 30);
+            int ne = 0;
+            if (lane == 0) ne = atomicAdd(&s_ne, n0 + n1 + n2 + n3);
+            ne = __shfl_sync(0xffffffffu, ne, 0);
+            if (ne + n0 + n1 + n2 + n3 <= EX_ENT) {
+                if (f0) s_ent[ne + __popc(b0 & lt)] = j;
+                if (f1) s_ent[ne + n0 + __popc(b1 & lt)] = j | (1 << 30);
+                if (f2) s_ent[ne + n0 + n1 + __popc(b2 & lt)] = j | (int)(2u << 30);
+                if (f3) s_ent[ne + n0 + n1 + n2 + __popc(b3 & lt)] = j | (int)(3u << 30);
             }
             if (lane == 0) {
-                s_mask[wib][0][h] = b0;
-                s_mask[wib][1][h] = b1;
-                s_mask[wib][2][h] = b2;
-                s_mask[wib][3][h] = b3;
-                s_off[wib][h] = (unsigned short)ne;
+                s_mask[0][h] = b0;
+                s_mask[1][h] = b1;
+                s_mask[2][h] = b2;
+                s_mask[3][h] = b3;
+                s_off[h] = (unsigned short)ne;
             }
-            ne += n0 + n1 + n2 + n3;
-            if (!fits) ne = EX_ENT + 1; // stays above the capacity
         }
-        if (ne > EX_ENT) {
-            if (lane == 0) v.ex_flag[(size_t)ci * v.ex_act + a] = 1;
-            __syncwarp();
+        nstat = __reduce_add_sync(0xffffffffu, nstat);
+        if (lane == 0 && nstat) atomicAdd(&s_nstat, nstat);
+        __syncthreads();
+        const int ne = s_ne;
+        if (ne > EX_ENT) { // (uniform)
+            if (t == 0) v.ex_flag[(size_t)ci * v.ex_act + a] = 1;
+            __syncthreads();
             continue;
         }
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) nstat += __shfl_xor_sync(0xffffffffu, nstat, o);
-        __syncwarp();
-        // 2 the listed terms, two per lane and round (independent chains)
-        for (int e0 = 0; e0 < ne; e0 += 64) {
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int e = e0 + 32 * h + lane;
-                if (e < ne) {
-                    const unsigned u = (unsigned)s_ent[wib][e];
-                    const int j = (int)(u & 0x3fffffffu);
-                    const bool nk = u & (1u << 30), nj = u & (2u << 30);
-                    const double ri[3] = {nk ? rn[0] : ro[0], nk ? rn[1] : ro[1], nk ? rn[2] : ro[2]};
-                    const double ei[3] = {nk ? v.tux[g] : v.ox[g], nk ? v.tuy[g] : v.oy[g], nk ? v.tuz[g] : v.oz[g]};
-                    const double rj[3] = {nj ? v.tnx[j] : v.px[j], nj ? v.tny[j] : v.py[j], nj ? v.tnz[j] : v.pz[j]};
-                    const double ej[3] = {nj ? v.tux[j] : v.ox[j], nj ? v.tuy[j] : v.oy[j], nj ? v.tuz[j] : v.oz[j]};
-                    double d[3];
-                    const double r2 = dist_fold(ri[0], ri[1], ri[2], rj[0], rj[1], rj[2], p.L, d);
-                    s_val[wib][e] = pair_exact(p.k, r2, d, ei, ej);
-                }
-            }
+        // 2 the listed terms, every lane busy
+        for (int e = t; e < ne; e += 128) {
+            const unsigned u = (unsigned)s_ent[e];
+            const int j = (int)(u & 0x3fffffffu);
+            const bool nk = u & (1u << 30), nj = u & (2u << 30);
+            const double ri[3] = {nk ? rn[0] : ro[0], nk ? rn[1] : ro[1], nk ? rn[2] : ro[2]};
+            const double ei[3] = {nk ? v.tux[g] : v.ox[g], nk ? v.tuy[g] : v.oy[g], nk ? v.tuz[g] : v.oz[g]};
+            const double rj[3] = {nj ? v.tnx[j] : v.px[j], nj ? v.tny[j] : v.py[j], nj ? v.tnz[j] : v.pz[j]};
+            const double ej[3] = {nj ? v.tux[j] : v.ox[j], nj ? v.tuy[j] : v.oy[j], nj ? v.tuz[j] : v.oz[j]};
+            double d[3];
+            const double r2 = dist_fold(ri[0], ri[1], ri[2], rj[0], rj[1], rj[2], p.L, d);
+            s_val[e] = pair_exact(p.k, r2, d, ei, ej);
         }
-        // colloid terms: lane 0 the old state, lane 1 the trial state
-        if (lane < 2 && p.k.coll_on) {
-            const double r3[3] = {lane ? rn[0] : ro[0], lane ? rn[1] : ro[1], lane ? rn[2] : ro[2]};
-            const double e3[3] = {lane ? v.tux[g] : v.ox[g], lane ? v.tuy[g] : v.oy[g], lane ? v.tuz[g] : v.oz[g]};
+        // colloid terms: the old state and the trial state
+        if (t >= 126 && p.k.coll_on) {
+            const bool nk = t & 1;
+            const double r3[3] = {nk ? rn[0] : ro[0], nk ? rn[1] : ro[1], nk ? rn[2] : ro[2]};
+            const double e3[3] = {nk ? v.tux[g] : v.ox[g], nk ? v.tuy[g] : v.oy[g], nk ? v.tuz[g] : v.oz[g]};
             const double u = colloid_rod(p.k, r3, e3, p.L);
-            if (lane == 0) hd->uo = u;
-            else hd->un = u;
+            if (nk) hd->un = u;
+            else hd->uo = u;
         }
-        __syncwarp();
-        // 3 the lane sums, in slot order
+        __syncthreads();
+        // 3 the lane sums, in slot order: warp 0 the slots before the own cell, warp 1 the own cell's, warp 2 those after
         const int J = ex_chunks(c.na);
-        const int c0 = q13 >> 5, c1 = (q13 + c.na - 1) >> 5;
-        double po = 0.0, pn = 0.0;
-        int ns = 0;
-        double2 *suf = rec + (size_t)(2 + 2 * J) * 32;
-        for (int h = 0; h < nch; h++) {
-            const unsigned b0 = s_mask[wib][0][h], b1 = s_mask[wib][1][h];
-            const unsigned b2 = s_mask[wib][2][h], b3 = s_mask[wib][3][h];
-            const int o0 = s_off[wib][h], o1 = o0 + __popc(b0);
-            const double t0 = (b0 >> lane) & 1u ? s_val[wib][o0 + __popc(b0 & lt)] : 0.0;
-            const double t1 = (b1 >> lane) & 1u ? s_val[wib][o1 + __popc(b1 & lt)] : 0.0;
-            const int q = 32 * h + lane;
-            const bool mine = q >= q13 && q < q13 + c.na;
-            if (h >= c0 && h <= c1) { // (uniform) a chunk of the own cell: every lane writes both rows
-                const int o2 = o1 + __popc(b1), o3 = o2 + __popc(b2);
-                const double t2 = (b2 >> lane) & 1u ? s_val[wib][o2 + __popc(b2 & lt)] : 0.0;
-                const double t3 = (b3 >> lane) & 1u ? s_val[wib][o3 + __popc(b3 & lt)] : 0.0;
-                rec[(size_t)(2 + h - c0) * 32 + lane] = mine ? make_double2(t0, t1) : make_double2(0.0, 0.0);
-                rec[(size_t)(2 + J + h - c0) * 32 + lane] = mine ? make_double2(t2, t3) : make_double2(0.0, 0.0);
-                const unsigned own = __ballot_sync(0xffffffffu, mine);
-                if (lane == 0) {
-                    hd->mask[0][h - c0] = b0 & own;
-                    hd->mask[1][h - c0] = b1 & own;
-                    hd->mask[2][h - c0] = b2 & own;
-                    hd->mask[3][h - c0] = b3 & own;
+        const int c0 = q13 >> 5, q14 = q13 + c.na, c1 = (q14 - 1) >> 5;
+        auto term = [&](unsigned m, int o) { return (m >> lane) & 1u ? s_val[o + __popc(m & lt)] : 0.0; };
+        if (w == 0) {
+            double po = 0.0, pn = 0.0;
+            for (int h = 0; h <= c0; h++) {
+                unsigned b0 = s_mask[0][h], b1 = s_mask[1][h];
+                const int o = s_off[h];
+                const double t0 = term(b0, o), t1 = term(b1, o + __popc(b0));
+                if (32 * h + lane < q13) {
+                    po += t0;
+                    pn += t1;
                 }
             }
-            if (q < q13) {
-                po += t0;
-                pn += t1;
-            } else if (!mine && (((b0 | b1) >> lane) & 1u)) {
-                if (ns < EX_SUF) suf[(size_t)ns * 32 + lane] = make_double2(t0, t1);
-                ns++;
-            }
-        }
-        rec[32 + lane] = make_double2(po, pn);
-        int nsuf = ns;
+            rec[32 + lane] = make_double2(po, pn);
+        } else if (w == 1) {
+            for (int h = c0; h < c0 + J; h++) { // chunks beyond the last one the cell touches are written as empty
+                const int q = 32 * h + lane;
+                const bool mine = q >= q13 && q < q14;
+                const unsigned own = __ballot_sync(0xffffffffu, mine);
+                unsigned m[4] = {0u, 0u, 0u, 0u};
+                double x[4] = {0.0, 0.0, 0.0, 0.0};
+                if (h <= c1) {
+                    int o = s_off[h];
 #pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) nsuf = max(nsuf, __shfl_xor_sync(0xffffffffu, nsuf, o));
-        if (nsuf > EX_SUF) {
-            if (lane == 0) v.ex_flag[(size_t)ci * v.ex_act + a] = 1;
-        } else {
-            for (int s = ns; s < nsuf; s++) suf[(size_t)s * 32 + lane] = make_double2(0.0, 0.0);
-            // chunks J covers beyond the last one the cell touches
-            for (int h = c1 - c0 + 1; h < J; h++) {
-                rec[(size_t)(2 + h) * 32 + lane] = make_double2(0.0, 0.0);
-                rec[(size_t)(2 + J + h) * 32 + lane] = make_double2(0.0, 0.0);
-                if (lane < 4) hd->mask[lane][h] = 0u;
+                    for (int i = 0; i < 4; i++) {
+                        m[i] = s_mask[i][h];
+                        x[i] = mine ? term(m[i], o) : 0.0;
+                        o += __popc(m[i]);
+                    }
+                }
+                rec[(size_t)(2 + h - c0) * 32 + lane] = make_double2(x[0], x[1]);
+                rec[(size_t)(2 + J + h - c0) * 32 + lane] = make_double2(x[2], x[3]);
+                if (lane < 4) {
+                    const unsigned mm = lane == 0 ? m[0] : (lane == 1 ? m[1] : (lane == 2 ? m[2] : m[3]));
+                    hd->mask[lane][h - c0] = mm & own;
+                }
             }
-            if (lane == 0) {
-                hd->nsuf = nsuf;
-                hd->nstat = nstat;
+        } else if (w == 2) {
+            int ns = 0;
+            double2 *suf = rec + (size_t)(2 + 2 * J) * 32;
+            for (int h = c1; h < nch; h++) {
+                const unsigned b0 = s_mask[0][h], b1 = s_mask[1][h];
+                const int o = s_off[h];
+                if (32 * h + lane >= q14 && (((b0 | b1) >> lane) & 1u)) {
+                    if (ns < EX_SUF) suf[(size_t)ns * 32 + lane] = make_double2(term(b0, o), term(b1, o + __popc(b0)));
+                    ns++;
+                }
+            }
+            const int nsuf = __reduce_max_sync(0xffffffffu, ns);
+            if (nsuf > EX_SUF) {
+                if (lane == 0) v.ex_flag[(size_t)ci * v.ex_act + a] = 1;
+            } else {
+                for (int s = ns; s < nsuf; s++) suf[(size_t)s * 32 + lane] = make_double2(0.0, 0.0);
+                if (lane == 0) {
+                    hd->nsuf = nsuf;
+                    hd->nstat = s_nstat;
+                }
             }
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -535,15 +547,154 @@ __device__ __forceinline__ void cp_row_async(void *dst, const void *src)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
-// Rows fetched ahead of an attempt, three attempts deep: the scratch rows come
-// from L2, and the chain of one attempt (a dozen additions, ten shuffles, the
-// test) is what remains.
-constexpr int EX_STAGES = 3;
-constexpr int EX_PF = 2 + 2 * EX_J + EX_PFS;
+// The attempts of one cell (J chunks of own-cell slots).  The records come from
+// L2, EX_STAGES - 1 attempts ahead (cp.async, fully unrolled: one warp runs
+// here, so every instruction of an attempt is latency); what remains is the
+// chain of one attempt: a dozen additions, the butterfly, the test.
+constexpr int EX_STAGES = 4;
+template <int J> struct ExactStage {
+    static constexpr int PF = 2 + 2 * J + EX_PFS; // rows fetched per attempt
+};
+
+template <int J>
+__device__ __forceinline__ void exact_decide_cell(const DevView &v, const CellView &c, int lane, int q13,
+                                                  const double2 *rows, double2 *buf)
+{
+    constexpr int PF = ExactStage<J>::PF, RPP = 2 + 2 * J + EX_SUF;
+    const Replica &p = v.rep[c.r];
+    const int na = c.na, c0 = q13 >> 5;
+    const double beta = p.k.beta;
+    const bool coll = p.k.coll_on;
+    const double2 *src = rows + lane;
+    double2 *mine = buf + lane;
+    int kf = 0, sf = 0; // next record to fetch and its stage
+    auto fetch = [&]() {
+        if (kf < na) {
+            double2 *dst = mine + sf * (PF * 32);
+#pragma unroll
+            for (int i = 0; i < PF; i++) cp_row_async(dst + i * 32, src + i * 32);
+            src += RPP * 32;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        kf++;
+        sf = sf == EX_STAGES - 1 ? 0 : sf + 1;
+    };
+#pragma unroll
+    for (int k = 0; k < EX_STAGES - 1; k++) fetch();
+    unsigned accm = 0u; // bit j: the particle at slot 32 (c0 + j) + lane was accepted
+    double dE_sum = 0.0, dE_abs = 0.0;
+    int nacc = 0, nhard = 0, st = 0;
+    for (int k = 0; k < na; k++) {
+        fetch();
+        asm volatile("cp.async.wait_group %0;" ::"n"(EX_STAGES - 1) : "memory");
+        __syncwarp();
+        const double2 *rw = mine + st * (PF * 32);
+        st = st == EX_STAGES - 1 ? 0 : st + 1;
+        const ExactHead *hd = reinterpret_cast<const ExactHead *>(rw - lane);
+        const int code = hd->code, nsuf = hd->nsuf;
+        const double lu = hd->lu;
+        double dE = 0.0;
+        if (code) {
+            nhard += code == 1;
+        } else {
+            double2 x[J], y[4];
+            double po = rw[32].x, pn = rw[32].y;
+#pragma unroll
+            for (int j = 0; j < J; j++) x[j] = rw[((accm >> j) & 1u ? 2 + J + j : 2 + j) * 32];
+#pragma unroll
+            for (int s = 0; s < 4; s++) y[s] = s < nsuf ? rw[(2 + 2 * J + s) * 32] : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                po += x[j].x;
+                pn += x[j].y;
+            }
+#pragma unroll
+            for (int s = 0; s < 4; s++) {
+                po += y[s].x;
+                pn += y[s].y;
+            }
+            for (int s = 4; s < nsuf; s++) {
+                const double2 z = s < EX_PFS ? rw[(2 + 2 * J + s) * 32]
+                                             : rows[((size_t)k * RPP + 2 + 2 * J + s) * 32 + lane];
+                po += z.x;
+                pn += z.y;
+            }
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) {
+                const double yo = __shfl_xor_sync(0xffffffffu, po, o), yn = __shfl_xor_sync(0xffffffffu, pn, o);
+                po = po + yo;
+                pn = pn + yn;
+            }
+            if (coll) {
+                po = po + hd->uo;
+                pn = pn + hd->un;
+            }
+            dE = pn - po;
+            if ((dE <= 0.0) || (lu <= -beta * dE)) {
+                const int q = q13 + k;
+                if (lane == (q & 31)) accm |= 1u << ((q >> 5) - c0);
+                dE_sum += dE;
+                dE_abs += fabs(dE);
+                nacc++;
+            }
+        }
+        if (v.rec_dE && lane == 0) {
+            const int id = v.id[c.cs + k];
+            v.rec_dE[p.p_off + id] = dE;
+            v.rec_lu[p.p_off + id] = lu;
+        }
+        __syncwarp(); // the stage may be refilled
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // a lane per particle: outcome, accepted trial state to the master arrays, and the pairs its attempt met
+    // (the partners before it that were accepted in their trial state, every other in its old one)
+    unsigned long long npairs = 0ull;
+    for (int k0 = 0; k0 < na; k0 += 32) {
+        const int k = k0 + lane, q = q13 + k, g = c.cs + k;
+        const bool on = k < na;
+        const unsigned m = __shfl_sync(0xffffffffu, accm, q & 31);
+        const bool acc = on && ((m >> ((q >> 5) - c0)) & 1u);
+        const ExactHead *hd = reinterpret_cast<const ExactHead *>(rows + (size_t)(on ? k : 0) * RPP * 32);
+        const int code = on ? hd->code : 3;
+        if (on) v.outcome[p.p_off + v.id[g]] = code == 1 ? 2 : (acc ? 1 : 0);
+        if (acc) {
+            v.px[g] = v.tnx[g];
+            v.py[g] = v.tny[g];
+            v.pz[g] = v.tnz[g];
+            v.ox[g] = v.tux[g];
+            v.oy[g] = v.tuy[g];
+            v.oz[g] = v.tuz[g];
+        }
+        int np = code ? 0 : hd->nstat;
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            const unsigned A = __ballot_sync(0xffffffffu, (accm >> j) & 1u); // accepted slots of chunk c0 + j
+            if (!code) {
+                const int d = q - 32 * (c0 + j); // slots of this chunk before the particle's own
+                const unsigned B = d <= 0 ? 0u : (d >= 32 ? A : A & ((1u << d) - 1u));
+                np += __popc((hd->mask[0][j] & ~B) | (hd->mask[2][j] & B)) +
+                      __popc((hd->mask[1][j] & ~B) | (hd->mask[3][j] & B));
+            }
+        }
+        npairs += (unsigned long long)np;
+    }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
+    if (lane == 0) {
+        v.cell_e0[c.cell] = dE_sum;
+        v.cell_abs[c.cell] = dE_abs;
+        v.cell_fp64[c.cell] = 0;
+        v.cell_n0[c.cell] = nacc;
+        v.cell_n1[c.cell] = nhard;
+        v.cell_pairs[c.cell] = npairs;
+        v.cell_cands[c.cell] = (unsigned long long)(c.total - 1) * (unsigned long long)na;
+    }
+    __syncwarp();
+}
 
 __global__ void __launch_bounds__(32) k_exact_decide(const __grid_constant__ DevView v, int ci, int b)
 {
-    extern __shared__ double2 ex_buf[]; // [EX_STAGES][EX_PF][32]
+    extern __shared__ double2 ex_buf[]; // [EX_STAGES][PF][32]
     __shared__ int s_first[27], s_base[28];
     const int lane = threadIdx.x;
     const int *off = v.act_off + ci * (v.R + 1);
@@ -553,122 +704,20 @@ __global__ void __launch_bounds__(32) k_exact_decide(const __grid_constant__ Dev
     for (int a = eb.lo + blockIdx.x; a < a1; a += gridDim.x) {
         CellView c;
         active_cell(v, off, ci, a, c);
-        const Replica &p = v.rep[c.r];
-        if (p.use_fast) continue;
+        if (v.rep[c.r].use_fast) continue;
         cell_stencil(v, c, lane, s_first, s_base);
         if (a >= eb.hi || v.ex_flag[(size_t)ci * v.ex_act + a]) {
             exact_cell_sequential(&v, c, lane, s_first, s_base);
             continue;
         }
-        const int na = c.na, J = ex_chunks(na), rpp = ex_rows_per_particle(na);
-        const int npf = 2 + 2 * J + EX_PFS;
-        const double2 *rows = v.ex_rows + (size_t)(er[a] - eb.row0) * 32 + lane;
-        const int q13 = s_base[c.own], c0 = q13 >> 5;
-        const double beta = p.k.beta;
-        const bool coll = p.k.coll_on;
-        auto fetch = [&](int k) {
-            if (k < na) {
-                const double2 *src = rows + (size_t)k * rpp * 32;
-                double2 *dst = ex_buf + (size_t)(k % EX_STAGES) * EX_PF * 32 + lane;
-                for (int i = 0; i < npf; i++) cp_row_async(dst + i * 32, src + (size_t)i * 32);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-#pragma unroll
-        for (int k = 0; k < EX_STAGES - 1; k++) fetch(k);
-        unsigned accm = 0u; // lane j: accepted particles at the slots of chunk c0 + j
-        double dE_sum = 0.0, dE_abs = 0.0;
-        int nacc = 0, nhard = 0;
-        unsigned long long npairs = 0ull;
-        for (int k = 0; k < na; k++) {
-            fetch(k + EX_STAGES - 1);
-            asm volatile("cp.async.wait_group %0;" ::"n"(EX_STAGES - 1) : "memory");
-            __syncwarp();
-            const double2 *rw = ex_buf + (size_t)(k % EX_STAGES) * EX_PF * 32 + lane;
-            const ExactHead *hd = reinterpret_cast<const ExactHead *>(rw - lane);
-            const int g = c.cs + k;
-            const int code = hd->code;
-            const double lu = hd->lu;
-            double dE = 0.0;
-            bool acc = false;
-            if (code) {
-                nhard += code == 1;
-            } else {
-                const int nsuf = hd->nsuf;
-                double po = rw[32].x, pn = rw[32].y;
-                for (int j = 0; j < J; j++) {
-                    const unsigned m = __shfl_sync(0xffffffffu, accm, j);
-                    const double2 x = rw[(2 + j + ((m >> lane) & 1u ? J : 0)) * 32];
-                    po += x.x;
-                    pn += x.y;
-                }
-                for (int s = 0; s < nsuf; s++) {
-                    const double2 x = s < EX_PFS ? rw[(2 + 2 * J + s) * 32]
-                                                 : rows[((size_t)k * rpp + 2 + 2 * J + s) * 32];
-                    po += x.x;
-                    pn += x.y;
-                }
-#pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) {
-                    const double yo = __shfl_xor_sync(0xffffffffu, po, o), yn = __shfl_xor_sync(0xffffffffu, pn, o);
-                    po = po + yo;
-                    pn = pn + yn;
-                }
-                if (coll) {
-                    po = po + hd->uo;
-                    pn = pn + hd->un;
-                }
-                dE = pn - po;
-                acc = (dE <= 0.0) || (lu <= -beta * dE);
-                if (lane < J)
-                    npairs += (unsigned long long)(__popc((hd->mask[0][lane] & ~accm) | (hd->mask[2][lane] & accm)) +
-                                                   __popc((hd->mask[1][lane] & ~accm) | (hd->mask[3][lane] & accm)));
-                if (lane == 0) npairs += (unsigned long long)hd->nstat;
-                if (acc) {
-                    const int q = q13 + k;
-                    if (lane == (q >> 5) - c0) accm |= 1u << (q & 31);
-                    dE_sum += dE;
-                    dE_abs += fabs(dE);
-                    nacc++;
-                }
-            }
-            if (lane == 0) {
-                const int id = v.id[g];
-                v.outcome[p.p_off + id] = code ? (code == 1 ? 2 : 0) : (acc ? 1 : 0);
-                if (v.rec_dE) {
-                    v.rec_dE[p.p_off + id] = dE;
-                    v.rec_lu[p.p_off + id] = lu;
-                }
-            }
-            __syncwarp(); // the stage may be refilled
+        const double2 *rows = v.ex_rows + (size_t)(er[a] - eb.row0) * 32;
+        const int q13 = s_base[c.own];
+        switch (ex_chunks(c.na)) {
+        case 2: exact_decide_cell<2>(v, c, lane, q13, rows, ex_buf); break;
+        case 3: exact_decide_cell<3>(v, c, lane, q13, rows, ex_buf); break;
+        case 5: exact_decide_cell<5>(v, c, lane, q13, rows, ex_buf); break;
+        default: exact_decide_cell<EX_J>(v, c, lane, q13, rows, ex_buf); break;
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        // accepted trial states to the master arrays
-        for (int k0 = 0; k0 < na; k0 += 32) {
-            const int k = k0 + lane, q = q13 + k;
-            const unsigned m = __shfl_sync(0xffffffffu, accm, k < na ? (q >> 5) - c0 : 0);
-            if (k < na && ((m >> (q & 31)) & 1u)) {
-                const int g = c.cs + k;
-                v.px[g] = v.tnx[g];
-                v.py[g] = v.tny[g];
-                v.pz[g] = v.tnz[g];
-                v.ox[g] = v.tux[g];
-                v.oy[g] = v.tuy[g];
-                v.oz[g] = v.tuz[g];
-            }
-        }
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
-        if (lane == 0) {
-            v.cell_e0[c.cell] = dE_sum;
-            v.cell_abs[c.cell] = dE_abs;
-            v.cell_fp64[c.cell] = 0;
-            v.cell_n0[c.cell] = nacc;
-            v.cell_n1[c.cell] = nhard;
-            v.cell_pairs[c.cell] = npairs;
-            v.cell_cands[c.cell] = (unsigned long long)(c.total - 1) * (unsigned long long)na;
-        }
-        __syncwarp();
     }
 }
 
@@ -860,15 +909,15 @@ void exact_scratch_size(int ntot, long long *cap, long long *alloc, int *nb)
 void exact_init()
 {
     cudaFuncSetAttribute(k_exact_decide, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         EX_STAGES * EX_PF * 32 * (int)sizeof(double2));
+                         EX_STAGES * ExactStage<EX_J>::PF * 32 * (int)sizeof(double2));
 }
 
 void launch_exact_offsets(const DevView &v, cudaStream_t s) { k_exact_offsets<<<v.nphase, 1024, 0, s>>>(v); }
 
 void launch_phase_exact(const DevView &v, cudaStream_t s, int ci, int grid)
 {
-    const int bytes = EX_STAGES * EX_PF * 32 * (int)sizeof(double2);
-    const int gt = min(grid, (v.ntot + 3) / 4), gd = min(grid, v.ex_act);
+    const int bytes = EX_STAGES * ExactStage<EX_J>::PF * 32 * (int)sizeof(double2);
+    const int gt = min(4 * grid, v.ntot), gd = min(grid, v.ex_act);
     for (int b = 0; b < v.ex_nb; b++) {
         k_exact_terms<<<gt, 128, 0, s>>>(v, ci, b);
         k_exact_decide<<<gd, 32, bytes, s>>>(v, ci, b);
