@@ -147,7 +147,8 @@ enum {
     LCMC_F_LISTCAP = 4,     /* the bits stay reserved                                                       */
     LCMC_F_NONFINITE = 8,   /* NaN/Inf energy change */
     LCMC_F_GRIDCAP = 16,    /* box grew past the allocated cell grid (cells kept wider) */
-    LCMC_F_DRIFT = 32       /* a periodic FP64 energy check was out of tolerance */
+    LCMC_F_DRIFT = 32,      /* a periodic FP64 energy check was out of tolerance */
+    LCMC_F_TIMEOUT = 64     /* a bounded wait inside a phase kernel gave up (the kernel returned cleanly) */
 };
 
 /* ---- parameters (host only) ---- */

@@ -38,6 +38,8 @@ struct lcmc_ctx {
     Replica *d_rep = nullptr;
     DevStats *d_stats = nullptr;
     int *d_act_off = nullptr, *d_p2r = nullptr;
+    int4 *d_act_tab = nullptr;
+    int act_max = 1; // most active cells of a colour phase
     double *d_x[2][6] = {{nullptr}};
     int *d_id[2] = {nullptr, nullptr};
     int *d_cid = nullptr, *d_rank = nullptr, *d_perm = nullptr, *d_scid = nullptr;
@@ -48,6 +50,7 @@ struct lcmc_ctx {
     double *d_cell_abs = nullptr;
     int *d_cell_fp64 = nullptr;
     int *d_p2c = nullptr, *d_resc_count = nullptr, *d_resc_list = nullptr;
+    int *d_retry_count = nullptr, *d_retry_list = nullptr;
     // FP64 colour phases (allocated when a replica first needs them)
     int *d_ex_p = nullptr;
     long long *d_ex_r = nullptr;
@@ -56,6 +59,10 @@ struct lcmc_ctx {
     long long ex_cap = 0, ex_alloc = 0;
     int ex_act = 0, ex_nb = 1;
     int nphase = 8; // colour phases per sweep (LCMC_MAX_COLOURS with a fine-grid replica)
+    int nrun = 8;   // of those, the ones any replica's box can take
+    // sweeps until an NPT box could reach the four cells per axis below which
+    // its moves need the FP64 kernel (the choice is looked over again by then)
+    long long safe_sweeps = 1ll << 40, since_choice = 0;
     // Replica groups of a batch: the colour phases of each group run on their
     // own stream (a branch of the sweep graph between the rebin and the
     // statistics), so the phases of different groups overlap instead of all
@@ -72,8 +79,8 @@ struct lcmc_ctx {
     double *d_red = nullptr;
     double *d_red_part = nullptr; // chunk partial sums
     int red_nchunk = 1;
-    double *d_trial_d[8] = {nullptr}; // tnx tny tnz tux tuy tuz tdU tlu
-    float *d_trial_f[3] = {nullptr};  // tdx tdy tdz
+    double *d_trial_d[7] = {nullptr}; // tnx tny tnz tux tuy tuz tlu
+    ActRec *d_act_rec = nullptr;
     unsigned char *d_thard = nullptr;
     float4 *d_cl4 = nullptr;
     float2 *d_cl2 = nullptr;
@@ -93,7 +100,7 @@ struct lcmc_ctx {
     std::vector<char> uploaded;
     // kernels
     int kernel_override = -1;
-    int fast_variant = 0;
+    FastChoice fast; // the FP32 phase kernel
     int need_amax = 0; // active-cell capacity the capacity rule asks for
     int need_min = 0;  // the smallest capacity lcmc_autotune may try: mean + 3 standard deviations of a cell's count
     int tuned_class = -1; // capacity class lcmc_autotune chose (kept while it holds the rule's capacity)
@@ -483,6 +490,8 @@ static DevView view(const lcmc_ctx *c, int parity)
     v.rep = c->d_rep;
     v.stats = c->d_stats;
     v.act_off = c->d_act_off;
+    v.act_tab = c->d_act_tab;
+    v.act_max = c->act_max;
     v.p2r = c->d_p2r;
     const int a = parity, b = parity ^ 1;
     v.px = c->d_x[a][0];
@@ -516,6 +525,8 @@ static DevView view(const lcmc_ctx *c, int parity)
     v.cell_fp64 = c->d_cell_fp64;
     v.p2c = c->d_p2c;
     v.resc_count = c->d_resc_count;
+    v.retry_count = c->d_retry_count;
+    v.retry_list = c->d_retry_list;
     v.nphase = c->nphase;
     v.r_lo = 0;
     v.r_hi = c->R;
@@ -540,11 +551,8 @@ static DevView view(const lcmc_ctx *c, int parity)
     v.tux = c->d_trial_d[3];
     v.tuy = c->d_trial_d[4];
     v.tuz = c->d_trial_d[5];
-    v.tdU = c->d_trial_d[6];
-    v.tlu = c->d_trial_d[7];
-    v.tdx = c->d_trial_f[0];
-    v.tdy = c->d_trial_f[1];
-    v.tdz = c->d_trial_f[2];
+    v.tlu = c->d_trial_d[6];
+    v.act_rec = c->d_act_rec;
     v.thard = c->d_thard;
     v.cl4 = c->d_cl4;
     v.cl2 = c->d_cl2;
@@ -571,18 +579,17 @@ static void free_ctx(lcmc_ctx *c)
         if (c->ev_join[g]) cudaEventDestroy(c->ev_join[g]);
     }
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
-    void *ptrs[] = {c->d_rep, c->d_stats, c->d_act_off, c->d_p2r, c->d_id[0], c->d_id[1], c->d_cid, c->d_rank,
+    void *ptrs[] = {c->d_rep, c->d_stats, c->d_act_off, c->d_act_tab, c->d_p2r, c->d_id[0], c->d_id[1], c->d_cid, c->d_rank,
                     c->d_perm, c->d_scid, c->d_cell_count, c->d_cell_start, c->d_block_sums, c->d_flag, c->d_cell_e0,
                     c->d_cell_e1, c->d_cell_n0, c->d_cell_n1, c->d_cell_pairs, c->d_cell_cands, c->d_outcome,
                     c->d_pe0, c->d_pe1, c->d_phard, c->d_red, c->d_red_part, c->d_cell_abs, c->d_cell_fp64,
-                    c->d_rec_dE, c->d_rec_lu, c->d_p2c, c->d_resc_count, c->d_resc_list, c->d_ex_p, c->d_ex_r, c->d_ex_flag,
+                    c->d_rec_dE, c->d_rec_lu, c->d_p2c, c->d_resc_count, c->d_resc_list, c->d_retry_count, c->d_retry_list, c->d_ex_p, c->d_ex_r, c->d_ex_flag,
                     c->d_ex_rows};
     for (void *p : ptrs)
         if (p) cudaFree(p);
-    for (int k = 0; k < 8; k++)
+    for (int k = 0; k < 7; k++)
         if (c->d_trial_d[k]) cudaFree(c->d_trial_d[k]);
-    for (int k = 0; k < 3; k++)
-        if (c->d_trial_f[k]) cudaFree(c->d_trial_f[k]);
+    if (c->d_act_rec) cudaFree(c->d_act_rec);
     if (c->d_thard) cudaFree(c->d_thard);
     if (c->d_cl4) cudaFree(c->d_cl4);
     if (c->d_cl2) cudaFree(c->d_cl2);
@@ -684,7 +691,7 @@ extern "C" int lcmc_cell_capacity(const lcmc_params *p, int *capacity, int *clas
 // tolerance of the periodic energy check.
 static void set_caps(lcmc_ctx *c)
 {
-    const int amax = fast_variant(c->fast_variant >> 1).amax;
+    const int amax = fast_variant(c->fast.cls).amax;
     for (int r = 0; r < c->R; r++) {
         Replica &rp = c->rep[r];
         const lcmc_params &p = c->params[r];
@@ -710,11 +717,77 @@ static int push_kernel_fields(lcmc_ctx *c)
     return LCMC_OK;
 }
 
+// What a sweep launches that depends on the replicas' boxes: the FP64 phase
+// kernels (a system on them, or an FP32 system with fewer than four cells along
+// an axis) and the colour phases.  An NPT box may cross the four cells while
+// sweeps run: the number of sweeps until it could (a volume move changes ln L
+// by at most dlnv_max / 3) says when to look again, and below 32 the FP64
+// kernels are launched all the time.
+static void box_launches(lcmc_ctx *c)
+{
+    c->any_exact = false;
+    c->safe_sweeps = 1ll << 40;
+    c->since_choice = 0;
+    c->nrun = 8;
+    for (int r = 0; r < c->R; r++) {
+        const Replica &rp = c->rep[r];
+        const double Lmin = std::min(rp.L[0], std::min(rp.L[1], rp.L[2]));
+        if (rp.kernel == 0 || grid_dim_host(Lmin, rp.wmin, rp.fine) < 4) {
+            c->any_exact = true;
+        } else if (rp.ensemble == 2 && rp.dlnv_max > 0.0) {
+            const long long safe = (long long)(3.0 * std::log(Lmin / (4.0 * rp.wmin)) / rp.dlnv_max) - 1;
+            if (safe < 32) c->any_exact = true;
+            else c->safe_sweeps = std::min(c->safe_sweeps, safe);
+        }
+        // colours: 2 per axis, 3 on an odd count of the fine grid; an NPT box may take any count
+        int ncol = rp.fine && rp.ensemble == 2 ? LCMC_MAX_COLOURS : 1;
+        for (int a = 0; a < 3 && ncol < LCMC_MAX_COLOURS; a++) {
+            const int nc = std::min(grid_dim_host(rp.L[a], rp.wmin, rp.fine), rp.nc_max);
+            ncol *= (nc & 1) && nc >= 3 ? 3 : 2;
+        }
+        c->nrun = std::max(c->nrun, ncol);
+    }
+}
+
+static bool same_pair_consts(const GBConsts &a, const GBConsts &b)
+{
+    return a.f_rc2 == b.f_rc2 && a.f_chi == b.f_chi && a.f_chi_sq == b.f_chi_sq && a.f_chip == b.f_chip &&
+           a.f_chip_sq == b.f_chip_sq && a.f_4eps0 == b.f_4eps0 && a.f_half_chi == b.f_half_chi &&
+           a.f_half_chip == b.f_half_chip && a.f_big == b.f_big;
+}
+
+// The shape of the FP32 phase kernel within its capacity class: the light one
+// when no system's rule asks for more than 40 particles per cell, the wide one
+// when a colour phase has at most one active cell per SM (the phase then takes
+// the latency of one cell).
+static void choose_fast_shape(lcmc_ctx *c)
+{
+    long long act = 0;
+    for (int r = 0; r < c->R; r++) {
+        long long cells = 1; // of the largest colour
+        for (int a = 0; a < 3; a++) {
+            const int nc = grid_dim_host(c->rep[r].L[a], c->rep[r].wmin, c->rep[r].fine);
+            cells *= (nc & 1) && nc >= 3 ? (nc + 2) / 3 : (nc + 1) / 2;
+        }
+        act += cells;
+    }
+    c->fast.light = c->fast.cls == 0 && c->need_amax <= 40;
+    c->fast.wide = act <= c->sms;
+    // blocks: the fewest per SM that take as many rounds over a phase's cells as the most that fit (fewer
+    // neighbours, so each round ends sooner)
+    const int fit = fast_blocks_per_sm(c->fast);
+    const long long rounds = (act + (long long)fit * c->sms - 1) / ((long long)fit * c->sms);
+    int per_sm = fit;
+    while (per_sm > 1 && (act + (long long)(per_sm - 1) * c->sms - 1) / ((long long)(per_sm - 1) * c->sms) == rounds)
+        per_sm--;
+    c->grid_fast = per_sm * c->sms;
+}
+
 // Kernel selection: FP32 kernel for precision_mode fp32 (boxes with >= 4
 // cells per axis; smaller boxes run the FP64 kernel), FP64 kernel otherwise.
 static void choose_kernels(lcmc_ctx *c)
 {
-    c->any_fast = c->any_exact = c->any_npt = false;
+    c->any_fast = c->any_npt = false;
     int need_amax = 0, need_min = 0;
     bool spec21 = true; // every system has mu = 2, nu = 1, sigma0 = 1
     for (int r = 0; r < c->R; r++) {
@@ -729,25 +802,25 @@ static void choose_kernels(lcmc_ctx *c)
             capacity_rule(p, rp.L[0], rp.wmin, rp.ensemble == 2) > fast_variant(fast_variant_count() - 1).amax)
             kern = 0;
         rp.kernel = kern;
-        int nc = grid_dim_host(rp.L[0], rp.wmin, rp.fine);
         if (kern == 1) {
             c->any_fast = true;
-            if (nc < 6) c->any_exact = true; // NPT boxes near the 4-cell threshold may switch
             const int want = capacity_rule(p, rp.L[0], rp.wmin, rp.ensemble == 2);
             if (want > need_amax) need_amax = want;
             need_min = std::max(need_min, capacity_floor(p, rp.L[0], rp.wmin));
-        } else {
-            c->any_exact = true;
         }
         if (rp.ensemble == 2) c->any_npt = true;
-        spec21 = spec21 && p.gb_mu_exponent == 2.0 && p.gb_nu_exponent == 1.0 && p.gb_sigma_sidetoside == 1.0;
+        spec21 = spec21 && p.gb_mu_exponent == 2.0 && p.gb_nu_exponent == 1.0 && p.gb_sigma_sidetoside == 1.0 &&
+                 same_pair_consts(rp.k, c->rep[0].k);
     }
     c->need_amax = need_amax;
     c->need_min = need_min;
     int cls = capacity_class(need_amax);
     if (c->tuned_class >= 0 && fast_variant(c->tuned_class).amax >= need_min) cls = c->tuned_class;
-    c->fast_variant = 2 * cls + (spec21 ? 1 : 0);
+    c->fast.cls = cls;
+    c->fast.spec21 = spec21;
+    choose_fast_shape(c);
     set_caps(c);
+    box_launches(c);
 }
 
 static int upload_replica_table(lcmc_ctx *c)
@@ -809,6 +882,9 @@ extern "C" int lcmc_create_batch(const lcmc_params *params, int n, lcmc_ctx **ou
         rp.sweep = 0ull;
         poff += rp.n;
         coff += rp.nc_max * rp.nc_max * rp.nc_max;
+        // at most ceil(nc / 2) cells of a colour per axis (two or three colours)
+        const int h = (rp.nc_max + 1) / 2;
+        c->act_max += h * h * h;
     }
     c->ntot = poff;
     c->ctot = coff;
@@ -864,6 +940,7 @@ extern "C" int lcmc_create_batch(const lcmc_params *params, int n, lcmc_ctx **ou
     ALLOC(c->d_rep, n);
     ALLOC(c->d_stats, n);
     ALLOC(c->d_act_off, c->nphase * (n + 1));
+    ALLOC(c->d_act_tab, (size_t)c->nphase * c->act_max);
     ALLOC(c->d_p2r, c->ntot);
     for (int a = 0; a < 2; a++) {
         for (int k = 0; k < 6; k++) ALLOC(c->d_x[a][k], c->ntot);
@@ -888,6 +965,8 @@ extern "C" int lcmc_create_batch(const lcmc_params *params, int n, lcmc_ctx **ou
     ALLOC(c->d_p2c, c->ctot);
     ALLOC(c->d_resc_count, c->nphase * c->ngroup);
     ALLOC(c->d_resc_list, (size_t)c->nphase * c->ngroup * c->ctot);
+    ALLOC(c->d_retry_count, c->nphase * c->ngroup);
+    ALLOC(c->d_retry_list, (size_t)c->nphase * c->ngroup * c->act_max);
     ALLOC(c->d_outcome, c->ntot);
     ALLOC(c->d_pe0, c->ntot);
     ALLOC(c->d_pe1, c->ntot);
@@ -900,11 +979,12 @@ extern "C" int lcmc_create_batch(const lcmc_params *params, int n, lcmc_ctx **ou
         c->red_nchunk = (nmax + LCMC_RED_CHUNK - 1) / LCMC_RED_CHUNK;
     }
     ALLOC(c->d_red_part, (size_t)n * c->red_nchunk * LCMC_RED_K);
-    for (int k = 0; k < 8; k++) ALLOC(c->d_trial_d[k], c->ntot);
-    for (int k = 0; k < 3; k++) ALLOC(c->d_trial_f[k], c->ntot);
+    for (int k = 0; k < 7; k++) ALLOC(c->d_trial_d[k], c->ntot);
+    ALLOC(c->d_act_rec, c->ntot);
     ALLOC(c->d_thard, c->ntot);
-    ALLOC(c->d_cl4, c->ntot);
-    ALLOC(c->d_cl2, c->ntot);
+    // the phase kernel copies cells in granules of 16 bytes: one entry past the last may be read
+    ALLOC(c->d_cl4, c->ntot + 2);
+    ALLOC(c->d_cl2, c->ntot + 2);
     ALLOC(c->d_feat_acc, (size_t)n * 512 * 7);
     ALLOC(c->d_feat_f, (size_t)n * LCMC_FEAT);
 #undef ALLOC
@@ -921,6 +1001,7 @@ extern "C" int lcmc_create_batch(const lcmc_params *params, int n, lcmc_ctx **ou
         for (int i = 0; i < c->rep[r].nc_max * c->rep[r].nc_max * c->rep[r].nc_max; i++) p2c[c->rep[r].cell_off + i] = r;
     cudaMemcpy(c->d_p2c, p2c.data(), sizeof(int) * c->ctot, cudaMemcpyHostToDevice);
     cudaMemset(c->d_resc_count, 0, sizeof(int) * c->nphase * c->ngroup);
+    cudaMemset(c->d_retry_count, 0, sizeof(int) * c->nphase * c->ngroup);
     cudaMemset(c->d_stats, 0, sizeof(DevStats) * n);
     cudaMemset(c->d_outcome, 0, c->ntot);
     cudaMemset(c->d_cell_e0, 0, sizeof(double) * c->ctot);
@@ -936,7 +1017,6 @@ extern "C" int lcmc_create_batch(const lcmc_params *params, int n, lcmc_ctx **ou
     c->grid_exact = 4 * c->sms;
     c->grid_energy = energy_exact_blocks_per_sm() * c->sms;
     c->grid_screen = screen_blocks_per_sm() * c->sms;
-    c->grid_fast = fast_blocks_per_sm(c->fast_variant) * c->sms;
     rescue_init();
     int rc = upload_replica_table(c);
     if (rc) {
@@ -963,22 +1043,44 @@ extern "C" int lcmc_destroy(lcmc_ctx *ctx)
 
 extern "C" int lcmc_num_replicas(const lcmc_ctx *ctx) { return ctx ? ctx->R : 0; }
 
-// Re-run the kernel choice on the replicas' current boxes (read back from the
-// device: NPT volume moves change them) and push the fields it sets.
-static int rechoose_kernels(lcmc_ctx *c)
+// The replicas' current boxes (NPT volume moves change them on the device).
+static int read_boxes(lcmc_ctx *c)
 {
     std::vector<Replica> dev(c->R);
     CUDA_TRY(c, cudaMemcpyAsync(dev.data(), c->d_rep, sizeof(Replica) * c->R, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     for (int r = 0; r < c->R; r++)
         for (int a = 0; a < 3; a++) c->rep[r].L[a] = dev[r].L[a];
-    const int old_variant = c->fast_variant;
+    return LCMC_OK;
+}
+
+// The box-dependent launches again, within a run of sweeps (no kernel changes).
+static int recheck_boxes(lcmc_ctx *c)
+{
+    int rc = read_boxes(c);
+    if (rc) return rc;
+    const bool old_exact = c->any_exact;
+    const int old_nrun = c->nrun;
+    box_launches(c);
+    if (old_exact != c->any_exact || old_nrun != c->nrun) invalidate_graphs(c);
+    return LCMC_OK;
+}
+
+// Re-run the kernel choice on the replicas' current boxes and push the fields
+// it sets.
+static int rechoose_kernels(lcmc_ctx *c)
+{
+    int brc = read_boxes(c);
+    if (brc) return brc;
+    const FastChoice old_fast_choice = c->fast;
     const bool old_fast = c->any_fast, old_exact = c->any_exact;
+    const int old_nrun = c->nrun, old_grid = c->grid_fast;
     choose_kernels(c);
     int rc = push_kernel_fields(c);
     if (rc) return rc;
-    c->grid_fast = fast_blocks_per_sm(c->fast_variant) * c->sms;
-    if (old_variant != c->fast_variant || old_fast != c->any_fast || old_exact != c->any_exact) invalidate_graphs(c);
+    if (!(old_fast_choice == c->fast) || old_fast != c->any_fast || old_exact != c->any_exact ||
+        old_nrun != c->nrun || old_grid != c->grid_fast)
+        invalidate_graphs(c);
     return LCMC_OK;
 }
 
@@ -1017,15 +1119,17 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
         vg.r_lo = c->grp_lo[g];
         vg.r_hi = c->grp_hi[g];
         vg.resc_count = c->d_resc_count + (size_t)g * c->nphase;
+        vg.retry_count = c->d_retry_count + (size_t)g * c->nphase;
+        vg.retry_list = c->d_retry_list + (size_t)g * c->nphase * c->act_max;
         vg.resc_list = c->d_resc_list + (size_t)g * c->nphase * c->ctot;
         if (c->d_ex_rows) vg.ex_rows = c->d_ex_rows + (size_t)g * c->ex_alloc * 32;
         cudaStream_t sg = g == 0 ? c->stream : c->side[g];
         if (g > 0) cudaStreamWaitEvent(sg, c->ev_fork, 0);
-        for (int ci = 0; ci < c->nphase; ci++) {
+        for (int ci = 0; ci < c->nrun; ci++) {
             if (c->any_exact) launch_phase_exact(vg, sg, ci, c->grid_exact);
             if (c->any_fast) {
-                launch_phase_fast(c->fast_variant, vg, sg, ci, c->grid_fast);
-                launch_phase_rescue(c->fast_variant & 1, vg, sg, ci, c->sms);
+                launch_phase_fast(c->fast, c->rep[0].k, vg, sg, ci, c->grid_fast);
+                launch_phase_rescue(c->fast.spec21, c->rep[0].k, vg, sg, ci, c->sms);
             }
         }
         if (g > 0) cudaEventRecord(c->ev_join[g], sg);
@@ -1038,7 +1142,7 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
         if (c->any_da || c->rec_cap > 0)
             launch_features(v, c->stream, c->any_da ? mlp_input(c->mlp) : nullptr, c->any_da ? mlp_ld(c->mlp) : 0,
                             c->grid_elem);
-        if (c->any_screen) launch_screen(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_screen, c->fast_variant & 1);
+        if (c->any_screen) launch_screen(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_screen, c->fast.spec21);
         if (c->any_da) {
             const int B = (2 * c->R + 127) / 128 * 128;
             const float *y = mlp_forward_device(c->mlp, B, c->stream);
@@ -1053,23 +1157,26 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
 }
 
 // Scratch of the FP64 colour phases, one set of records per replica group.
-// Active cells of a phase: at most ceil(nc / 2) per axis (two or three colours).
 static int ensure_exact_scratch(lcmc_ctx *c)
 {
-    if (!c->any_exact || c->d_ex_rows) return LCMC_OK;
-    long long act = 0;
+    if (!c->any_exact) return LCMC_OK;
+    const long long act = c->act_max;
     int most = 1; // particles of the largest replica group
-    for (int r = 0; r < c->R; r++) {
-        const long long h = (c->rep[r].nc_max + 1) / 2;
-        act += h * h * h;
-    }
     for (int g = 0; g < c->ngroup; g++) {
         int n = 0;
-        for (int r = c->grp_lo[g]; r < c->grp_hi[g]; r++) n += c->rep[r].n;
+        for (int r = c->grp_lo[g]; r < c->grp_hi[g]; r++)
+            // an FP32 system comes here only with three cells or fewer along an axis
+            if (c->rep[r].kernel == 0 || grid_dim_host(c->rep[r].L[0], c->rep[r].wmin, c->rep[r].fine) < 6) n += c->rep[r].n;
         most = std::max(most, n);
     }
     long long cap, alloc;
     exact_scratch_size(most, &cap, &alloc, &c->ex_nb);
+    if (c->d_ex_rows && alloc <= c->ex_alloc) return LCMC_OK;
+    if (c->d_ex_rows) { // more replicas need it than before
+        CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+        cudaFree(c->d_ex_rows);
+        c->d_ex_rows = nullptr;
+    }
     const size_t np = (size_t)c->nphase;
     if (!c->d_ex_p) CUDA_TRY(c, dalloc(&c->d_ex_p, np * (act + 1)));
     if (!c->d_ex_r) CUDA_TRY(c, dalloc(&c->d_ex_r, np * (act + 1)));
@@ -1090,6 +1197,7 @@ static int check_flags(lcmc_ctx *c)
     int f = 0;
     for (auto &s : st) f |= s.flags;
     if (f & (F_CELLCAP | F_STENCILCAP | F_LISTCAP)) return set_err(c, LCMC_ECELLCAP, "cell capacity exceeded");
+    if (f & F_TIMEOUT) return set_err(c, LCMC_ETIMEOUT, "a copy inside a phase kernel did not land");
     if (f & F_NONFINITE) return set_err(c, LCMC_ENUMERIC, "non-finite energy change");
     if (f & F_DRIFT) {
         char b[200];
@@ -1184,6 +1292,11 @@ extern "C" int lcmc_sweep(lcmc_ctx *ctx, int n_sweeps)
     for (int r = 0; r < ctx->R; r++)
         if (!ctx->uploaded[r]) return set_err(ctx, LCMC_EINVAL, "replica has no configuration (upload or init first)");
     for (int s = 0; s < n_sweeps; s++) {
+        if (ctx->since_choice >= ctx->safe_sweeps) {
+            int rc = recheck_boxes(ctx);
+            if (rc) return rc;
+        }
+        ctx->since_choice++;
         const int par = ctx->cur;
         if (!ctx->graph[par]) {
             int rc = ensure_exact_scratch(ctx);
@@ -1273,7 +1386,7 @@ extern "C" int lcmc_kernels_per_sweep(lcmc_ctx *ctx)
     // energy, chunk sums, accept, scale; surrogate: 2 feature kernels, 2 GEMMs + 3 small kernels, stage 1;
     // recording; history: chunk sums, rows; sweep counter
     const int exact = ctx->any_exact ? 2 * ctx->ex_nb : 0;
-    int n = 8 + (int)ctx->any_exact + ctx->ngroup * ctx->nphase * (exact + 2 * (int)ctx->any_fast) +
+    int n = 8 + (int)ctx->any_exact + ctx->ngroup * ctx->nrun * (exact + 2 * (int)ctx->any_fast) +
             5 * (int)ctx->any_npt + 3;
     if (ctx->any_npt && (ctx->any_da || ctx->rec_cap > 0)) n += 2;
     if (ctx->any_npt && ctx->any_da) n += 6;
@@ -1777,12 +1890,12 @@ void tune_cache_append(const char *path, const std::string &key, const TuneChoic
 
 static int apply_tuning(lcmc_ctx *c, const TuneChoice &ch)
 {
-    c->fast_variant = 2 * ch.variant_class + (c->fast_variant & 1);
+    c->fast.cls = ch.variant_class;
     c->tuned_class = ch.variant_class;
+    choose_fast_shape(c);
     set_caps(c);
     int prc = push_kernel_fields(c);
     if (prc) return prc;
-    c->grid_fast = fast_blocks_per_sm(c->fast_variant) * c->sms;
     for (int r = 0; r < c->R; r++) {
         Replica &rp = c->rep[r];
         rp.vol_cells = ch.vol_cells;
@@ -1802,7 +1915,7 @@ extern "C" int lcmc_autotune(lcmc_ctx *ctx, int sweeps, const char *cache_path, 
     if (ctx->hist_cap > 0 || ctx->rec_cap > 0)
         return set_err(ctx, LCMC_EINVAL, "autotune before recording history or volume samples");
     const std::string key = tune_key(ctx);
-    TuneChoice best{ctx->fast_variant >> 1, 1};
+    TuneChoice best{ctx->fast.cls, 1};
     double best_ms = 0.0;
     lcmc_tuning res;
     memset(&res, 0, sizeof(res));
@@ -1817,7 +1930,7 @@ extern "C" int lcmc_autotune(lcmc_ctx *ctx, int sweeps, const char *cache_path, 
         for (int r = 0; r < ctx->R; r++)
             npt4 = npt4 || (ctx->rep[r].ensemble == 2 && grid_dim_host(ctx->rep[r].L[0], ctx->rep[r].wmin, ctx->rep[r].fine) >= 4);
         for (int v = 0; v < fast_variant_count(); v++) {
-            if (!ctx->any_fast && v != (ctx->fast_variant >> 1)) continue;
+            if (!ctx->any_fast && v != ctx->fast.cls) continue;
             // classes below mean + 3 standard deviations of a cell's count are not tried (the largest always is)
             if (ctx->any_fast && fast_variant(v).amax < ctx->need_min && v != fast_variant_count() - 1) continue;
             cand.push_back({v, 1});

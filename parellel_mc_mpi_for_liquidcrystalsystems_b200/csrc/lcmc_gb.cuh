@@ -205,7 +205,7 @@ __device__ __forceinline__ float pair_fast_21(const FastK &k, float dx, float dy
 }
 
 // FP32 constants of a system for the FP32 pair term.
-__device__ __forceinline__ FastK fast_consts(const GBConsts &k)
+__host__ __device__ __forceinline__ FastK fast_consts(const GBConsts &k)
 {
     FastK K;
     K.rc2 = k.f_rc2;
@@ -225,35 +225,140 @@ __device__ __forceinline__ FastK fast_consts(const GBConsts &k)
     return K;
 }
 
+// Two FP32 values in one 64-bit register pair: sm_100's packed FP32 operations
+// do both in one instruction, each with the rounding of the scalar operation.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 x, float &lo, float &hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x));
+}
+__device__ __forceinline__ f32x2 dup2(float x) { return pack2(x, x); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_ftz(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_ftz(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ f32x2 rsqrt2(f32x2 x)
+{
+    float a, b;
+    unpack2(x, a, b);
+    return pack2(rsqrt_ftz(a), rsqrt_ftz(b));
+}
+__device__ __forceinline__ f32x2 rcp2(f32x2 x)
+{
+    float a, b;
+    unpack2(x, a, b);
+    return pack2(rcp_ftz(a), rcp_ftz(b));
+}
+// x0 y0 + x1 y1 + x2 y2
+__device__ __forceinline__ f32x2 dot2(f32x2 x0, f32x2 y0, f32x2 x1, f32x2 y1, f32x2 x2, f32x2 y2)
+{
+    return fma2(x2, y2, fma2(x0, y0, mul2(x1, y1)));
+}
+
+// pair_fast_21 of two configurations at once, with every rounding of the
+// scalar term as nvcc contracts it (so both give the same bits, and the term
+// does not depend on how a caller is compiled).  The reciprocal square roots
+// and reciprocals flush subnormal arguments, which only two coincident centres
+// (r^2 < 1e-38) have: their term is not finite either way.  Half the issue
+// slots of two scalar terms on the FMA pipe.
+__device__ __forceinline__ void pair_fast_21x2(const FastK &k, f32x2 dx, f32x2 dy, f32x2 dz, f32x2 r2, f32x2 eix,
+                                               f32x2 eiy, f32x2 eiz, f32x2 ejx, f32x2 ejy, f32x2 ejz, float &v0,
+                                               float &v1)
+{
+    const f32x2 one = dup2(1.0f), neg = dup2(-1.0f);
+    const f32x2 ir = rsqrt2(r2);
+    const f32x2 a = dot2(dx, eix, dy, eiy, dz, eiz); // without 1 / r
+    const f32x2 b = mul2(dot2(dx, ejx, dy, ejy, dz, ejz), ir);
+    const f32x2 c = dot2(eix, ejx, eiy, ejy, eiz, ejz);
+    const f32x2 s = fma2(a, ir, b), d = fma2(a, ir, mul2(b, neg));
+    const f32x2 d2 = mul2(d, d);
+    const f32x2 sp = fma2(s, s, d2), sm = fma2(s, s, mul2(d2, neg));
+    const f32x2 c2 = mul2(c, c);
+    const f32x2 eps1 = rsqrt2(fma2(dup2(-k.chi_sq), c2, one));
+    const f32x2 q1 = fma2(mul2(dup2(-k.chi), c), sm, sp);
+    const f32x2 s_chi = fma2(mul2(dup2(-k.half_chi), q1), mul2(eps1, eps1), one);
+    const f32x2 inv2 = rcp2(fma2(dup2(-k.chip_sq), c2, one));
+    const f32x2 q2 = fma2(mul2(dup2(-k.chip), c), sm, sp);
+    const f32x2 eps2 = fma2(mul2(dup2(-k.half_chip), q2), inv2, one);
+    const f32x2 dr = add2(fma2(r2, ir, mul2(rsqrt2(s_chi), neg)), one);
+    const f32x2 R = rcp2(dr);
+    const f32x2 R2 = mul2(R, R);
+    const f32x2 R6 = mul2(mul2(R2, R2), R2);
+    const f32x2 v = mul2(mul2(mul2(dup2(k.four_eps0), mul2(mul2(eps1, eps2), eps2)), R6), add2(R6, neg));
+    float dr0, dr1;
+    unpack2(dr, dr0, dr1);
+    unpack2(v, v0, v1);
+    v0 = dr0 < 0.001f ? 1.0e9f : v0;
+    v1 = dr1 < 0.001f ? 1.0e9f : v1;
+}
+
 template <bool SPEC21>
 __device__ __forceinline__ float pair_fast_t(const FastK &k, float dx, float dy, float dz, float r2, float eix,
                                              float eiy, float eiz, float ejx, float ejy, float ejz);
 
+__device__ __forceinline__ float dot_rn(float x0, float y0, float x1, float y1, float x2, float y2)
+{
+    return __fmaf_rn(x2, y2, __fmaf_rn(x0, y0, __fmul_rn(x1, y1)));
+}
+
+// Any exponents and sigma0.  Every rounding written out, so that the bits do not
+// depend on how a caller is compiled.
 __device__ __forceinline__ float pair_fast(const FastK &k, float dx, float dy, float dz, float r2, float eix,
                                            float eiy, float eiz, float ejx, float ejy, float ejz)
 {
-    float ir = rsqrtf(r2);
-    float r = r2 * ir;
-    float a = (dx * eix + dy * eiy + dz * eiz) * ir;
-    float b = (dx * ejx + dy * ejy + dz * ejz) * ir;
-    float c = eix * ejx + eiy * ejy + eiz * ejz;
-    float s = a + b, d = a - b;
-    float s2 = s * s, d2 = d * d;
-    float sp = s2 + d2, sm = s2 - d2;
-    float c2 = c * c;
-    float eps1 = rsqrtf(1.0f - k.chi_sq * c2);
-    float inv1 = eps1 * eps1;
-    float s_chi = 1.0f - k.half_chi * (sp - k.chi * c * sm) * inv1;
-    float inv2 = __fdividef(1.0f, 1.0f - k.chip_sq * c2);
-    float eps2 = 1.0f - k.half_chip * (sp - k.chip * c * sm) * inv2;
-    float e1 = k.nu_code == 1 ? eps1 : (k.nu_code == 2 ? eps1 * eps1 : __powf(eps1, k.nu));
-    float e2 = k.mu_code == 2 ? eps2 * eps2 : (k.mu_code == 1 ? eps2 : __powf(eps2, k.mu));
-    float sigma = k.sigma0 * rsqrtf(s_chi);
-    float dr = r - sigma + k.sigma0;
-    float R = __fdividef(k.sigma0, dr);
-    float R2 = R * R;
-    float R6 = R2 * R2 * R2;
-    float v = k.four_eps0 * (e1 * e2) * R6 * (R6 - 1.0f);
+    const float ir = rsqrtf(r2);
+    const float a = dot_rn(dx, eix, dy, eiy, dz, eiz); // without 1 / r
+    const float b = __fmul_rn(dot_rn(dx, ejx, dy, ejy, dz, ejz), ir);
+    const float c = dot_rn(eix, ejx, eiy, ejy, eiz, ejz);
+    const float s = __fmaf_rn(a, ir, b), d = __fmaf_rn(a, ir, -b);
+    const float d2 = __fmul_rn(d, d);
+    const float sp = __fmaf_rn(s, s, d2), sm = __fmaf_rn(s, s, -d2);
+    const float c2 = __fmul_rn(c, c);
+    const float eps1 = rsqrtf(__fmaf_rn(-k.chi_sq, c2, 1.0f));
+    const float q1 = __fmaf_rn(-__fmul_rn(k.chi, c), sm, sp);
+    const float s_chi = __fmaf_rn(-__fmul_rn(k.half_chi, q1), __fmul_rn(eps1, eps1), 1.0f);
+    const float inv2 = __fdividef(1.0f, __fmaf_rn(-k.chip_sq, c2, 1.0f));
+    const float q2 = __fmaf_rn(-__fmul_rn(k.chip, c), sm, sp);
+    const float eps2 = __fmaf_rn(-__fmul_rn(k.half_chip, q2), inv2, 1.0f);
+    const float e1 = k.nu_code == 1 ? eps1 : (k.nu_code == 2 ? __fmul_rn(eps1, eps1) : __powf(eps1, k.nu));
+    const float e2 = k.mu_code == 2 ? __fmul_rn(eps2, eps2) : (k.mu_code == 1 ? eps2 : __powf(eps2, k.mu));
+    const float dr = __fadd_rn(__fmaf_rn(r2, ir, -__fmul_rn(k.sigma0, rsqrtf(s_chi))), k.sigma0);
+    const float R = __fdividef(k.sigma0, dr);
+    const float R2 = __fmul_rn(R, R);
+    const float R6 = __fmul_rn(__fmul_rn(R2, R2), R2);
+    const float v = __fmul_rn(__fmul_rn(__fmul_rn(k.four_eps0, __fmul_rn(e1, e2)), R6), __fadd_rn(R6, -1.0f));
     return dr < 0.001f ? 1.0e9f : v;
 }
 
@@ -271,5 +376,35 @@ __device__ __forceinline__ float pair_fast_t<false>(const FastK &k, float dx, fl
                                                     float eiy, float eiz, float ejx, float ejy, float ejz)
 {
     return pair_fast(k, dx, dy, dz, r2, eix, eiy, eiz, ejx, ejy, ejz);
+}
+
+// Terms of two configurations (separations and orientations in pairs), and
+// whether each is within the cutoff.
+template <bool SPEC21>
+__device__ __forceinline__ void pair_fast_x2(const FastK &k, f32x2 dx, f32x2 dy, f32x2 dz, f32x2 eix, f32x2 eiy,
+                                             f32x2 eiz, f32x2 ejx, f32x2 ejy, f32x2 ejz, float &v0, float &v1, bool &in0,
+                                             bool &in1)
+{
+    const f32x2 r2 = dot2(dx, dx, dy, dy, dz, dz);
+    float q0, q1;
+    unpack2(r2, q0, q1);
+    in0 = q0 < k.rc2;
+    in1 = q1 < k.rc2;
+    if (SPEC21) {
+        pair_fast_21x2(k, dx, dy, dz, r2, eix, eiy, eiz, ejx, ejy, ejz, v0, v1);
+    } else {
+        float x[2], y[2], z[2], a0[2], a1[2], a2[2], b0[2], b1[2], b2[2];
+        unpack2(dx, x[0], x[1]);
+        unpack2(dy, y[0], y[1]);
+        unpack2(dz, z[0], z[1]);
+        unpack2(eix, a0[0], a0[1]);
+        unpack2(eiy, a1[0], a1[1]);
+        unpack2(eiz, a2[0], a2[1]);
+        unpack2(ejx, b0[0], b0[1]);
+        unpack2(ejy, b1[0], b1[1]);
+        unpack2(ejz, b2[0], b2[1]);
+        v0 = pair_fast(k, x[0], y[0], z[0], q0, a0[0], a1[0], a2[0], b0[0], b1[0], b2[0]);
+        v1 = pair_fast(k, x[1], y[1], z[1], q1, a0[1], a1[1], a2[1], b0[1], b1[1], b2[1]);
+    }
 }
 } // namespace lcmc

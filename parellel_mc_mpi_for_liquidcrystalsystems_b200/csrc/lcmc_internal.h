@@ -26,6 +26,25 @@ __host__ __device__ __forceinline__ int axis_colour_cell(int nc, int k, int b, i
     return j < q ? b + 3 * j : 3 * q + (r == 2 ? b : 0);
 }
 
+// Colour of cell i along an axis, and its index among the cells of that colour
+// (the inverse of axis_colour_cell).
+__host__ __device__ __forceinline__ void axis_colour_of(int nc, int k, int i, int *b, int *j)
+{
+    if (k != 3) {
+        *b = i & 1;
+        *j = i >> 1;
+        return;
+    }
+    const int q = nc / 3, r = nc - 3 * q;
+    if (i < 3 * q) {
+        *b = i % 3;
+        *j = i / 3;
+    } else {
+        *b = r == 1 ? 1 : i - 3 * q;
+        *j = q;
+    }
+}
+
 // Derived constants of one system (get_system_const, MCnptColloid.c:2752-2783,
 // with chi computed after kappa^2).  FP64, plus FP32 copies for the FP32 kernel.
 struct GBConsts {
@@ -102,7 +121,18 @@ struct DevStats {
 };
 
 // error flag bits (mirrors LCMC_F_* in lcmc.h)
-constexpr int F_CELLCAP = 1, F_STENCILCAP = 2, F_LISTCAP = 4, F_NONFINITE = 8, F_GRIDCAP = 16, F_DRIFT = 32;
+constexpr int F_CELLCAP = 1, F_STENCILCAP = 2, F_LISTCAP = 4, F_NONFINITE = 8, F_GRIDCAP = 16, F_DRIFT = 32,
+              F_TIMEOUT = 64;
+
+// One particle's attempt in an FP32 colour phase, written by the gather: old (a)
+// and trial (b) state relative to the cell origin, in pairs (ax, bx, ay, by),
+// (az, bz, aux, bux), (auy, buy, auz, buz); the trial as the write-back stores it.
+struct alignas(16) ActRec {
+    float4 p0, p1, p2;
+    double tdU, tlu; // colloid-term change, log of the Metropolis draw
+    float reach;     // length of the displacement
+    int code, id, pad; // trial code (thard), particle id
+};
 
 // Launch view of the device buffers, passed by value to every kernel.
 // particles per chunk of the two-level reductions (sums over a replica)
@@ -117,6 +147,9 @@ struct DevView {
     Replica *rep;       // [R]
     DevStats *stats;    // [R]
     int *act_off;       // [nphase * (R + 1)] active-cell prefix per phase
+    int4 *act_tab;      // [nphase][act_max] active cells of a phase: cell, replica, coordinates (8 bits each) with
+                        // the count of its particles above them (at most 255), first particle slot
+    int act_max;
     int nphase;         // colour phases per sweep: 8, or LCMC_MAX_COLOURS with a fine-grid replica
     int r_lo, r_hi;     // replicas whose cells the phase kernels attempt (a group of a batch: [r_lo, r_hi))
     int ngroup;         // replica groups (resc_count/resc_list hold one set of phases per group)
@@ -142,6 +175,8 @@ struct DevView {
     int *resc_count;           // [nphase] cells the FP32 kernel handed over to the FP64 kernel, per colour phase
                                // (per group: a group's view points at its own nphase counts and lists)
     int *resc_list;            // [nphase x ctot] their codes: cell * 4 + mode (1 large term, 2 capacity)
+    int *retry_count;          // [nphase] cells above the light or class kernel's own capacity, run again in FP32 with
+    int *retry_list;           // the largest one: [nphase x act_max] indices into act_tab (per group likewise)
     int *cell_fp64;            // per cell: 0 FP32, 1 attempted in FP64 (large term), 2 (capacity)
     // FP64 colour phases: per phase the particle and record-row prefixes over the
     // active cells ([nphase][ex_act + 1]), cells attempted sequentially
@@ -157,12 +192,11 @@ struct DevView {
     double *scratch_d;         // [R * 8] small reductions
     double *red_part;          // [R x red_nchunk x LCMC_RED_K] per-chunk partial sums
     int red_nchunk;            // chunks of LCMC_RED_CHUNK particles per replica (largest replica)
-    // this sweep's trial moves, by sorted slot (tdU and the displacement: FP32 kernel systems)
+    // this sweep's trial moves, by sorted slot (act_rec: FP32 kernel systems)
     double *tnx, *tny, *tnz;   // new position, wrapped
     double *tux, *tuy, *tuz;   // new orientation, normalised
-    double *tdU;               // colloid-term change
     double *tlu;               // log of the Metropolis draw
-    float *tdx, *tdy, *tdz;    // displacement
+    ActRec *act_rec;           // FP32 copies of both states and what else an attempt needs
     unsigned char *thard;      // 0 evaluate, 1 colloid hard-core reject, 3 leaves its cell (rejected)
     // FP32 copy of the state of FP32-kernel systems, relative to each particle's
     // own cell origin: (x, y, z, ux) and (uy, uz), unit orientation; written by

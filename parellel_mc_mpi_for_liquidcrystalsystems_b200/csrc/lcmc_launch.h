@@ -23,15 +23,26 @@ int energy_exact_blocks_per_sm(); // resident blocks of 128 threads per SM
 
 // lcmc_sweep_fast.cu (FP32)
 struct FastVariant {
-    int threads, amax, seg, lcap; // active-cell capacity, staged candidates per warp, list capacity
+    int amax; // active-cell capacity of a class
+};
+// The FP32 phase kernel a context runs
+struct FastChoice {
+    int cls = 0;        // capacity class
+    bool spec21 = true; // mu = 2, nu = 1, sigma0 = 1 and the same pair constants in every replica
+    bool light = false; // class 0 for systems of at most 40 particles per cell
+    bool wide = false;  // 512 threads per cell: fewer active cells than SMs
+    bool operator==(const FastChoice &o) const
+    {
+        return cls == o.cls && spec21 == o.spec21 && light == o.light && wide == o.wide;
+    }
 };
 int fast_variant_count();
 FastVariant fast_variant(int i);
-void launch_phase_fast(int variant, const DevView &v, cudaStream_t s, int ci, int grid);
-// FP64 attempts of the cells the FP32 kernel handed over in colour phase ci
-void launch_phase_rescue(bool spec21, const DevView &v, cudaStream_t s, int ci, int grid);
+void launch_phase_fast(const FastChoice &c, const GBConsts &k, const DevView &v, cudaStream_t s, int ci, int grid);
+int fast_blocks_per_sm(const FastChoice &c);
+// retries (FP32, the largest capacity) and FP64 attempts of the cells the FP32 kernel left in colour phase ci
+void launch_phase_rescue(bool spec21, const GBConsts &k, const DevView &v, cudaStream_t s, int ci, int grid);
 void rescue_init(); // once per process before the first hand-over launch
-int fast_blocks_per_sm(int variant);
 
 // lcmc_misc.cu
 void launch_q_chunk_sums(const DevView &v, cudaStream_t s); // Q-tensor chunk sums of every replica

@@ -76,7 +76,10 @@ __global__ void k_sweep_setup(DevView v)
         p.vol_state = 0;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < v.nphase * v.ngroup; i += blockDim.x) v.resc_count[i] = 0;
+    for (int i = threadIdx.x; i < v.nphase * v.ngroup; i += blockDim.x) {
+        v.resc_count[i] = 0;
+        v.retry_count[i] = 0;
+    }
     if ((int)threadIdx.x < v.nphase) {
         int ci = threadIdx.x;
         int *off = v.act_off + ci * (v.R + 1);
@@ -214,13 +217,33 @@ __global__ void k_scatter(DevView v)
 
 // Warp per cell: order the cell's slots by particle id (ids are unique inside
 // a replica).  Writes the gather source of every destination slot to `rank`
-// (reused as the second permutation buffer).
+// (reused as the second permutation buffer), and enters the cell in the table of
+// its colour phase's active cells, so that the phase kernels find a cell with
+// one load (their order is the enumeration of act_off: x fastest).
 __global__ void k_sort_cells(DevView v)
 {
     int lane = threadIdx.x & 31;
     int warps = (gridDim.x * blockDim.x) >> 5;
     for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < v.ctot; c += warps) {
         int s = v.cell_start[c], e = v.cell_start[c + 1], n = e - s;
+        if (lane == 0) {
+            const int r = v.p2c[c];
+            const Replica &p = v.rep[r];
+            const int l = c - p.cell_off, nc0 = p.nc[0], nc1 = p.nc[1];
+            if (l < nc0 * nc1 * p.nc[2]) { // a used cell
+                const int x = l % nc0, y = (l / nc0) % nc1, z = l / (nc0 * nc1);
+                int bx, by, bz, jx, jy, jz;
+                axis_colour_of(nc0, p.kc[0], x, &bx, &jx);
+                axis_colour_of(nc1, p.kc[1], y, &by, &jy);
+                axis_colour_of(p.nc[2], p.kc[2], z, &bz, &jz);
+                const int col = bx + p.kc[0] * (by + p.kc[1] * bz);
+                int ci = 0;
+                while (ci < p.ncol - 1 && p.perm[ci] != col) ci++;
+                const int a = v.act_off[ci * (v.R + 1) + r] +
+                              (jz * axis_colour_count(nc1, p.kc[1], by) + jy) * axis_colour_count(nc0, p.kc[0], bx) + jx;
+                v.act_tab[(size_t)ci * v.act_max + a] = make_int4(c, r, (int)((unsigned)(x | y << 8 | z << 16) | (unsigned)min(n, 255) << 24), s);
+            }
+        }
         for (int a = lane; a < n; a += 32) {
             int src = v.perm[s + a];
             int my = v.id[src];
@@ -234,7 +257,8 @@ __global__ void k_sort_cells(DevView v)
 // Permute into the other buffer and build this sweep's trial move of every
 // particle (a particle is attempted once per sweep from its sweep-start state,
 // so the trial is known now): new state, log of the Metropolis draw, trial code,
-// and for systems on the FP32 kernel the displacement and colloid-term change.
+// and for systems on the FP32 kernel the colloid-term change and the FP32 copies
+// of both states (the phase kernels then do no FP64 square root or division).
 __global__ void k_gather(DevView v)
 {
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < v.ntot; g += gridDim.x * blockDim.x) {
@@ -268,10 +292,6 @@ __global__ void k_gather(DevView v)
         if (!p.use_fast) continue;
         double dU = 0.0;
         if (code == 0 && p.k.coll_on) dU = colloid_rod(p.k, rn, en, p.L) - colloid_rod(p.k, ro, eo, p.L);
-        v.tdx[g] = (float)dsp[0];
-        v.tdy[g] = (float)dsp[1];
-        v.tdz[g] = (float)dsp[2];
-        v.tdU[g] = dU;
         // FP32 copy relative to the particle's own cell origin
         const double lx = fold_rel(ro[0], p.shift[0] + (double)cx * p.w[0], 0.5 * p.w[0], p.L[0], 1.0 / p.L[0]);
         const double ly = fold_rel(ro[1], p.shift[1] + (double)cy * p.w[1], 0.5 * p.w[1], p.L[1], 1.0 / p.L[1]);
@@ -280,6 +300,20 @@ __global__ void k_gather(DevView v)
         unit_f32(eo[0], eo[1], eo[2], ux, uy, uz);
         v.cl4[g] = make_float4((float)lx, (float)ly, (float)lz, ux);
         v.cl2[g] = make_float2(uy, uz);
+        float bx, by, bz;
+        unit_f32(en[0], en[1], en[2], bx, by, bz);
+        const float dx = (float)dsp[0], dy = (float)dsp[1], dz = (float)dsp[2];
+        ActRec ar;
+        ar.p0 = make_float4((float)lx, (float)lx + dx, (float)ly, (float)ly + dy);
+        ar.p1 = make_float4((float)lz, (float)lz + dz, ux, bx);
+        ar.p2 = make_float4(uy, by, uz, bz);
+        ar.tdU = dU;
+        ar.tlu = log_unit(u);
+        ar.reach = sqrtf(dx * dx + dy * dy + dz * dz);
+        ar.code = code;
+        ar.id = id;
+        ar.pad = 0;
+        v.act_rec[g] = ar;
     }
 }
 

@@ -21,52 +21,65 @@
 // (MCnptColloid.c:2491-2563) for the sequential in-cell order (ascending id);
 // only the decisions depend on each other, through a triangular system.
 //
-// Phases per cell:
-//   1 stencil  27 cells (>= 4 cells per axis, no duplicates)
-//   2 active   phase-start state and precomputed trial of each particle of the
-//              cell, coordinates relative to the cell origin (FP32)
-//   3 staging  the 26 static cells -> shared memory (float4 x,y,z,ux + float2
-//              uy,uz), read from the FP32 copy of the state (coordinates
-//              relative to each particle's own cell origin, folded across the
-//              periodic seam by the gather) plus the stencil offset, pruned to
-//              the cell box grown by rc + max_displacement/2; warp w compacts its
-//              quarter of the candidates into its own segment (no block barrier
-//              per round)
-//   4 tasks    warps take tasks from a shared queue:
-//              particle task (two particles k, k + 1): cutoff test of every
-//                staged candidate, loaded once, against both old positions
-//                with radius rc + |displacement| (covers old and new state),
-//                warp segment by warp segment, ballot compaction into two
-//                lists, then FP32 Gay-Berne for old and new state over both
-//                lists together, lane sums in FP64
+// What bounds it: one cell's attempt is a chain of short stages (staging, reach
+// tests, pair terms, decisions, write-back) with a block barrier between them,
+// so an SM needs several cells in flight, and how many is set by the shared
+// memory of one (36-74 KB); with six blocks of four warps the schedulers issue
+// in 58 % of the cycles (the pair terms take 37 % of the instructions, the
+// MUFU pipe is at 29 %, DRAM at 3 %).  Stages of a cell:
+//   1 copies   the 26 static cells' FP32 states (float4 x,y,z,ux and float2
+//              uy,uz, relative to each particle's own cell origin) come into
+//              shared memory as bulk copies that ran under the previous cell's
+//              decisions; the stencil offset is added, and each candidate gets
+//              a half-precision test vector
+//   2 tests    which candidates lie within reach (cutoff plus displacement) of
+//              a particle's old position, eight particles and sixteen
+//              candidates per matrix instruction (mma m16n8k8); the sign bits
+//              become the particle's candidate list.  The same tests on the
+//              FP32 pipes, 16 instructions per 32 pairs with ballots and prefix
+//              counts, were half of the old kernel's task time
+//   3 tasks    warps take tasks from a shared queue:
+//              particle task (two particles): Gay-Berne terms of the old and
+//                the trial state over both lists, packed FP32 operations (both
+//                states in one instruction), lane sums of new - old in FP64
 //              pair task: 32 unordered in-cell pairs, 4 terms each
-//              (old/new x old/new), differences formed in FP64
-//   5 sums     warp 0, thread per particle: static + colloid + later in-cell
-//              partners (per-particle trial data was prefetched into shared
-//              memory in step 2)
-//   6 decide   warp 0: Metropolis decisions in id order (fixed-point passes
-//              over the triangular system the sequential order defines)
-//   7 write    accepted trial states to the FP64 master arrays
+//              (old/new x old/new)
+//   4 base     four threads per particle: static + colloid + later in-cell
+//              partners
+//   5 decide   warp 0: Metropolis decisions in id order; warp 1 looks up the
+//              next cell's stencil and starts its copies, threads 32 + k fetch
+//              the next cell's records and this cell's FP64 trial states
+//   6 write    accepted trial states to the FP64 master arrays
+// The list order, and so every sum, depends neither on the block size nor on
+// the capacity class: a system's moves do not depend on how it is batched.
+// One B200, 1,048,576 rods at rho* = 0.32 (5832 cells per phase), all eight
+// phases: 1.97 ms before the tests went to matrix instructions and the terms to
+// packed operations, 1.51 ms now; 262,144 rods at 0.28: 0.57 -> 0.46 ms; a grid
+// of at most one cell per SM (wide blocks): 0.32 -> 0.19 ms (32,768 rods NPT).
 //
 // FP64 for overlaps: FP32 rounding of a pair term is relative to the term,
 // and near an overlap (R^12 up to 1e36 just above the 1e9 clamp) it exceeds
 // any energy scale, so a decision or a running energy built from such terms
 // is meaningless.  A static pair whose FP32 term (old or new state) exceeds
 // f_big in magnitude, hits the overlap clamp or is not finite is evaluated
-// again in FP64 from the master arrays (its flat stencil index is kept with
-// the staged candidate), both states, on the one-fold minimum image; the lane
+// again in FP64 from the master arrays, both states, on the one-fold minimum image; the lane
 // sums are FP64, so such terms carry FP64 rounding only.  A cell with such an
-// in-cell term (whose pair differences are kept in FP32), or above the
-// kernel's capacity (particles, staged candidates or list entries), makes no
-// move here and is handed over to k_phase_rescue, which attempts it from the
-// same phase-start state in FP64.  Below f_big the FP32 terms carry an absolute
+// in-cell term (whose pair differences are kept in FP32) makes no move here and
+// is handed over to k_phase_rescue, which attempts it from the same phase-start
+// state in FP64; a cell above this kernel's capacity (particles, staged
+// candidates or list entries) is run again there in FP32 with the largest
+// capacity, and in FP64 when its class does not hold it.  Below f_big the FP32 terms carry an absolute
 // error of at most about 2e-4 f_big / 100 (1.9e-4 relative, stated per pair),
 // so decisions differ from FP64 only at near-ties.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "lcmc_gb.cuh"
 #include "lcmc_internal.h"
 #include "lcmc_rng.cuh"
+#include "lcmc_tc.cuh"
 #include "lcmc_trial.cuh"
 
 namespace lcmc {
@@ -130,26 +143,50 @@ __device__ __forceinline__ BigPair big_pair64(const double *__restrict__ px, con
     return b;
 }
 
-template <int NT, int AMAX, int SEG, int LW>
+template <int AMAX, int CCAP, int LCAP>
 struct FastSmem {
-    static constexpr int NW = NT / 32;
     static constexpr int NPAIR = AMAX * (AMAX - 1) / 2;
-    float4 cpos[NW * SEG];     // x, y, z, ux of the static candidates (segment per warp)
-    float2 cori[NW * SEG];     // uy, uz
-    unsigned short cidx[NW * SEG]; // flat stencil index of each (to find its FP64 state for a large term)
-    // in-cell pair terms rounded to FP32: C - A, B - A, D - C (for a later particle the scan adds
-    // D - C if the earlier partner moved, B - A if it stayed)
-    float pCA[NPAIR], pBA[NPAIR], pDC[NPAIR];
-    // old (a) and trial (b) state of each active particle, relative to the cell
-    // origin: [0] = (ax, ay, az, aux), [1] = (auy, auz, bx, by), [2] = (bz, bux, buy, buz)
+    float4 cpos[CCAP]; // x, y, z, ux of the static cells' particles, cell by cell
+    float2 cori[CCAP]; // uy, uz
+    union {
+        // half-precision test vectors (x, y, z, |c|^2 rounded down) of the
+        // candidates, relative to the cell centre, scaled; dead once the lists stand
+        uint2 ch[CCAP + 16];
+        // in-cell pair terms rounded to FP32: C - A, and (B - A, D - C) (for a later particle the decisions
+        // add D - C if the earlier partner moved, B - A if it stayed)
+        struct {
+            float2 pBD[NPAIR];
+            float pCA[NPAIR];
+        };
+    };
+    // old (a) and trial (b) state of each active particle, relative to the cell origin, in pairs:
+    // [0] = (ax, bx, ay, by), [1] = (az, bz, aux, bux), [2] = (auy, buy, auz, buz)
     float4 pst[AMAX][3];
-    float rad2[AMAX];
-    double Sold[AMAX], Snew[AMAX];
+    union {
+        struct {
+            uint2 qh[AMAX]; // (-2x, -2y, -2z, 1) of a particle (the reach tests)
+            float qc[AMAX]; // |q|^2 - reach^2 of a particle (1e30: nothing in reach)
+        };
+        struct {
+            // static part of dE (the task queue), then all of it that does not depend on a decision
+            double Sdif[AMAX];
+        };
+    };
     double tdU[AMAX], tlu[AMAX]; // colloid dU of the trial, log of the Metropolis draw
-    int pid[AMAX];        // particle id (outcome slot)
+    unsigned long long pairs;
+    uint64_t full; // mbarrier: the static cells' copies have landed
+    unsigned short lst[AMAX], lcnt[AMAX]; // a particle's part of the list
+    union {
+        unsigned short list[LCAP]; // candidates in reach, particle by particle
+        // from the end of the task queue to the next cell's reach tests, thread 32 + k's own fetches:
+        // the next cell's particle k, and the FP64 trial state of this cell's
+        struct {
+            ActRec next[AMAX];
+            double wn[AMAX][6];
+        };
+    };
     unsigned char hard[AMAX];
-    int acc[AMAX];
-    unsigned short wlist[NW][2][LW]; // per warp: candidate lists of the task's two particles
+    unsigned char acc[AMAX];
     // pairs whose FP32 term is above f_big (overlaps), evaluated in FP64 by the
     // fix-up pass after the task queue: static pairs (particle k << 16 | staged
     // candidate) and in-cell pairs (pair index)
@@ -157,12 +194,13 @@ struct FastSmem {
     unsigned int bigs[BIGCAP];
     unsigned short bigp[BIGCAP];
     int nbigs, nbigp;
-    int st_start[27], st_cnt[27], st_pre[28];
-    int segcnt[NW];
-    int task;
+    struct Stencil {
+        int start[27], cnt[27], pos[28]; // stencil cells: first slot, particles, place of the copy
+        int skip;                        // 0 runs here, 1 not an FP32 cell, 2 above a capacity
+    } st[2]; // the cell that runs and the next
+    int nlist, task;
     int overflow;
     int big; // a pair term above f_big (or clamped, or non-finite): attempt the cell in FP64
-    unsigned long long pairs;
 };
 
 // Hand a cell over to the FP64 phase kernel (k_phase_rescue, launched after
@@ -197,7 +235,7 @@ __device__ __forceinline__ double term64(const Replica &p, const double ri[3], c
 //     ascending staged order, both states in FP64, added to its static sums
 //     (a fixed order: the bits do not depend on scheduling).
 template <int NT, typename SM, bool SPEC21>
-__device__ __noinline__ void fixup_big(const DevView *__restrict__ vp, int r, int g0, int na, SM &sm)
+__device__ __noinline__ void fixup_big(const DevView *__restrict__ vp, int r, int g0, int na, int which, SM &sm)
 {
     const DevView &v = *vp;
     const Replica &p = v.rep[r];
@@ -226,8 +264,7 @@ __device__ __noinline__ void fixup_big(const DevView *__restrict__ vp, int r, in
             sm.big = 1;
         } else {
             sm.pCA[idx] = (float)(term[2] - term[0]);
-            sm.pBA[idx] = (float)(term[1] - term[0]);
-            sm.pDC[idx] = (float)(term[3] - term[2]);
+            sm.pBD[idx] = make_float2((float)(term[1] - term[0]), (float)(term[3] - term[2]));
         }
     }
     unsigned long long extra = 0ull;
@@ -244,467 +281,614 @@ __device__ __noinline__ void fixup_big(const DevView *__restrict__ vp, int r, in
             }
             if (best == (1 << 30)) break;
             last = best;
-            const int f = sm.cidx[best];
-            int sl = 0, hi = 27;
+            int sl = 0, hi = 27; // the candidate's cell: the last that begins at or before it
+            // (a cell without particles shares the place of the next one, or lies before a gap: never picked)
             while (hi - sl > 1) {
                 const int mid = (sl + hi) >> 1;
-                if (sm.st_pre[mid] <= f) sl = mid;
+                if (sm.st[which].pos[mid] <= best) sl = mid;
                 else hi = mid;
             }
             const BigPair b = big_pair64<SPEC21>(v.px, v.py, v.pz, v.ox, v.oy, v.oz, v.tnx, v.tny, v.tnz, v.tux,
-                                                 v.tuy, v.tuz, v.rep + r, g0 + k, sm.st_start[sl] + (f - sm.st_pre[sl]));
+                                                 v.tuy, v.tuz, v.rep + r, g0 + k,
+                                                 sm.st[which].start[sl] + best - sm.st[which].pos[sl]);
             so += b.e0;
             sn += b.e1;
             extra += (unsigned long long)b.n;
             any = true;
         }
         if (any) {
-            sm.Sold[k] += so;
-            sm.Snew[k] += sn;
+            sm.Sdif[k] += sn - so;
         }
     }
     if (extra) atomicAdd(&sm.pairs, extra);
 }
 
-// resident CTAs per SM the register budget is sized for: the 48-particle
-// class (36.9 KB of shared memory) fits six per SM at 80 registers, the
-// 56-particle class (44.5 KB) five at 102, the 64-particle class is limited to
-// three by its shared memory
-template <int AMAX> struct FastMinBlocks { static constexpr int value = AMAX <= 48 ? 6 : (AMAX <= 56 ? 5 : 3); };
-
-template <int NT, int AMAX, int SEG, int LW, bool SPEC21>
-__global__ void __launch_bounds__(NT, FastMinBlocks<AMAX>::value) k_phase_fast(const __grid_constant__ DevView v, int ci)
+#define FAST_ILP 1
+// D += A B of a 16 x 8 tile (half-precision operands, FP32 accumulators).
+__device__ __forceinline__ void mma_16x8x8(float (&d)[4], unsigned a0, unsigned a1, unsigned b0, float c0, float c1)
 {
-    using SM = FastSmem<NT, AMAX, SEG, LW>;
-    constexpr int NW = SM::NW;
-    static_assert(AMAX <= 64, "the scan warp holds two particles per lane");
-    static_assert(AMAX + 32 <= NT, "threads 32 .. 32 + AMAX - 1 write the particles back");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %8, %7, %8};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(b0), "f"(c0), "f"(c1));
+}
+
+__device__ __forceinline__ unsigned h2_bits(__half2 h) { return *reinterpret_cast<unsigned *>(&h); }
+
+// Sums over the warp of two values per lane: lanes 0-15 get the sum of a, 16-31
+// of b (one exchange halves the values a lane carries).
+__device__ __forceinline__ double warp_sum2(double a, double b, int lane)
+{
+    const bool up = lane & 16;
+    const double s = up ? a : b;
+    double x = (up ? b : a) + __shfl_xor_sync(0xffffffffu, s, 16);
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     tc::smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(tc::smem_u32(bar))
+                 : "memory");
+}
+
+// One warp: the stencil of active cell `rec`, and the places of its 26 static
+// cells' copies in shared memory.  Cells that cannot run here are marked.
+template <typename ST, int AMAX, int CCAP>
+__device__ __forceinline__ void prepare_stencil(const DevView &v, ST &st, const int4 rec, int lane)
+{
+    const Replica &p = v.rep[rec.y];
+    const int nc0 = p.nc[0], nc1 = p.nc[1], nc2 = p.nc[2];
+    int start = 0, cnt = 0;
+    if (lane < 27) {
+        int x = (rec.z & 255) + lane % 3 - 1, y = ((rec.z >> 8) & 255) + (lane / 3) % 3 - 1,
+            z = ((rec.z >> 16) & 255) + lane / 9 - 1;
+        x += x < 0 ? nc0 : (x >= nc0 ? -nc0 : 0);
+        y += y < 0 ? nc1 : (y >= nc1 ? -nc1 : 0);
+        z += z < 0 ? nc2 : (z >= nc2 ? -nc2 : 0);
+        const int c = p.cell_off + (z * nc1 + y) * nc0 + x;
+        start = v.cell_start[c];
+        cnt = v.cell_start[c + 1] - start;
+    }
+    const int na = __shfl_sync(0xffffffffu, cnt, 13);
+    // a cell's copy keeps the parity of its slots (granules of two entries); cells that follow one another in
+    // memory (a row's, usually) follow one another here, others begin a granule of their own
+    int end = lane < 27 ? start + cnt : 0;
+    const int e12 = __shfl_sync(0xffffffffu, end, 12);
+    const int s13 = lane == 13 ? e12 : start;
+    if (lane == 13) end = e12; // the cell itself has no copy
+    int prev = __shfl_up_sync(0xffffffffu, end, 1);
+    if (lane == 0) prev = -1;
+    const int pad = lane >= 27 || s13 == prev ? 0 : (lane > 0 ? prev & 1 : 0) + (s13 & 1);
+    const int own = lane < 27 ? end - s13 : 0;
+    int pos = pad + own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, pos, o);
+        if (lane >= o) pos += y;
+    }
+    const int all = __shfl_sync(0xffffffffu, pos, 31);
+    if (lane < 27) {
+        st.start[lane] = start;
+        st.cnt[lane] = cnt;
+        st.pos[lane] = pos - own;
+    }
+    if (lane == 27) st.pos[27] = all;
+    if (lane == 0) st.skip = !p.use_fast ? 1 : (na > AMAX || na > p.cap || all + 1 > CCAP ? 2 : 0);
+}
+
+// One warp: the copies of a prepared cell's static cells (one bulk copy per
+// cell and array, in granules of 16 bytes), completing on sm.full.
+template <typename SM>
+__device__ __forceinline__ void copy_static(const DevView &v, SM &sm, int which, int lane)
+{
+    const auto &st = sm.st[which];
+    if (st.skip) return; // (uniform)
+    const int start = lane < 27 ? st.start[lane] : 0, cnt = lane < 27 && lane != 13 ? st.cnt[lane] : 0;
+    const int n = cnt == 0 ? 0 : ((start + cnt + 1) & ~1) - (start & ~1); // entries copied
+    const unsigned bytes = 24u * __reduce_add_sync(0xffffffffu, (unsigned)n);
+    tc::fence_proxy_async_smem(); // the block's reads and writes of the last cell's copies came before its barrier
+    if (lane == 0) tc::mbar_arrive_expect_tx(&sm.full, bytes);
+    __syncwarp();
+    if (n > 0) {
+        const int pos = st.pos[lane] & ~1, from = start & ~1;
+        bulk_load(&sm.cpos[pos], v.cl4 + from, (unsigned)n * 16u, &sm.full);
+        bulk_load(&sm.cori[pos], v.cl2 + from, (unsigned)n * 8u, &sm.full);
+    }
+}
+
+template <int BYTES>
+__device__ __forceinline__ void fetch_async(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(tc::smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The fetch of one particle's attempt record.
+__device__ __forceinline__ void fetch_rec(ActRec *dst, const ActRec *src)
+{
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(ActRec); i += 16) fetch_async<16>((char *)dst + i, (const char *)src + i);
+}
+
+constexpr unsigned FAST_WAIT_TRIES = 1u << 24; // mbarrier tries before a block gives up
+
+// Cells a retry left to the FP64 attempts of its block.
+struct RetryFailed {
+    int n;
+    int cell[32]; // cell * 4 + mode
+};
+
+// The FP32 attempts of a block: active cells a, a + step, ... below `total` of
+// phase ci (RETRY: of the phase's retry list).
+template <int NT, int AMAX, int CCAP, int LCAP, bool SPEC21, bool RETRY>
+__device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &ku, int ci, unsigned char *smem_raw, int a,
+                                                const int total, const int step, RetryFailed *failed)
+{
+    using SM = FastSmem<AMAX, CCAP, LCAP>;
+    constexpr int NW = NT / 32;
+    static_assert(AMAX <= 64, "the decision warp holds two particles per lane");
+    static_assert(AMAX + 32 <= NT, "threads 32 .. 32 + AMAX - 1 hold a particle each");
+    static_assert(AMAX % 8 == 0 && CCAP % 2 == 0, "test tiles of eight particles; copies of 16 bytes");
     SM &sm = *reinterpret_cast<SM *>(smem_raw);
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const unsigned lt = (1u << lane) - 1u;
-    const int *off = v.act_off + ci * (v.R + 1);
-    const int total = off[v.r_hi]; // this launch's replicas: active cells [off[r_lo], off[r_hi])
+    const int4 *tab = v.act_tab + (size_t)ci * v.act_max;
+    const int *list = v.retry_list + (size_t)ci * v.act_max;
+    auto entry = [&](int i) { return tab[RETRY ? list[i] : i]; };
+    if (a >= total) return;
+    if (t == 0) {
+        tc::mbar_init(&sm.full, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    int4 rec = entry(a); // cell, replica, coordinates (8 bits each) and count of the particles (capped), first slot
+    int4 nxt = a + step < total ? entry(a + step) : make_int4(0, 0, 0, 0);
+    const int kw = t - 32; // thread 32 + k: particle k
+    if (w == 1) {
+        prepare_stencil<typename SM::Stencil, AMAX, CCAP>(v, sm.st[0], rec, lane);
+        __syncwarp();
+        copy_static(v, sm, 0, lane);
+    }
+    if (kw >= 0 && kw < AMAX && kw < (int)((unsigned)rec.z >> 24)) fetch_rec(&sm.next[kw], v.act_rec + rec.w + kw);
+    unsigned phase = 0;
+    int which = 0, id = 0; // id: of particle kw of the cell that runs
+    __syncthreads();
 
-    for (int a = off[v.r_lo] + blockIdx.x; a < total; a += gridDim.x) {
-        const int r = find_replica_f(off, v.R, a);
+    for (;;) {
+        const int cell = rec.x, r = rec.y, g0 = rec.w;
         const Replica &p = v.rep[r];
-        if (!p.use_fast) continue; // uniform across the block
-        const int col = p.perm[ci];
-        const int bx = col % p.kc[0], by = (col / p.kc[0]) % p.kc[1], bz = col / (p.kc[0] * p.kc[1]);
-        const int nc0 = p.nc[0], nc1 = p.nc[1], nc2 = p.nc[2];
-        const int nax = axis_colour_count(nc0, p.kc[0], bx), nay = axis_colour_count(nc1, p.kc[1], by);
-        int loc = a - off[r];
-        const int cx = axis_colour_cell(nc0, p.kc[0], bx, loc % nax);
-        loc /= nax;
-        const int cy = axis_colour_cell(nc1, p.kc[1], by, loc % nay);
-        const int cz = axis_colour_cell(nc2, p.kc[2], bz, loc / nay);
-        const int cell = p.cell_off + (cz * nc1 + cy) * nc0 + cx;
-        const double w0 = p.w[0], w1 = p.w[1], w2 = p.w[2];
-        const FastK K = fast_consts(p.k);
-
-        // ---- 1 stencil ----
-        if (t < 27) {
-            int x = cx + t % 3 - 1, y = cy + (t / 3) % 3 - 1, z = cz + t / 9 - 1;
-            x += x < 0 ? nc0 : (x >= nc0 ? -nc0 : 0);
-            y += y < 0 ? nc1 : (y >= nc1 ? -nc1 : 0);
-            z += z < 0 ? nc2 : (z >= nc2 ? -nc2 : 0);
-            const int c = p.cell_off + (z * nc1 + y) * nc0 + x;
-            const int s = v.cell_start[c];
-            sm.st_start[t] = s;
-            sm.st_cnt[t] = v.cell_start[c + 1] - s;
-        }
-        if (t == 0) {
-            sm.overflow = 0;
-            sm.big = 0;
-            sm.nbigs = 0;
-            sm.nbigp = 0;
-            sm.pairs = 0ull;
-            sm.task = 0;
-        }
-        __syncthreads();
-        if (t < 32) { // prefix over the 26 static cells (slot 13 = the active cell excluded)
-            int c = (t < 27 && t != 13) ? sm.st_cnt[t] : 0;
-            int inc = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += y;
-            }
-            if (t < 27) sm.st_pre[t] = inc - c;
-            if (t == 26) sm.st_pre[27] = inc;
-        }
-        __syncthreads();
-        const int na = sm.st_cnt[13];
-        const int g0 = sm.st_start[13];
-        const int S26 = sm.st_pre[27];
-        if (na > AMAX || na > p.cap) { // above capacity: the whole cell in FP64
-            if (t == 0) hand_over(v, ci, cell, 2);
-            __syncthreads();
-            continue;
-        }
-
-        // ---- 2 active particles: phase-start state and precomputed trial ----
-        const float rcf = (float)p.k.rc;
-        for (int k = t; k < na; k += NT) {
-            const int g = g0 + k;
-            const float4 c4 = v.cl4[g]; // relative to this cell's origin
-            const float2 c2 = v.cl2[g];
-            const float dx = v.tdx[g], dy = v.tdy[g], dz = v.tdz[g];
-            sm.pst[k][0] = c4;
-            sm.pst[k][1] = make_float4(c2.x, c2.y, c4.x + dx, c4.y + dy);
-            float tux, tuy, tuz; // the trial orientation as the FP32 state copy will hold it
-            unit_f32(v.tux[g], v.tuy[g], v.tuz[g], tux, tuy, tuz);
-            sm.pst[k][2] = make_float4(c4.z + dz, tux, tuy, tuz);
-            const float rr = rcf + sqrtf(dx * dx + dy * dy + dz * dz) + 1e-3f;
-            const unsigned char hd = v.thard[g];
-            sm.rad2[k] = hd ? -1.0f : rr * rr;
-            sm.hard[k] = hd;
-            sm.tdU[k] = v.tdU[g];
-            sm.tlu[k] = v.tlu[g];
-            sm.pid[k] = v.id[g];
-        }
-
-        // ---- 3 staging: warp w takes a contiguous quarter of the 26 static cells'
-        //      particles and compacts the kept ones into its own segment ----
-        {
-            const float wx = (float)w0, wy = (float)w1, wz = (float)w2;
-            const float hb = 0.5f * (float)p.k.max_disp + 1e-3f;
-            const float prune2 = K.rc2 * 1.0002f + 1e-3f;
-            const int fb = (int)(((long long)S26 * w) / NW), fe = (int)(((long long)S26 * (w + 1)) / NW);
-            int cnt = 0;
-            // two candidates per lane per round, all six coordinates loaded at
-            // once: the global loads of a round are independent of each other
-            for (int base = fb; base < fe; base += 64) {
-                float x[2], y[2], z[2], ux[2], uy[2], uz[2];
-                bool keep[2];
-                int fi[2];
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int f = base + 32 * h + lane;
-                    fi[h] = f;
-                    keep[h] = false;
-                    x[h] = y[h] = z[h] = ux[h] = uy[h] = uz[h] = 0.0f;
-                    if (f < fe) {
-                        // largest stencil slot whose prefix is <= f (slot 13 has an empty range;
-                        // an empty slot's prefix is the end of the previous range, so it is never picked)
-                        int sl = 0, hi = 27;
-                        while (hi - sl > 1) {
-                            const int mid = (sl + hi) >> 1;
-                            if (sm.st_pre[mid] <= f) sl = mid;
-                            else hi = mid;
-                        }
-                        const int g = sm.st_start[sl] + (f - sm.st_pre[sl]);
-                        const float4 c4 = v.cl4[g]; // relative to its own cell's origin
-                        const float2 c2 = v.cl2[g];
-                        // stencil offset of slot sl is (sl % 3, sl / 3 % 3, sl / 9) - 1 cells
-                        x[h] = c4.x + (float)(sl % 3 - 1) * wx;
-                        y[h] = c4.y + (float)((sl / 3) % 3 - 1) * wy;
-                        z[h] = c4.z + (float)(sl / 9 - 1) * wz;
-                        const float qx = fmaxf(fmaxf(-hb - x[h], x[h] - (wx + hb)), 0.0f);
-                        const float qy = fmaxf(fmaxf(-hb - y[h], y[h] - (wy + hb)), 0.0f);
-                        const float qz = fmaxf(fmaxf(-hb - z[h], z[h] - (wz + hb)), 0.0f);
-                        keep[h] = qx * qx + qy * qy + qz * qz < prune2;
-                        ux[h] = c4.w;
-                        uy[h] = c2.x;
-                        uz[h] = c2.y;
-                    }
-                }
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const unsigned bal = __ballot_sync(0xffffffffu, keep[h]);
-                    const int pos = cnt + __popc(bal & lt);
-                    if (keep[h] && pos < SEG) {
-                        sm.cpos[w * SEG + pos] = make_float4(x[h], y[h], z[h], ux[h]);
-                        sm.cori[w * SEG + pos] = make_float2(uy[h], uz[h]);
-                        sm.cidx[w * SEG + pos] = (unsigned short)fi[h];
-                    }
-                    cnt += __popc(bal);
-                }
-            }
-            if (lane == 0) {
-                sm.segcnt[w] = cnt < SEG ? cnt : SEG;
-                if (cnt > SEG) sm.overflow = 2;
-            }
-        }
-        __syncthreads();
-        if (sm.overflow) { // staged candidates above a warp segment's capacity
-            if (t == 0) hand_over(v, ci, cell, 2);
-            __syncthreads();
-            continue;
-        }
-        // ---- 4 task queue: particle tasks (two particles each: cutoff test +
-        //      pair sums) and in-cell pair tasks ----
-        const int nptask = (na + 1) >> 1;
-        const int npair = na * (na - 1) / 2;
-        const int ntask = nptask + (npair + 31) / 32;
+        const FastK K = SPEC21 ? ku : fast_consts(p.k);
+        int mode = sm.st[which].skip; // 0 runs here, 1 not an FP32 cell, 2 handed over (capacity), 3 handed over (terms)
+        const int na = sm.st[which].cnt[13];
+        const bool more = a + step < total;
+        int s26 = 0;
         unsigned long long npairs = 0ull;
+        if (mode == 0) {
+            // ---- 1 the prepared cell's copies: offsets and test vectors ----
+            const float wx = (float)p.w[0], wy = (float)p.w[1], wz = (float)p.w[2];
+            const float wmax = fmaxf(wx, fmaxf(wy, wz));
+            const float mc = 2.0f * wmax; // above any candidate's coordinate from the cell centre (1.5 cells)
+            // power of two that brings mc into [4, 8): half precision then rounds a coordinate by at most 2^-11 of it
+            const float sc = __int_as_float((129 + 127 - ((__float_as_int(mc) >> 23) & 0xff)) << 23);
+            // sqrt(3) axes, a candidate's and a particle's rounding, and the FP32 sums' own
+            const float slack = 1.75f / 2048.0f * (mc + 0.5f * wmax) + 1e-3f;
+            if (t == 0) {
+                sm.overflow = 0;
+                sm.big = 0;
+                sm.nbigs = 0;
+                sm.nbigp = 0;
+                sm.pairs = 0ull;
+                sm.nlist = 0;
+                sm.task = 0;
+            }
+            if (kw >= 0 && kw < ((na + 7) & ~7)) { // particle kw: states, trial, test vector
+                uint2 qh = make_uint2(0u, 0x3c000000u); // (0, 0, 0, 1)
+                float qc = 1e30f;
+                if (kw < na) {
+                    fetch_wait();
+                    const ActRec ar = sm.next[kw];
+                    sm.pst[kw][0] = ar.p0;
+                    sm.pst[kw][1] = ar.p1;
+                    sm.pst[kw][2] = ar.p2;
+                    sm.hard[kw] = (unsigned char)ar.code;
+                    sm.tdU[kw] = ar.tdU;
+                    sm.tlu[kw] = ar.tlu;
+                    id = ar.id;
+                    if (!ar.code) {
+                        const float rr = ((float)p.k.rc + ar.reach + 1e-3f + slack) * sc;
+                        const __half2 xy = __floats2half2_rn((ar.p0.x - 0.5f * wx) * sc, (ar.p0.z - 0.5f * wy) * sc);
+                        const __half2 z1 = __floats2half2_rn((ar.p1.x - 0.5f * wz) * sc, -0.5f);
+                        const float fx = __low2float(xy), fy = __high2float(xy), fz = __low2float(z1);
+                        qc = fx * fx + fy * fy + fz * fz - rr * rr;
+                        const __half2 m2 = __floats2half2_rn(-2.0f, -2.0f);
+                        qh = make_uint2(h2_bits(__hmul2(xy, m2)), h2_bits(__hmul2(z1, m2)));
+                    }
+                }
+                sm.qh[kw] = qh;
+                sm.qc[kw] = qc;
+            }
+            const auto &st = sm.st[which];
+            const int ncand = st.pos[27]; // places of the copies
+            if (w == 0) s26 = __reduce_add_sync(0xffffffffu, lane < 27 && lane != 13 ? st.cnt[lane] : 0);
+            bool ok = tc::mbar_wait_bounded(&sm.full, phase, FAST_WAIT_TRIES);
+            phase ^= 1u;
+#pragma unroll 2
+            for (int s = w; s < 27; s += NW) {
+                const int pos = st.pos[s], cnt = s == 13 ? 0 : st.cnt[s];
+                // places between two copies: far from everything
+                const int gap = s == 0 ? 0 : st.pos[s - 1] + (s == 14 ? 0 : st.cnt[s - 1]);
+                if (gap + lane < pos) sm.ch[gap + lane] = make_uint2(0u, 0x7b000000u);
+                const float ox = (float)(s % 3 - 1) * wx, oy = (float)((s / 3) % 3 - 1) * wy, oz = (float)(s / 9 - 1) * wz;
+                for (int i = lane; i < cnt; i += 32) {
+                    float4 c = sm.cpos[pos + i]; // relative to its own cell's origin
+                    c.x += ox;
+                    c.y += oy;
+                    c.z += oz;
+                    sm.cpos[pos + i] = c;
+                    const __half2 xy = __floats2half2_rn((c.x - 0.5f * wx) * sc, (c.y - 0.5f * wy) * sc);
+                    const __half hz = __float2half_rn((c.z - 0.5f * wz) * sc);
+                    const float fx = __low2float(xy), fy = __high2float(xy), fz = __half2float(hz);
+                    const __half hs = __float2half_rd(fx * fx + fy * fy + fz * fz);
+                    sm.ch[pos + i] = make_uint2(h2_bits(xy), h2_bits(__halves2half2(hz, hs)));
+                }
+            }
+            if (t < 16) sm.ch[ncand + t] = make_uint2(0u, 0x7b000000u); // beyond the last: likewise
+            if (__syncthreads_or(!ok)) { // (uniform) the copies did not land within the limit: flag it and leave
+                if (t == 0) atomicOr(&v.stats[r].flags, F_TIMEOUT);
+                tc::mbar_wait_bounded(&sm.full, phase ^ 1u, FAST_WAIT_TRIES);
+                return;
+            }
+        // ---- 2 reach tests of eight particles against every candidate ----
+        for (int task = w; task < (na + 7) >> 3; task += NW) {
+            {
+                // test_tile: which candidates lie within reach of eight particles' old positions (cutoff plus the
+                // trial's displacement, so both states are covered), by matrix instructions: a candidate's row
+                // (x, y, z, |c|^2) times a particle's column (-2x, -2y, -2z, 1) plus |q|^2 - reach^2 is negative
+                // when it is in reach.  The operands are in half precision; `slack` covers their rounding (2^-11
+                // of a coordinate each) and |c|^2 is rounded down, so every pair inside the cutoff is in the
+                // list, and the few beyond it add nothing (the pair evaluation tests the FP32 distance).
+                // Lanes q >= 2 carry the unused half of the inner dimension: their column entries are zero.
+                // A sign bit is shifted into the lane's mask for each row: lane 4 g + q holds the candidates
+                // 8 z + g of particles 2 q and 2 q + 1, the first in the highest bit.
+                constexpr int NB = (CCAP + 255) / 256;
+                const int g = lane >> 2, q = lane & 3, k0 = 8 * task;
+                const uint2 bq = sm.qh[k0 + g];
+                const unsigned b0 = q == 0 ? bq.x : (q == 1 ? bq.y : 0u);
+                const float c0 = sm.qc[k0 + 2 * q], c1 = sm.qc[k0 + 2 * q + 1];
+                const unsigned *ah = reinterpret_cast<const unsigned *>(sm.ch) + 2 * g + (q & 1);
+                unsigned m0[NB], m1[NB];
+                const int nmt = (ncand + 15) >> 4;
+                int n0 = 0, n1 = 0;
+#pragma unroll
+                for (int b = 0; b < NB; b++) {
+                    unsigned x0 = 0u, x1 = 0u;
+                    const int e = min(16, nmt - 16 * b);
+#pragma unroll 4
+                    for (int i = 0; i < e; i++) {
+                        const unsigned a0 = ah[32 * (16 * b + i)], a1 = ah[32 * (16 * b + i) + 16];
+                        float d[4];
+                        mma_16x8x8(d, a0, a1, b0, c0, c1);
+                        x0 = __funnelshift_l(__float_as_uint(d[0]), x0, 1);
+                        x1 = __funnelshift_l(__float_as_uint(d[1]), x1, 1);
+                        x0 = __funnelshift_l(__float_as_uint(d[2]), x0, 1);
+                        x1 = __funnelshift_l(__float_as_uint(d[3]), x1, 1);
+                    }
+                    if (e <= 0) x0 = x1 = 0u;
+                    else if (e < 16) {
+                        x0 <<= 32 - 2 * e;
+                        x1 <<= 32 - 2 * e;
+                    }
+                    m0[b] = x0;
+                    m1[b] = x1;
+                    n0 += __popc(x0);
+                    n1 += __popc(x1);
+                }
+                // offsets: lanes of a particle (stride 4) in order, then the particles
+                int i0 = n0, i1 = n1;
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    const int y0 = __shfl_up_sync(0xffffffffu, i0, o), y1 = __shfl_up_sync(0xffffffffu, i1, o);
+                    if (lane >= o) {
+                        i0 += y0;
+                        i1 += y1;
+                    }
+                }
+                const int t0 = __shfl_sync(0xffffffffu, i0, 28 + q), t1 = __shfl_sync(0xffffffffu, i1, 28 + q);
+                int s = t0 + t1;
+                {
+                    int y = __shfl_up_sync(0xffffffffu, s, 1, 4);
+                    if (q >= 1) s += y;
+                    y = __shfl_up_sync(0xffffffffu, s, 2, 4);
+                    if (q >= 2) s += y;
+                }
+                const int all = __shfl_sync(0xffffffffu, s, 3);
+                int base = 0;
+                if (lane == 0) base = atomicAdd(&sm.nlist, all);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                const bool fits = base + all <= LCAP;
+                base += s - t0 - t1;
+                if (g == 0) {
+                    sm.lst[k0 + 2 * q] = (unsigned short)base;
+                    sm.lst[k0 + 2 * q + 1] = (unsigned short)(base + t0);
+                    sm.lcnt[k0 + 2 * q] = (unsigned short)(fits ? t0 : 0);
+                    sm.lcnt[k0 + 2 * q + 1] = (unsigned short)(fits ? t1 : 0);
+                }
+                if (!fits) {
+                    if (lane == 0) sm.overflow = 1;
+                } else {
+                    unsigned short *l0 = sm.list + base + i0 - n0, *l1 = sm.list + base + t0 + i1 - n1;
+#pragma unroll
+                    for (int b = 0; b < NB; b++) {
+                        const int c = 256 * b + g;
+                        unsigned x0 = m0[b], x1 = m1[b];
+                        while (x0 | x1) { // both particles' next candidates (two independent chains)
+                            const int z0 = __clz(x0), z1 = __clz(x1); // 32 when exhausted
+                            if (x0) *l0++ = (unsigned short)(c + 8 * z0);
+                            if (x1) *l1++ = (unsigned short)(c + 8 * z1);
+                            x0 &= 0x7fffffffu >> z0;
+                            x1 &= 0x7fffffffu >> z1;
+                        }
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        // ---- 3 task queue: Gay-Berne terms of two particles' lists, old and trial state; in-cell pairs ----
+        const int nptask = (na + 1) >> 1, npair = na * (na - 1) / 2;
+        const int ntask2 = nptask + (npair + 31) / 32;
         for (;;) {
             int task = 0;
-            if (lane == 0) task = *(volatile int *)&sm.big ? ntask : atomicAdd(&sm.task, 1);
+            if (lane == 0) task = sm.overflow ? ntask2 : atomicAdd(&sm.task, 1);
             task = __shfl_sync(0xffffffffu, task, 0);
-            if (task >= ntask) break;
-            if (task < nptask) {
-                const int ka = 2 * task, kb = 2 * task + 1;
-                const bool has_b = kb < na;
-                const float R2a = sm.rad2[ka];
-                const float R2b = has_b ? sm.rad2[kb] : -1.0f;
-                double soa = 0.0, sna = 0.0, sob = 0.0, snb = 0.0;
-                int np = 0;
-                if (R2a > 0.0f || R2b > 0.0f) {
-                    const float4 qa = sm.pst[ka][0];
-                    const float4 qb = has_b ? sm.pst[kb][0] : qa;
-                    int ca = 0, cb = 0;
-                    // cutoff test of every staged candidate, warp segment by warp segment
-#pragma unroll 1
-                    for (int i = 0; i < NW; i++) {
-                        const int s0 = i * SEG, sc = sm.segcnt[i];
-                        for (int base = 0; base < sc; base += 64) {
-                            bool pa[2], pb[2];
-#pragma unroll
-                            for (int h = 0; h < 2; h++) {
-                                const int j = base + 32 * h + lane;
-                                pa[h] = pb[h] = false;
-                                if (j < sc) {
-                                    const float4 c = sm.cpos[s0 + j];
-                                    float dx = c.x - qa.x, dy = c.y - qa.y, dz = c.z - qa.z;
-                                    pa[h] = dx * dx + dy * dy + dz * dz < R2a;
-                                    dx = c.x - qb.x;
-                                    dy = c.y - qb.y;
-                                    dz = c.z - qb.z;
-                                    pb[h] = dx * dx + dy * dy + dz * dz < R2b;
-                                }
-                            }
-#pragma unroll
-                            for (int h = 0; h < 2; h++) {
-                                const unsigned ba = __ballot_sync(0xffffffffu, pa[h]);
-                                const unsigned bb = __ballot_sync(0xffffffffu, pb[h]);
-                                const int pa_ = ca + __popc(ba & lt), pb_ = cb + __popc(bb & lt);
-                                const unsigned short sl = (unsigned short)(s0 + base + 32 * h + lane);
-                                if (pa[h] && pa_ < LW) sm.wlist[w][0][pa_] = sl;
-                                if (pb[h] && pb_ < LW) sm.wlist[w][1][pb_] = sl;
-                                ca += __popc(ba);
-                                cb += __popc(bb);
-                            }
-                        }
-                    }
-                    if (ca > LW || cb > LW) {
-                        if (lane == 0) sm.overflow = 1;
-                        ca = ca < LW ? ca : LW;
-                        cb = cb < LW ? cb : LW;
-                    }
-                    __syncwarp();
-                    // FP64 lane sums of the FP32 terms.  Entries [0, ca) belong to
-                    // particle a, [ca, ca + cb) to particle b.  An entry with a term
-                    // FP32 cannot carry is listed for the FP64 fix-up pass.
-                    for (int q = lane; q < ca + cb; q += 32) {
-                        const bool isa = q < ca;
-                        const int j = isa ? sm.wlist[w][0][q] : sm.wlist[w][1][q - ca];
-                        const int k = isa ? ka : kb;
-                        const float4 P0 = sm.pst[k][0], P1 = sm.pst[k][1], P2 = sm.pst[k][2];
-                        const float4 c = sm.cpos[j];
-                        const float2 u = sm.cori[j];
-                        float dx = c.x - P0.x, dy = c.y - P0.y, dz = c.z - P0.z;
-                        float r2 = dx * dx + dy * dy + dz * dz;
-                        const float e0 = pair_fast_t<SPEC21>(K, dx, dy, dz, r2, P0.w, P1.x, P1.y, c.w, u.x, u.y);
-                        const bool in0 = r2 < K.rc2;
-                        dx = c.x - P1.z;
-                        dy = c.y - P1.w;
-                        dz = c.z - P2.x;
-                        r2 = dx * dx + dy * dy + dz * dz;
-                        const float e1 = pair_fast_t<SPEC21>(K, dx, dy, dz, r2, P2.y, P2.z, P2.w, c.w, u.x, u.y);
-                        const bool in1 = r2 < K.rc2;
-                        int nin = (int)in0 + (int)in1;
-                        double d0 = in0 ? (double)e0 : 0.0, d1 = in1 ? (double)e1 : 0.0;
-                        if ((in0 && !(fabsf(e0) <= K.big)) || (in1 && !(fabsf(e1) <= K.big))) {
-                            const int slot = atomicAdd(&sm.nbigs, 1);
-                            if (slot < SM::BIGCAP) sm.bigs[slot] = ((unsigned)k << 16) | (unsigned)j;
-                            else sm.overflow = 1;
-                            d0 = d1 = 0.0;
-                            nin = 0;
-                        }
-                        if (isa) {
-                            soa += d0;
-                            sna += d1;
-                        } else {
-                            sob += d0;
-                            snb += d1;
-                        }
-                        np += nin;
-                    }
-                    __syncwarp();
-                }
-#pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) {
-                    soa += __shfl_xor_sync(0xffffffffu, soa, o);
-                    sna += __shfl_xor_sync(0xffffffffu, sna, o);
-                    sob += __shfl_xor_sync(0xffffffffu, sob, o);
-                    snb += __shfl_xor_sync(0xffffffffu, snb, o);
-                    np += __shfl_xor_sync(0xffffffffu, np, o);
-                }
-                if (lane == 0) {
-                    sm.Sold[ka] = soa;
-                    sm.Snew[ka] = sna;
-                    if (has_b) {
-                        sm.Sold[kb] = sob;
-                        sm.Snew[kb] = snb;
-                    }
-                }
-                npairs += (unsigned long long)np;
-            } else {
-                const int idx = (task - nptask) * 32 + lane;
-                int npin = 0;
-                if (idx < npair) {
-                    int q = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)idx)) * 0.5f);
-                    while (q * (q - 1) / 2 > idx) q--;
-                    while ((q + 1) * q / 2 <= idx) q++;
-                    const int pp = idx - q * (q - 1) / 2;
-                    float A, B, Cc, D;
+            if (task >= ntask2) break;
+            if (task >= nptask) { // 32 in-cell pairs, four terms each
+            const int idx = (task - nptask) * 32 + lane;
+            int npin = 0;
+            if (idx < npair) {
+                int q = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)idx)) * 0.5f);
+                while (q * (q - 1) / 2 > idx) q--;
+                while ((q + 1) * q / 2 <= idx) q++;
+                const int pp = idx - q * (q - 1) / 2;
+                float A, B, Cc, D;
+                {
+                    // q's states in pairs against p's old (A, B) and trial state (C, D)
                     const float4 Q0 = sm.pst[q][0], Q1 = sm.pst[q][1], Q2 = sm.pst[q][2];
                     const float4 R0 = sm.pst[pp][0], R1 = sm.pst[pp][1], R2 = sm.pst[pp][2];
-                    // a(.) = (X0.x, X0.y, X0.z), u_a = (X0.w, X1.x, X1.y); b(.) = (X1.z, X1.w, X2.x), u_b = (X2.y, X2.z, X2.w)
-                    {
-                        float dx = Q0.x - R0.x, dy = Q0.y - R0.y, dz = Q0.z - R0.z;
-                        float r2 = dx * dx + dy * dy + dz * dz;
-                        A = pair_fast_t<SPEC21>(K, dx, dy, dz, r2, R0.w, R1.x, R1.y, Q0.w, Q1.x, Q1.y);
-                        A = r2 < K.rc2 ? A : 0.0f;
-                        npin += 2 * (r2 < K.rc2);
-                    }
-                    {
-                        float dx = Q1.z - R0.x, dy = Q1.w - R0.y, dz = Q2.x - R0.z;
-                        float r2 = dx * dx + dy * dy + dz * dz;
-                        B = pair_fast_t<SPEC21>(K, dx, dy, dz, r2, R0.w, R1.x, R1.y, Q2.y, Q2.z, Q2.w);
-                        B = r2 < K.rc2 ? B : 0.0f;
-                        npin += (r2 < K.rc2);
-                    }
-                    {
-                        float dx = Q0.x - R1.z, dy = Q0.y - R1.w, dz = Q0.z - R2.x;
-                        float r2 = dx * dx + dy * dy + dz * dz;
-                        Cc = pair_fast_t<SPEC21>(K, dx, dy, dz, r2, R2.y, R2.z, R2.w, Q0.w, Q1.x, Q1.y);
-                        Cc = r2 < K.rc2 ? Cc : 0.0f;
-                        npin += (r2 < K.rc2);
-                    }
-                    {
-                        float dx = Q1.z - R1.z, dy = Q1.w - R1.w, dz = Q2.x - R2.x;
-                        float r2 = dx * dx + dy * dy + dz * dz;
-                        D = pair_fast_t<SPEC21>(K, dx, dy, dz, r2, R2.y, R2.z, R2.w, Q2.y, Q2.z, Q2.w);
-                        D = r2 < K.rc2 ? D : 0.0f;
-                    }
-                    // a particle that cannot move (colloid hard core, or a trial out of the cell) keeps
-                    // its old state: terms with its trial state are never used, so they are dropped
-                    // before the size test (p hard: C and D unused; q hard: B and D unused)
-                    const bool hp = sm.hard[pp] != 0, hq = sm.hard[q] != 0;
-                    if (hq) B = D = 0.0f;
-                    if (hp) Cc = D = 0.0f;
-                    if (hp && hq) A = 0.0f;
-                    if (!(fabsf(A) <= K.big && fabsf(B) <= K.big && fabsf(Cc) <= K.big && fabsf(D) <= K.big)) {
-                        const int slot = atomicAdd(&sm.nbigp, 1); // the fix-up pass rewrites this pair
-                        if (slot < SM::BIGCAP) sm.bigp[slot] = (unsigned short)idx;
-                        else sm.overflow = 1;
-                    }
-                    // differences in FP64, then rounded (each term is at most f_big here)
-                    const double a = A, b = B, c = Cc, d = D;
-                    sm.pCA[idx] = (float)(c - a);
-                    sm.pBA[idx] = (float)(b - a);
-                    sm.pDC[idx] = (float)(d - c);
+                    const f32x2 qx = pack2(Q0.x, Q0.y), qy = pack2(Q0.z, Q0.w), qz = pack2(Q1.x, Q1.y);
+                    const f32x2 ux = pack2(Q1.z, Q1.w), uy = pack2(Q2.x, Q2.y), uz = pack2(Q2.z, Q2.w);
+                    const f32x2 neg = dup2(-1.0f);
+                    bool in0, in1;
+                    pair_fast_x2<SPEC21>(K, fma2(dup2(R0.x), neg, qx), fma2(dup2(R0.z), neg, qy), fma2(dup2(R1.x), neg, qz),
+                                         dup2(R1.z), dup2(R2.x), dup2(R2.z), ux, uy, uz, A, B, in0, in1);
+                    A = in0 ? A : 0.0f;
+                    B = in1 ? B : 0.0f;
+                    npin += 2 * (int)in0 + (int)in1;
+                    pair_fast_x2<SPEC21>(K, fma2(dup2(R0.y), neg, qx), fma2(dup2(R0.w), neg, qy), fma2(dup2(R1.y), neg, qz),
+                                         dup2(R1.w), dup2(R2.y), dup2(R2.w), ux, uy, uz, Cc, D, in0, in1);
+                    Cc = in0 ? Cc : 0.0f;
+                    D = in1 ? D : 0.0f;
+                    npin += (int)in0;
+                }
+                // a particle that cannot move (colloid hard core, or a trial out of the cell) keeps
+                // its old state: terms with its trial state are never used, so they are dropped
+                // before the size test (p hard: C and D unused; q hard: B and D unused)
+                const bool hp = sm.hard[pp] != 0, hq = sm.hard[q] != 0;
+                if (hq) B = D = 0.0f;
+                if (hp) Cc = D = 0.0f;
+                if (hp && hq) A = 0.0f;
+                if (!(fabsf(A) <= K.big && fabsf(B) <= K.big && fabsf(Cc) <= K.big && fabsf(D) <= K.big)) {
+                    const int slot = atomicAdd(&sm.nbigp, 1); // the fix-up pass rewrites this pair
+                    if (slot < SM::BIGCAP) sm.bigp[slot] = (unsigned short)idx;
+                    else sm.overflow = 1;
+                }
+                // differences in FP64, then rounded (each term is at most f_big here)
+                const double a = A, b = B, c = Cc, d = D;
+                sm.pCA[idx] = (float)(c - a);
+                sm.pBD[idx] = make_float2((float)(b - a), (float)(d - c));
+            }
+                npairs += (unsigned long long)__reduce_add_sync(0xffffffffu, npin);
+                continue;
+            }
+            const int ka = 2 * task, kb = ka + 1; // kb = na has an empty list (its tile's padding)
+            const int ca = sm.lcnt[ka], cb = kb < na ? sm.lcnt[kb] : 0;
+            const int la = sm.lst[ka], lb = (kb < na ? sm.lst[kb] : 0) - ca;
+            double sa = 0.0, sb = 0.0; // new minus old of either particle
+            int np = 0;
+            // FP64 lane sums of the FP32 terms.  Entries [0, ca) belong to
+            // particle a, [ca, ca + cb) to particle b.  An entry with a term
+            // FP32 cannot carry is listed for the FP64 fix-up pass.
+            // Two entries per lane and step: their chains of a dozen dependent
+            // operations and five MUFU calls run side by side.
+            const int n = ca + cb;
+            const f32x2 neg = dup2(-1.0f);
+            for (int q0 = 0; q0 < n; q0 += 32 * FAST_ILP) {
+                int jj[FAST_ILP], kk[FAST_ILP];
+                float e0[FAST_ILP], e1[FAST_ILP];
+                bool in0[FAST_ILP], in1[FAST_ILP];
+#pragma unroll
+                for (int h = 0; h < FAST_ILP; h++) {
+                    const int q = q0 + 32 * h + lane;
+                    const bool isa = q < ca;
+                    const int j = q < n ? sm.list[(isa ? la : lb) + q] : 0;
+                    const int k = isa ? ka : min(kb, na - 1);
+                    jj[h] = j;
+                    kk[h] = k;
+                    const float4 P0 = sm.pst[k][0], P1 = sm.pst[k][1], P2 = sm.pst[k][2];
+                    const float4 c = sm.cpos[j];
+                    const float2 u = sm.cori[j];
+                    pair_fast_x2<SPEC21>(K, fma2(pack2(P0.x, P0.y), neg, dup2(c.x)),
+                                         fma2(pack2(P0.z, P0.w), neg, dup2(c.y)),
+                                         fma2(pack2(P1.x, P1.y), neg, dup2(c.z)), pack2(P1.z, P1.w), pack2(P2.x, P2.y),
+                                         pack2(P2.z, P2.w), dup2(c.w), dup2(u.x), dup2(u.y), e0[h], e1[h], in0[h],
+                                         in1[h]);
+                    e0[h] = in0[h] && q < n ? e0[h] : 0.0f; // beyond the cutoff
+                    e1[h] = in1[h] && q < n ? e1[h] : 0.0f;
+                    np += (int)(in0[h] && q < n) + (int)(in1[h] && q < n);
                 }
 #pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) npin += __shfl_xor_sync(0xffffffffu, npin, o);
-                npairs += (unsigned long long)npin;
+                for (int h = 0; h < FAST_ILP; h++) {
+                    const bool isa = q0 + 32 * h + lane < ca;
+                    if (!(fmaxf(fabsf(e0[h]), fabsf(e1[h])) <= K.big) || e0[h] != e0[h] || e1[h] != e1[h]) {
+                        const int slot = atomicAdd(&sm.nbigs, 1);
+                        if (slot < SM::BIGCAP) sm.bigs[slot] = ((unsigned)kk[h] << 16) | (unsigned)jj[h];
+                        else sm.overflow = 1;
+                        np -= (int)(in0[h]) + (int)(in1[h]); // the fix-up counts its pairs
+                        e0[h] = e1[h] = 0.0f;
+                    }
+                    const double d = (double)e1[h] - (double)e0[h];
+                    if (isa) sa += d;
+                    else sb += d;
+                }
             }
+            __syncwarp();
+            const double sum = warp_sum2(sa, sb, lane);
+            if (lane == 0) sm.Sdif[ka] = sum;
+            if (lane == 16 && kb < na) sm.Sdif[kb] = sum;
+            npairs += (unsigned long long)__reduce_add_sync(0xffffffffu, np);
         }
         if (lane == 0 && npairs) atomicAdd(&sm.pairs, npairs);
+        tc::fence_proxy_async_smem(); // the next cell's copies overwrite what this cell read and wrote
         __syncthreads();
         if (!sm.overflow && (sm.nbigs | sm.nbigp)) { // (uniform) FP64 fix-up of the listed pairs
-            fixup_big<NT, SM, SPEC21>(&v, r, g0, na, sm);
+            fixup_big<NT, SM, SPEC21>(&v, r, g0, na, which, sm);
             __syncthreads();
         }
-        if (sm.overflow || sm.big) { // a capacity exceeded, or an in-cell term too large to keep in FP32
-            if (t == 0) hand_over(v, ci, cell, sm.overflow ? 2 : 1);
-            __syncthreads();
-            continue;
-        }
-
-        // ---- 5+6 warp 0: decision-independent part of dE (thread per particle),
-        //      then the Metropolis decisions in id order; meanwhile thread
-        //      32 + k loads the FP64 trial state of particle k for step 7 ----
-        const int kw = t - 32; // write-back particle of this thread
-        double wn[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        if (w != 0 && kw < na) {
-            const int g = g0 + kw;
-            wn[0] = v.tnx[g];
-            wn[1] = v.tny[g];
-            wn[2] = v.tnz[g];
-            wn[3] = v.tux[g];
-            wn[4] = v.tuy[g];
-            wn[5] = v.tuz[g];
-        }
-        if (w == 0) {
-            // decision-independent part of dE_k: static cells, colloid, and the
-            // in-cell partners after k (still at their old state when k is tried)
-            double e0 = 0.0, e1 = 0.0;
-            for (int h = 0; h < 2; h++) {
-                const int k = lane + 32 * h;
-                if (k >= na) break;
-                double sc = 0.0, sd = 0.0;
-                int m = k + 1;
-                for (; m + 1 < na; m += 2) {
-                    sc += (double)sm.pCA[tri(k, m)];
-                    sd += (double)sm.pCA[tri(k, m + 1)];
+        // a capacity exceeded, or an in-cell term too large to keep in FP32
+        if (sm.overflow || sm.big) mode = sm.overflow ? 2 : 3;
+        // ---- 4 the part of dE that no decision changes: static cells, colloid, and the in-cell partners after k
+        //      (still at their old state when k is tried); four threads per particle ----
+        if (mode == 0) {
+            for (int k0 = 0; k0 < na; k0 += NT / 4) {
+                const int k = k0 + (t >> 2);
+                double s0 = 0.0, s1 = 0.0;
+                if (k < na) {
+                    for (int m = k + 1 + (t & 3); m < na; m += 8) {
+                        const int m1 = m + 4;
+                        s0 += (double)sm.pCA[m * (m - 1) / 2 + k];
+                        s1 += (double)(m1 < na ? sm.pCA[m1 * (m1 - 1) / 2 + k] : 0.0f);
+                    }
                 }
-                if (m < na) sc += (double)sm.pCA[tri(k, m)];
-                const double d = (sm.Snew[k] - sm.Sold[k]) + (sc + sd) + sm.tdU[k];
-                if (h == 0) e0 = d;
-                else e1 = d;
+                s0 += s1;
+                s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+                s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+                if ((t & 3) == 0 && k < na) sm.Sdif[k] = sm.Sdif[k] + s0 + sm.tdU[k];
             }
-            // Metropolis decisions in id order.  dE_k = base_k + sum over earlier
-            // m of (D - C if m accepted, else B - A): a triangular system, solved
-            // by fixed-point rounds in parallel.  Each round recomputes every
-            // dE_k from the current guess of the earlier decisions, adding the
-            // terms in increasing m exactly as a sequential scan would; after
-            // pass r the first r decisions are final, and a pass that changes
-            // no decision has reached the unique solution (usually the second
-            // or third pass), so the decisions and dE_k equal the sequential
-            // scan's bits.
+            __syncthreads();
+        }
+        } // mode == 0
+
+        // ---- 5 warp 0: the Metropolis decisions in id order; meanwhile warp 1 prepares the next cell (its copies run under the decisions), thread
+        //      32 + k loads the next cell's particle k and the FP64 trial state of this cell's ----
+        // dE_k = base_k + sum over earlier m of (D - C if m was accepted, else
+        // B - A): lane k carries dE_k (and lane k - 32 the particles from 32 on);
+        // step m decides particle m, whose sum is then complete, and adds m's
+        // term to every later particle's.  Both terms are converted ahead of the
+        // step, so its chain is the test, the vote and one addition.
+        unsigned acc0 = 0u, acc1 = 0u, hc0 = 0u, hc1 = 0u;
+        double x0 = 0.0, x1 = 0.0;
+        if (w == 0 && mode == 0) {
             const double beta = p.k.beta;
             const bool v0 = lane < na, v1 = lane + 32 < na;
-            const unsigned hd0 = __ballot_sync(0xffffffffu, v0 && sm.hard[lane]);
-            const unsigned hd1 = __ballot_sync(0xffffffffu, v1 && sm.hard[lane + 32]);
+            const bool go0 = v0 && !sm.hard[lane], go1 = v1 && !sm.hard[lane + 32];
             const double lu0 = v0 ? sm.tlu[lane] : 0.0, lu1 = v1 ? sm.tlu[lane + 32] : 0.0;
-            unsigned acc0 = 0u, acc1 = 0u;
-            double x0 = e0, x1 = e1;
-            for (int round = 0; round <= na; round++) {
-                x0 = e0;
-                x1 = e1;
-                if (v0) {
-                    const int kb = tri(0, lane);
-                    for (int m = 0; m < lane; m++) x0 += (double)((acc0 >> m) & 1u ? sm.pDC[kb + m] : sm.pBA[kb + m]);
+            x0 = v0 ? sm.Sdif[lane] : 0.0;
+            x1 = v1 ? sm.Sdif[lane + 32] : 0.0;
+            const float2 *row0 = sm.pBD + (lane * (lane - 1)) / 2, *row1 = sm.pBD + ((lane + 32) * (lane + 31)) / 2;
+            if (na <= 32) { // (uniform)
+                for (int m0 = 0; m0 < na; m0 += 4) {
+                    double ba[4], dc[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const float2 q = v0 && m0 + i < lane ? row0[m0 + i] : make_float2(0.0f, 0.0f);
+                        ba[i] = (double)q.x;
+                        dc[i] = (double)q.y;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const bool a0 = go0 && ((x0 <= 0.0) || (lu0 <= -beta * x0));
+                        const unsigned bit = __ballot_sync(0xffffffffu, a0) & (1u << (m0 + i));
+                        acc0 |= bit;
+                        x0 += bit ? dc[i] : ba[i];
+                    }
                 }
-                if (v1) {
-                    const int k = lane + 32, kb = tri(0, k);
-                    for (int m = 0; m < 32; m++) x1 += (double)((acc0 >> m) & 1u ? sm.pDC[kb + m] : sm.pBA[kb + m]);
-                    for (int m = 32; m < k; m++)
-                        x1 += (double)((acc1 >> (m - 32)) & 1u ? sm.pDC[kb + m] : sm.pBA[kb + m]);
+            } else {
+                for (int m = 0; m < na; m++) {
+                    const float2 q0 = m < lane ? row0[m] : make_float2(0.0f, 0.0f);
+                    const float2 q1 = v1 && m < lane + 32 ? row1[m] : make_float2(0.0f, 0.0f);
+                    const double ba0 = (double)q0.x, dc0 = (double)q0.y, ba1 = (double)q1.x, dc1 = (double)q1.y;
+                    const double xm = m < 32 ? x0 : x1;
+                    const bool am = (m < 32 ? go0 : go1) && ((xm <= 0.0) || ((m < 32 ? lu0 : lu1) <= -beta * xm));
+                    const unsigned bit = __ballot_sync(0xffffffffu, am) & (1u << (m & 31));
+                    if (m < 32) acc0 |= bit;
+                    else acc1 |= bit;
+                    x0 += bit ? dc0 : ba0;
+                    x1 += bit ? dc1 : ba1;
                 }
-                const bool a0 = v0 && !((hd0 >> lane) & 1u) && ((x0 <= 0.0) || (lu0 <= -beta * x0));
-                const bool a1 = v1 && !((hd1 >> lane) & 1u) && ((x1 <= 0.0) || (lu1 <= -beta * x1));
-                const unsigned n0 = __ballot_sync(0xffffffffu, a0), n1 = __ballot_sync(0xffffffffu, a1);
-                if (n0 == acc0 && n1 == acc1) break;
-                acc0 = n0;
-                acc1 = n1;
             }
             if (v0) sm.acc[lane] = (acc0 >> lane) & 1u;
             if (v1) sm.acc[lane + 32] = (acc1 >> lane) & 1u;
+            // colloid hard-core rejects (code 1) counted apart from moves that leave their cell (code 3)
+            hc0 = __ballot_sync(0xffffffffu, v0 && sm.hard[lane] == 1);
+            hc1 = __ballot_sync(0xffffffffu, v1 && sm.hard[lane + 32] == 1);
             if (v.rec_dE) {
                 if (v0) {
-                    v.rec_dE[p.p_off + sm.pid[lane]] = ((hd0 >> lane) & 1u) ? 0.0 : x0;
-                    v.rec_lu[p.p_off + sm.pid[lane]] = lu0;
+                    v.rec_dE[p.p_off + v.id[g0 + lane]] = sm.hard[lane] ? 0.0 : x0;
+                    v.rec_lu[p.p_off + v.id[g0 + lane]] = lu0;
                 }
                 if (v1) {
-                    v.rec_dE[p.p_off + sm.pid[lane + 32]] = ((hd1 >> lane) & 1u) ? 0.0 : x1;
-                    v.rec_lu[p.p_off + sm.pid[lane + 32]] = lu1;
+                    v.rec_dE[p.p_off + v.id[g0 + lane + 32]] = sm.hard[lane + 32] ? 0.0 : x1;
+                    v.rec_lu[p.p_off + v.id[g0 + lane + 32]] = lu1;
                 }
             }
+        }
+        // (the list is read no more: every thread has passed the barrier after the task queue)
+        if (w != 0) {
+            if (w == 1 && more) {
+                prepare_stencil<typename SM::Stencil, AMAX, CCAP>(v, sm.st[which ^ 1], nxt, lane);
+                __syncwarp();
+                copy_static(v, sm, which ^ 1, lane);
+            }
+            if (mode == 0 && kw < na) {
+                const int g = g0 + kw;
+                fetch_async<8>(&sm.wn[kw][0], v.tnx + g);
+                fetch_async<8>(&sm.wn[kw][1], v.tny + g);
+                fetch_async<8>(&sm.wn[kw][2], v.tnz + g);
+                fetch_async<8>(&sm.wn[kw][3], v.tux + g);
+                fetch_async<8>(&sm.wn[kw][4], v.tuy + g);
+                fetch_async<8>(&sm.wn[kw][5], v.tuz + g);
+            }
+            if (more && kw < AMAX && kw < (int)((unsigned)nxt.z >> 24)) fetch_rec(&sm.next[kw], v.act_rec + nxt.w + kw);
+        }
+        if (mode >= 2 && t == 0) {
+            if (RETRY) failed->cell[failed->n++] = cell * 4 + (mode == 2 ? 2 : 1);
+            else if (mode == 2 && na <= p.cap) // above this kernel's capacity, not the class's
+                v.retry_list[(size_t)ci * v.act_max + atomicAdd(&v.retry_count[ci], 1)] = a;
+            else hand_over(v, ci, cell, mode == 2 ? 2 : 1);
+        }
+        __syncthreads();
+
+        // ---- 6 write-back ----
+        if (mode == 0 && kw >= 0 && kw < na) {
+            const int k = kw, g = g0 + k;
+            const int acc = sm.acc[k];
+            if (acc) {
+                fetch_wait();
+                v.px[g] = sm.wn[k][0];
+                v.py[g] = sm.wn[k][1];
+                v.pz[g] = sm.wn[k][2];
+                v.ox[g] = sm.wn[k][3];
+                v.oy[g] = sm.wn[k][4];
+                v.oz[g] = sm.wn[k][5];
+                const float4 P0 = sm.pst[k][0], P1 = sm.pst[k][1], P2 = sm.pst[k][2];
+                v.cl4[g] = make_float4(P0.y, P0.w, P1.y, P1.w);
+                v.cl2[g] = make_float2(P2.y, P2.w);
+            }
+            v.outcome[p.p_off + id] = sm.hard[k] == 1 ? 2 : acc;
+        }
+        // warp 0, while the others go on: the cell's results
+        if (w == 0 && mode == 0) {
             // accepted dE summed in a fixed (butterfly) order
             double dsum = ((acc0 >> lane) & 1u ? x0 : 0.0) + ((acc1 >> lane) & 1u ? x1 : 0.0);
             double dabs = ((acc0 >> lane) & 1u ? fabs(x0) : 0.0) + ((acc1 >> lane) & 1u ? fabs(x1) : 0.0);
@@ -713,9 +897,6 @@ __global__ void __launch_bounds__(NT, FastMinBlocks<AMAX>::value) k_phase_fast(c
                 dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
                 dabs += __shfl_xor_sync(0xffffffffu, dabs, o);
             }
-            // colloid hard-core rejects (code 1) counted apart from moves that leave their cell (code 3)
-            const unsigned hc0 = __ballot_sync(0xffffffffu, v0 && sm.hard[lane] == 1);
-            const unsigned hc1 = __ballot_sync(0xffffffffu, v1 && sm.hard[lane + 32] == 1);
             const int nacc = __popc(acc0) + __popc(acc1), nhard = __popc(hc0) + __popc(hc1);
             if (lane == 0) {
                 if (!(dsum - dsum == 0.0)) atomicOr(&v.stats[r].flags, F_NONFINITE);
@@ -725,30 +906,29 @@ __global__ void __launch_bounds__(NT, FastMinBlocks<AMAX>::value) k_phase_fast(c
                 v.cell_n0[cell] = nacc;
                 v.cell_n1[cell] = nhard;
                 v.cell_pairs[cell] = sm.pairs;
-                v.cell_cands[cell] = (unsigned long long)na * (unsigned long long)(S26 + na - 1);
+                v.cell_cands[cell] = (unsigned long long)na * (unsigned long long)(s26 + na - 1);
             }
         }
-        __syncthreads();
-
-        // ---- 7 write-back ----
-        if (w != 0 && kw < na) {
-            const int k = kw, g = g0 + k;
-            const int acc = sm.acc[k];
-            if (acc) {
-                v.px[g] = wn[0];
-                v.py[g] = wn[1];
-                v.pz[g] = wn[2];
-                v.ox[g] = wn[3];
-                v.oy[g] = wn[4];
-                v.oz[g] = wn[5];
-                const float4 P1 = sm.pst[k][1], P2 = sm.pst[k][2];
-                v.cl4[g] = make_float4(P1.z, P1.w, P2.x, P2.y);
-                v.cl2[g] = make_float2(P2.z, P2.w);
-            }
-            v.outcome[p.p_off + sm.pid[k]] = sm.hard[k] == 1 ? 2 : acc;
-        }
-        __syncthreads();
+        if (!more) break;
+        rec = nxt;
+        a += step;
+        if (a + step < total) nxt = entry(a + step);
+        which ^= 1;
     }
+    if (RETRY) { // the block comes back with the barrier's memory
+        __syncthreads();
+        if (t == 0) asm volatile("mbarrier.inval.shared.b64 [%0];" ::"r"(tc::smem_u32(&sm.full)) : "memory");
+    }
+}
+
+template <int NT, int MINB, int AMAX, int CCAP, int LCAP, bool SPEC21>
+__global__ void __launch_bounds__(NT, MINB)
+    k_phase_fast(const __grid_constant__ DevView v, const __grid_constant__ FastK ku, int ci)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int *off = v.act_off + ci * (v.R + 1); // this launch's replicas: active cells [off[r_lo], off[r_hi])
+    phase_fast_body<NT, AMAX, CCAP, LCAP, SPEC21, false>(v, ku, ci, smem_raw, off[v.r_lo] + (int)blockIdx.x, off[v.r_hi],
+                                                         (int)gridDim.x, nullptr);
 }
 
 // FP64 attempts of the cells the FP32 phase kernel handed over in colour phase
@@ -771,99 +951,67 @@ __global__ void __launch_bounds__(NT, FastMinBlocks<AMAX>::value) k_phase_fast(c
 // FP32 kernel changes nothing in the chain.
 constexpr int RESCUE_CAP = 1024; // particles of a staged stencil (48 KB of shared memory)
 
+#define FAST_RETRY 64, 1664, 7168 // active particles, places of the static cells' particles, list entries
+
 template <int NT, bool SPEC21>
-__global__ void __launch_bounds__(NT) k_phase_rescue(DevView v, int ci)
+__global__ void __launch_bounds__(NT) k_phase_rescue(const __grid_constant__ DevView v, const __grid_constant__ FastK ku, int ci)
 {
     constexpr int NW = NT / 32;
-    extern __shared__ double sx[]; // [6][RESCUE_CAP]: x, y, z, ux, uy, uz of the staged stencil
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *sx = reinterpret_cast<double *>(smem_raw); // [6][RESCUE_CAP]: x, y, z, ux, uy, uz of the staged stencil
     __shared__ int st_start[27], st_cnt[27], pre[28];
     __shared__ double spo[NW], spn[NW];
     __shared__ int snp[NW];
+    __shared__ RetryFailed failed;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const int count = v.resc_count[ci];
-    for (int e = blockIdx.x; e < count; e += gridDim.x) {
-        const int code = v.resc_list[(size_t)ci * v.ctot + e];
-        const int cell = code >> 2, mode = code & 3;
-        const int r = v.p2c[cell];
-        const Replica &p = v.rep[r];
-        const int nc0 = p.nc[0], nc1 = p.nc[1], nc2 = p.nc[2];
-        const int loc = cell - p.cell_off;
-        const int cx = loc % nc0, cy = (loc / nc0) % nc1, cz = loc / (nc0 * nc1);
-        if (t < 27) {
-            int x = cx + t % 3 - 1, y = cy + (t / 3) % 3 - 1, z = cz + t / 9 - 1;
-            x += x < 0 ? nc0 : (x >= nc0 ? -nc0 : 0);
-            y += y < 0 ? nc1 : (y >= nc1 ? -nc1 : 0);
-            z += z < 0 ? nc2 : (z >= nc2 ? -nc2 : 0);
-            const int c = p.cell_off + (z * nc1 + y) * nc0 + x;
-            st_start[t] = v.cell_start[c];
-            st_cnt[t] = v.cell_start[c + 1] - v.cell_start[c];
-        }
+    const int nretry = v.retry_count[ci], count = v.resc_count[ci];
+    if (nretry == 0 && count == 0) return;
+    // Rounds of at most 32 retries of this block, each followed by the FP64 attempts of those that failed; the
+    // cells handed over by the phase kernel come with the first round.
+    for (int a0 = blockIdx.x; a0 == (int)blockIdx.x || a0 < nretry; a0 += 32 * gridDim.x) {
+        if (t == 0) failed.n = 0;
+        tc::fence_proxy_async_smem(); // the staged states of the last round's cells come before this round's copies
         __syncthreads();
-        if (t < 32) {
-            const int c = t < 27 ? st_cnt[t] : 0;
-            int inc = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += y;
-            }
-            if (t < 27) pre[t] = inc - c;
-            if (t == 26) pre[27] = inc;
-        }
+        const int a1 = min(nretry, a0 + 32 * (int)gridDim.x);
+        if (a0 < a1) phase_fast_body<NT, FAST_RETRY, SPEC21, true>(v, ku, ci, smem_raw, a0, a1, (int)gridDim.x, &failed);
         __syncthreads();
-        const int total = pre[27];
-        const int g0 = st_start[13], na = st_cnt[13];
-        const bool staged = total <= RESCUE_CAP;
-        if (staged) {
-            for (int f = t; f < total; f += NT) {
-                int sl = 0, hi = 27;
-                while (hi - sl > 1) {
-                    const int mid = (sl + hi) >> 1;
-                    if (pre[mid] <= f) sl = mid;
-                    else hi = mid;
-                }
-                const int j = st_start[sl] + (f - pre[sl]);
-                sx[f] = v.px[j];
-                sx[RESCUE_CAP + f] = v.py[j];
-                sx[2 * RESCUE_CAP + f] = v.pz[j];
-                sx[3 * RESCUE_CAP + f] = v.ox[j];
-                sx[4 * RESCUE_CAP + f] = v.oy[j];
-                sx[5 * RESCUE_CAP + f] = v.oz[j];
+        const int mine = a0 == (int)blockIdx.x && count > a0 ? (count - a0 + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+        for (int e = 0; e < failed.n + mine; e++) {
+            const int code = e < failed.n ? failed.cell[e]
+                                          : v.resc_list[(size_t)ci * v.ctot + a0 + (e - failed.n) * (int)gridDim.x];
+            const int cell = code >> 2, mode = code & 3;
+            const int r = v.p2c[cell];
+            const Replica &p = v.rep[r];
+            const int nc0 = p.nc[0], nc1 = p.nc[1], nc2 = p.nc[2];
+            const int loc = cell - p.cell_off;
+            const int cx = loc % nc0, cy = (loc / nc0) % nc1, cz = loc / (nc0 * nc1);
+            if (t < 27) {
+                int x = cx + t % 3 - 1, y = cy + (t / 3) % 3 - 1, z = cz + t / 9 - 1;
+                x += x < 0 ? nc0 : (x >= nc0 ? -nc0 : 0);
+                y += y < 0 ? nc1 : (y >= nc1 ? -nc1 : 0);
+                z += z < 0 ? nc2 : (z >= nc2 ? -nc2 : 0);
+                const int c = p.cell_off + (z * nc1 + y) * nc0 + x;
+                st_start[t] = v.cell_start[c];
+                st_cnt[t] = v.cell_start[c + 1] - v.cell_start[c];
             }
             __syncthreads();
-        }
-        double dsum = 0.0, dabs = 0.0;
-        int nacc = 0, nhard = 0;
-        unsigned long long npairs = 0ull;
-        for (int k = 0; k < na; k++) {
-            const int g = g0 + k;
-            const int id = v.id[g];
-            const unsigned char code = v.thard[g];
-            if (code) { // colloid hard-core reject (1) or a move out of the cell (3): no energy evaluation
-                if (t == 0) {
-                    v.outcome[p.p_off + id] = code == 1 ? 2 : 0;
-                    if (v.rec_dE) {
-                        v.rec_dE[p.p_off + id] = 0.0;
-                        v.rec_lu[p.p_off + id] = v.tlu[g];
-                    }
+            if (t < 32) {
+                const int c = t < 27 ? st_cnt[t] : 0;
+                int inc = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += y;
                 }
-                nhard += code == 1;
-                continue;
+                if (t < 27) pre[t] = inc - c;
+                if (t == 26) pre[27] = inc;
             }
-            const double ro[3] = {v.px[g], v.py[g], v.pz[g]};
-            const double eo[3] = {v.ox[g], v.oy[g], v.oz[g]};
-            const double rn[3] = {v.tnx[g], v.tny[g], v.tnz[g]};
-            const double en[3] = {v.tux[g], v.tuy[g], v.tuz[g]};
-            double po = 0.0, pn = 0.0;
-            int np = 0;
-            const int fk = pre[13] + k; // this particle's own entry
-            for (int f = t; f < total; f += NT) {
-                if (f == fk) continue;
-                double rj[3], ej[3];
-                if (staged) {
-                    rj[0] = sx[f], rj[1] = sx[RESCUE_CAP + f], rj[2] = sx[2 * RESCUE_CAP + f];
-                    ej[0] = sx[3 * RESCUE_CAP + f], ej[1] = sx[4 * RESCUE_CAP + f], ej[2] = sx[5 * RESCUE_CAP + f];
-                } else {
+            __syncthreads();
+            const int total = pre[27];
+            const int g0 = st_start[13], na = st_cnt[13];
+            const bool staged = total <= RESCUE_CAP;
+            if (staged) {
+                for (int f = t; f < total; f += NT) {
                     int sl = 0, hi = 27;
                     while (hi - sl > 1) {
                         const int mid = (sl + hi) >> 1;
@@ -871,85 +1019,132 @@ __global__ void __launch_bounds__(NT) k_phase_rescue(DevView v, int ci)
                         else hi = mid;
                     }
                     const int j = st_start[sl] + (f - pre[sl]);
-                    rj[0] = v.px[j], rj[1] = v.py[j], rj[2] = v.pz[j];
-                    ej[0] = v.ox[j], ej[1] = v.oy[j], ej[2] = v.oz[j];
+                    sx[f] = v.px[j];
+                    sx[RESCUE_CAP + f] = v.py[j];
+                    sx[2 * RESCUE_CAP + f] = v.pz[j];
+                    sx[3 * RESCUE_CAP + f] = v.ox[j];
+                    sx[4 * RESCUE_CAP + f] = v.oy[j];
+                    sx[5 * RESCUE_CAP + f] = v.oz[j];
                 }
-                double d[3];
-                double r2 = dist_fold(ro[0], ro[1], ro[2], rj[0], rj[1], rj[2], p.L, d);
-                if (r2 < p.k.rc2) {
-                    po += SPEC21 ? pair_energy64_21(p.k, r2, d, eo, ej) : pair_exact(p.k, r2, d, eo, ej);
-                    np++;
-                }
-                r2 = dist_fold(rn[0], rn[1], rn[2], rj[0], rj[1], rj[2], p.L, d);
-                if (r2 < p.k.rc2) {
-                    pn += SPEC21 ? pair_energy64_21(p.k, r2, d, en, ej) : pair_exact(p.k, r2, d, en, ej);
-                    np++;
-                }
+                __syncthreads();
             }
+            double dsum = 0.0, dabs = 0.0;
+            int nacc = 0, nhard = 0;
+            unsigned long long npairs = 0ull;
+            for (int k = 0; k < na; k++) {
+                const int g = g0 + k;
+                const int id = v.id[g];
+                const unsigned char code = v.thard[g];
+                if (code) { // colloid hard-core reject (1) or a move out of the cell (3): no energy evaluation
+                    if (t == 0) {
+                        v.outcome[p.p_off + id] = code == 1 ? 2 : 0;
+                        if (v.rec_dE) {
+                            v.rec_dE[p.p_off + id] = 0.0;
+                            v.rec_lu[p.p_off + id] = v.tlu[g];
+                        }
+                    }
+                    nhard += code == 1;
+                    continue;
+                }
+                const double ro[3] = {v.px[g], v.py[g], v.pz[g]};
+                const double eo[3] = {v.ox[g], v.oy[g], v.oz[g]};
+                const double rn[3] = {v.tnx[g], v.tny[g], v.tnz[g]};
+                const double en[3] = {v.tux[g], v.tuy[g], v.tuz[g]};
+                double po = 0.0, pn = 0.0;
+                int np = 0;
+                const int fk = pre[13] + k; // this particle's own entry
+                for (int f = t; f < total; f += NT) {
+                    if (f == fk) continue;
+                    double rj[3], ej[3];
+                    if (staged) {
+                        rj[0] = sx[f], rj[1] = sx[RESCUE_CAP + f], rj[2] = sx[2 * RESCUE_CAP + f];
+                        ej[0] = sx[3 * RESCUE_CAP + f], ej[1] = sx[4 * RESCUE_CAP + f], ej[2] = sx[5 * RESCUE_CAP + f];
+                    } else {
+                        int sl = 0, hi = 27;
+                        while (hi - sl > 1) {
+                            const int mid = (sl + hi) >> 1;
+                            if (pre[mid] <= f) sl = mid;
+                            else hi = mid;
+                        }
+                        const int j = st_start[sl] + (f - pre[sl]);
+                        rj[0] = v.px[j], rj[1] = v.py[j], rj[2] = v.pz[j];
+                        ej[0] = v.ox[j], ej[1] = v.oy[j], ej[2] = v.oz[j];
+                    }
+                    double d[3];
+                    double r2 = dist_fold(ro[0], ro[1], ro[2], rj[0], rj[1], rj[2], p.L, d);
+                    if (r2 < p.k.rc2) {
+                        po += SPEC21 ? pair_energy64_21(p.k, r2, d, eo, ej) : pair_exact(p.k, r2, d, eo, ej);
+                        np++;
+                    }
+                    r2 = dist_fold(rn[0], rn[1], rn[2], rj[0], rj[1], rj[2], p.L, d);
+                    if (r2 < p.k.rc2) {
+                        pn += SPEC21 ? pair_energy64_21(p.k, r2, d, en, ej) : pair_exact(p.k, r2, d, en, ej);
+                        np++;
+                    }
+                }
 #pragma unroll
-            for (int o = 16; o >= 1; o >>= 1) {
-                po += __shfl_xor_sync(0xffffffffu, po, o);
-                pn += __shfl_xor_sync(0xffffffffu, pn, o);
-                np += __shfl_xor_sync(0xffffffffu, np, o);
+                for (int o = 16; o >= 1; o >>= 1) {
+                    po += __shfl_xor_sync(0xffffffffu, po, o);
+                    pn += __shfl_xor_sync(0xffffffffu, pn, o);
+                    np += __shfl_xor_sync(0xffffffffu, np, o);
+                }
+                if (lane == 0) {
+                    spo[w] = po;
+                    spn[w] = pn;
+                    snp[w] = np;
+                }
+                __syncthreads();
+                if (t == 0) {
+                    double so = spo[0], sn = spn[0];
+                    int sp = snp[0];
+                    for (int q = 1; q < NW; q++) {
+                        so += spo[q];
+                        sn += spn[q];
+                        sp += snp[q];
+                    }
+                    const double dE = (sn - so) + v.act_rec[g].tdU;
+                    const double lu = v.tlu[g];
+                    const bool acc = (dE <= 0.0) || (lu <= -p.k.beta * dE);
+                    if (acc) {
+                        v.px[g] = rn[0];
+                        v.py[g] = rn[1];
+                        v.pz[g] = rn[2];
+                        v.ox[g] = en[0];
+                        v.oy[g] = en[1];
+                        v.oz[g] = en[2];
+                        if (staged) {
+                            const int fk = pre[13] + k;
+                            sx[fk] = rn[0], sx[RESCUE_CAP + fk] = rn[1], sx[2 * RESCUE_CAP + fk] = rn[2];
+                            sx[3 * RESCUE_CAP + fk] = en[0], sx[4 * RESCUE_CAP + fk] = en[1], sx[5 * RESCUE_CAP + fk] = en[2];
+                        }
+                        const ActRec &ar = v.act_rec[g];
+                        v.cl4[g] = make_float4(ar.p0.y, ar.p0.w, ar.p1.y, ar.p1.w);
+                        v.cl2[g] = make_float2(ar.p2.y, ar.p2.w);
+                        dsum += dE;
+                        dabs += fabs(dE);
+                        nacc++;
+                    }
+                    v.outcome[p.p_off + id] = acc ? 1 : 0;
+                    if (v.rec_dE) {
+                        v.rec_dE[p.p_off + id] = dE;
+                        v.rec_lu[p.p_off + id] = lu;
+                    }
+                    npairs += (unsigned long long)sp;
+                }
+                __syncthreads(); // the accepted state is visible to the next attempt
             }
-            if (lane == 0) {
-                spo[w] = po;
-                spn[w] = pn;
-                snp[w] = np;
+            if (t == 0) {
+                if (!(dsum - dsum == 0.0)) atomicOr(&v.stats[r].flags, F_NONFINITE);
+                v.cell_e0[cell] = dsum;
+                v.cell_abs[cell] = dabs;
+                v.cell_n0[cell] = nacc;
+                v.cell_n1[cell] = nhard;
+                v.cell_pairs[cell] = npairs;
+                v.cell_cands[cell] = (unsigned long long)na * (unsigned long long)(total > 0 ? total - 1 : 0);
+                v.cell_fp64[cell] = mode;
             }
             __syncthreads();
-            if (t == 0) {
-                double so = spo[0], sn = spn[0];
-                int sp = snp[0];
-                for (int q = 1; q < NW; q++) {
-                    so += spo[q];
-                    sn += spn[q];
-                    sp += snp[q];
-                }
-                const double dE = (sn - so) + v.tdU[g];
-                const double lu = v.tlu[g];
-                const bool acc = (dE <= 0.0) || (lu <= -p.k.beta * dE);
-                if (acc) {
-                    v.px[g] = rn[0];
-                    v.py[g] = rn[1];
-                    v.pz[g] = rn[2];
-                    v.ox[g] = en[0];
-                    v.oy[g] = en[1];
-                    v.oz[g] = en[2];
-                    if (staged) {
-                        const int fk = pre[13] + k;
-                        sx[fk] = rn[0], sx[RESCUE_CAP + fk] = rn[1], sx[2 * RESCUE_CAP + fk] = rn[2];
-                        sx[3 * RESCUE_CAP + fk] = en[0], sx[4 * RESCUE_CAP + fk] = en[1], sx[5 * RESCUE_CAP + fk] = en[2];
-                    }
-                    const float4 c4 = v.cl4[g];
-                    float tux, tuy, tuz;
-                    unit_f32(en[0], en[1], en[2], tux, tuy, tuz);
-                    v.cl4[g] = make_float4(c4.x + v.tdx[g], c4.y + v.tdy[g], c4.z + v.tdz[g], tux);
-                    v.cl2[g] = make_float2(tuy, tuz);
-                    dsum += dE;
-                    dabs += fabs(dE);
-                    nacc++;
-                }
-                v.outcome[p.p_off + id] = acc ? 1 : 0;
-                if (v.rec_dE) {
-                    v.rec_dE[p.p_off + id] = dE;
-                    v.rec_lu[p.p_off + id] = lu;
-                }
-                npairs += (unsigned long long)sp;
-            }
-            __syncthreads(); // the accepted state is visible to the next attempt
         }
-        if (t == 0) {
-            if (!(dsum - dsum == 0.0)) atomicOr(&v.stats[r].flags, F_NONFINITE);
-            v.cell_e0[cell] = dsum;
-            v.cell_abs[cell] = dabs;
-            v.cell_n0[cell] = nacc;
-            v.cell_n1[cell] = nhard;
-            v.cell_pairs[cell] = npairs;
-            v.cell_cands[cell] = (unsigned long long)na * (unsigned long long)(total > 0 ? total - 1 : 0);
-            v.cell_fp64[cell] = mode;
-        }
-        __syncthreads();
     }
 }
 
@@ -959,75 +1154,99 @@ __global__ void __launch_bounds__(NT) k_phase_rescue(DevView v, int ci)
 
 namespace lcmc {
 
-// (threads, active capacity, staged candidates per warp segment, per-warp list capacity)
-// the shared memory of the 48- and 56-particle classes lets six and five
-// blocks share an SM's 228 KB (1 KB of it reserved per block)
-static_assert(sizeof(FastSmem<128, 48, 160, 160>) + 1024 <= 233472 / 6, "48-class: six blocks per SM");
-static_assert(sizeof(FastSmem<128, 56, 176, 192>) + 1024 <= 233472 / 5, "56-class: five blocks per SM");
-static const FastVariant kVariants[] = {{128, 48, 160, 160}, {128, 56, 176, 192}, {128, 64, 288, 384}};
+// Capacity classes: (active particles, places of the static cells' particles, list entries).
+// "Light" is the 48-particle class for systems whose capacity rule asks for at most 40.
+#define FAST40 40, 780, 2688
+#define FAST48 48, 832, 3456
+#define FAST56 56, 1040, 4096
+#define FAST64 64, 1440, 5376
+static_assert(sizeof(FastSmem<FAST40>) + 1024 <= 233472 / 6, "light: six blocks per SM");
+static_assert(sizeof(FastSmem<FAST48>) + 1024 <= 233472 / 5, "48-class: five blocks per SM");
+static_assert(sizeof(FastSmem<FAST56>) + 1024 <= 233472 / 4, "56-class: four blocks per SM");
+static_assert(sizeof(FastSmem<FAST64>) + 1024 <= 233472 / 3, "64-class: three blocks per SM");
+static const FastVariant kVariants[] = {{48}, {56}, {64}};
 
 int fast_variant_count() { return (int)(sizeof(kVariants) / sizeof(kVariants[0])); }
 FastVariant fast_variant(int i) { return kVariants[i]; }
 
-template <int NT, int AMAX, int SEG, int LW, bool S21>
-static void launch_v(const DevView &v, cudaStream_t s, int ci, int grid)
-{
-    const int bytes = (int)sizeof(FastSmem<NT, AMAX, SEG, LW>);
-    k_phase_fast<NT, AMAX, SEG, LW, S21><<<grid, NT, bytes, s>>>(v, ci);
-}
-
-template <int NT, int AMAX, int SEG, int LW, bool S21>
-static int occupancy_v()
-{
-    const int bytes = (int)sizeof(FastSmem<NT, AMAX, SEG, LW>);
-    cudaFuncSetAttribute(k_phase_fast<NT, AMAX, SEG, LW, S21>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_phase_fast<NT, AMAX, SEG, LW, S21>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_phase_fast<NT, AMAX, SEG, LW, S21>, NT, bytes);
-    return n > 0 ? n : 1;
-}
-
-// variant = 2 * capacity class + (mu = 2, nu = 1, sigma0 = 1 specialisation)
-void launch_phase_fast(int variant, const DevView &v, cudaStream_t s, int ci, int grid)
-{
-    switch (variant) {
-    case 0: launch_v<128, 48, 160, 160, false>(v, s, ci, grid); break;
-    case 1: launch_v<128, 48, 160, 160, true>(v, s, ci, grid); break;
-    case 2: launch_v<128, 56, 176, 192, false>(v, s, ci, grid); break;
-    case 3: launch_v<128, 56, 176, 192, true>(v, s, ci, grid); break;
-    case 4: launch_v<128, 64, 288, 384, false>(v, s, ci, grid); break;
-    default: launch_v<128, 64, 288, 384, true>(v, s, ci, grid); break;
+template <int NT, int MINB, int AMAX, int CCAP, int LCAP, bool S21>
+struct FastLaunch {
+    static constexpr int bytes = (int)sizeof(FastSmem<AMAX, CCAP, LCAP>);
+    static void launch(const DevView &v, const FastK &k, cudaStream_t s, int ci, int grid)
+    {
+        k_phase_fast<NT, MINB, AMAX, CCAP, LCAP, S21><<<grid, NT, bytes, s>>>(v, k, ci);
     }
+    static int blocks()
+    {
+        auto k = k_phase_fast<NT, MINB, AMAX, CCAP, LCAP, S21>;
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        int n = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, NT, bytes);
+        return n > 0 ? n : 1;
+    }
+};
+
+// Threads: four warps per cell where a phase has more cells than SMs (1,048,576
+// rods, all phases: 1.48 ms; three warps 1.60, five 1.53, six at five blocks
+// 1.66), sixteen where it has not and a phase takes one cell's latency (32,768
+// rods NPT: 0.19 ms against 0.30 with four).  The light shape holds six blocks
+// per SM where the class's own 48-particle arrays leave five (1.48 against 1.60).
+// The kernel of a variant: class, specialisation (mu = 2, nu = 1, sigma0 = 1, the
+// same pair constants in every replica), light, wide (a block per SM).
+template <typename F>
+static auto with_variant(const FastChoice &c, F f)
+{
+#define FAST_PICK(...) (c.wide ? f(FastLaunch<512, 1, __VA_ARGS__>()) : f(FastLaunch<FAST_NT, __VA_ARGS__>()))
+#define FAST_NT 128, 6
+    if (c.cls == 0 && c.light) return c.spec21 ? FAST_PICK(FAST40, true) : FAST_PICK(FAST40, false);
+#undef FAST_NT
+#define FAST_NT 128, 5
+    if (c.cls == 0) return c.spec21 ? FAST_PICK(FAST48, true) : FAST_PICK(FAST48, false);
+#undef FAST_NT
+#define FAST_NT 128, 4
+    if (c.cls == 1) return c.spec21 ? FAST_PICK(FAST56, true) : FAST_PICK(FAST56, false);
+#undef FAST_NT
+#define FAST_NT 128, 3
+    return c.spec21 ? FAST_PICK(FAST64, true) : FAST_PICK(FAST64, false);
+#undef FAST_NT
+#undef FAST_PICK
 }
 
-void launch_phase_rescue(bool spec21, const DevView &v, cudaStream_t s, int ci, int grid)
+void launch_phase_fast(const FastChoice &c, const GBConsts &k, const DevView &v, cudaStream_t s, int ci, int grid)
 {
-    const int bytes = 6 * RESCUE_CAP * (int)sizeof(double);
-    if (spec21) k_phase_rescue<256, true><<<grid, 256, bytes, s>>>(v, ci);
-    else k_phase_rescue<256, false><<<grid, 256, bytes, s>>>(v, ci);
+    const FastK K = fast_consts(k);
+    with_variant(c, [&](auto l) {
+        decltype(l)::launch(v, K, s, ci, grid);
+        return 0;
+    });
+}
+
+static constexpr int rescue_bytes()
+{
+    return std::max(6 * RESCUE_CAP * (int)sizeof(double), (int)sizeof(FastSmem<FAST_RETRY>));
+}
+
+void launch_phase_rescue(bool spec21, const GBConsts &k, const DevView &v, cudaStream_t s, int ci, int grid)
+{
+    const FastK K = fast_consts(k);
+    if (spec21) k_phase_rescue<256, true><<<grid, 256, rescue_bytes(), s>>>(v, K, ci);
+    else k_phase_rescue<256, false><<<grid, 256, rescue_bytes(), s>>>(v, K, ci);
 }
 
 // Opts the hand-over kernel in to its dynamic shared memory (call once).
 void rescue_init()
 {
-    const int bytes = 6 * RESCUE_CAP * (int)sizeof(double);
+    const int bytes = rescue_bytes();
     cudaFuncSetAttribute(k_phase_rescue<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     cudaFuncSetAttribute(k_phase_rescue<256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-// Also opts the variant in to its dynamic shared memory size: call once
-// before the first launch of a variant.
-int fast_blocks_per_sm(int variant)
+// Also opts the kernel in to its dynamic shared memory size: call once
+// before the first launch of a choice.
+int fast_blocks_per_sm(const FastChoice &c)
 {
-    switch (variant) {
-    case 0: return occupancy_v<128, 48, 160, 160, false>();
-    case 1: return occupancy_v<128, 48, 160, 160, true>();
-    case 2: return occupancy_v<128, 56, 176, 192, false>();
-    case 3: return occupancy_v<128, 56, 176, 192, true>();
-    case 4: return occupancy_v<128, 64, 288, 384, false>();
-    default: return occupancy_v<128, 64, 288, 384, true>();
-    }
+    return with_variant(c, [](auto l) { return decltype(l)::blocks(); });
 }
 
 } // namespace lcmc
