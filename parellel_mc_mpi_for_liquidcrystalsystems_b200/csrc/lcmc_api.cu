@@ -107,6 +107,7 @@ struct lcmc_ctx {
     bool checks_off = false; // no periodic energy checks (autotune trials)
     int grid_elem = 0, grid_exact = 0, grid_fast = 0, grid_energy = 0, grid_screen = 0;
     bool any_fast = false, any_exact = false, any_npt = false;
+    bool any_small = false; // a box may have fewer than four cells along an axis, or takes the per-particle energies
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     bool timed = false;
@@ -725,20 +726,21 @@ static int push_kernel_fields(lcmc_ctx *c)
 // kernels are launched all the time.
 static void box_launches(lcmc_ctx *c)
 {
-    c->any_exact = false;
+    c->any_exact = c->any_small = false;
     c->safe_sweeps = 1ll << 40;
     c->since_choice = 0;
     c->nrun = 8;
     for (int r = 0; r < c->R; r++) {
         const Replica &rp = c->rep[r];
         const double Lmin = std::min(rp.L[0], std::min(rp.L[1], rp.L[2]));
-        if (rp.kernel == 0 || grid_dim_host(Lmin, rp.wmin, rp.fine) < 4) {
-            c->any_exact = true;
-        } else if (rp.ensemble == 2 && rp.dlnv_max > 0.0) {
+        bool small = grid_dim_host(Lmin, rp.wmin, rp.fine) < 4;
+        if (!small && rp.ensemble == 2 && rp.dlnv_max > 0.0) {
             const long long safe = (long long)(3.0 * std::log(Lmin / (4.0 * rp.wmin)) / rp.dlnv_max) - 1;
-            if (safe < 32) c->any_exact = true;
+            if (safe < 32) small = true;
             else c->safe_sweeps = std::min(c->safe_sweeps, safe);
         }
+        c->any_exact = c->any_exact || rp.kernel == 0 || small;
+        c->any_small = c->any_small || small || !rp.vol_cells;
         // colours: 2 per axis, 3 on an odd count of the fine grid; an NPT box may take any count
         int ncol = rp.fine && rp.ensemble == 2 ? LCMC_MAX_COLOURS : 1;
         for (int a = 0; a < 3 && ncol < LCMC_MAX_COLOURS; a++) {
@@ -1059,10 +1061,10 @@ static int recheck_boxes(lcmc_ctx *c)
 {
     int rc = read_boxes(c);
     if (rc) return rc;
-    const bool old_exact = c->any_exact;
+    const bool old_exact = c->any_exact, old_small = c->any_small;
     const int old_nrun = c->nrun;
     box_launches(c);
-    if (old_exact != c->any_exact || old_nrun != c->nrun) invalidate_graphs(c);
+    if (old_exact != c->any_exact || old_small != c->any_small || old_nrun != c->nrun) invalidate_graphs(c);
     return LCMC_OK;
 }
 
@@ -1073,13 +1075,13 @@ static int rechoose_kernels(lcmc_ctx *c)
     int brc = read_boxes(c);
     if (brc) return brc;
     const FastChoice old_fast_choice = c->fast;
-    const bool old_fast = c->any_fast, old_exact = c->any_exact;
+    const bool old_fast = c->any_fast, old_exact = c->any_exact, old_small = c->any_small;
     const int old_nrun = c->nrun, old_grid = c->grid_fast;
     choose_kernels(c);
     int rc = push_kernel_fields(c);
     if (rc) return rc;
     if (!(old_fast_choice == c->fast) || old_fast != c->any_fast || old_exact != c->any_exact ||
-        old_nrun != c->nrun || old_grid != c->grid_fast)
+        old_small != c->any_small || old_nrun != c->nrun || old_grid != c->grid_fast)
         invalidate_graphs(c);
     return LCMC_OK;
 }
@@ -1142,13 +1144,13 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
         if (c->any_da || c->rec_cap > 0)
             launch_features(v, c->stream, c->any_da ? mlp_input(c->mlp) : nullptr, c->any_da ? mlp_ld(c->mlp) : 0,
                             c->grid_elem);
-        if (c->any_screen) launch_screen(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_screen, c->fast.spec21);
+        if (c->any_screen) launch_screen(v, c->stream, c->grid_screen, c->fast.spec21);
         if (c->any_da) {
             const int B = (2 * c->R + 127) / 128 * 128;
             const float *y = mlp_forward_device(c->mlp, B, c->stream);
             launch_da_stage1(v, c->stream, y);
         }
-        launch_volume_finish(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_energy);
+        launch_volume_finish(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_energy, c->any_small);
     }
     cudaEventRecordWithFlags(c->ev[3], c->stream, cudaEventRecordExternal);
     launch_sweep_advance(v, c->stream);
@@ -1220,7 +1222,7 @@ static void enqueue_energy_check(lcmc_ctx *c, int all)
     enqueue_rebin(c, c->cur);
     c->cur ^= 1;
     DevView v = view(c, c->cur);
-    launch_energy_exact(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, 0, c->grid_energy);
+    launch_total_energy(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_energy, true, c->any_small);
     launch_energy_check(v, c->stream, c->d_pe0, all);
 }
 
@@ -1387,7 +1389,7 @@ extern "C" int lcmc_kernels_per_sweep(lcmc_ctx *ctx)
     // recording; history: chunk sums, rows; sweep counter
     const int exact = ctx->any_exact ? 2 * ctx->ex_nb : 0;
     int n = 8 + (int)ctx->any_exact + ctx->ngroup * ctx->nrun * (exact + 2 * (int)ctx->any_fast) +
-            5 * (int)ctx->any_npt + 3;
+            (5 + (int)ctx->any_small) * (int)ctx->any_npt + 3;
     if (ctx->any_npt && (ctx->any_da || ctx->rec_cap > 0)) n += 2;
     if (ctx->any_npt && ctx->any_da) n += 6;
     if (ctx->any_npt && ctx->any_screen) n += 3; // screen energies, chunk sums, stage 1
@@ -1583,13 +1585,13 @@ extern "C" int lcmc_last_sweep_timing(lcmc_ctx *ctx, double ms[4])
 
 // Rebin (no sweep) and recompute the FP64 total energy of every replica with
 // the FP64 kernel; resets the running energies.
-static int recompute_energy(lcmc_ctx *c, int replica_only)
+static int recompute_energy(lcmc_ctx *c, int replica_only, bool cells)
 {
     enqueue_rebin(c, c->cur);
     c->cur ^= 1;
     DevView v = view(c, c->cur);
-    launch_energy_exact(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, 0, c->grid_energy);
-    launch_energy_reduce(v, c->stream, c->d_pe0, replica_only);
+    launch_total_energy(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_energy, cells, c->any_small);
+    launch_energy_reduce(v, c->stream, c->d_pe0, replica_only, cells);
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     CUDA_TRY(c, cudaGetLastError());
     return LCMC_OK;
@@ -1599,7 +1601,7 @@ extern "C" int lcmc_total_energy(lcmc_ctx *ctx, int replica, int precision, doub
 {
     if (!ctx || replica < 0 || replica >= ctx->R || !energy) return LCMC_EINVAL;
     (void)precision; // pair terms of the recompute always run in FP64 (B200 FP64 rate is ample here)
-    int rc = recompute_energy(ctx, replica);
+    int rc = recompute_energy(ctx, replica, true);
     if (rc) return rc;
     CUDA_TRY(ctx, cudaMemcpy(energy, ctx->d_red + replica, sizeof(double), cudaMemcpyDeviceToHost));
     return LCMC_OK;
@@ -1658,7 +1660,7 @@ extern "C" int lcmc_upload(lcmc_ctx *ctx, int replica, const double *px, const d
     bool all = true;
     for (int r = 0; r < ctx->R; r++) all = all && ctx->uploaded[r];
     if (!all) return LCMC_OK; // energies are computed once every replica holds a configuration
-    int e = recompute_energy(ctx, -1);
+    int e = recompute_energy(ctx, -1, false);
     if (e) return e;
     // zero the drift of the first recompute
     std::vector<DevStats> st(ctx->R);
@@ -1903,6 +1905,7 @@ static int apply_tuning(lcmc_ctx *c, const TuneChoice &ch)
                                     sizeof(int), cudaMemcpyHostToDevice, c->stream));
     }
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    box_launches(c);
     invalidate_graphs(c);
     return LCMC_OK;
 }

@@ -168,7 +168,7 @@ struct DevView {
     int *cell_start;    // [ctot + 1]
     int *block_sums;    // scan scratch
     double *cell_e0, *cell_e1; // per-cell FP64 sums (sweep dE / energies)
-    int *cell_n0, *cell_n1;    // per-cell counts (accepted / hard-core)
+    int *cell_n0, *cell_n1;    // per-cell counts (accepted / hard-core; of the energies: centres in the colloid at V')
     unsigned long long *cell_pairs, *cell_cands;
     double *cell_abs;          // per cell: sum of |dE| of the accepted moves
     int *p2c;                  // [ctot] replica of each cell slot

@@ -18,7 +18,10 @@ void exact_init(); // before the first FP64 colour phase
 void exact_scratch_size(int ntot, long long *cap, long long *alloc, int *nb);
 void launch_exact_offsets(const DevView &v, cudaStream_t s); // after the rebin, before the colour phases
 void launch_phase_exact(const DevView &v, cudaStream_t s, int ci, int grid);
-void launch_energy_exact(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int scaled, int grid);
+void launch_volume_energies(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid,
+                            bool per_particle);
+void launch_total_energy(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid, bool cells,
+                         bool per_particle);
 int energy_exact_blocks_per_sm(); // resident blocks of 128 threads per SM
 
 // lcmc_sweep_fast.cu (FP32)
@@ -49,12 +52,13 @@ void launch_q_chunk_sums(const DevView &v, cudaStream_t s); // Q-tensor chunk su
 // chunk sums of (e0, e1, hard) of the NPT replicas not rejected at stage 1
 void launch_chunk_sums_volume(const DevView &v, cudaStream_t s, const double *e0, const double *e1, const int *hard);
 // FP32-pair screen of the volume move: energies at V and V', chunk sums, stage 1
-void launch_screen(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid, bool spec21);
+void launch_screen(const DevView &v, cudaStream_t s, int grid, bool spec21);
+void launch_chunk_sums_screen(const DevView &v, cudaStream_t s);
 int screen_blocks_per_sm();
-void launch_energy_reduce(const DevView &v, cudaStream_t s, const double *e0, int replica_only);
-// FP64 energy check of the due replicas (all = every replica) from per-particle energies e0
+// from launch_total_energy's sums (its `cells`)
+void launch_energy_reduce(const DevView &v, cudaStream_t s, const double *e0, int replica_only, bool cells);
+// FP64 energy check of the due replicas (all = every replica) from launch_total_energy's sums with cells = true
 void launch_energy_check(const DevView &v, cudaStream_t s, const double *e0, int all);
-void launch_volume(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid);
 void launch_order_sums(const DevView &v, cudaStream_t s, int r, double *out);
 void launch_to_id_order(const DevView &v, cudaStream_t s, int r, int grid);
 void launch_validate_upload(const double *const x[6], int *id, int n, const double L[3], double R2, int *flag,
@@ -77,7 +81,8 @@ void launch_da_stage1(const DevView &v, cudaStream_t s, const float *y);
 void launch_record_samples(const DevView &v, cudaStream_t s);
 void launch_hist_record(const DevView &v, cudaStream_t s);
 void launch_volume_propose(const DevView &v, cudaStream_t s);
-void launch_volume_finish(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid);
+void launch_volume_finish(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid,
+                          bool per_particle);
 
 // lcmc_noalloc.cu (allocation-free FP64 total energy on a caller's stream)
 int total_energy_noalloc(const GBConsts &k, int n, const double *px, const double *py, const double *pz,

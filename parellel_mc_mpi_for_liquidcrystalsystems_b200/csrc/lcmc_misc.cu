@@ -5,6 +5,7 @@
 #include "lcmc_internal.h"
 #include "lcmc_reduce.cuh"
 #include "lcmc_rng.cuh"
+#include "lcmc_volume_cells.cuh"
 
 namespace lcmc {
 
@@ -16,29 +17,47 @@ namespace lcmc {
 //   mode 0: k = 0 sum of e0 (total energy)
 //   mode 1: k = 0, 1, 2 sums of e0, e1 and hard-core hits (NPT replicas whose
 //           volume move was not screened out)
+//   mode 3: the same of the screen's energies
+//           (modes 0, 1, 3: over the cells' sums where a cell kernel served the
+//           replica, else over the particles')
 //   mode 2: k = 0..5 Q-tensor sums u_x u_x, u_x u_y, u_x u_z, u_y u_y, u_y u_z,
 //           u_z u_z (compute_liquid_crystal_order_parameters,
 //           MCnptColloid.c:2149-2167, in FP64)
+template <int MODE>
+__device__ __forceinline__ bool by_cells(const Replica &p)
+{
+    return MODE == 0 ? cells_serve<2>(p) : (MODE == 1 ? cells_serve<0>(p) : (MODE == 3 && cells_serve<1>(p)));
+}
+// items a replica's sums of `mode` run over
+template <int MODE>
+__device__ __forceinline__ int sum_items(const Replica &p)
+{
+    return by_cells<MODE>(p) ? p.nc[0] * p.nc[1] * p.nc[2] : p.n;
+}
+
 template <int K, int MODE>
-__global__ void __launch_bounds__(256) k_chunk_sums(DevView v, const double *e0, const double *e1, const int *hard)
+__global__ void __launch_bounds__(256) k_chunk_sums(DevView v, const double *e0, const double *e1, const int *hard,
+                                                    bool use_cells)
 {
     const int c = blockIdx.x, r = blockIdx.y;
     const Replica &p = v.rep[r];
+    if ((MODE == 1 || MODE == 3) && (p.ensemble != 2 || p.vol_stage1 == 0)) return;
+    const bool cells = use_cells && by_cells<MODE>(p);
+    const int n = cells ? p.nc[0] * p.nc[1] * p.nc[2] : p.n, off = cells ? p.cell_off : p.p_off;
     const int i0 = c * LCMC_RED_CHUNK;
-    if (i0 >= p.n) return;
-    if (MODE == 1 && (p.ensemble != 2 || p.vol_stage1 == 0)) return;
-    const int i1 = min(p.n, i0 + LCMC_RED_CHUNK);
+    if (i0 >= n) return;
+    const int i1 = min(n, i0 + LCMC_RED_CHUNK);
     double s[K];
 #pragma unroll
     for (int k = 0; k < K; k++) s[k] = 0.0;
     for (int i = i0 + (int)threadIdx.x; i < i1; i += blockDim.x) {
-        const int g = p.p_off + i;
+        const int g = off + i;
         if (MODE == 0) {
-            s[0] += e0[g];
-        } else if (MODE == 1) {
-            s[0] += e0[g];
-            s[1] += e1[g];
-            s[2] += hard[g] ? 1.0 : 0.0;
+            s[0] += cells ? v.cell_e0[g] : e0[g];
+        } else if (MODE == 1 || MODE == 3) {
+            s[0] += cells ? v.cell_e0[g] : e0[g];
+            s[1] += cells ? v.cell_e1[g] : e1[g];
+            s[2] += (cells ? v.cell_n1[g] : hard[g]) ? 1.0 : 0.0;
         } else {
             const double x = v.ox[g], y = v.oy[g], z = v.oz[g];
             s[0] += x * x;
@@ -57,12 +76,12 @@ __global__ void __launch_bounds__(256) k_chunk_sums(DevView v, const double *e0,
 
 // Block per replica: total energy from the chunk sums.  Resets the running
 // energy to the recomputed value and records the drift.
-__global__ void __launch_bounds__(256) k_energy_reduce(DevView v, int replica_only)
+__global__ void __launch_bounds__(256) k_energy_reduce(DevView v, int replica_only, bool use_cells)
 {
     const int r = blockIdx.x;
     if (replica_only >= 0 && r != replica_only) return;
     double s[1];
-    finish_sums<1>(v, r, s);
+    finish_sums<1>(v, r, use_cells ? sum_items<0>(v.rep[r]) : v.rep[r].n, s);
     if (threadIdx.x == 0) {
         const double tot = s[0];
         DevStats &st = v.stats[r];
@@ -91,7 +110,7 @@ __global__ void __launch_bounds__(256) k_energy_check(DevView v, int all)
     const bool due = all || (p.check_every > 0 && p.sweep % (unsigned long long)p.check_every == 0ull);
     if (!due) return;
     double s[1];
-    finish_sums<1>(v, r, s);
+    finish_sums<1>(v, r, sum_items<0>(v.rep[r]), s);
     if (threadIdx.x == 0) {
         const double tot = s[0];
         DevStats &st = v.stats[r];
@@ -147,7 +166,7 @@ __global__ void __launch_bounds__(256) k_volume_accept(DevView v)
         return;
     }
     double su[3];
-    finish_sums<3>(v, r, su);
+    finish_sums<3>(v, r, sum_items<1>(p), su);
     if (threadIdx.x == 0) {
         const double U0 = su[0], U1 = su[1];
         const bool H = su[2] > 0.0;
@@ -258,32 +277,31 @@ namespace lcmc {
 
 static dim3 chunk_grid(const DevView &v) { return dim3(v.red_nchunk, v.R); }
 
-void launch_energy_reduce(const DevView &v, cudaStream_t s, const double *e0, int replica_only)
+void launch_energy_reduce(const DevView &v, cudaStream_t s, const double *e0, int replica_only, bool cells)
 {
-    k_chunk_sums<1, 0><<<chunk_grid(v), 256, 0, s>>>(v, e0, nullptr, nullptr);
-    k_energy_reduce<<<v.R, 256, 0, s>>>(v, replica_only);
+    k_chunk_sums<1, 0><<<chunk_grid(v), 256, 0, s>>>(v, e0, nullptr, nullptr, cells);
+    k_energy_reduce<<<v.R, 256, 0, s>>>(v, replica_only, cells);
 }
 
 void launch_energy_check(const DevView &v, cudaStream_t s, const double *e0, int all)
 {
-    k_chunk_sums<1, 0><<<chunk_grid(v), 256, 0, s>>>(v, e0, nullptr, nullptr);
+    k_chunk_sums<1, 0><<<chunk_grid(v), 256, 0, s>>>(v, e0, nullptr, nullptr, true);
     k_energy_check<<<v.R, 256, 0, s>>>(v, all);
 }
 
 void launch_chunk_sums_volume(const DevView &v, cudaStream_t s, const double *e0, const double *e1, const int *hard)
 {
-    k_chunk_sums<3, 1><<<chunk_grid(v), 256, 0, s>>>(v, e0, e1, hard);
+    k_chunk_sums<3, 1><<<chunk_grid(v), 256, 0, s>>>(v, e0, e1, hard, true);
+}
+
+void launch_chunk_sums_screen(const DevView &v, cudaStream_t s)
+{
+    k_chunk_sums<3, 3><<<chunk_grid(v), 256, 0, s>>>(v, nullptr, nullptr, nullptr, true);
 }
 
 void launch_q_chunk_sums(const DevView &v, cudaStream_t s)
 {
-    k_chunk_sums<6, 2><<<chunk_grid(v), 256, 0, s>>>(v, nullptr, nullptr, nullptr);
-}
-
-void launch_volume(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid)
-{
-    launch_volume_propose(v, s);
-    launch_volume_finish(v, s, e0, e1, hard, grid);
+    k_chunk_sums<6, 2><<<chunk_grid(v), 256, 0, s>>>(v, nullptr, nullptr, nullptr, false);
 }
 
 void launch_volume_propose(const DevView &v, cudaStream_t s) { k_volume_propose<<<1, 256, 0, s>>>(v); }
@@ -291,9 +309,10 @@ void launch_volume_propose(const DevView &v, cudaStream_t s) { k_volume_propose<
 // exact FP64 energies of the current and the scaled configuration (skipped for
 // replicas the surrogate screened out), the acceptance test, optional sample
 // recording, and the scaling of accepted replicas.
-void launch_volume_finish(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid)
+void launch_volume_finish(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid,
+                          bool per_particle)
 {
-    launch_energy_exact(v, s, e0, e1, hard, 1, grid);
+    launch_volume_energies(v, s, e0, e1, hard, grid, per_particle);
     launch_chunk_sums_volume(v, s, e0, e1, hard);
     k_volume_accept<<<v.R, 256, 0, s>>>(v);
     if (v.rec_cap > 0) launch_record_samples(v, s);

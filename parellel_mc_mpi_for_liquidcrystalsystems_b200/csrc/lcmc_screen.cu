@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(256) k_screen_stage1(DevView v)
     Replica &p = v.rep[r];
     if (p.ensemble != 2 || p.da_kind != 2 || !p.use_fast) return;
     double su[3];
-    finish_sums<3>(v, r, su);
+    finish_sums<3>(v, r, p.nc[0] * p.nc[1] * p.nc[2], su);
     if (threadIdx.x == 0) {
         if (su[2] > 0.0) { // a rod centre inside the colloid at V': the exact test rejects too
             p.vol_dU_sur = 0.0;
@@ -63,18 +63,18 @@ __global__ void __launch_bounds__(256) k_screen_stage1(DevView v)
 int screen_blocks_per_sm()
 {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_volume_cells<false, true>, 128, 0) != cudaSuccess || b < 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cell_energy<1, true>, 128, 0) != cudaSuccess || b < 1) {
         cudaGetLastError();
         b = 4;
     }
     return b;
 }
 
-void launch_screen(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid, bool spec21)
+void launch_screen(const DevView &v, cudaStream_t s, int grid, bool spec21)
 {
-    if (spec21) k_volume_cells<false, true><<<grid, 128, 0, s>>>(v, e0, e1, hard);
-    else k_volume_cells<false, false><<<grid, 128, 0, s>>>(v, e0, e1, hard);
-    launch_chunk_sums_volume(v, s, e0, e1, hard);
+    if (spec21) k_cell_energy<1, true><<<grid, 128, 0, s>>>(v);
+    else k_cell_energy<1, false><<<grid, 128, 0, s>>>(v);
+    launch_chunk_sums_screen(v, s);
     k_screen_stage1<<<v.R, 256, 0, s>>>(v);
 }
 

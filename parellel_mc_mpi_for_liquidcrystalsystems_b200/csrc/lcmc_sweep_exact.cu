@@ -745,7 +745,8 @@ constexpr int EQ = 96; // queue entries per warp: < 32 pending + 64 from one chu
 #endif
 
 template <bool SCALED>
-__global__ void __launch_bounds__(128, LCMC_ENERGY_MIN_BLOCKS) k_energy_exact(DevView v, double *e0, double *e1, int *hard)
+__global__ void __launch_bounds__(128, LCMC_ENERGY_MIN_BLOCKS) k_energy_exact(DevView v, double *e0, double *e1, int *hard,
+                                                                                      bool all)
 {
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -754,20 +755,19 @@ __global__ void __launch_bounds__(128, LCMC_ENERGY_MIN_BLOCKS) k_energy_exact(De
     __shared__ int s_start[4][28]; // flat index of the first candidate of each cell
     __shared__ int s_base[4][28];  // particle slot minus flat index, per cell
     __shared__ int s_qj[4][EQ];    // queued candidate slot, configuration in bit 31
-    if (SCALED) { // nothing to do when the cell kernel serves every NPT replica needing the energies
-        bool any = false;
-        for (int r = 0; r < v.R && !any; r++) {
-            const Replica &p = v.rep[r];
-            any = p.ensemble == 2 && !(p.da_on && !p.vol_stage1) && !volume_cells_serves<true>(p);
-        }
-        if (!any) return;
+    // nothing to do when the cell kernel serves every replica that needs the energies
+    bool any = false;
+    for (int r = lane; r < v.R; r += 32) {
+        const Replica &p = v.rep[r];
+        any = any || (SCALED ? p.ensemble == 2 && !(p.da_on && !p.vol_stage1) && !cells_serve<0>(p) : all || !cells_serve<2>(p));
     }
+    if (!__any_sync(0xffffffffu, any)) return;
     for (int i = blockIdx.x * nw + wib; i < v.ntot; i += gridDim.x * nw) {
         const int r = v.p2r[i];
         const Replica &p = v.rep[r];
         const int nc0 = p.nc[0], nc1 = p.nc[1], nc2 = p.nc[2];
         // NVT, screened out, or served by the cell kernel (>= 4 cells per axis)
-        if (SCALED && (p.ensemble != 2 || (p.da_on && !p.vol_stage1) || volume_cells_serves<true>(p))) continue;
+        if (SCALED ? p.ensemble != 2 || (p.da_on && !p.vol_stage1) || cells_serve<0>(p) : !all && cells_serve<2>(p)) continue;
         const int own = v.scid[i];
         const int cell = own - p.cell_off;
         const int cx = cell % nc0, cy = (cell / nc0) % nc1, cz = cell / (nc0 * nc1);
@@ -934,34 +934,41 @@ int energy_exact_blocks_per_sm()
     return b;
 }
 
-// resident blocks of the cell kernel on this device (queried once)
-static int volume_cells_grid()
+// resident blocks of a cell kernel on this device (queried once)
+template <int MODE>
+static int cell_energy_grid()
 {
-    static int grid = 0;
-    if (!grid) {
+    static const int grid = [] {
         int dev = 0, sms = 0, b = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_volume_cells<true, false>, 128, 0) != cudaSuccess ||
-            b < 1) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cell_energy<MODE, false>, 128, 0) != cudaSuccess || b < 1) {
             cudaGetLastError();
             b = 2;
         }
-        grid = b * (sms > 0 ? sms : 1);
-    }
+        return b * (sms > 0 ? sms : 1);
+    }();
     return grid;
 }
 
-// scaled = 1: the volume move's U(V), U(V') -- the cell kernel for systems with
-// >= 4 cells per axis, the per-particle kernel for the rest
-void launch_energy_exact(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int scaled, int grid)
+// The volume move's U(V), U(V'): the cell kernel for systems with >= 4 cells
+// per axis, the per-particle kernel for the rest (launched when there may be any).
+void launch_volume_energies(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid,
+                            bool per_particle)
 {
-    if (scaled) {
-        k_volume_cells<true, false><<<volume_cells_grid(), 128, 0, s>>>(v, e0, e1, hard);
-        k_energy_exact<true><<<grid, 128, 0, s>>>(v, e0, e1, hard);
-    } else {
-        k_energy_exact<false><<<grid, 128, 0, s>>>(v, e0, e1, hard);
-    }
+    k_cell_energy<0, false><<<cell_energy_grid<0>(), 128, 0, s>>>(v);
+    if (per_particle) k_energy_exact<true><<<grid, 128, 0, s>>>(v, e0, e1, hard, false);
+}
+
+// The total energy, likewise; cells = false: per particle for every system.
+// That is the order an uploaded configuration's energy is summed in: a start
+// with overlapping rods has terms of 1e20 and more, whose rounding stays in the
+// running energy after the overlaps have gone.
+void launch_total_energy(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid, bool cells,
+                         bool per_particle)
+{
+    if (cells) k_cell_energy<2, false><<<cell_energy_grid<2>(), 128, 0, s>>>(v);
+    if (!cells || per_particle) k_energy_exact<false><<<grid, 128, 0, s>>>(v, e0, e1, hard, !cells);
 }
 
 } // namespace lcmc

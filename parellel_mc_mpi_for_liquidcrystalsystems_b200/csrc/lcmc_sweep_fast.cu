@@ -304,16 +304,6 @@ __device__ __noinline__ void fixup_big(const DevView *__restrict__ vp, int r, in
 }
 
 #define FAST_ILP 1
-// D += A B of a 16 x 8 tile (half-precision operands, FP32 accumulators).
-__device__ __forceinline__ void mma_16x8x8(float (&d)[4], unsigned a0, unsigned a1, unsigned b0, float c0, float c1)
-{
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %8, %7, %8};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a0), "r"(a1), "r"(b0), "f"(c0), "f"(c1));
-}
-
-__device__ __forceinline__ unsigned h2_bits(__half2 h) { return *reinterpret_cast<unsigned *>(&h); }
-
 // Sums over the warp of two values per lane: lanes 0-15 get the sum of a, 16-31
 // of b (one exchange halves the values a lane carries).
 __device__ __forceinline__ double warp_sum2(double a, double b, int lane)
@@ -503,7 +493,7 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
                         const float fx = __low2float(xy), fy = __high2float(xy), fz = __low2float(z1);
                         qc = fx * fx + fy * fy + fz * fz - rr * rr;
                         const __half2 m2 = __floats2half2_rn(-2.0f, -2.0f);
-                        qh = make_uint2(h2_bits(__hmul2(xy, m2)), h2_bits(__hmul2(z1, m2)));
+                        qh = make_uint2(tc::h2_bits(__hmul2(xy, m2)), tc::h2_bits(__hmul2(z1, m2)));
                     }
                 }
                 sm.qh[kw] = qh;
@@ -531,7 +521,7 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
                     const __half hz = __float2half_rn((c.z - 0.5f * wz) * sc);
                     const float fx = __low2float(xy), fy = __high2float(xy), fz = __half2float(hz);
                     const __half hs = __float2half_rd(fx * fx + fy * fy + fz * fz);
-                    sm.ch[pos + i] = make_uint2(h2_bits(xy), h2_bits(__halves2half2(hz, hs)));
+                    sm.ch[pos + i] = make_uint2(tc::h2_bits(xy), tc::h2_bits(__halves2half2(hz, hs)));
                 }
             }
             if (t < 16) sm.ch[ncand + t] = make_uint2(0u, 0x7b000000u); // beyond the last: likewise
@@ -569,7 +559,7 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
                     for (int i = 0; i < e; i++) {
                         const unsigned a0 = ah[32 * (16 * b + i)], a1 = ah[32 * (16 * b + i) + 16];
                         float d[4];
-                        mma_16x8x8(d, a0, a1, b0, c0, c1);
+                        tc::mma_16x8x8(d, a0, a1, b0, c0, c1);
                         x0 = __funnelshift_l(__float_as_uint(d[0]), x0, 1);
                         x1 = __funnelshift_l(__float_as_uint(d[1]), x1, 1);
                         x0 = __funnelshift_l(__float_as_uint(d[2]), x0, 1);

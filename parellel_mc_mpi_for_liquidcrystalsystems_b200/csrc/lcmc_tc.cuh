@@ -3,6 +3,7 @@
 // mbarrier, bounded mbarrier waits and TMEM loads.  Encodings follow the PTX
 // ISA for tcgen05 (the same fields CUTLASS's cute/arch/mma_sm100_desc.hpp names).
 #pragma once
+#include <cuda_fp16.h>
 #include <stdint.h>
 
 namespace lcmc {
@@ -154,6 +155,20 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16])
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
+
+// D = A B + C of a 16 x 8 tile on the warp-level matrix path (half-precision
+// operands, inner dimension 8, FP32 accumulators; C the same in every row): the
+// reach tests, whose 8-column tiles of a few dozen rows are far below a tcgen05
+// tile.  Lane 4 g + q holds rows g and g + 8 of A (elements 2q, 2q + 1), column g
+// of B, and columns 2q, 2q + 1 of D in rows g (d[0], d[1]) and g + 8 (d[2], d[3]).
+__device__ __forceinline__ void mma_16x8x8(float (&d)[4], unsigned a0, unsigned a1, unsigned b0, float c0, float c1)
+{
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %8, %7, %8};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(b0), "f"(c0), "f"(c1));
+}
+
+__device__ __forceinline__ unsigned h2_bits(__half2 h) { return *reinterpret_cast<unsigned *>(&h); }
 
 } // namespace tc
 } // namespace lcmc
