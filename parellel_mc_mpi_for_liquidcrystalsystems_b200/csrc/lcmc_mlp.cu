@@ -13,8 +13,17 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
+#include <atomic>
+#include <condition_variable>
+#include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
+
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
 
 #include "../../include/lcmc.h"
 #include "lcmc_rng.cuh"
@@ -429,7 +438,7 @@ __device__ __forceinline__ float dsilu(float z)
 }
 
 // Z += bias; H = silu(Z) (BF16, row-major B x H) and its transpose (H x B)
-__global__ void k_bias_act(float *Z, const float *bias, bf16 *Hb, bf16 *HbT, float *Hf, int Bn, int Hn)
+__global__ void k_bias_act(float *Z, const float *bias, bf16 *Hb, bf16 *HbT, int Bn, int Hn)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Bn * Hn; i += gridDim.x * blockDim.x) {
         const int b = i / Hn, h = i % Hn;
@@ -439,18 +448,25 @@ __global__ void k_bias_act(float *Z, const float *bias, bf16 *Hb, bf16 *HbT, flo
         const bf16 ab = __float2bfloat16(a);
         Hb[i] = ab;
         if (HbT) HbT[(size_t)h * Bn + b] = ab;
-        if (Hf) Hf[i] = a;
     }
 }
 
-// y = A2 . w3 + b3 (warp per row); optionally dy = 2 (y - t) / n_valid for rows < n_valid
-__global__ void k_out_layer(const float *A2, const float *w3, const float *b3, float *y, const float *target,
-                            float *dy, float *loss, int Bn, int Hn, int n_valid)
+// Second hidden layer and output, warp per row: Z2 += b2, A2 = silu(Z2),
+// y = A2 . w3 + b3; with a target also dy = 2 (y - t) / n_valid for rows <
+// n_valid and the row's share of the loss.
+__global__ void k_act_out(float *Z2, const float *b2, const float *w3, const float *b3, float *A2, float *y,
+                          const float *target, float *dy, float *row_loss, int Bn, int Hn, int n_valid)
 {
     const int lane = threadIdx.x & 31;
     for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < Bn; r += (gridDim.x * blockDim.x) >> 5) {
         float s = 0.0f;
-        for (int h = lane; h < Hn; h += 32) s += A2[(size_t)r * Hn + h] * w3[h];
+        for (int h = lane; h < Hn; h += 32) {
+            const size_t i = (size_t)r * Hn + h;
+            const float z = Z2[i] + b2[h], a = silu(z);
+            Z2[i] = z;
+            A2[i] = a;
+            s += a * w3[h];
+        }
         for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) {
             const float v = s + b3[0];
@@ -458,45 +474,88 @@ __global__ void k_out_layer(const float *A2, const float *w3, const float *b3, f
             if (target) {
                 const float e = r < n_valid ? v - target[r] : 0.0f;
                 dy[r] = 2.0f * e / (float)n_valid;
-                atomicAdd(loss, e * e / (float)n_valid);
+                row_loss[r] = e * e / (float)n_valid;
             }
         }
     }
 }
 
-// dZ2 = (dy w3) * silu'(Z2); also dw3 += dy A2 (atomics), db3 += dy; writes dZ2 (B x H) and dZ2^T (H x B) in BF16
-__global__ void k_back_out(const float *dy, const float *w3, const float *Z2, const float *A2, float *gw3, float *gb3,
-                           bf16 *dZ2b, bf16 *dZ2bT, float *dZ2f, int Bn, int Hn)
+// A layer's backward pass by columns: a block takes BK_COLS of the Hn columns and
+// every row.  The sums over the batch are the block's own (no atomics, nothing to
+// clear) and run in the rows' order, from shared memory, a thread per sum: 256
+// dependent additions take 0.6 us, less than one more launch.
+constexpr int BK_COLS = 4, BK_THREADS = 256, BK_ROWS = BK_THREADS / BK_COLS;
+
+// dZ2 = (dy w3) * silu'(Z2) in BF16 (B x H and its transpose); gradients of w3
+// and b2, and (block 0) of b3 and the batch loss.
+__global__ void __launch_bounds__(BK_THREADS) k_back_out(const float *dy, const float *row_loss, const float *w3,
+                                                         const float *Z2, const float *A2, float *gw3, float *gb2,
+                                                         float *gb3, float *loss, bf16 *dZ2b, bf16 *dZ2bT, int Bn, int Hn)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Bn * Hn; i += gridDim.x * blockDim.x) {
-        const int b = i / Hn, h = i % Hn;
-        const float g = dy[b] * w3[h] * dsilu(Z2[i]);
-        const bf16 gb = __float2bfloat16(g);
-        dZ2b[i] = gb;
-        dZ2bT[(size_t)h * Bn + b] = gb;
-        dZ2f[i] = g;
-        atomicAdd(&gw3[h], dy[b] * A2[i]);
-        if (h == 0) atomicAdd(gb3, dy[b]);
+    __shared__ float term[2 * BK_COLS + 2][BK_THREADS]; // per column: w3, b2; then b3 and the loss
+    const int c = threadIdx.x % BK_COLS, h = blockIdx.x * BK_COLS + c;
+    float sum = 0.0f;
+    for (int b0 = 0; b0 < Bn; b0 += BK_THREADS) {
+        const int rows = min(BK_THREADS, Bn - b0);
+        __syncthreads();
+        for (int r = threadIdx.x / BK_COLS; r < rows; r += BK_ROWS) {
+            const int b = b0 + r;
+            const size_t i = (size_t)b * Hn + h;
+            const float d = dy[b], g = d * w3[h] * dsilu(Z2[i]);
+            const bf16 gb = __float2bfloat16(g);
+            dZ2b[i] = gb;
+            dZ2bT[(size_t)h * Bn + b] = gb;
+            term[c][r] = __fmul_rn(d, A2[i]);
+            term[BK_COLS + c][r] = g;
+            if (c == 0) {
+                term[2 * BK_COLS][r] = d;
+                term[2 * BK_COLS + 1][r] = row_loss[b];
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 2 * BK_COLS + 2) {
+#pragma unroll 16
+            for (int r = 0; r < rows; r++) sum += term[threadIdx.x][r];
+        }
     }
+    const int t = threadIdx.x;
+    if (t < BK_COLS) gw3[h] = sum;
+    else if (t < 2 * BK_COLS) gb2[h] = sum;
+    else if (t < 2 * BK_COLS + 2 && blockIdx.x == 0) (t == 2 * BK_COLS ? gb3 : loss)[0] = sum;
 }
 
-// dZ1 = dH1 * silu'(Z1) -> dZ1^T (H x B) in BF16; db1 accumulated
-__global__ void k_back_hidden(const float *dH, const float *Z, bf16 *dZbT, float *gbias, int Bn, int Hn)
+// dZ1 = dH1 * silu'(Z1) -> dZ1^T (H x B) in BF16, and the gradient of b1
+__global__ void __launch_bounds__(BK_THREADS) k_back_hidden(const float *dH, const float *Z, bf16 *dZbT, float *gbias,
+                                                            int Bn, int Hn)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Bn * Hn; i += gridDim.x * blockDim.x) {
-        const int b = i / Hn, h = i % Hn;
-        const float g = dH[i] * dsilu(Z[i]);
-        dZbT[(size_t)h * Bn + b] = __float2bfloat16(g);
-        atomicAdd(&gbias[h], g);
+    __shared__ float term[BK_COLS][BK_THREADS];
+    const int c = threadIdx.x % BK_COLS, h = blockIdx.x * BK_COLS + c;
+    float sum = 0.0f;
+    for (int b0 = 0; b0 < Bn; b0 += BK_THREADS) {
+        const int rows = min(BK_THREADS, Bn - b0);
+        __syncthreads();
+        for (int r = threadIdx.x / BK_COLS; r < rows; r += BK_ROWS) {
+            const size_t i = (size_t)(b0 + r) * Hn + h;
+            const float g = dH[i] * dsilu(Z[i]);
+            dZbT[(size_t)h * Bn + b0 + r] = __float2bfloat16(g);
+            term[c][r] = g;
+        }
+        __syncthreads();
+        if (threadIdx.x < BK_COLS) {
+#pragma unroll 16
+            for (int r = 0; r < rows; r++) sum += term[threadIdx.x][r];
+        }
     }
+    if (threadIdx.x < BK_COLS) gbias[h] = sum;
 }
 
-__global__ void k_colsum(const float *X, float *out, int Bn, int Hn)
+// rows pos[r] of the data set -> row r of X (16 bytes per thread and step)
+__global__ void k_gather_rows(const bf16 *D, const int *pos, bf16 *X, int rows, int K1)
 {
-    for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < Hn; h += gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        for (int b = 0; b < Bn; b++) s += X[(size_t)b * Hn + h];
-        out[h] += s;
+    const int per = K1 / 8;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows * per; i += gridDim.x * blockDim.x) {
+        const int r = i / per, c = i - r * per;
+        reinterpret_cast<uint4 *>(X)[i] = reinterpret_cast<const uint4 *>(D)[(size_t)pos[r] * per + c];
     }
 }
 
@@ -532,9 +591,10 @@ __global__ void k_weights_bf16(const float *W, bf16 *Wb, bf16 *WbT, int rows, in
     }
 }
 
-// Adam (Kingma & Ba 2015), FP32 master weights
+// Adam (Kingma & Ba 2015), FP32 master weights; the BF16 copies of W1 (the first
+// n1 parameters) and W2 (H x H from o2, with its transpose) are written along.
 __global__ void k_adam(float *w, const float *g, float *m, float *v, int n, float lr, float b1, float b2, float eps,
-                       float c1, float c2)
+                       float c1, float c2, bf16 *W1b, int n1, bf16 *W2b, bf16 *W2bT, int o2, int H)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float gi = g[i];
@@ -542,7 +602,16 @@ __global__ void k_adam(float *w, const float *g, float *m, float *v, int n, floa
         const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
         m[i] = mi;
         v[i] = vi;
-        w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        w[i] = wi;
+        if (i < n1) {
+            W1b[i] = __float2bfloat16(wi);
+        } else if (i >= o2 && i < o2 + H * H) {
+            const int j = i - o2;
+            const bf16 x = __float2bfloat16(wi);
+            W2b[j] = x;
+            W2bT[(j % H) * H + j / H] = x;
+        }
     }
 }
 
@@ -562,11 +631,22 @@ struct lcmc_mlp {
     size_t np = 0;
     bf16 *W1b = nullptr, *W2b = nullptr, *W2bT = nullptr;
     // activations (bmax rows)
-    bf16 *X = nullptr, *XT = nullptr, *H1 = nullptr, *H1T = nullptr, *H2 = nullptr, *dZ2 = nullptr, *dZ2T = nullptr,
-         *dZ1T = nullptr;
-    float *Xf = nullptr, *Z1 = nullptr, *Z2 = nullptr, *A2 = nullptr, *y = nullptr, *t = nullptr, *dy = nullptr,
-          *dZ2f = nullptr, *dH1 = nullptr, *loss = nullptr;
+    bf16 *X = nullptr, *XT = nullptr, *H1 = nullptr, *H1T = nullptr, *dZ2 = nullptr, *dZ2T = nullptr, *dZ1T = nullptr;
+    float *Z1 = nullptr, *Z2 = nullptr, *A2 = nullptr, *y = nullptr, *t = nullptr, *dy = nullptr, *row_loss = nullptr,
+          *dH1 = nullptr, *loss = nullptr;
     int *err = nullptr;
+    // host rows on their way to the device
+    static constexpr int SLOTS = 2, STAGE_ROWS = 128;
+    uint16_t *stage = nullptr; // pinned, SLOTS x STAGE_ROWS rows of k1 BF16 values each
+    cudaEvent_t sent[SLOTS] = {nullptr, nullptr};
+    int slot = 0;
+    // training: the rows (BF16), an epoch's targets and places of its rows, its losses (grown as needed)
+    bf16 *rows = nullptr;
+    float *et = nullptr, *losses = nullptr;
+    int *pos = nullptr;
+    size_t rows_n = 0, et_n = 0, losses_n = 0, pos_n = 0;
+    float *yall = nullptr; // a predict call's outputs (grown as needed)
+    size_t yall_n = 0;
     long long step = 0;
     std::string msg;
 };
@@ -581,9 +661,12 @@ extern "C" int lcmc_mlp_destroy(lcmc_mlp *m)
 {
     if (!m) return LCMC_EINVAL;
     if (m->s) cudaStreamSynchronize(m->s);
-    void *ptrs[] = {m->P, m->G, m->Mm, m->Vv, m->W1b, m->W2b, m->W2bT, m->X, m->XT, m->H1, m->H1T, m->H2, m->dZ2,
-                    m->dZ2T, m->dZ1T, m->Xf, m->Z1, m->Z2, m->A2, m->y, m->t, m->dy, m->dZ2f, m->dH1, m->loss,
-                    m->err};
+    void *ptrs[] = {m->P, m->G, m->Mm, m->Vv, m->W1b, m->W2b, m->W2bT, m->X, m->XT, m->H1, m->H1T, m->dZ2,
+                    m->dZ2T, m->dZ1T, m->Z1, m->Z2, m->A2, m->y, m->t, m->dy, m->row_loss, m->dH1, m->loss,
+                    m->err, m->yall, m->rows, m->et, m->losses, m->pos};
+    if (m->stage) cudaFreeHost(m->stage);
+    for (cudaEvent_t ev : m->sent)
+        if (ev) cudaEventDestroy(ev);
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (m->s) cudaStreamDestroy(m->s);
@@ -631,22 +714,27 @@ extern "C" int lcmc_mlp_create(int n_in, int hidden, int max_batch, uint64_t see
     MA(m->XT, (size_t)B * K1 * 2);
     MA(m->H1, (size_t)B * H * 2);
     MA(m->H1T, (size_t)B * H * 2);
-    MA(m->H2, (size_t)B * H * 2);
     MA(m->dZ2, (size_t)B * H * 2);
     MA(m->dZ2T, (size_t)B * H * 2);
     MA(m->dZ1T, (size_t)B * H * 2);
-    MA(m->Xf, (size_t)B * K1 * 4);
     MA(m->Z1, (size_t)B * H * 4);
     MA(m->Z2, (size_t)B * H * 4);
     MA(m->A2, (size_t)B * H * 4);
     MA(m->y, (size_t)B * 4);
     MA(m->t, (size_t)B * 4);
     MA(m->dy, (size_t)B * 4);
-    MA(m->dZ2f, (size_t)B * H * 4);
+    MA(m->row_loss, (size_t)B * 4);
     MA(m->dH1, (size_t)B * H * 4);
     MA(m->loss, 4);
     MA(m->err, 4);
 #undef MA
+    e = cudaMallocHost((void **)&m->stage, (size_t)lcmc_mlp::SLOTS * lcmc_mlp::STAGE_ROWS * K1 * 2);
+    for (cudaEvent_t &ev : m->sent)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+        lcmc_mlp_destroy(m);
+        return LCMC_ENOMEM;
+    }
     m->W1 = m->P;
     m->b1 = m->W1 + (size_t)H * K1;
     m->W2 = m->b1 + H;
@@ -667,11 +755,11 @@ extern "C" int lcmc_mlp_create(int n_in, int hidden, int max_batch, uint64_t see
     for (size_t i = 0; i < (size_t)H * H; i++) host[o2 + i] = uni(o2 + i, a2);
     const size_t o3 = o2 + (size_t)H * H + H;
     for (int h = 0; h < H; h++) host[o3 + h] = uni(o3 + h, a3);
-    cudaMemcpy(m->P, host.data(), m->np * 4, cudaMemcpyHostToDevice);
+    // on the network's own stream: the conversions below follow the copy
+    cudaMemcpyAsync(m->P, host.data(), m->np * 4, cudaMemcpyHostToDevice, m->s);
     cudaMemsetAsync(m->Mm, 0, m->np * 4, m->s);
     cudaMemsetAsync(m->Vv, 0, m->np * 4, m->s);
     cudaMemsetAsync(m->X, 0, (size_t)B * K1 * 2, m->s);
-    cudaMemsetAsync(m->Xf, 0, (size_t)B * K1 * 4, m->s);
     cudaMemsetAsync(m->err, 0, 4, m->s);
     k_weights_bf16<<<256, 256, 0, m->s>>>(m->W1, m->W1b, nullptr, H, K1);
     k_weights_bf16<<<64, 256, 0, m->s>>>(m->W2, m->W2b, m->W2bT, H, H);
@@ -684,16 +772,17 @@ extern "C" int lcmc_mlp_create(int n_in, int hidden, int max_batch, uint64_t see
     return LCMC_OK;
 }
 
-// forward on the B (multiple of 128) rows of m->X -> activations A2
-static void mlp_forward_s(lcmc_mlp *m, int B, cudaStream_t s)
+// forward on B (a multiple of 128) rows of X -> activations A2, outputs y; with
+// targets t also dy and the rows' losses
+static void mlp_forward_s(lcmc_mlp *m, const bf16 *X, int B, const float *t, int n_valid, cudaStream_t s)
 {
     const int H = m->hid, K1 = m->k1;
-    gemm_tc(m->X, K1, m->W1b, K1, m->Z1, H, B, H, K1, 0, m->err, s);
-    k_bias_act<<<(B * H + 255) / 256, 256, 0, s>>>(m->Z1, m->b1, m->H1, m->H1T, nullptr, B, H);
+    gemm_tc(X, K1, m->W1b, K1, m->Z1, H, B, H, K1, 0, m->err, s);
+    k_bias_act<<<(B * H + 255) / 256, 256, 0, s>>>(m->Z1, m->b1, m->H1, m->H1T, B, H);
     gemm_tc(m->H1, H, m->W2b, H, m->Z2, H, B, H, H, 0, m->err, s);
-    k_bias_act<<<(B * H + 255) / 256, 256, 0, s>>>(m->Z2, m->b2, m->H2, nullptr, m->A2, B, H);
+    k_act_out<<<(B * 32 + 255) / 256, 256, 0, s>>>(m->Z2, m->b2, m->w3, m->b3, m->A2, m->y, t, m->dy, m->row_loss, B, H,
+                                                   n_valid);
 }
-static void mlp_forward(lcmc_mlp *m, int B) { mlp_forward_s(m, B, m->s); }
 
 namespace lcmc {
 // In-sweep inference: the sweep's kernels write the BF16 input rows into
@@ -705,87 +794,217 @@ int mlp_bmax(lcmc_mlp *m) { return m->bmax; }
 int mlp_n_in(lcmc_mlp *m) { return m->n_in; }
 const float *mlp_forward_device(lcmc_mlp *m, int B, cudaStream_t s)
 {
-    mlp_forward_s(m, B, s);
-    k_out_layer<<<(B * 32 + 255) / 256, 256, 0, s>>>(m->A2, m->w3, m->b3, m->y, nullptr, nullptr, nullptr, B, m->hid,
-                                                     B);
+    mlp_forward_s(m, m->X, B, nullptr, B, s);
     return m->y;
 }
 int *mlp_err(lcmc_mlp *m) { return m->err; }
 } // namespace lcmc
 
-// rows of host features (n x n_in, FP32) -> m->X (BF16, padded to k1 columns, B rows)
-static void load_batch(lcmc_mlp *m, const float *x, int n, int B)
+// ---------------------------------------------------------------------------
+// Host rows to the device.  Feature rows come as FP32 in pageable memory, 16 KB
+// each; copied as they are, the driver moves them at 8-10 GB/s through its own
+// staging, and that was nearly all of a call.  Here host threads round them to
+// BF16, which the network takes, into pinned buffers whose copies run while the
+// next rows are converted: half the bytes on the link.  Predictions of 4096 rows
+// 8.2 -> 2.2 ms, an epoch of 2048 rows in batches of 256 10.6 -> 2.2 ms; bound by
+// the threads' reads of the FP32 rows (67 MB in 4096 of them).
+// ---------------------------------------------------------------------------
+
+// float -> BF16, round to nearest even, NaN to 0x7fff as __float2bfloat16 does
+static inline uint16_t bf16_bits(float f)
 {
-    const int K1 = m->k1;
-    cudaMemset2DAsync(m->Xf, (size_t)K1 * 4, 0, (size_t)K1 * 4, B, m->s);
-    cudaMemcpy2DAsync(m->Xf, (size_t)K1 * 4, x, (size_t)m->n_in * 4, (size_t)m->n_in * 4, n, cudaMemcpyHostToDevice,
-                      m->s);
-    k_f32_to_bf16<<<512, 256, 0, m->s>>>(m->Xf, m->X, B * K1);
+    uint32_t u;
+    memcpy(&u, &f, 4);
+    if ((u & 0x7fffffffu) > 0x7f800000u) return 0x7fff;
+    return (uint16_t)((u + 0x7fffu + ((u >> 16) & 1u)) >> 16);
+}
+
+static void convert_row(const float *x, int n_in, int k1, uint16_t *dst)
+{
+    int i = 0;
+#ifdef __SSE2__
+    const __m128i one = _mm_set1_epi32(1), bias = _mm_set1_epi32(0x7fff), qnan = _mm_set1_epi32(0x7fff);
+    for (; i + 8 <= n_in; i += 8) {
+        __m128i r[2];
+        for (int h = 0; h < 2; h++) {
+            const __m128 f = _mm_loadu_ps(x + i + 4 * h);
+            const __m128i u = _mm_castps_si128(f), nan = _mm_castps_si128(_mm_cmpunord_ps(f, f));
+            const __m128i v = _mm_add_epi32(_mm_add_epi32(u, bias), _mm_and_si128(_mm_srli_epi32(u, 16), one));
+            r[h] = _mm_or_si128(_mm_andnot_si128(nan, _mm_srai_epi32(v, 16)), _mm_and_si128(nan, qnan));
+        }
+        _mm_storeu_si128((__m128i *)(dst + i), _mm_packs_epi32(r[0], r[1]));
+    }
+#endif
+    for (; i < n_in; i++) dst[i] = bf16_bits(x[i]);
+    for (; i < k1; i++) dst[i] = 0;
+}
+
+// The threads of one call: rows [0, n) of a batch split among them.  They live
+// from the first batch to the end of the call.
+class RowConverter {
+public:
+    RowConverter(size_t values)
+    {
+        // one thread for small calls (starting a thread takes as long as converting a few hundred KB)
+        const unsigned hw = std::thread::hardware_concurrency();
+        const int want = (int)std::min<size_t>(values >> 19, std::min(hw ? hw : 1u, 12u));
+        try {
+            threads_.reserve(want > 1 ? want - 1 : 0);
+            for (int i = 1; i < want; i++) threads_.emplace_back([this] { work(); });
+        } catch (...) { // fewer threads then
+        }
+    }
+    ~RowConverter()
+    {
+        {
+            std::lock_guard<std::mutex> l(mu_);
+            stop_.store(true);
+        }
+        cv_.notify_all();
+        for (auto &t : threads_) t.join();
+    }
+    // rows idx[r] (idx null: r) of x -> rows r of dst
+    void run(const float *x, const int *idx, int n, int n_in, int k1, uint16_t *dst)
+    {
+        x_ = x, idx_ = idx, n_ = n, n_in_ = n_in, k1_ = k1, dst_ = dst;
+        next_.store(0);
+        busy_.store((int)threads_.size());
+        {
+            std::lock_guard<std::mutex> l(mu_);
+            gen_.fetch_add(1);
+        }
+        cv_.notify_all();
+        rows();
+        while (busy_.load() > 0) std::this_thread::yield(); // (the last rows of other threads)
+    }
+
+private:
+    void rows()
+    {
+        constexpr int STEP = 8;
+        for (int r0; (r0 = next_.fetch_add(STEP)) < n_;)
+            for (int r = r0; r < std::min(n_, r0 + STEP); r++)
+                convert_row(x_ + (size_t)(idx_ ? idx_[r] : r) * n_in_, n_in_, k1_, dst_ + (size_t)r * k1_);
+    }
+    void work()
+    {
+        long long seen = 0;
+        for (;;) {
+            // the next part follows within some 10 us: look for it before sleeping
+            for (int i = 0; i < 64 && gen_.load() == seen && !stop_.load(); i++) std::this_thread::yield();
+            if (gen_.load() == seen) {
+                std::unique_lock<std::mutex> l(mu_);
+                cv_.wait(l, [&] { return stop_.load() || gen_.load() != seen; });
+            }
+            if (stop_.load()) return;
+            seen = gen_.load();
+            rows();
+            busy_.fetch_sub(1);
+        }
+    }
+    std::vector<std::thread> threads_;
+    std::mutex mu_;
+    std::condition_variable cv_;
+    std::atomic<int> next_{0}, busy_{0};
+    std::atomic<long long> gen_{0};
+    std::atomic<bool> stop_{false};
+    const float *x_ = nullptr;
+    const int *idx_ = nullptr;
+    int n_ = 0, n_in_ = 0, k1_ = 0;
+    uint16_t *dst_ = nullptr;
+};
+
+// Rows idx[0 .. n) (idx null: the first n) of the caller's features to rows [0, B)
+// of dst on the network's stream, zeros beyond n.
+static cudaError_t send_rows(lcmc_mlp *m, RowConverter &rc, const float *x, const int *idx, int n, int B, bf16 *dst)
+{
+    cudaError_t e;
+    const size_t row = (size_t)m->k1 * 2;
+    constexpr int step = lcmc_mlp::STAGE_ROWS;
+    for (int off = 0; off < n; off += step) {
+        const int i = m->slot, c = std::min(step, n - off);
+        m->slot = (i + 1) % lcmc_mlp::SLOTS;
+        if ((e = cudaEventSynchronize(m->sent[i])) != cudaSuccess) return e; // its last copy has left
+        uint16_t *stage = m->stage + (size_t)i * lcmc_mlp::STAGE_ROWS * m->k1;
+        rc.run(idx ? x : x + (size_t)off * m->n_in, idx ? idx + off : nullptr, c, m->n_in, m->k1, stage);
+        e = cudaMemcpyAsync(dst + (size_t)off * m->k1, stage, (size_t)c * row, cudaMemcpyHostToDevice, m->s);
+        if (e != cudaSuccess) return e;
+        if ((e = cudaEventRecord(m->sent[i], m->s)) != cudaSuccess) return e;
+    }
+    if (B > n) return cudaMemsetAsync((char *)dst + (size_t)n * row, 0, (size_t)(B - n) * row, m->s);
+    return cudaSuccess;
+}
+
+template <typename T>
+static cudaError_t grow(T **p, size_t *have, size_t want)
+{
+    if (want <= *have) return cudaSuccess;
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+    *have = 0;
+    cudaError_t e = cudaMalloc((void **)p, want * sizeof(T));
+    if (e == cudaSuccess) *have = want;
+    return e;
 }
 
 extern "C" int lcmc_mlp_predict(lcmc_mlp *m, const float *x, int n, float *y)
 {
     if (!m || !x || !y || n < 0) return LCMC_EINVAL;
-    for (int off = 0; off < n; off += m->bmax) {
-        const int nb = n - off < m->bmax ? n - off : m->bmax;
-        const int B = (nb + 127) / 128 * 128;
-        load_batch(m, x + (size_t)off * m->n_in, nb, B);
-        mlp_forward(m, B);
-        k_out_layer<<<(B * 32 + 255) / 256, 256, 0, m->s>>>(m->A2, m->w3, m->b3, m->y, nullptr, nullptr, nullptr, B,
-                                                             m->hid, nb);
-        cudaMemcpyAsync(y + off, m->y, (size_t)nb * 4, cudaMemcpyDeviceToHost, m->s);
+    cudaError_t e = cudaSuccess;
+    if (n > 0) {
+        // outputs gather on the device: one copy back, after the last rows
+        if ((e = grow(&m->yall, &m->yall_n, (size_t)(n + 127) / 128 * 128)) != cudaSuccess) return mlp_fail(m, "predict", e);
+        RowConverter rc((size_t)n * m->n_in);
+        for (int off = 0; off < n && e == cudaSuccess; off += m->bmax) {
+            const int nb = n - off < m->bmax ? n - off : m->bmax;
+            const int B = (nb + 127) / 128 * 128;
+            e = send_rows(m, rc, x + (size_t)off * m->n_in, nullptr, nb, B, m->X);
+            if (e != cudaSuccess) break;
+            mlp_forward_s(m, m->X, B, nullptr, nb, m->s);
+            e = cudaMemcpyAsync(m->yall + off, m->y, (size_t)nb * 4, cudaMemcpyDeviceToDevice, m->s);
+        }
+        if (e == cudaSuccess) e = cudaMemcpyAsync(y, m->yall, (size_t)n * 4, cudaMemcpyDeviceToHost, m->s);
     }
-    cudaError_t e = cudaStreamSynchronize(m->s);
+    const cudaError_t es = cudaStreamSynchronize(m->s);
+    if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) return mlp_fail(m, "predict", e);
     int err = 0;
     cudaMemcpy(&err, m->err, 4, cudaMemcpyDeviceToHost);
     return err ? LCMC_ETIMEOUT : LCMC_OK;
 }
 
-// Forward + backward on rows [0, n) of a host batch: gradients in m->G, MSE in m->loss.
-static void mlp_backward(lcmc_mlp *m, const float *x, const float *t, int n);
-
-// One Adam step on rows [0, n) of the given host batch; returns the batch MSE.
-static int mlp_step(lcmc_mlp *m, const float *x, const float *t, int n, float lr, float *loss_out)
-{
-    const int H = m->hid, K1 = m->k1;
-    mlp_backward(m, x, t, n);
-    m->step++;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.0f - powf(b1, (float)m->step), c2 = 1.0f - powf(b2, (float)m->step);
-    k_adam<<<512, 256, 0, m->s>>>(m->P, m->G, m->Mm, m->Vv, (int)m->np, lr, b1, b2, 1e-8f, c1, c2);
-    // padding columns of W1 stay exactly zero: their gradient is zero (zero inputs)
-    k_weights_bf16<<<256, 256, 0, m->s>>>(m->W1, m->W1b, nullptr, H, K1);
-    k_weights_bf16<<<64, 256, 0, m->s>>>(m->W2, m->W2b, m->W2bT, H, H);
-    if (loss_out) cudaMemcpyAsync(loss_out, m->loss, 4, cudaMemcpyDeviceToHost, m->s);
-    return LCMC_OK;
-}
-
-static void mlp_backward(lcmc_mlp *m, const float *x, const float *t, int n)
+// Forward + backward on n rows of X (zeros beyond, up to a multiple of 128; so
+// the targets t): gradients in m->G, MSE in *loss.
+static void mlp_backward(lcmc_mlp *m, const bf16 *X, const float *t, int n, float *loss)
 {
     const int H = m->hid, K1 = m->k1;
     const int B = (n + 127) / 128 * 128;
-    load_batch(m, x, n, B);
-    cudaMemsetAsync(m->t, 0, (size_t)B * 4, m->s);
-    cudaMemcpyAsync(m->t, t, (size_t)n * 4, cudaMemcpyHostToDevice, m->s);
-    cudaMemsetAsync(m->G, 0, m->np * 4, m->s);
-    cudaMemsetAsync(m->loss, 0, 4, m->s);
-    mlp_forward(m, B);
+    mlp_forward_s(m, X, B, t, n, m->s);
     float *gW1 = m->G, *gb1 = gW1 + (size_t)H * K1, *gW2 = gb1 + H, *gb2 = gW2 + (size_t)H * H, *gw3 = gb2 + H,
           *gb3 = gw3 + H;
-    k_out_layer<<<(B * 32 + 255) / 256, 256, 0, m->s>>>(m->A2, m->w3, m->b3, m->y, m->t, m->dy, m->loss, B, H, n);
-    k_back_out<<<(B * H + 255) / 256, 256, 0, m->s>>>(m->dy, m->w3, m->Z2, m->A2, gw3, gb3, m->dZ2, m->dZ2T, m->dZ2f,
-                                                      B, H);
-    k_colsum<<<1, 128, 0, m->s>>>(m->dZ2f, gb2, B, H);
+    k_back_out<<<H / BK_COLS, BK_THREADS, 0, m->s>>>(m->dy, m->row_loss, m->w3, m->Z2, m->A2, gw3, gb2, gb3, loss, m->dZ2,
+                                                     m->dZ2T, B, H);
     // dW2 = dZ2^T H1: (H x B) . (H x B)^T
     gemm_tc(m->dZ2T, B, m->H1T, B, gW2, H, H, H, B, 0, m->err, m->s);
     // dH1 = dZ2 W2: (B x H) . (W2^T)^T
     gemm_tc(m->dZ2, H, m->W2bT, H, m->dH1, H, B, H, H, 0, m->err, m->s);
-    k_back_hidden<<<(B * H + 255) / 256, 256, 0, m->s>>>(m->dH1, m->Z1, m->dZ1T, gb1, B, H);
+    k_back_hidden<<<H / BK_COLS, BK_THREADS, 0, m->s>>>(m->dH1, m->Z1, m->dZ1T, gb1, B, H);
     // dW1 = dZ1^T X: (H x B) . (X^T)^T with X^T = K1 x B
     dim3 tg((K1 + 31) / 32, (B + 31) / 32), tb(32, 8);
-    k_transpose_bf16<<<tg, tb, 0, m->s>>>(m->X, m->XT, B, K1);
+    k_transpose_bf16<<<tg, tb, 0, m->s>>>(X, m->XT, B, K1);
     gemm_tc(m->dZ1T, B, m->XT, B, gW1, K1, H, K1, B, 0, m->err, m->s);
+}
+
+// One Adam step on the gradients in m->G.
+static void mlp_update(lcmc_mlp *m, float lr)
+{
+    const int H = m->hid, K1 = m->k1;
+    m->step++;
+    const float b1 = 0.9f, b2 = 0.999f;
+    const float c1 = 1.0f - powf(b1, (float)m->step), c2 = 1.0f - powf(b2, (float)m->step);
+    // padding columns of W1 stay exactly zero: their gradient is zero (zero inputs)
+    k_adam<<<512, 256, 0, m->s>>>(m->P, m->G, m->Mm, m->Vv, (int)m->np, lr, b1, b2, 1e-8f, c1, c2, m->W1b, H * K1, m->W2b,
+                                  m->W2bT, (int)(m->W2 - m->P), H);
 }
 
 extern "C" int lcmc_mlp_num_params(const lcmc_mlp *m) { return m ? (int)m->np : 0; }
@@ -793,10 +1012,19 @@ extern "C" int lcmc_mlp_num_params(const lcmc_mlp *m) { return m ? (int)m->np : 
 extern "C" int lcmc_mlp_gradients(lcmc_mlp *m, const float *x, const float *t, int n, float *grad, float *loss)
 {
     if (!m || !x || !t || !grad || n <= 0 || n > m->bmax) return LCMC_EINVAL;
-    mlp_backward(m, x, t, n);
+    const int B = (n + 127) / 128 * 128;
+    cudaError_t e;
+    {
+        RowConverter rc((size_t)n * m->n_in);
+        e = send_rows(m, rc, x, nullptr, n, B, m->X);
+    }
+    if (e != cudaSuccess) return mlp_fail(m, "gradients", e);
+    cudaMemsetAsync(m->t, 0, (size_t)B * 4, m->s);
+    cudaMemcpyAsync(m->t, t, (size_t)n * 4, cudaMemcpyHostToDevice, m->s);
+    mlp_backward(m, m->X, m->t, n, m->loss);
     cudaMemcpyAsync(grad, m->G, m->np * 4, cudaMemcpyDeviceToHost, m->s);
     if (loss) cudaMemcpyAsync(loss, m->loss, 4, cudaMemcpyDeviceToHost, m->s);
-    cudaError_t e = cudaStreamSynchronize(m->s);
+    e = cudaStreamSynchronize(m->s);
     if (e != cudaSuccess) return mlp_fail(m, "gradients", e);
     int err = 0;
     cudaMemcpy(&err, m->err, 4, cudaMemcpyDeviceToHost);
@@ -813,7 +1041,7 @@ extern "C" int lcmc_mlp_get_params(lcmc_mlp *m, float *params)
 extern "C" int lcmc_mlp_set_params(lcmc_mlp *m, const float *params)
 {
     if (!m || !params) return LCMC_EINVAL;
-    cudaError_t e = cudaMemcpy(m->P, params, m->np * 4, cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMemcpyAsync(m->P, params, m->np * 4, cudaMemcpyHostToDevice, m->s);
     if (e != cudaSuccess) return mlp_fail(m, "set_params", e);
     k_weights_bf16<<<256, 256, 0, m->s>>>(m->W1, m->W1b, nullptr, m->hid, m->k1);
     k_weights_bf16<<<64, 256, 0, m->s>>>(m->W2, m->W2b, m->W2bT, m->hid, m->hid);
@@ -821,17 +1049,35 @@ extern "C" int lcmc_mlp_set_params(lcmc_mlp *m, const float *params)
     return e == cudaSuccess ? LCMC_OK : mlp_fail(m, "set_params", e);
 }
 
+// The rows cross the link once: the first epoch sends each batch's and, if there
+// are more epochs, keeps them on the device in the order in which it took them;
+// the later epochs gather from there.  Rows that would take more than
+// TRAIN_KEEP_BYTES, or for which there is no room, are sent in every epoch.
+// Nothing waits for a step: the losses stay on the device until the last one.
+constexpr size_t TRAIN_KEEP_BYTES = (size_t)1 << 30;
+
 extern "C" int lcmc_mlp_train(lcmc_mlp *m, const float *x, const float *t, int n, int epochs, int batch, float lr,
                               uint64_t seed, float *final_loss)
 {
     if (!m || !x || !t || n <= 0 || epochs <= 0 || batch <= 0 || batch > m->bmax) return LCMC_EINVAL;
-    std::vector<int> idx(n);
+    std::vector<int> idx(n), at(n); // a batch's rows; their places on the device
     for (int i = 0; i < n; i++) idx[i] = i;
-    std::vector<float> bx((size_t)batch * m->n_in), bt(batch);
     uint32_t key[2];
     seed_key(seed, key);
-    float last = 0.0f;
-    for (int ep = 0; ep < epochs; ep++) {
+    const int nb = n / batch, used = nb * batch, B = (batch + 127) / 128 * 128, K1 = m->k1;
+    std::vector<float> et(n), losses(std::max(nb, 1));
+    std::vector<int> place(n);
+    cudaError_t e = grow(&m->et, &m->et_n, (size_t)n);
+    if (e == cudaSuccess) e = grow(&m->losses, &m->losses_n, losses.size());
+    if (e != cudaSuccess) return mlp_fail(m, "train", e);
+    bool keep = epochs > 1 && nb > 0 && (size_t)n * K1 * 2 <= TRAIN_KEEP_BYTES;
+    if (keep && (grow(&m->pos, &m->pos_n, (size_t)n) != cudaSuccess ||
+                 grow(&m->rows, &m->rows_n, (size_t)n * K1) != cudaSuccess)) {
+        cudaGetLastError();
+        keep = false;
+    }
+    RowConverter rc((size_t)n * m->n_in);
+    for (int ep = 0; ep < epochs && e == cudaSuccess && nb > 0; ep++) {
         for (int i = n - 1; i > 0; i--) { // shuffle
             U4 o = draw(key, (uint32_t)i, (uint64_t)ep, 0x301u);
             int j = (int)(o.x % (uint32_t)(i + 1));
@@ -839,25 +1085,44 @@ extern "C" int lcmc_mlp_train(lcmc_mlp *m, const float *x, const float *t, int n
             idx[i] = idx[j];
             idx[j] = tmp;
         }
-        double acc = 0.0;
-        int nb = 0;
-        for (int off = 0; off + batch <= n; off += batch) {
-            for (int r = 0; r < batch; r++) {
-                memcpy(&bx[(size_t)r * m->n_in], x + (size_t)idx[off + r] * m->n_in, sizeof(float) * m->n_in);
-                bt[r] = t[idx[off + r]];
-            }
-            float l = 0.0f;
-            mlp_step(m, bx.data(), bt.data(), batch, lr, &l);
-            cudaError_t e = cudaStreamSynchronize(m->s);
-            if (e != cudaSuccess) return mlp_fail(m, "train", e);
-            acc += l;
-            nb++;
+        const bool gather = ep > 0 && keep;
+        for (int i = 0; i < n; i++) {
+            et[i] = t[idx[i]];
+            if (ep == 0) place[idx[i]] = i;
+            at[i] = place[idx[i]];
         }
-        last = nb ? (float)(acc / nb) : 0.0f;
+        // (pageable memory: the copies have left it when the calls return)
+        e = cudaMemcpyAsync(m->et, et.data(), (size_t)n * 4, cudaMemcpyHostToDevice, m->s);
+        if (e == cudaSuccess && gather) e = cudaMemcpyAsync(m->pos, at.data(), (size_t)n * 4, cudaMemcpyHostToDevice, m->s);
+        for (int k = 0; k < nb && e == cudaSuccess; k++) {
+            const int off = k * batch;
+            if (gather) {
+                k_gather_rows<<<512, 256, 0, m->s>>>(m->rows, m->pos + off, m->X, batch, K1);
+                if (B > batch)
+                    e = cudaMemsetAsync(m->X + (size_t)batch * K1, 0, (size_t)(B - batch) * K1 * 2, m->s);
+            } else {
+                e = send_rows(m, rc, x, idx.data() + off, batch, B, m->X);
+                if (e == cudaSuccess && keep)
+                    e = cudaMemcpyAsync(m->rows + (size_t)off * K1, m->X, (size_t)batch * K1 * 2,
+                                        cudaMemcpyDeviceToDevice, m->s);
+            }
+            if (e != cudaSuccess) break;
+            mlp_backward(m, m->X, m->et + off, batch, m->losses + k);
+            mlp_update(m, lr);
+        }
+        if (ep == 0 && keep && e == cudaSuccess && used < n) // rows that no batch of the first epoch took
+            e = send_rows(m, rc, x, idx.data() + used, n - used, n - used, m->rows + (size_t)used * K1);
     }
+    if (e == cudaSuccess && nb > 0)
+        e = cudaMemcpyAsync(losses.data(), m->losses, (size_t)nb * 4, cudaMemcpyDeviceToHost, m->s);
+    const cudaError_t es = cudaStreamSynchronize(m->s);
+    if (e == cudaSuccess) e = es;
+    if (e != cudaSuccess) return mlp_fail(m, "train", e);
+    double acc = 0.0; // the last epoch's
+    for (int k = 0; k < nb; k++) acc += losses[k];
     int err = 0;
     cudaMemcpy(&err, m->err, 4, cudaMemcpyDeviceToHost);
-    if (final_loss) *final_loss = last;
+    if (final_loss) *final_loss = nb ? (float)(acc / nb) : 0.0f;
     return err ? LCMC_ETIMEOUT : LCMC_OK;
 }
 

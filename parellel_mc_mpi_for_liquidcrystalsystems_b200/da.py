@@ -52,7 +52,8 @@ class Surrogate:
         squared loss."""
         y = np.asarray(slope, dtype=np.float64)
         keep = np.isfinite(y) & (np.abs(y) <= max_abs)
-        x = np.ascontiguousarray(np.asarray(x)[keep], dtype=np.float32)
+        x = np.asarray(x)
+        x = np.ascontiguousarray(x if keep.all() else x[keep], dtype=np.float32)
         y = y[keep]
         if len(y) == 0:
             raise ValueError("no training sample with |slope| <= max_abs")
