@@ -674,6 +674,18 @@ extern "C" int lcmc_mlp_destroy(lcmc_mlp *m)
     return LCMC_OK;
 }
 
+template <typename T>
+static cudaError_t grow(T **p, size_t *have, size_t want)
+{
+    if (want <= *have) return cudaSuccess;
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+    *have = 0;
+    cudaError_t e = cudaMalloc((void **)p, want * sizeof(T));
+    if (e == cudaSuccess) *have = want;
+    return e;
+}
+
 // Weights: uniform(-a, a) with a = sqrt(6 / (fan_in + fan_out)) (Glorot & Bengio
 // 2010), from Philox so that a seed fixes the network.
 extern "C" int lcmc_mlp_create(int n_in, int hidden, int max_batch, uint64_t seed, lcmc_mlp **out)
@@ -731,6 +743,9 @@ extern "C" int lcmc_mlp_create(int n_in, int hidden, int max_batch, uint64_t see
     e = cudaMallocHost((void **)&m->stage, (size_t)lcmc_mlp::SLOTS * lcmc_mlp::STAGE_ROWS * K1 * 2);
     for (cudaEvent_t &ev : m->sent)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = grow(&m->yall, &m->yall_n, (size_t)1 << 16);
+    if (e == cudaSuccess) e = grow(&m->et, &m->et_n, (size_t)1 << 16);
+    if (e == cudaSuccess) e = grow(&m->losses, &m->losses_n, (size_t)1 << 10);
     if (e != cudaSuccess) {
         lcmc_mlp_destroy(m);
         return LCMC_ENOMEM;
@@ -933,18 +948,6 @@ static cudaError_t send_rows(lcmc_mlp *m, RowConverter &rc, const float *x, cons
     }
     if (B > n) return cudaMemsetAsync((char *)dst + (size_t)n * row, 0, (size_t)(B - n) * row, m->s);
     return cudaSuccess;
-}
-
-template <typename T>
-static cudaError_t grow(T **p, size_t *have, size_t want)
-{
-    if (want <= *have) return cudaSuccess;
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-    *have = 0;
-    cudaError_t e = cudaMalloc((void **)p, want * sizeof(T));
-    if (e == cudaSuccess) *have = want;
-    return e;
 }
 
 extern "C" int lcmc_mlp_predict(lcmc_mlp *m, const float *x, int n, float *y)

@@ -16,6 +16,7 @@
 #include "lcmc_gb.cuh"
 #include "lcmc_internal.h"
 #include "lcmc_rng.cuh"
+#include "lcmc_tc.cuh"
 #include "lcmc_trial.cuh"
 #include "lcmc_volume_cells.cuh"
 
@@ -125,7 +126,7 @@ __device__ __forceinline__ void cell_stencil(const DevView &v, CellView &c, int 
 //                   trial state through a compacted list with all lanes busy,
 //                   then the lane sums of the canonical order as far as they do
 //                   not depend on a decision;
-//   k_exact_decide  warp per cell: for each attempt in ascending id, the lane
+//   k_exact_decide  block per cell: for each attempt in ascending id, the lane
 //                   sums completed with the chosen in-cell terms and the static
 //                   terms after them, the xor butterfly, the Metropolis test.
 // The order of every FP64 addition is the canonical one (lane q mod 32 adds the
@@ -138,7 +139,8 @@ __device__ __forceinline__ void cell_stencil(const DevView &v, CellView &c, int 
 //   1            sums over the static slots before the own cell
 //   2 .. 1+J     own-cell slots, partner in its old state (J chunks of 32 slots)
 //   2+J .. 1+2J  own-cell slots, partner in its trial state
-//   2+2J ..      the lane's static terms after the own cell, in order (nsuf rows)
+//   2+2J ..      the lane's static terms after the own cell, in order (nsuf rows, a
+//                multiple of four; zeros at the end)
 // The records of a phase lie in a scratch of ex_cap rows; a phase with more is
 // run in ex_nb batches of cells.  A cell above a capacity (particles, stencil,
 // in-cutoff terms, terms after the own cell in one lane) is attempted by
@@ -149,7 +151,6 @@ constexpr int EX_CH = 96;    // chunks of 32 stencil slots
 constexpr int EX_ENT = 640;  // in-cutoff terms of a particle
 constexpr int EX_SUF = 12;   // static terms after the own cell, per lane
 constexpr int EX_J = 9;      // most chunks an own cell touches
-constexpr int EX_PFS = 6;    // of the suffix rows, those fetched ahead
 
 // chunks of 32 slots that na consecutive slots can touch, rounded up to a class
 // (2, 3, 5, 9) the decisions are unrolled for (chunks beyond the cell's are empty)
@@ -431,9 +432,10 @@ __global__ void __launch_bounds__(128) k_exact_terms(const __grid_constant__ Dev
             if (nsuf > EX_SUF) {
                 if (lane == 0) v.ex_flag[(size_t)ci * v.ex_act + a] = 1;
             } else {
-                for (int s = ns; s < nsuf; s++) suf[(size_t)s * 32 + lane] = make_double2(0.0, 0.0);
+                const int nsuf4 = (nsuf + 3) & ~3; // the decisions take them four at a time
+                for (int s = ns; s < nsuf4; s++) suf[(size_t)s * 32 + lane] = make_double2(0.0, 0.0);
                 if (lane == 0) {
-                    hd->nsuf = nsuf;
+                    hd->nsuf = nsuf4;
                     hd->nstat = s_nstat;
                 }
             }
@@ -541,26 +543,282 @@ __device__ __noinline__ void exact_cell_sequential(const DevView *__restrict__ v
     __syncwarp();
 }
 
+// The attempts of one cell (J chunks of own-cell slots), D = 3 at a time: attempt
+// k + d depends on the outcomes of k .. k + d - 1, so a warp evaluates it for
+// each of their 2^d patterns (2^D - 1 warps), and every warp then follows the
+// outcomes through the decisions.  What a warp does is what one alone would do
+// per attempt: a dozen additions, the butterfly, the test, all of it latency, so
+// three attempts take the time of one plus a barrier.  The records come from L2
+// by bulk copies, a round ahead.  A cell of 125 particles: 58 us with one warp,
+// 31 us; 15 warps for four attempts 33 us, three warps with 1, 2 and 4 chains
+// each 46 us (the instructions of a warp count, not its waits).
+constexpr int EX_SMS = 148;
+constexpr int EX_DEPTH = 3, EX_WARPS = 8; // attempts of a round and the warps of a block (the eighth is a double)
+template <int J> struct ExactStage {
+    static constexpr int PF = 2 + 2 * J + EX_SUF;      // rows copied per attempt
+    static constexpr int D = J <= 5 ? EX_DEPTH : 2;    // attempts of a round
+    static constexpr int BYTES = 2 * D * PF * 32 * 16; // this round's records and the next one's
+};
+constexpr int ex_max(int a, int b) { return a > b ? a : b; }
+constexpr int EX_BYTES = ex_max(ex_max(ExactStage<2>::BYTES, ExactStage<3>::BYTES),
+                                ex_max(ExactStage<5>::BYTES, ExactStage<EX_J>::BYTES));
+
+constexpr unsigned EX_WAIT_TRIES = 1u << 24; // mbarrier tries before a block gives up
+
+struct ExactShared {
+    uint64_t full[2];       // mbarriers: a half's records have landed
+    double dE[EX_NA];       // energy change of an accepted attempt, else 0
+    int failed;             // a copy did not land
+    unsigned pairs[EX_WARPS], hard[EX_WARPS];
+    CellView c;
+    int first[27], base[28];
+};
+
+// false: a copy did not land (the flag is set)
+template <int J>
+__device__ __forceinline__ bool exact_decide_cell(const DevView &v, const CellView &c, int q13, const double2 *rows,
+                                                  double2 *buf, ExactShared &sh, unsigned &phase)
+{
+    constexpr int PF = ExactStage<J>::PF, RPP = 2 + 2 * J + EX_SUF, D = ExactStage<J>::D, W = (1 << D) - 1;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const Replica &p = v.rep[c.r];
+    const int na = c.na, c0 = q13 >> 5;
+    const double beta = p.k.beta;
+    const bool coll = p.k.coll_on;
+    // warp w: the attempt at depth wd of a round, for the pattern wh of outcomes before it (the eighth as the seventh)
+    const int wi = min(w, W - 1), wd = 31 - __clz(wi + 1), wh = wi + 1 - (1 << wd);
+    // lanes of this warp that report its decision: the block's count is then the decisions' bits, 1 << w for warp w
+    const bool report = w < W - (W == 7) ? lane < (1 << w) : W == 7;
+    auto fetch = [&](int k0, int half) { // attempts k0 .. k0 + D - 1
+        const int n = min(D, na - k0);
+        if (t != EX_WARPS * 32 - 32 || n <= 0) return;
+        tc::fence_proxy_async_smem(); // the block's reads of the records there came before its barrier
+        tc::mbar_arrive_expect_tx(&sh.full[half], (uint32_t)n * (PF * 512));
+        for (int d = 0; d < n; d++)
+            tc::bulk_load(buf + (half * D + d) * (PF * 32), rows + (size_t)(k0 + d) * RPP * 32, PF * 512, &sh.full[half]);
+    };
+    fetch(0, 0);
+    fetch(D, 1);
+    bool ok = true;
+    if (na > 0) { // (uniform; an empty cell copies nothing)
+        ok = tc::mbar_wait_bounded(&sh.full[0], phase & 1u, EX_WAIT_TRIES);
+        phase ^= 1u;
+    }
+    if (!ok) sh.failed = 1;
+    __syncthreads();
+    ok = !sh.failed;
+    unsigned accm = 0u; // bit j: the particle at slot 32 (c0 + j) + lane was accepted
+    int half = 0;
+    for (int k0 = 0; k0 < na && ok; k0 += D, half ^= 1) {
+        const int k = k0 + wd, q0 = q13 + k0;
+        const int mine = (lane - q0) & 31, jm = ((q0 + mine) >> 5) - c0; // this lane's slot is the round's mine-th
+        double dE = 0.0, lu = 0.0;
+        bool acc = false;
+        if (w < EX_WARPS && k < na) {
+            const unsigned am = accm | ((unsigned)((wh >> mine) & 1) << jm); // with the pattern
+            const double2 *rw = buf + (half * D + wd) * (PF * 32) + lane;
+            const ExactHead *hd = reinterpret_cast<const ExactHead *>(rw - lane);
+            struct { double lu; int code, nsuf; } h; // one load
+            static_assert(offsetof(ExactHead, lu) == 16 && offsetof(ExactHead, code) == 24 && offsetof(ExactHead, nsuf) == 28, "layout");
+            *reinterpret_cast<int4 *>(&h) = *reinterpret_cast<const int4 *>(&hd->lu);
+            lu = h.lu;
+            if (!h.code) {
+                double2 x[J], y[4];
+                double po = rw[32].x, pn = rw[32].y;
+#pragma unroll
+                for (int j = 0; j < J; j++) x[j] = rw[(2 + j) * 32 + ((am >> j) & 1u) * (J * 32)];
+#pragma unroll
+                for (int j = 0; j < J; j++) {
+                    po += x[j].x;
+                    pn += x[j].y;
+                }
+#pragma unroll
+                for (int s0 = 0; s0 < EX_SUF; s0 += 4) {
+                    if (s0 >= h.nsuf) break; // (uniform)
+#pragma unroll
+                    for (int s = 0; s < 4; s++) y[s] = rw[(2 + 2 * J + s0 + s) * 32];
+#pragma unroll
+                    for (int s = 0; s < 4; s++) {
+                        po += y[s].x;
+                        pn += y[s].y;
+                    }
+                }
+                // the butterfly of both sums: the first level leaves the old state's to the lower lanes and the trial
+                // state's to the upper ones (the additions are those of two butterflies)
+                const bool up = lane & 16;
+                double e = (up ? pn : po) + __shfl_xor_sync(0xffffffffu, up ? po : pn, 16);
+#pragma unroll
+                for (int o = 8; o >= 1; o >>= 1) e = e + __shfl_xor_sync(0xffffffffu, e, o);
+                if (coll) e = e + (up ? hd->un : hd->uo);
+                const double other = __shfl_xor_sync(0xffffffffu, e, 16);
+                dE = up ? e - other : other - e;
+                acc = (dE <= 0.0) || (lu <= -beta * dE);
+            }
+        }
+        if (w == EX_WARPS - 1 && k0 + D < na) { // the next round's records
+            if (!tc::mbar_wait_bounded(&sh.full[half ^ 1], (phase >> (half ^ 1)) & 1u, EX_WAIT_TRIES)) sh.failed = 1;
+        }
+        if (k0 + D < na) phase ^= 1u << (half ^ 1);
+        const int m = __syncthreads_count(acc && report); // bit w: warp w's attempt was accepted
+        fetch(k0 + 2 * D, half);                          // over this round's
+        const int a0 = m & 1, a1 = (m >> (1 + a0)) & 1, h2 = a0 | (a1 << 1);
+        const int hist = D == 2 ? h2 : h2 | (((m >> (3 + h2)) & 1) << 2); // bit d: attempt k0 + d was accepted
+        accm |= (unsigned)((hist >> mine) & 1) << jm;
+        if (w < W && k < na && wh == (hist & ((1 << wd) - 1)) && lane == 0) { // this warp's pattern came about
+            sh.dE[k] = (hist >> wd) & 1 ? dE : 0.0;
+            if (v.rec_dE) {
+                const int id = v.id[c.cs + k];
+                v.rec_dE[p.p_off + id] = dE;
+                v.rec_lu[p.p_off + id] = lu;
+            }
+        }
+        ok = !sh.failed;
+    }
+    if (!ok) { // (uniform) copies still on their way are waited for, again with a limit
+        __syncthreads();
+        if (t == 0) atomicOr(&v.stats[c.r].flags, F_TIMEOUT);
+        tc::mbar_wait_bounded(&sh.full[0], phase & 1u, EX_WAIT_TRIES);
+        tc::mbar_wait_bounded(&sh.full[1], (phase >> 1) & 1u, EX_WAIT_TRIES);
+        return false;
+    }
+    // a lane per particle: outcome, accepted trial state to the master arrays, and the pairs its attempt met
+    // (the partners before it that were accepted in their trial state, every other in its old one)
+    unsigned A[J]; // accepted slots of chunk c0 + j
+#pragma unroll
+    for (int j = 0; j < J; j++) A[j] = __ballot_sync(0xffffffffu, (accm >> j) & 1u);
+    unsigned npairs = 0u, nhard = 0u;
+    for (int k = 32 * w + lane; k < na; k += 32 * EX_WARPS) {
+        const int q = q13 + k, g = c.cs + k;
+        const ExactHead *hd = reinterpret_cast<const ExactHead *>(rows + (size_t)k * RPP * 32);
+        const int code = hd->code, id = v.id[g];
+        unsigned mk[4][J];
+        int np = 0;
+        if (!code) {
+            np = hd->nstat;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < J; j++) mk[i][j] = hd->mask[i][j];
+        }
+        bool acc = false;
+#pragma unroll
+        for (int j = 0; j < J; j++)
+            if ((q >> 5) - c0 == j) acc = (A[j] >> (q & 31)) & 1u;
+        v.outcome[p.p_off + id] = code == 1 ? 2 : (acc ? 1 : 0);
+        if (acc) {
+            v.px[g] = v.tnx[g];
+            v.py[g] = v.tny[g];
+            v.pz[g] = v.tnz[g];
+            v.ox[g] = v.tux[g];
+            v.oy[g] = v.tuy[g];
+            v.oz[g] = v.tuz[g];
+        }
+        if (!code) {
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                const int d = q - 32 * (c0 + j); // slots of this chunk before the particle's own
+                const unsigned B = d <= 0 ? 0u : (d >= 32 ? A[j] : A[j] & ((1u << d) - 1u));
+                np += __popc((mk[0][j] & ~B) | (mk[2][j] & B)) + __popc((mk[1][j] & ~B) | (mk[3][j] & B));
+            }
+        }
+        npairs += (unsigned)np;
+        nhard += code == 1;
+    }
+    npairs = __reduce_add_sync(0xffffffffu, npairs);
+    nhard = __reduce_add_sync(0xffffffffu, nhard);
+    if (lane == 0) sh.pairs[w] = npairs, sh.hard[w] = nhard;
+    __syncthreads();
+    if (t == 0) {
+        unsigned long long n = 0ull;
+        int nh = 0, nacc = 0;
+        for (int i = 0; i < EX_WARPS; i++) n += sh.pairs[i], nh += sh.hard[i];
+#pragma unroll
+        for (int j = 0; j < J; j++) nacc += __popc(A[j]);
+        double dE_sum = 0.0, dE_abs = 0.0; // in the attempts' order (0 for those that were not accepted)
+#pragma unroll 8
+        for (int k = 0; k < na; k++) {
+            dE_sum += sh.dE[k];
+            dE_abs += fabs(sh.dE[k]);
+        }
+        v.cell_e0[c.cell] = dE_sum;
+        v.cell_abs[c.cell] = dE_abs;
+        v.cell_fp64[c.cell] = 0;
+        v.cell_n0[c.cell] = nacc;
+        v.cell_n1[c.cell] = nh;
+        v.cell_pairs[c.cell] = n;
+        v.cell_cands[c.cell] = (unsigned long long)(c.total - 1) * (unsigned long long)na;
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(EX_WARPS * 32) k_exact_decide(const __grid_constant__ DevView v, int ci, int b)
+{
+    extern __shared__ double2 ex_buf[]; // [2][D][PF][32]
+    __shared__ ExactShared sh;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        tc::mbar_init(&sh.full[0], 1);
+        tc::mbar_init(&sh.full[1], 1);
+        sh.failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    unsigned phase = 0u; // bit h: parity of full[h]'s next completion
+    const int *off = v.act_off + ci * (v.R + 1);
+    const long long *er = v.ex_r + (size_t)ci * (v.ex_act + 1);
+    const ExactBatch eb = exact_batch(v, off, er, b);
+    const int a1 = b == v.ex_nb - 1 ? off[v.r_hi] : eb.hi; // the last batch takes the cells beyond the scratch
+    for (int a = eb.lo + blockIdx.x; a < a1; a += gridDim.x) {
+        __syncthreads(); // the cell before this one is done with the shared memory
+        if (threadIdx.x < 32) {
+            CellView c;
+            active_cell(v, off, ci, a, c);
+            if (!v.rep[c.r].use_fast) cell_stencil(v, c, lane, sh.first, sh.base);
+            if (lane == 0) sh.c = c;
+        }
+        __syncthreads();
+        const CellView c = sh.c;
+        if (v.rep[c.r].use_fast) continue;
+        if (a >= eb.hi || v.ex_flag[(size_t)ci * v.ex_act + a]) {
+            if (threadIdx.x < 32) exact_cell_sequential(&v, c, lane, sh.first, sh.base);
+            continue;
+        }
+        const double2 *rows = v.ex_rows + (size_t)(er[a] - eb.row0) * 32;
+        const int q13 = sh.base[c.own];
+        bool ok;
+        switch (ex_chunks(c.na)) {
+        case 2: ok = exact_decide_cell<2>(v, c, q13, rows, ex_buf, sh, phase); break;
+        case 3: ok = exact_decide_cell<3>(v, c, q13, rows, ex_buf, sh, phase); break;
+        case 5: ok = exact_decide_cell<5>(v, c, q13, rows, ex_buf, sh, phase); break;
+        default: ok = exact_decide_cell<EX_J>(v, c, q13, rows, ex_buf, sh, phase); break;
+        }
+        if (!ok) return; // (uniform)
+    }
+}
+
 __device__ __forceinline__ void cp_row_async(void *dst, const void *src)
 {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
-// The attempts of one cell (J chunks of own-cell slots).  The records come from
-// L2, EX_STAGES - 1 attempts ahead (cp.async, fully unrolled: one warp runs
-// here, so every instruction of an attempt is latency); what remains is the
-// chain of one attempt: a dozen additions, the butterfly, the test.
+// The attempts of one cell by one warp, for phases with more cells than the chip
+// has SMs: several such blocks share an SM, and evaluating only what is needed
+// costs less than the patterns (262,144 particles: 6.3 ms of phases per sweep,
+// 7.0 ms with a block of eight warps per cell).  Records EX_STAGES - 1 attempts
+// ahead (cp.async), of the suffix rows EX_PFS.
+constexpr int EX_PFS = 6;
 constexpr int EX_STAGES = 4;
-template <int J> struct ExactStage {
+template <int J> struct ExactPipe {
     static constexpr int PF = 2 + 2 * J + EX_PFS; // rows fetched per attempt
 };
 
+constexpr int EX_PIPE_BYTES = EX_STAGES * ExactPipe<EX_J>::PF * 32 * 16;
+
 template <int J>
-__device__ __forceinline__ void exact_decide_cell(const DevView &v, const CellView &c, int lane, int q13,
+__device__ __forceinline__ void exact_decide_cell_warp(const DevView &v, const CellView &c, int lane, int q13,
                                                   const double2 *rows, double2 *buf)
 {
-    constexpr int PF = ExactStage<J>::PF, RPP = 2 + 2 * J + EX_SUF;
+    constexpr int PF = ExactPipe<J>::PF, RPP = 2 + 2 * J + EX_SUF;
     const Replica &p = v.rep[c.r];
     const int na = c.na, c0 = q13 >> 5;
     const double beta = p.k.beta;
@@ -692,7 +950,7 @@ __device__ __forceinline__ void exact_decide_cell(const DevView &v, const CellVi
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(32) k_exact_decide(const __grid_constant__ DevView v, int ci, int b)
+__global__ void __launch_bounds__(32) k_exact_decide_warp(const __grid_constant__ DevView v, int ci, int b)
 {
     extern __shared__ double2 ex_buf[]; // [EX_STAGES][PF][32]
     __shared__ int s_first[27], s_base[28];
@@ -713,10 +971,10 @@ __global__ void __launch_bounds__(32) k_exact_decide(const __grid_constant__ Dev
         const double2 *rows = v.ex_rows + (size_t)(er[a] - eb.row0) * 32;
         const int q13 = s_base[c.own];
         switch (ex_chunks(c.na)) {
-        case 2: exact_decide_cell<2>(v, c, lane, q13, rows, ex_buf); break;
-        case 3: exact_decide_cell<3>(v, c, lane, q13, rows, ex_buf); break;
-        case 5: exact_decide_cell<5>(v, c, lane, q13, rows, ex_buf); break;
-        default: exact_decide_cell<EX_J>(v, c, lane, q13, rows, ex_buf); break;
+        case 2: exact_decide_cell_warp<2>(v, c, lane, q13, rows, ex_buf); break;
+        case 3: exact_decide_cell_warp<3>(v, c, lane, q13, rows, ex_buf); break;
+        case 5: exact_decide_cell_warp<5>(v, c, lane, q13, rows, ex_buf); break;
+        default: exact_decide_cell_warp<EX_J>(v, c, lane, q13, rows, ex_buf); break;
         }
     }
 }
@@ -908,19 +1166,21 @@ void exact_scratch_size(int ntot, long long *cap, long long *alloc, int *nb)
 
 void exact_init()
 {
-    cudaFuncSetAttribute(k_exact_decide, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         EX_STAGES * ExactStage<EX_J>::PF * 32 * (int)sizeof(double2));
+    cudaFuncSetAttribute(k_exact_decide, cudaFuncAttributeMaxDynamicSharedMemorySize, EX_BYTES);
+    cudaFuncSetAttribute(k_exact_decide_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, EX_PIPE_BYTES);
 }
 
 void launch_exact_offsets(const DevView &v, cudaStream_t s) { k_exact_offsets<<<v.nphase, 1024, 0, s>>>(v); }
 
 void launch_phase_exact(const DevView &v, cudaStream_t s, int ci, int grid)
 {
-    const int bytes = EX_STAGES * ExactStage<EX_J>::PF * 32 * (int)sizeof(double2);
     const int gt = min(4 * grid, v.ntot), gd = min(grid, v.ex_act);
     for (int b = 0; b < v.ex_nb; b++) {
         k_exact_terms<<<gt, 128, 0, s>>>(v, ci, b);
-        k_exact_decide<<<gd, 32, bytes, s>>>(v, ci, b);
+        // up to a cell per SM the patterns' warps are idle ones: 1000 particles (one active cell or eight) 0.655 ->
+        // 0.48 ms of phases per sweep, 8192 (27) 0.51 -> 0.465; 65,536 (343) would take 1.72 instead of 1.50
+        if (v.ex_act <= EX_SMS) k_exact_decide<<<gd, EX_WARPS * 32, EX_BYTES, s>>>(v, ci, b);
+        else k_exact_decide_warp<<<gd, 32, EX_PIPE_BYTES, s>>>(v, ci, b);
     }
 }
 

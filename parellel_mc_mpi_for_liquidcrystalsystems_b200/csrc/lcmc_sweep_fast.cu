@@ -316,14 +316,6 @@ __device__ __forceinline__ double warp_sum2(double a, double b, int lane)
     return x;
 }
 
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, uint64_t *bar)
-{
-    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     tc::smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(tc::smem_u32(bar))
-                 : "memory");
-}
-
 // One warp: the stencil of active cell `rec`, and the places of its 26 static
 // cells' copies in shared memory.  Cells that cannot run here are marked.
 template <typename ST, int AMAX, int CCAP>
@@ -384,8 +376,8 @@ __device__ __forceinline__ void copy_static(const DevView &v, SM &sm, int which,
     __syncwarp();
     if (n > 0) {
         const int pos = st.pos[lane] & ~1, from = start & ~1;
-        bulk_load(&sm.cpos[pos], v.cl4 + from, (unsigned)n * 16u, &sm.full);
-        bulk_load(&sm.cori[pos], v.cl2 + from, (unsigned)n * 8u, &sm.full);
+        tc::bulk_load(&sm.cpos[pos], v.cl4 + from, (unsigned)n * 16u, &sm.full);
+        tc::bulk_load(&sm.cori[pos], v.cl2 + from, (unsigned)n * 8u, &sm.full);
     }
 }
 

@@ -97,6 +97,16 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr)
     return d;
 }
 
+// Copy of `bytes` (a multiple of 16, from and to 16-byte boundaries) into shared
+// memory, completing on the mbarrier's transaction count.
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
 // ---- TMA (no multicast) ----
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes)
 {
