@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(256) k_chunk_sums(DevView v, const double *e0,
     const int c = blockIdx.x, r = blockIdx.y;
     const Replica &p = v.rep[r];
     if ((MODE == 1 || MODE == 3) && (p.ensemble != 2 || p.vol_stage1 == 0)) return;
+    if (MODE == 3 && !cells_serve<1>(p)) return; // a box below the FP32 kernel's four cells: no screen, no sums
     const bool cells = use_cells && by_cells<MODE>(p);
     const int n = cells ? p.nc[0] * p.nc[1] * p.nc[2] : p.n, off = cells ? p.cell_off : p.p_off;
     const int i0 = c * LCMC_RED_CHUNK;
