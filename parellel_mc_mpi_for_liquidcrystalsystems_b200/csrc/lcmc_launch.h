@@ -6,6 +6,38 @@
 
 namespace lcmc {
 
+// Launch of a kernel of the FP64 colour phases.  The next such kernel in the
+// stream may be launched while this one runs: each calls phase_begin() first,
+// which waits until all that came before it in the stream is complete and
+// visible, so only the launch itself overlaps (8192 particles, 27 phases of two
+// kernels: 0.465 -> 0.350 ms per sweep).  The FP32 phase kernels gained 1 % from
+// it in small systems and lost 4 % in batches, where the early blocks of the
+// hand-over kernel took the other streams' shared memory: they are launched
+// plainly.
+template <typename... P, typename... A>
+inline void launch_phase(void (*f)(P...), int grid, int block, int smem, cudaStream_t s, const A &...a)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, f, P(a)...);
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void phase_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 // lcmc_rebin.cu
 void launch_rebin(const DevView &v, cudaStream_t s, int grid);
 // per-cell results of the colour phases into the statistics and the running

@@ -15,6 +15,7 @@
 
 #include "lcmc_gb.cuh"
 #include "lcmc_internal.h"
+#include "lcmc_launch.h"
 #include "lcmc_rng.cuh"
 #include "lcmc_tc.cuh"
 #include "lcmc_trial.cuh"
@@ -255,6 +256,7 @@ __device__ __forceinline__ ExactBatch exact_batch(const DevView &v, const int *o
 
 __global__ void __launch_bounds__(128) k_exact_terms(const __grid_constant__ DevView v, int ci, int b)
 {
+    phase_begin();
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const unsigned lt = (1u << lane) - 1u;
     __shared__ int s_first[27], s_base[28];
@@ -754,6 +756,7 @@ __device__ __forceinline__ bool exact_decide_cell(const DevView &v, const CellVi
 __global__ void __launch_bounds__(EX_WARPS * 32) k_exact_decide(const __grid_constant__ DevView v, int ci, int b)
 {
     extern __shared__ double2 ex_buf[]; // [2][D][PF][32]
+    phase_begin();
     __shared__ ExactShared sh;
     const int lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -953,6 +956,7 @@ __device__ __forceinline__ void exact_decide_cell_warp(const DevView &v, const C
 __global__ void __launch_bounds__(32) k_exact_decide_warp(const __grid_constant__ DevView v, int ci, int b)
 {
     extern __shared__ double2 ex_buf[]; // [EX_STAGES][PF][32]
+    phase_begin();
     __shared__ int s_first[27], s_base[28];
     const int lane = threadIdx.x;
     const int *off = v.act_off + ci * (v.R + 1);
@@ -1145,7 +1149,6 @@ __global__ void __launch_bounds__(128, LCMC_ENERGY_MIN_BLOCKS) k_energy_exact(De
 
 } // namespace lcmc
 
-#include "lcmc_launch.h"
 
 namespace lcmc {
 
@@ -1176,11 +1179,11 @@ void launch_phase_exact(const DevView &v, cudaStream_t s, int ci, int grid)
 {
     const int gt = min(4 * grid, v.ntot), gd = min(grid, v.ex_act);
     for (int b = 0; b < v.ex_nb; b++) {
-        k_exact_terms<<<gt, 128, 0, s>>>(v, ci, b);
+        launch_phase(k_exact_terms, gt, 128, 0, s, v, ci, b);
         // up to a cell per SM the patterns' warps are idle ones: 1000 particles (one active cell or eight) 0.655 ->
         // 0.48 ms of phases per sweep, 8192 (27) 0.51 -> 0.465; 65,536 (343) would take 1.72 instead of 1.50
-        if (v.ex_act <= EX_SMS) k_exact_decide<<<gd, EX_WARPS * 32, EX_BYTES, s>>>(v, ci, b);
-        else k_exact_decide_warp<<<gd, 32, EX_PIPE_BYTES, s>>>(v, ci, b);
+        if (v.ex_act <= EX_SMS) launch_phase(k_exact_decide, gd, EX_WARPS * 32, EX_BYTES, s, v, ci, b);
+        else launch_phase(k_exact_decide_warp, gd, 32, EX_PIPE_BYTES, s, v, ci, b);
     }
 }
 
