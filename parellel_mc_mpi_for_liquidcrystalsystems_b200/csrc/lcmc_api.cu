@@ -102,6 +102,8 @@ struct lcmc_ctx {
     int kernel_override = -1;
     FastChoice fast; // the FP32 phase kernel
     int need_amax = 0; // active-cell capacity the capacity rule asks for
+    int fit = 0;       // blocks per SM of the FP32 phase kernel fit_of
+    FastChoice fit_of;
     int need_min = 0;  // the smallest capacity lcmc_autotune may try: mean + 3 standard deviations of a cell's count
     int tuned_class = -1; // capacity class lcmc_autotune chose (kept while it holds the rule's capacity)
     bool checks_off = false; // no periodic energy checks (autotune trials)
@@ -758,26 +760,47 @@ static bool same_pair_consts(const GBConsts &a, const GBConsts &b)
            a.f_half_chip == b.f_half_chip && a.f_big == b.f_big;
 }
 
-// The shape of the FP32 phase kernel within its capacity class: the light one
-// when no system's rule asks for more than 40 particles per cell, the wide one
-// when a colour phase has at most one active cell per SM (the phase then takes
-// the latency of one cell).
+// The shape of the FP32 phase kernel: the class's own, or the light one when no
+// system's rule asks for more than 40 particles per cell, but one whose arrays
+// hold the neighbour cells' particles (cells are as wide as the box allows, so
+// they can be fuller than the class's liquid): a cell above them is run again by
+// the hand-over kernel, and the phase waits for it, 24 us, as long as the phase
+// itself (30,157 rods, 30 to a cell, 810 candidates in the mean: 0.34 ms of phases
+// per sweep with the class's 780 or 832 places, 0.19 with 1040).  The wide one when a colour
+// phase has at most one active cell per SM (the phase then takes the latency of
+// one cell).
 static void choose_fast_shape(lcmc_ctx *c)
 {
-    long long act = 0;
+    long long act = 0, above[FAST_SHAPES] = {};
     for (int r = 0; r < c->R; r++) {
-        long long cells = 1; // of the largest colour
+        const Replica &rp = c->rep[r];
+        long long cells = 1, all = 1; // of the largest colour; of the box
+        double V = 1.0;
         for (int a = 0; a < 3; a++) {
-            const int nc = grid_dim_host(c->rep[r].L[a], c->rep[r].wmin, c->rep[r].fine);
+            const int nc = grid_dim_host(rp.L[a], rp.wmin, rp.fine);
             cells *= (nc & 1) && nc >= 3 ? (nc + 2) / 3 : (nc + 1) / 2;
+            all *= nc;
+            V *= rp.L[a];
         }
         act += cells;
+        // 26 cells at the density outside the colloid, two (ideal-gas) standard deviations and the copies' padding
+        const double free = std::max(V - 4.18879 * rp.k.coll_R * rp.k.coll_R * rp.k.coll_R, 0.5 * V);
+        const double mean = 26.0 * rp.n / all * V / free, need = mean + 2.0 * std::sqrt(mean) + 20.0;
+        for (int s = 0; s < FAST_SHAPES; s++)
+            if (need > fast_shape_candidates(s)) above[s] += cells;
     }
-    c->fast.light = c->fast.cls == 0 && c->need_amax <= 40;
+    int shape = c->fast.cls == 0 && c->need_amax <= 40 ? 0 : 1 + c->fast.cls;
+    // (a batch keeps a shape that a few of its cells do not fit)
+    while (shape < FAST_SHAPES - 1 && above[shape] * 20 > act) shape++;
+    c->fast.shape = shape;
     c->fast.wide = act <= c->sms;
     // blocks: the fewest per SM that take as many rounds over a phase's cells as the most that fit (fewer
     // neighbours, so each round ends sooner)
-    const int fit = fast_blocks_per_sm(c->fast);
+    if (c->fit == 0 || !c->fast.same_kernel(c->fit_of)) {
+        c->fit = fast_blocks_per_sm(c->fast);
+        c->fit_of = c->fast;
+    }
+    const int fit = c->fit;
     const long long rounds = (act + (long long)fit * c->sms - 1) / ((long long)fit * c->sms);
     int per_sm = fit;
     while (per_sm > 1 && (act + (long long)(per_sm - 1) * c->sms - 1) / ((long long)(per_sm - 1) * c->sms) == rounds)

@@ -64,13 +64,14 @@ struct FastVariant {
 struct FastChoice {
     int cls = 0;        // capacity class
     bool spec21 = true; // mu = 2, nu = 1, sigma0 = 1 and the same pair constants in every replica
-    bool light = false; // class 0 for systems of at most 40 particles per cell
-    bool wide = false;  // 512 threads per cell: fewer active cells than SMs
-    bool operator==(const FastChoice &o) const
-    {
-        return cls == o.cls && spec21 == o.spec21 && light == o.light && wide == o.wide;
-    }
+    int shape = 1;      // block shape: 0 for at most 40 particles per cell, 1 + class by class
+    bool wide = false;  // 512 threads per cell: at most a cell per SM
+    // the same kernel (the class is only a capacity)
+    bool same_kernel(const FastChoice &o) const { return spec21 == o.spec21 && wide == o.wide && shape == o.shape; }
+    bool operator==(const FastChoice &o) const { return cls == o.cls && same_kernel(o); }
 };
+constexpr int FAST_SHAPES = 4;
+int fast_shape_candidates(int shape); // places of the static cells' particles
 int fast_variant_count();
 FastVariant fast_variant(int i);
 void launch_phase_fast(const FastChoice &c, const GBConsts &k, const DevView &v, cudaStream_t s, int ci, int grid);

@@ -1151,6 +1151,14 @@ static const FastVariant kVariants[] = {{48}, {56}, {64}};
 int fast_variant_count() { return (int)(sizeof(kVariants) / sizeof(kVariants[0])); }
 FastVariant fast_variant(int i) { return kVariants[i]; }
 
+static constexpr int shape_candidates(int, int ccap, int) { return ccap; }
+int fast_shape_candidates(int shape)
+{
+    constexpr int n[FAST_SHAPES] = {shape_candidates(FAST40), shape_candidates(FAST48), shape_candidates(FAST56),
+                                    shape_candidates(FAST64)};
+    return n[shape];
+}
+
 template <int NT, int MINB, int AMAX, int CCAP, int LCAP, bool S21>
 struct FastLaunch {
     static constexpr int bytes = (int)sizeof(FastSmem<AMAX, CCAP, LCAP>);
@@ -1174,24 +1182,18 @@ struct FastLaunch {
 // 1.66), sixteen where it has not and a phase takes one cell's latency (32,768
 // rods NPT: 0.19 ms against 0.30 with four).  The light shape holds six blocks
 // per SM where the class's own 48-particle arrays leave five (1.48 against 1.60).
-// The kernel of a variant: class, specialisation (mu = 2, nu = 1, sigma0 = 1, the
-// same pair constants in every replica), light, wide (a block per SM).
+// The kernel of a variant: shape, specialisation (mu = 2, nu = 1, sigma0 = 1, the
+// same pair constants in every replica), wide (a block per SM).
 template <typename F>
 static auto with_variant(const FastChoice &c, F f)
 {
-#define FAST_PICK(...) (c.wide ? f(FastLaunch<512, 1, __VA_ARGS__>()) : f(FastLaunch<FAST_NT, __VA_ARGS__>()))
-#define FAST_NT 128, 6
-    if (c.cls == 0 && c.light) return c.spec21 ? FAST_PICK(FAST40, true) : FAST_PICK(FAST40, false);
-#undef FAST_NT
-#define FAST_NT 128, 5
-    if (c.cls == 0) return c.spec21 ? FAST_PICK(FAST48, true) : FAST_PICK(FAST48, false);
-#undef FAST_NT
-#define FAST_NT 128, 4
-    if (c.cls == 1) return c.spec21 ? FAST_PICK(FAST56, true) : FAST_PICK(FAST56, false);
-#undef FAST_NT
-#define FAST_NT 128, 3
-    return c.spec21 ? FAST_PICK(FAST64, true) : FAST_PICK(FAST64, false);
-#undef FAST_NT
+#define FAST_PICK(MINB, ...)                                                                                           \
+    (c.wide ? (c.spec21 ? f(FastLaunch<512, 1, __VA_ARGS__, true>()) : f(FastLaunch<512, 1, __VA_ARGS__, false>()))    \
+            : (c.spec21 ? f(FastLaunch<128, MINB, __VA_ARGS__, true>()) : f(FastLaunch<128, MINB, __VA_ARGS__, false>())))
+    if (c.shape == 0) return FAST_PICK(6, FAST40);
+    if (c.shape == 1) return FAST_PICK(5, FAST48);
+    if (c.shape == 2) return FAST_PICK(4, FAST56);
+    return FAST_PICK(3, FAST64);
 #undef FAST_PICK
 }
 
