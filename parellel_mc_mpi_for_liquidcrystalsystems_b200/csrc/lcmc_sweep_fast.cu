@@ -303,7 +303,6 @@ __device__ __noinline__ void fixup_big(const DevView *__restrict__ vp, int r, in
     if (extra) atomicAdd(&sm.pairs, extra);
 }
 
-#define FAST_ILP 1
 // Sums over the warp of two values per lane: lanes 0-15 get the sum of a, 16-31
 // of b (one exchange halves the values a lane carries).
 __device__ __forceinline__ double warp_sum2(double a, double b, int lane)
@@ -681,48 +680,32 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
             // FP64 lane sums of the FP32 terms.  Entries [0, ca) belong to
             // particle a, [ca, ca + cb) to particle b.  An entry with a term
             // FP32 cannot carry is listed for the FP64 fix-up pass.
-            // Two entries per lane and step: their chains of a dozen dependent
-            // operations and five MUFU calls run side by side.
             const int n = ca + cb;
             const f32x2 neg = dup2(-1.0f);
-            for (int q0 = 0; q0 < n; q0 += 32 * FAST_ILP) {
-                int jj[FAST_ILP], kk[FAST_ILP];
-                float e0[FAST_ILP], e1[FAST_ILP];
-                bool in0[FAST_ILP], in1[FAST_ILP];
-#pragma unroll
-                for (int h = 0; h < FAST_ILP; h++) {
-                    const int q = q0 + 32 * h + lane;
-                    const bool isa = q < ca;
-                    const int j = q < n ? sm.list[(isa ? la : lb) + q] : 0;
-                    const int k = isa ? ka : min(kb, na - 1);
-                    jj[h] = j;
-                    kk[h] = k;
-                    const float4 P0 = sm.pst[k][0], P1 = sm.pst[k][1], P2 = sm.pst[k][2];
-                    const float4 c = sm.cpos[j];
-                    const float2 u = sm.cori[j];
-                    pair_fast_x2<SPEC21>(K, fma2(pack2(P0.x, P0.y), neg, dup2(c.x)),
-                                         fma2(pack2(P0.z, P0.w), neg, dup2(c.y)),
-                                         fma2(pack2(P1.x, P1.y), neg, dup2(c.z)), pack2(P1.z, P1.w), pack2(P2.x, P2.y),
-                                         pack2(P2.z, P2.w), dup2(c.w), dup2(u.x), dup2(u.y), e0[h], e1[h], in0[h],
-                                         in1[h]);
-                    e0[h] = in0[h] && q < n ? e0[h] : 0.0f; // beyond the cutoff
-                    e1[h] = in1[h] && q < n ? e1[h] : 0.0f;
-                    np += (int)(in0[h] && q < n) + (int)(in1[h] && q < n);
+            for (int q = lane; q < n; q += 32) {
+                const bool isa = q < ca;
+                const int j = sm.list[(isa ? la : lb) + q], k = isa ? ka : kb;
+                const float4 P0 = sm.pst[k][0], P1 = sm.pst[k][1], P2 = sm.pst[k][2];
+                const float4 c = sm.cpos[j];
+                const float2 u = sm.cori[j];
+                float e0, e1;
+                bool in0, in1;
+                pair_fast_x2<SPEC21>(K, fma2(pack2(P0.x, P0.y), neg, dup2(c.x)), fma2(pack2(P0.z, P0.w), neg, dup2(c.y)),
+                                     fma2(pack2(P1.x, P1.y), neg, dup2(c.z)), pack2(P1.z, P1.w), pack2(P2.x, P2.y),
+                                     pack2(P2.z, P2.w), dup2(c.w), dup2(u.x), dup2(u.y), e0, e1, in0, in1);
+                e0 = in0 ? e0 : 0.0f; // beyond the cutoff
+                e1 = in1 ? e1 : 0.0f;
+                if (!(fmaxf(fabsf(e0), fabsf(e1)) <= K.big) || e0 != e0 || e1 != e1) {
+                    const int slot = atomicAdd(&sm.nbigs, 1);
+                    if (slot < SM::BIGCAP) sm.bigs[slot] = ((unsigned)k << 16) | (unsigned)j;
+                    else sm.overflow = 1;
+                    e0 = e1 = 0.0f; // the fix-up counts its pairs
+                } else {
+                    np += (int)in0 + (int)in1;
                 }
-#pragma unroll
-                for (int h = 0; h < FAST_ILP; h++) {
-                    const bool isa = q0 + 32 * h + lane < ca;
-                    if (!(fmaxf(fabsf(e0[h]), fabsf(e1[h])) <= K.big) || e0[h] != e0[h] || e1[h] != e1[h]) {
-                        const int slot = atomicAdd(&sm.nbigs, 1);
-                        if (slot < SM::BIGCAP) sm.bigs[slot] = ((unsigned)kk[h] << 16) | (unsigned)jj[h];
-                        else sm.overflow = 1;
-                        np -= (int)(in0[h]) + (int)(in1[h]); // the fix-up counts its pairs
-                        e0[h] = e1[h] = 0.0f;
-                    }
-                    const double d = (double)e1[h] - (double)e0[h];
-                    if (isa) sa += d;
-                    else sb += d;
-                }
+                const double d = (double)e1 - (double)e0;
+                if (isa) sa += d;
+                else sb += d;
             }
             __syncwarp();
             const double sum = warp_sum2(sa, sb, lane);
