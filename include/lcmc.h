@@ -88,10 +88,10 @@ typedef struct {
     /* added keys */
     uint64_t rng_seed;
     int total_mc_sweeps;             /* sweeps of a run_simulation driver run; 0 = ceil(total_mc_cycles / num_particles) */
-    int cell_capacity;               /* active-cell capacity of the FP32 kernel (<= 48: small class, six
-                                        blocks per SM; <= 64: large class); 0 = automatic: NVT from the
-                                        creation density, NPT the large class.  A cell holding more
-                                        particles is attempted in FP64 (counted in overcap_cells) */
+    int cell_capacity;               /* active-cell capacity of the FP32 kernel (classes of 48, 56 and 64);
+                                        0 = automatic, from the creation density.  A cell holding more
+                                        particles than its class is attempted in FP64 (counted in
+                                        overcap_cells) */
     double npt_max_dlnV;
     int volume_moves_per_sweep;      /* 0 or 1 */
     int precision_mode;              /* LCMC_PREC_FP64 / LCMC_PREC_FP32 */
@@ -132,8 +132,8 @@ typedef struct {
     int kernel;                  /* 0 = FP64 kernel, 1 = FP32 kernel */
     int64_t volume_stage1_rejected; /* volume moves the surrogate rejected (no exact energy computed) */
     int64_t fp64_cells;          /* FP32-kernel cell attempts run in FP64: a pair term above 100 eps0 (an
-                                    overlap), or the cell above the kernel's capacity */
-    int64_t overcap_cells;       /* of which: above the cell, staged-candidate or list capacity */
+                                    overlap), or the cell above its class or the largest arrays */
+    int64_t overcap_cells;       /* of which: above the class, staged-candidate or list capacity */
     int64_t energy_checks;       /* periodic FP64 energy checks run */
     int64_t drift_breaches;      /* checks out of tolerance */
     double drift_bound;          /* tolerance of the last check (absolute energy) */
@@ -143,7 +143,7 @@ typedef struct {
 /* error_flags bits */
 enum {
     LCMC_F_CELLCAP = 1,     /* not set by this version: a cell above the FP32 kernel's capacity (active,    */
-    LCMC_F_STENCILCAP = 2,  /* staged-candidate or list) is attempted in FP64 and counted in overcap_cells; */
+    LCMC_F_STENCILCAP = 2,  /* staged-candidate or list) is run by the hand-over kernel (overcap_cells);   */
     LCMC_F_LISTCAP = 4,     /* the bits stay reserved                                                       */
     LCMC_F_NONFINITE = 8,   /* NaN/Inf energy change */
     LCMC_F_GRIDCAP = 16,    /* box grew past the allocated cell grid (cells kept wider) */
@@ -343,8 +343,8 @@ int lcmc_cell_capacity(const lcmc_params *p, int *capacity, int *class_capacity)
 
 /* Autotuner (no counterpart in the reference): times `sweeps` sweeps (after
  * one warm-up sweep) of every candidate configuration -- each FP32 phase-kernel
- * capacity class the capacity rule allows (the per-block tile of the active
- * cell: threads, cell capacity, staged candidates per warp, list capacity) and,
+ * capacity class the capacity rule allows (its block shape: cell capacity,
+ * places of the neighbour cells' particles, list capacity) and,
  * for NPT systems with >= 4 cells per axis, the per-cell or the per-particle
  * kernel for the volume move's exact energies -- and keeps the fastest.  The
  * state, statistics, sweep counters and last outcomes are restored after every
