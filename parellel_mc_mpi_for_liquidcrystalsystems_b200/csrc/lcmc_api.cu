@@ -71,6 +71,8 @@ struct lcmc_ctx {
     int grp_lo[kMaxGroups] = {}, grp_hi[kMaxGroups] = {};
     cudaStream_t side[kMaxGroups] = {};
     cudaEvent_t ev_fork = nullptr, ev_join[kMaxGroups] = {};
+    cudaStream_t xside[kMaxGroups] = {}; // FP64 phases beside FP32 ones
+    cudaEvent_t ev_xjoin[kMaxGroups] = {};
     unsigned char *d_outcome = nullptr;
     double *d_rec_dE = nullptr, *d_rec_lu = nullptr; // move records (lcmc_record_moves)
     std::vector<unsigned long long> sweeps; // host mirror of every replica's sweep counter
@@ -580,6 +582,8 @@ static void free_ctx(lcmc_ctx *c)
     for (int g = 0; g < kMaxGroups; g++) {
         if (c->side[g]) cudaStreamDestroy(c->side[g]);
         if (c->ev_join[g]) cudaEventDestroy(c->ev_join[g]);
+        if (c->xside[g]) cudaStreamDestroy(c->xside[g]);
+        if (c->ev_xjoin[g]) cudaEventDestroy(c->ev_xjoin[g]);
     }
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     void *ptrs[] = {c->d_rep, c->d_stats, c->d_act_off, c->d_act_tab, c->d_p2r, c->d_id[0], c->d_id[1], c->d_cid, c->d_rank,
@@ -1137,7 +1141,7 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
     cudaEventRecordWithFlags(c->ev[1], c->stream, cudaEventRecordExternal);
     DevView v = view(c, parity ^ 1);
     if (c->any_exact) launch_exact_offsets(v, c->stream);
-    if (c->ngroup > 1) cudaEventRecord(c->ev_fork, c->stream);
+    if (c->ngroup > 1 || (c->any_exact && c->any_fast)) cudaEventRecord(c->ev_fork, c->stream);
     for (int g = 0; g < c->ngroup; g++) {
         // group g's phases: its replicas' cells, its own hand-over lists, its own stream
         DevView vg = v;
@@ -1150,16 +1154,20 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
         if (c->d_ex_rows) vg.ex_rows = c->d_ex_rows + (size_t)g * c->ex_alloc * 32;
         cudaStream_t sg = g == 0 ? c->stream : c->side[g];
         if (g > 0) cudaStreamWaitEvent(sg, c->ev_fork, 0);
-        for (int ci = 0; ci < c->nrun; ci++) {
-            if (c->any_exact) launch_phase_exact(vg, sg, ci, c->grid_exact);
-            if (c->any_fast) {
-                launch_phase_fast(c->fast, c->rep[0].k, vg, sg, ci, c->grid_fast);
-                launch_phase_rescue(c->fast.spec21, c->rep[0].k, vg, sg, ci, c->sms);
-            }
+        // the FP64 phases of a context that also has FP32 ones run beside them, on a branch of their own: a replica
+        // takes one kind or the other in a sweep, and replicas do not interact
+        cudaStream_t sx = c->any_exact && c->any_fast ? c->xside[g] : sg;
+        if (sx != sg) cudaStreamWaitEvent(sx, c->ev_fork, 0);
+        for (int ci = 0; ci < c->nrun && c->any_exact; ci++) launch_phase_exact(vg, sx, ci, c->grid_exact);
+        for (int ci = 0; ci < c->nrun && c->any_fast; ci++) {
+            launch_phase_fast(c->fast, c->rep[0].k, vg, sg, ci, c->grid_fast);
+            launch_phase_rescue(c->fast.spec21, c->rep[0].k, vg, sg, ci, c->sms);
         }
+        if (sx != sg) cudaEventRecord(c->ev_xjoin[g], sx);
         if (g > 0) cudaEventRecord(c->ev_join[g], sg);
     }
     for (int g = 1; g < c->ngroup; g++) cudaStreamWaitEvent(c->stream, c->ev_join[g], 0);
+    for (int g = 0; g < c->ngroup && c->any_exact && c->any_fast; g++) cudaStreamWaitEvent(c->stream, c->ev_xjoin[g], 0);
     cudaEventRecordWithFlags(c->ev[2], c->stream, cudaEventRecordExternal);
     launch_sweep_stats(v, c->stream);
     if (c->any_npt) {
@@ -1185,6 +1193,11 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
 static int ensure_exact_scratch(lcmc_ctx *c)
 {
     if (!c->any_exact) return LCMC_OK;
+    for (int g = 0; g < c->ngroup && c->any_fast; g++) { // the branches of their own
+        if (!c->ev_fork) CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+        if (!c->xside[g]) CUDA_TRY(c, cudaStreamCreateWithFlags(&c->xside[g], cudaStreamNonBlocking));
+        if (!c->ev_xjoin[g]) CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_xjoin[g], cudaEventDisableTiming));
+    }
     const long long act = c->act_max;
     int most = 1; // particles of the largest replica group
     for (int g = 0; g < c->ngroup; g++) {
