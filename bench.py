@@ -272,10 +272,9 @@ def kernel_traffic():
     k_phase_fast launch on this workload and where the figure comes from: a
     fixed ncu capture (ncu cannot run inside the timed process), so it is
     the same in every run and is refreshed when the kernel changes."""
-    return 45.368576e6 + 1.271808e6, ("fixed, from one ncu --set full capture of k_phase_fast launches 265-266 "
-                                      "of `bench.py --steps 3 --warmup 3 --e2e-steps 1 --cpu-seconds 2 "
-                                      "--port-seconds 0 --da-sweeps 0 --jammed-steps 0 --batch-steps 0` (45.4 MB "
-                                      "read + 1.3 MB written per launch); not measured in this run")
+    return 47.222980e6 + 1.815793e6, ("fixed, from ncu (dram__bytes_read.sum + dram__bytes_write.sum) over 17 "
+                                      "k_phase_fast launches of this workload, 22-24 sweeps from the lattice start "
+                                      "(47.2 MB read + 1.8 MB written per launch); not measured in this run")
 
 
 # ---------------------------------------------------------------------------

