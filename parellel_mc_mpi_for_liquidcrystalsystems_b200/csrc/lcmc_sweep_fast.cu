@@ -435,6 +435,7 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
     if (kw >= 0 && kw < AMAX && kw < (int)((unsigned)rec.z >> 24)) fetch_rec(&sm.next[kw], v.act_rec + rec.w + kw);
     unsigned phase = 0;
     int which = 0, id = 0; // id: of particle kw of the cell that runs
+    fetch_wait();          // (a first cell that does not run here reads no record)
     __syncthreads();
 
     for (;;) {
@@ -468,7 +469,6 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
                 uint2 qh = make_uint2(0u, 0x3c000000u); // (0, 0, 0, 1)
                 float qc = 1e30f;
                 if (kw < na) {
-                    fetch_wait();
                     const ActRec ar = sm.next[kw];
                     sm.pst[kw][0] = ar.p0;
                     sm.pst[kw][1] = ar.p1;
@@ -835,11 +835,14 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
         __syncthreads();
 
         // ---- 6 write-back ----
+        // Every thread's own fetches have landed before its cell ends, read or not: the next cell's list (and, after a
+        // retry, the staged FP64 states) take the place of this cell's trial states, and the fetches of the cell after a
+        // skipped one that of its records.
+        fetch_wait();
         if (mode == 0 && kw >= 0 && kw < na) {
             const int k = kw, g = g0 + k;
             const int acc = sm.acc[k];
             if (acc) {
-                fetch_wait();
                 v.px[g] = sm.wn[k][0];
                 v.py[g] = sm.wn[k][1];
                 v.pz[g] = sm.wn[k][2];
