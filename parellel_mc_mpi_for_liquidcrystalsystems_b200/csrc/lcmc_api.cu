@@ -58,6 +58,7 @@ struct lcmc_ctx {
     double2 *d_ex_rows = nullptr;
     long long ex_cap = 0, ex_alloc = 0;
     int ex_act = 0, ex_nb = 1;
+    int ex_need = 1, ex_have = 0; // particles of the largest group they are for: of the current boxes, of the scratch
     int nphase = 8; // colour phases per sweep (LCMC_MAX_COLOURS with a fine-grid replica)
     int nrun = 8;   // of those, the ones any replica's box can take
     // sweeps until an NPT box could reach the four cells per axis below which
@@ -736,8 +737,14 @@ static void box_launches(lcmc_ctx *c)
     c->safe_sweeps = 1ll << 40;
     c->since_choice = 0;
     c->nrun = 8;
-    for (int r = 0; r < c->R; r++) {
+    int n64 = 0; // particles of group g that the FP64 phases may take
+    c->ex_need = 1;
+    for (int r = 0, g = 0; r < c->R; r++) {
         const Replica &rp = c->rep[r];
+        if (r == c->grp_hi[g]) {
+            n64 = 0;
+            g++;
+        }
         const double Lmin = std::min(rp.L[0], std::min(rp.L[1], rp.L[2]));
         bool small = grid_dim_host(Lmin, rp.wmin, rp.fine) < 4;
         if (!small && rp.ensemble == 2 && rp.dlnv_max > 0.0) {
@@ -746,6 +753,8 @@ static void box_launches(lcmc_ctx *c)
             else c->safe_sweeps = std::min(c->safe_sweeps, safe);
         }
         c->any_exact = c->any_exact || rp.kernel == 0 || small;
+        if (rp.kernel == 0 || small) n64 += rp.n;
+        c->ex_need = std::max(c->ex_need, n64);
         c->any_small = c->any_small || small || !rp.vol_cells;
         // colours: 2 per axis, 3 on an odd count of the fine grid; an NPT box may take any count
         int ncol = rp.fine && rp.ensemble == 2 ? LCMC_MAX_COLOURS : 1;
@@ -1083,6 +1092,9 @@ static int read_boxes(lcmc_ctx *c)
     return LCMC_OK;
 }
 
+// The FP64 phases need more scratch than there is (the graphs hold its address and sizes).
+static bool exact_grows(const lcmc_ctx *c) { return c->any_exact && c->ex_need > c->ex_have; }
+
 // The box-dependent launches again, within a run of sweeps (no kernel changes).
 static int recheck_boxes(lcmc_ctx *c)
 {
@@ -1091,7 +1103,8 @@ static int recheck_boxes(lcmc_ctx *c)
     const bool old_exact = c->any_exact, old_small = c->any_small;
     const int old_nrun = c->nrun;
     box_launches(c);
-    if (old_exact != c->any_exact || old_small != c->any_small || old_nrun != c->nrun) invalidate_graphs(c);
+    if (old_exact != c->any_exact || old_small != c->any_small || old_nrun != c->nrun || exact_grows(c))
+        invalidate_graphs(c);
     return LCMC_OK;
 }
 
@@ -1108,7 +1121,7 @@ static int rechoose_kernels(lcmc_ctx *c)
     int rc = push_kernel_fields(c);
     if (rc) return rc;
     if (!(old_fast_choice == c->fast) || old_fast != c->any_fast || old_exact != c->any_exact ||
-        old_small != c->any_small || old_nrun != c->nrun || old_grid != c->grid_fast)
+        old_small != c->any_small || old_nrun != c->nrun || old_grid != c->grid_fast || exact_grows(c))
         invalidate_graphs(c);
     return LCMC_OK;
 }
@@ -1198,31 +1211,30 @@ static int ensure_exact_scratch(lcmc_ctx *c)
         if (!c->xside[g]) CUDA_TRY(c, cudaStreamCreateWithFlags(&c->xside[g], cudaStreamNonBlocking));
         if (!c->ev_xjoin[g]) CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_xjoin[g], cudaEventDisableTiming));
     }
+    if (!exact_grows(c)) return LCMC_OK;
     const long long act = c->act_max;
-    int most = 1; // particles of the largest replica group
-    for (int g = 0; g < c->ngroup; g++) {
-        int n = 0;
-        for (int r = c->grp_lo[g]; r < c->grp_hi[g]; r++)
-            // an FP32 system comes here only with three cells or fewer along an axis
-            if (c->rep[r].kernel == 0 || grid_dim_host(c->rep[r].L[0], c->rep[r].wmin, c->rep[r].fine) < 6) n += c->rep[r].n;
-        most = std::max(most, n);
-    }
     long long cap, alloc;
-    exact_scratch_size(most, &cap, &alloc, &c->ex_nb);
-    if (c->d_ex_rows && alloc <= c->ex_alloc) return LCMC_OK;
-    if (c->d_ex_rows) { // more replicas need it than before
-        CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        cudaFree(c->d_ex_rows);
-        c->d_ex_rows = nullptr;
-    }
+    int nb;
+    exact_scratch_size(c->ex_need, &cap, &alloc, &nb);
+    // what a captured graph holds changes: the sizes, and the rows' address where they grow
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    invalidate_graphs(c);
     const size_t np = (size_t)c->nphase;
     if (!c->d_ex_p) CUDA_TRY(c, dalloc(&c->d_ex_p, np * (act + 1)));
     if (!c->d_ex_r) CUDA_TRY(c, dalloc(&c->d_ex_r, np * (act + 1)));
     if (!c->d_ex_flag) CUDA_TRY(c, dalloc(&c->d_ex_flag, np * act));
-    CUDA_TRY(c, dalloc(&c->d_ex_rows, (size_t)c->ngroup * alloc * 32));
+    if (alloc > c->ex_alloc) {
+        if (c->d_ex_rows) cudaFree(c->d_ex_rows);
+        c->d_ex_rows = nullptr;
+        c->ex_alloc = 0;
+        c->ex_have = 0;
+        CUDA_TRY(c, dalloc(&c->d_ex_rows, (size_t)c->ngroup * alloc * 32));
+        c->ex_alloc = alloc;
+    }
     c->ex_act = (int)act;
     c->ex_cap = cap;
-    c->ex_alloc = alloc;
+    c->ex_nb = nb;
+    c->ex_have = c->ex_need;
     exact_init();
     return LCMC_OK;
 }
