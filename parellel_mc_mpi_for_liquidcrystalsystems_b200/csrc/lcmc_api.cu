@@ -1938,8 +1938,11 @@ void tune_cache_append(const char *path, const std::string &key, const TuneChoic
 
 } // namespace
 
+// (the boxes as they are on the device: the block shape and what box_launches grants follow from them)
 static int apply_tuning(lcmc_ctx *c, const TuneChoice &ch)
 {
+    int brc = read_boxes(c);
+    if (brc) return brc;
     c->fast.cls = ch.variant_class;
     c->tuned_class = ch.variant_class;
     choose_fast_shape(c);
@@ -1976,6 +1979,8 @@ extern "C" int lcmc_autotune(lcmc_ctx *ctx, int sweeps, const char *cache_path, 
         res.from_cache = 1;
     } else {
         // candidates: every capacity class the capacity rule allows, each volume-energy kernel that applies
+        int brc = read_boxes(ctx);
+        if (brc) return brc;
         std::vector<TuneChoice> cand;
         bool npt4 = false; // an NPT replica on the per-cell volume kernel's grid (>= 4 cells per axis)
         for (int r = 0; r < ctx->R; r++)
@@ -2078,6 +2083,10 @@ extern "C" int lcmc_autotune(lcmc_ctx *ctx, int sweeps, const char *cache_path, 
         }
         release();
         ctx->checks_off = false;
+        if (rc || best_ms < 0.0) { // the restored boxes, not the last trial's
+            const int b = recheck_boxes(ctx);
+            if (b) return b;
+        }
         if (rc) return rc;
         if (best_ms < 0.0) return set_err(ctx, LCMC_ECELLCAP, "no candidate ran");
         rc = apply_tuning(ctx, best);
