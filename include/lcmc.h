@@ -272,10 +272,12 @@ int lcmc_mlp_set_params(lcmc_mlp *m, const float *params);
 /* C[M x N] = A[M x K] B[N x K]^T with A, B rounded to BF16, FP32 accumulate, on
  * the tensor cores (host arrays; K a multiple of 64).  For tests. */
 int lcmc_gemm_bf16(const float *A, const float *B, float *C, int M, int N, int K);
-/* Limit, in tries, of the tensor-core kernels' bounded mbarrier waits for
- * launches made from now on (0 restores the default, 2^24).  A wait that runs
- * out sets the kernel's error flag, waits (with the full bound) for the MMAs
- * it issued, frees its TMEM and returns; the call then reports LCMC_ETIMEOUT.
+/* Limit, in tries, of the bounded mbarrier waits of the tensor-core kernels and
+ * of the sweep's phase kernels, for launches made from now on (0 restores the
+ * default, 2^24).  A wait that runs out sets the kernel's error flag, waits
+ * (with the full bound) for the MMAs and copies it issued, frees its TMEM and
+ * returns; the call then reports LCMC_ETIMEOUT, and the cells a phase kernel
+ * had not come to make no moves in that sweep.
  * For tests of that path (a limit of 1 makes the first wait give up).  Sweep
  * graphs captured earlier keep the limit they were captured with.  No
  * counterpart in the reference. */

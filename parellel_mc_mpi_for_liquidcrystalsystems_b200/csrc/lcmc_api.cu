@@ -498,6 +498,7 @@ static DevView view(const lcmc_ctx *c, int parity)
     v.act_off = c->d_act_off;
     v.act_tab = c->d_act_tab;
     v.act_max = c->act_max;
+    v.wait_tries = wait_limit() - 1;
     v.p2r = c->d_p2r;
     const int a = parity, b = parity ^ 1;
     v.px = c->d_x[a][0];

@@ -150,6 +150,8 @@ struct DevView {
     int4 *act_tab;      // [nphase][act_max] active cells of a phase: cell, replica, coordinates (8 bits each) with
                         // the count of its particles above them (at most 255), first particle slot
     int act_max;
+    unsigned wait_tries; // mbarrier tries of a phase kernel's wait: one below lcmc_set_wait_limit's limit, so that a
+                         // limit of 1 gives up without a look (a first look mostly finds the copies landed)
     int nphase;         // colour phases per sweep: 8, or LCMC_MAX_COLOURS with a fine-grid replica
     int r_lo, r_hi;     // replicas whose cells the phase kernels attempt (a group of a batch: [r_lo, r_hi))
     int ngroup;         // replica groups (resc_count/resc_list hold one set of phases per group)

@@ -101,6 +101,7 @@ void launch_validate_upload(const double *const x[6], int *id, int n, const doub
 struct lcmc_mlp;
 namespace lcmc {
 // lcmc_mlp.cu (in-sweep surrogate inference)
+unsigned wait_limit(); // what lcmc_set_wait_limit set
 void *mlp_input(lcmc_mlp *m);
 int mlp_ld(lcmc_mlp *m);
 int mlp_bmax(lcmc_mlp *m);

@@ -414,11 +414,12 @@ void gemm_tc(const bf16 *A, int lda, const bf16 *B, int ldb, float *C, int ldc, 
 
 } // namespace lcmc
 
-// Limit of the tensor-core kernels' bounded mbarrier waits, in tries, for
-// launches made from now on (0 restores the default).  A wait that runs out
-// sets the kernel's error flag, drains the MMAs in flight with the full bound,
-// frees its TMEM and returns; the call reports LCMC_ETIMEOUT.  For tests of
-// that path: a limit of 1 makes the first wait give up.
+// Limit of the kernels' bounded mbarrier waits (the GEMMs' here, the sweep's
+// phase kernels'), in tries, for launches made and graphs captured from now on
+// (0 restores the default).  A wait that runs out sets the kernel's error flag,
+// waits for what is in flight with the full bound, frees its TMEM and returns;
+// the call reports LCMC_ETIMEOUT.  For tests of that path: a limit of 1 makes
+// the first wait give up.
 extern "C" int lcmc_set_wait_limit(unsigned int tries)
 {
     lcmc::g_wait_iters = tries ? (uint32_t)tries : lcmc::kWaitIters;
@@ -426,6 +427,8 @@ extern "C" int lcmc_set_wait_limit(unsigned int tries)
 }
 
 namespace lcmc {
+
+unsigned wait_limit() { return g_wait_iters; }
 
 // ---------------------------------------------------------------------------
 // MLP kernels (FP32 CUDA cores)

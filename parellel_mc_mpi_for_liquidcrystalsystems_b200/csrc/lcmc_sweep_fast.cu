@@ -394,7 +394,7 @@ __device__ __forceinline__ void fetch_rec(ActRec *dst, const ActRec *src)
     for (int i = 0; i < (int)sizeof(ActRec); i += 16) fetch_async<16>((char *)dst + i, (const char *)src + i);
 }
 
-constexpr unsigned FAST_WAIT_TRIES = 1u << 24; // mbarrier tries before a block gives up
+constexpr unsigned FAST_WAIT_TRIES = 1u << 24; // mbarrier tries for the copies of a block that leaves
 
 // Cells a retry left to the FP64 attempts of its block.
 struct RetryFailed {
@@ -493,7 +493,7 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
             const auto &st = sm.st[which];
             const int ncand = st.pos[27]; // places of the copies
             if (w == 0) s26 = __reduce_add_sync(0xffffffffu, lane < 27 && lane != 13 ? st.cnt[lane] : 0);
-            bool ok = tc::mbar_wait_bounded(&sm.full, phase, FAST_WAIT_TRIES);
+            bool ok = tc::mbar_wait_bounded(&sm.full, phase, v.wait_tries);
             phase ^= 1u;
 #pragma unroll 2
             for (int s = w; s < 27; s += NW) {
@@ -516,10 +516,10 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
                 }
             }
             if (t < 16) sm.ch[ncand + t] = make_uint2(0u, 0x7b000000u); // beyond the last: likewise
-            if (__syncthreads_or(!ok)) { // (uniform) the copies did not land within the limit: flag it and leave
-                if (t == 0) atomicOr(&v.stats[r].flags, F_TIMEOUT);
+            if (__syncthreads_or(!ok)) { // (uniform) the copies did not land within the limit: flag it and leave,
+                if (t == 0) atomicOr(&v.stats[r].flags, F_TIMEOUT); // the copies waited for (no others are on their way)
                 tc::mbar_wait_bounded(&sm.full, phase ^ 1u, FAST_WAIT_TRIES);
-                return;
+                break;
             }
         // ---- 2 reach tests of eight particles against every candidate ----
         for (int task = w; task < (na + 7) >> 3; task += NW) {
