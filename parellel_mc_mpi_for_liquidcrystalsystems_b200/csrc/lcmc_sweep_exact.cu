@@ -566,12 +566,12 @@ constexpr int ex_max(int a, int b) { return a > b ? a : b; }
 constexpr int EX_BYTES = ex_max(ex_max(ExactStage<2>::BYTES, ExactStage<3>::BYTES),
                                 ex_max(ExactStage<5>::BYTES, ExactStage<EX_J>::BYTES));
 
-constexpr unsigned EX_WAIT_TRIES = 1u << 24; // mbarrier tries before a block gives up
+constexpr unsigned EX_WAIT_TRIES = 1u << 24; // mbarrier tries for the copies of a block that leaves
 
 struct ExactShared {
     uint64_t full[2];       // mbarriers: a half's records have landed
     double dE[EX_NA];       // energy change of an accepted attempt, else 0
-    int failed;             // a copy did not land
+    int failed[2];          // a half's records did not land
     unsigned pairs[EX_WARPS], hard[EX_WARPS];
     CellView c;
     int first[27], base[28];
@@ -602,17 +602,15 @@ __device__ __forceinline__ bool exact_decide_cell(const DevView &v, const CellVi
     };
     fetch(0, 0);
     fetch(D, 1);
-    bool ok = true;
     if (na > 0) { // (uniform; an empty cell copies nothing)
-        ok = tc::mbar_wait_bounded(&sh.full[0], phase & 1u, EX_WAIT_TRIES);
+        if (!tc::mbar_wait_bounded(&sh.full[0], phase & 1u, v.wait_tries)) sh.failed[0] = 1;
         phase ^= 1u;
     }
-    if (!ok) sh.failed = 1;
     __syncthreads();
-    ok = !sh.failed;
+    bool ok = !sh.failed[0];
     unsigned accm = 0u; // bit j: the particle at slot 32 (c0 + j) + lane was accepted
-    int half = 0;
-    for (int k0 = 0; k0 < na && ok; k0 += D, half ^= 1) {
+    int half = 0, k0 = 0;
+    for (; k0 < na && ok; k0 += D, half ^= 1) {
         const int k = k0 + wd, q0 = q13 + k0;
         const int mine = (lane - q0) & 31, jm = ((q0 + mine) >> 5) - c0; // this lane's slot is the round's mine-th
         double dE = 0.0, lu = 0.0;
@@ -659,7 +657,7 @@ __device__ __forceinline__ bool exact_decide_cell(const DevView &v, const CellVi
             }
         }
         if (w == EX_WARPS - 1 && k0 + D < na) { // the next round's records
-            if (!tc::mbar_wait_bounded(&sh.full[half ^ 1], (phase >> (half ^ 1)) & 1u, EX_WAIT_TRIES)) sh.failed = 1;
+            if (!tc::mbar_wait_bounded(&sh.full[half ^ 1], (phase >> (half ^ 1)) & 1u, v.wait_tries)) sh.failed[half ^ 1] = 1;
         }
         if (k0 + D < na) phase ^= 1u << (half ^ 1);
         const int m = __syncthreads_count(acc && report); // bit w: warp w's attempt was accepted
@@ -675,13 +673,16 @@ __device__ __forceinline__ bool exact_decide_cell(const DevView &v, const CellVi
                 v.rec_lu[p.p_off + id] = lu;
             }
         }
-        ok = !sh.failed;
+        // written before this round's barrier; the next round writes the other half's, the one after that comes past
+        // the next barrier: every thread reads the same
+        ok = !sh.failed[half ^ 1];
     }
-    if (!ok) { // (uniform) copies still on their way are waited for, again with a limit
-        __syncthreads();
+    if (!ok) { // (uniform) the records of the round at k0 did not land
         if (t == 0) atomicOr(&v.stats[c.r].flags, F_TIMEOUT);
-        tc::mbar_wait_bounded(&sh.full[0], phase & 1u, EX_WAIT_TRIES);
-        tc::mbar_wait_bounded(&sh.full[1], (phase >> 1) & 1u, EX_WAIT_TRIES);
+        // copies still on their way are waited for, again with a limit: that round's (its parity was stepped on) and,
+        // if there is one, the round after's
+        tc::mbar_wait_bounded(&sh.full[half], ((phase >> half) & 1u) ^ 1u, EX_WAIT_TRIES);
+        if (k0 + D < na) tc::mbar_wait_bounded(&sh.full[half ^ 1], (phase >> (half ^ 1)) & 1u, EX_WAIT_TRIES);
         return false;
     }
     // a lane per particle: outcome, accepted trial state to the master arrays, and the pairs its attempt met
@@ -763,7 +764,7 @@ __global__ void __launch_bounds__(EX_WARPS * 32) k_exact_decide(const __grid_con
     if (threadIdx.x == 0) {
         tc::mbar_init(&sh.full[0], 1);
         tc::mbar_init(&sh.full[1], 1);
-        sh.failed = 0;
+        sh.failed[0] = sh.failed[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     unsigned phase = 0u; // bit h: parity of full[h]'s next completion

@@ -38,6 +38,8 @@ SYSTEMS = {
     "fp32": lambda: system(60000, 0.30, 1),        # several cells per block
     "fp32_wide": lambda: system(8000, 0.30, 1),    # a block of 512 threads per cell
     "fp32_retry": slab_system,
+    "fp64": lambda: system(2000, 0.30, 0),         # records of a cell's attempts copied a round ahead
+    "fp64_cells": lambda: system(30000, 0.30, 0),  # a block per cell, a hundred cells
 }
 
 
