@@ -828,7 +828,7 @@ static void choose_kernels(lcmc_ctx *c)
 {
     c->any_fast = c->any_npt = false;
     int need_amax = 0, need_min = 0;
-    bool spec21 = true; // every system has mu = 2, nu = 1, sigma0 = 1
+    bool spec21 = true, one_k = true; // every system has mu = 2, nu = 1, sigma0 = 1; the same pair constants
     for (int r = 0; r < c->R; r++) {
         Replica &rp = c->rep[r];
         const lcmc_params &p = c->params[r];
@@ -848,8 +848,8 @@ static void choose_kernels(lcmc_ctx *c)
             need_min = std::max(need_min, capacity_floor(p, rp.L[0], rp.wmin));
         }
         if (rp.ensemble == 2) c->any_npt = true;
-        spec21 = spec21 && p.gb_mu_exponent == 2.0 && p.gb_nu_exponent == 1.0 && p.gb_sigma_sidetoside == 1.0 &&
-                 same_pair_consts(rp.k, c->rep[0].k);
+        spec21 = spec21 && p.gb_mu_exponent == 2.0 && p.gb_nu_exponent == 1.0 && p.gb_sigma_sidetoside == 1.0;
+        one_k = one_k && same_pair_consts(rp.k, c->rep[0].k);
     }
     c->need_amax = need_amax;
     c->need_min = need_min;
@@ -857,6 +857,7 @@ static void choose_kernels(lcmc_ctx *c)
     if (c->tuned_class >= 0 && fast_variant(c->tuned_class).amax >= need_min) cls = c->tuned_class;
     c->fast.cls = cls;
     c->fast.spec21 = spec21;
+    c->fast.one_k = one_k;
     choose_fast_shape(c);
     set_caps(c);
     box_launches(c);
@@ -1175,7 +1176,7 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
         for (int ci = 0; ci < c->nrun && c->any_exact; ci++) launch_phase_exact(vg, sx, ci, c->grid_exact);
         for (int ci = 0; ci < c->nrun && c->any_fast; ci++) {
             launch_phase_fast(c->fast, c->rep[0].k, vg, sg, ci, c->grid_fast);
-            launch_phase_rescue(c->fast.spec21, c->rep[0].k, vg, sg, ci, c->sms);
+            launch_phase_rescue(c->fast.spec21, vg, sg, ci, c->sms);
         }
         if (sx != sg) cudaEventRecord(c->ev_xjoin[g], sx);
         if (g > 0) cudaEventRecord(c->ev_join[g], sg);

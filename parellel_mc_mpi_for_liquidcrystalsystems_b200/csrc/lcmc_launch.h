@@ -63,11 +63,15 @@ struct FastVariant {
 // The FP32 phase kernel a context runs
 struct FastChoice {
     int cls = 0;        // capacity class
-    bool spec21 = true; // mu = 2, nu = 1, sigma0 = 1 and the same pair constants in every replica
+    bool spec21 = true; // mu = 2, nu = 1, sigma0 = 1 in every replica
+    bool one_k = true;  // the same pair constants in every replica: they come with the launch
     int shape = 1;      // block shape: 0 for at most 40 particles per cell, 1 + class by class
     bool wide = false;  // 512 threads per cell: at most a cell per SM
     // the same kernel (the class is only a capacity)
-    bool same_kernel(const FastChoice &o) const { return spec21 == o.spec21 && wide == o.wide && shape == o.shape; }
+    bool same_kernel(const FastChoice &o) const
+    {
+        return spec21 == o.spec21 && one_k == o.one_k && wide == o.wide && shape == o.shape;
+    }
     bool operator==(const FastChoice &o) const { return cls == o.cls && same_kernel(o); }
 };
 constexpr int FAST_SHAPES = 4;
@@ -77,7 +81,7 @@ FastVariant fast_variant(int i);
 void launch_phase_fast(const FastChoice &c, const GBConsts &k, const DevView &v, cudaStream_t s, int ci, int grid);
 int fast_blocks_per_sm(const FastChoice &c);
 // retries (FP32, the largest capacity) and FP64 attempts of the cells the FP32 kernel left in colour phase ci
-void launch_phase_rescue(bool spec21, const GBConsts &k, const DevView &v, cudaStream_t s, int ci, int grid);
+void launch_phase_rescue(bool spec21, const DevView &v, cudaStream_t s, int ci, int grid);
 void rescue_init(); // once per process before the first hand-over launch
 
 // lcmc_misc.cu

@@ -403,8 +403,9 @@ struct RetryFailed {
 };
 
 // The FP32 attempts of a block: active cells a, a + step, ... below `total` of
-// phase ci (RETRY: of the phase's retry list).
-template <int NT, int AMAX, int CCAP, int LCAP, bool SPEC21, bool RETRY>
+// phase ci (RETRY: of the phase's retry list).  ONE_K: the pair constants are
+// the launch's, ku, else each cell's replica's.
+template <int NT, int AMAX, int CCAP, int LCAP, bool SPEC21, bool ONE_K, bool RETRY>
 __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &ku, int ci, unsigned char *smem_raw, int a,
                                                 const int total, const int step, RetryFailed *failed)
 {
@@ -441,7 +442,7 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
     for (;;) {
         const int cell = rec.x, r = rec.y, g0 = rec.w;
         const Replica &p = v.rep[r];
-        const FastK K = SPEC21 ? ku : fast_consts(p.k);
+        const FastK K = ONE_K ? ku : fast_consts(p.k);
         int mode = sm.st[which].skip; // 0 runs here, 1 not an FP32 cell, 2 handed over (capacity), 3 handed over (terms)
         const int na = sm.st[which].cnt[13];
         const bool more = a + step < total;
@@ -889,14 +890,14 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
     }
 }
 
-template <int NT, int MINB, int AMAX, int CCAP, int LCAP, bool SPEC21>
+template <int NT, int MINB, int AMAX, int CCAP, int LCAP, bool SPEC21, bool ONE_K>
 __global__ void __launch_bounds__(NT, MINB)
     k_phase_fast(const __grid_constant__ DevView v, const __grid_constant__ FastK ku, int ci)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int *off = v.act_off + ci * (v.R + 1); // this launch's replicas: active cells [off[r_lo], off[r_hi])
-    phase_fast_body<NT, AMAX, CCAP, LCAP, SPEC21, false>(v, ku, ci, smem_raw, off[v.r_lo] + (int)blockIdx.x, off[v.r_hi],
-                                                         (int)gridDim.x, nullptr);
+    phase_fast_body<NT, AMAX, CCAP, LCAP, SPEC21, ONE_K, false>(v, ku, ci, smem_raw, off[v.r_lo] + (int)blockIdx.x,
+                                                                off[v.r_hi], (int)gridDim.x, nullptr);
 }
 
 // FP64 attempts of the cells the FP32 phase kernel handed over in colour phase
@@ -922,7 +923,7 @@ constexpr int RESCUE_CAP = 1024; // particles of a staged stencil (48 KB of shar
 #define FAST_RETRY 64, 1664, 7168 // active particles, places of the static cells' particles, list entries
 
 template <int NT, bool SPEC21>
-__global__ void __launch_bounds__(NT) k_phase_rescue(const __grid_constant__ DevView v, const __grid_constant__ FastK ku, int ci)
+__global__ void __launch_bounds__(NT) k_phase_rescue(const __grid_constant__ DevView v, int ci)
 {
     constexpr int NW = NT / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -941,7 +942,7 @@ __global__ void __launch_bounds__(NT) k_phase_rescue(const __grid_constant__ Dev
         tc::fence_proxy_async_smem(); // the staged states of the last round's cells come before this round's copies
         __syncthreads();
         const int a1 = min(nretry, a0 + 32 * (int)gridDim.x);
-        if (a0 < a1) phase_fast_body<NT, FAST_RETRY, SPEC21, true>(v, ku, ci, smem_raw, a0, a1, (int)gridDim.x, &failed);
+        if (a0 < a1) phase_fast_body<NT, FAST_RETRY, SPEC21, false, true>(v, FastK(), ci, smem_raw, a0, a1, (int)gridDim.x, &failed);
         __syncthreads();
         const int mine = a0 == (int)blockIdx.x && count > a0 ? (count - a0 + (int)gridDim.x - 1) / (int)gridDim.x : 0;
         for (int e = 0; e < failed.n + mine; e++) {
@@ -1145,16 +1146,16 @@ int fast_shape_candidates(int shape)
     return n[shape];
 }
 
-template <int NT, int MINB, int AMAX, int CCAP, int LCAP, bool S21>
+template <int NT, int MINB, int AMAX, int CCAP, int LCAP, bool S21, bool K1>
 struct FastLaunch {
     static constexpr int bytes = (int)sizeof(FastSmem<AMAX, CCAP, LCAP>);
     static void launch(const DevView &v, const FastK &k, cudaStream_t s, int ci, int grid)
     {
-        k_phase_fast<NT, MINB, AMAX, CCAP, LCAP, S21><<<grid, NT, bytes, s>>>(v, k, ci);
+        k_phase_fast<NT, MINB, AMAX, CCAP, LCAP, S21, K1><<<grid, NT, bytes, s>>>(v, k, ci);
     }
     static int blocks()
     {
-        auto k = k_phase_fast<NT, MINB, AMAX, CCAP, LCAP, S21>;
+        auto k = k_phase_fast<NT, MINB, AMAX, CCAP, LCAP, S21, K1>;
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         int n = 0;
@@ -1168,19 +1169,24 @@ struct FastLaunch {
 // 1.66), sixteen where it has not and a phase takes one cell's latency (32,768
 // rods NPT: 0.19 ms against 0.30 with four).  The light shape holds six blocks
 // per SM where the class's own 48-particle arrays leave five (1.48 against 1.60).
-// The kernel of a variant: shape, specialisation (mu = 2, nu = 1, sigma0 = 1, the
-// same pair constants in every replica), wide (a block per SM).
+// The kernel of a variant: shape, wide (a block per SM), specialisation (mu = 2,
+// nu = 1, sigma0 = 1; of that, whether all replicas have the same pair constants,
+// which then come as a kernel argument).  Twelve systems of 30,000 rods of three
+// kappas, all phases and the rest of a sweep: 1.26 ms with the general terms, 1.04
+// with these and each replica's constants; 1.05 when all have one kappa.
 template <typename F>
 static auto with_variant(const FastChoice &c, F f)
 {
-#define FAST_PICK(MINB, ...)                                                                                           \
-    (c.wide ? (c.spec21 ? f(FastLaunch<512, 1, __VA_ARGS__, true>()) : f(FastLaunch<512, 1, __VA_ARGS__, false>()))    \
-            : (c.spec21 ? f(FastLaunch<128, MINB, __VA_ARGS__, true>()) : f(FastLaunch<128, MINB, __VA_ARGS__, false>())))
+#define FAST_SPEC(NT, MINB, ...)                                                                                       \
+    (!c.spec21 ? f(FastLaunch<NT, MINB, __VA_ARGS__, false, false>())                                                  \
+               : c.one_k ? f(FastLaunch<NT, MINB, __VA_ARGS__, true, true>()) : f(FastLaunch<NT, MINB, __VA_ARGS__, true, false>()))
+#define FAST_PICK(MINB, ...) (c.wide ? FAST_SPEC(512, 1, __VA_ARGS__) : FAST_SPEC(128, MINB, __VA_ARGS__))
     if (c.shape == 0) return FAST_PICK(6, FAST40);
     if (c.shape == 1) return FAST_PICK(5, FAST48);
     if (c.shape == 2) return FAST_PICK(4, FAST56);
     return FAST_PICK(3, FAST64);
 #undef FAST_PICK
+#undef FAST_SPEC
 }
 
 void launch_phase_fast(const FastChoice &c, const GBConsts &k, const DevView &v, cudaStream_t s, int ci, int grid)
@@ -1197,11 +1203,10 @@ static constexpr int rescue_bytes()
     return std::max(6 * RESCUE_CAP * (int)sizeof(double), (int)sizeof(FastSmem<FAST_RETRY>));
 }
 
-void launch_phase_rescue(bool spec21, const GBConsts &k, const DevView &v, cudaStream_t s, int ci, int grid)
+void launch_phase_rescue(bool spec21, const DevView &v, cudaStream_t s, int ci, int grid)
 {
-    const FastK K = fast_consts(k);
-    if (spec21) k_phase_rescue<256, true><<<grid, 256, rescue_bytes(), s>>>(v, K, ci);
-    else k_phase_rescue<256, false><<<grid, 256, rescue_bytes(), s>>>(v, K, ci);
+    if (spec21) k_phase_rescue<256, true><<<grid, 256, rescue_bytes(), s>>>(v, ci);
+    else k_phase_rescue<256, false><<<grid, 256, rescue_bytes(), s>>>(v, ci);
 }
 
 // Opts the hand-over kernel in to its dynamic shared memory (call once).
