@@ -777,12 +777,12 @@ __global__ void __launch_bounds__(EX_WARPS * 32) k_exact_decide(const __grid_con
         if (threadIdx.x < 32) {
             CellView c;
             active_cell(v, off, ci, a, c);
-            if (!v.rep[c.r].use_fast) cell_stencil(v, c, lane, sh.first, sh.base);
+            if (!v.rep[c.r].use_fast && c.na > 0) cell_stencil(v, c, lane, sh.first, sh.base);
             if (lane == 0) sh.c = c;
         }
         __syncthreads();
         const CellView c = sh.c;
-        if (v.rep[c.r].use_fast) continue;
+        if (v.rep[c.r].use_fast || c.na == 0) continue; // (an empty cell has its results from the rebin)
         if (a >= eb.hi || v.ex_flag[(size_t)ci * v.ex_act + a]) {
             if (threadIdx.x < 32) exact_cell_sequential(&v, c, lane, sh.first, sh.base);
             continue;
@@ -968,7 +968,7 @@ __global__ void __launch_bounds__(32) k_exact_decide_warp(const __grid_constant_
     for (int a = eb.lo + blockIdx.x; a < a1; a += gridDim.x) {
         CellView c;
         active_cell(v, off, ci, a, c);
-        if (v.rep[c.r].use_fast) continue;
+        if (v.rep[c.r].use_fast || c.na == 0) continue; // (an empty cell has its results from the rebin)
         cell_stencil(v, c, lane, s_first, s_base);
         if (a >= eb.hi || v.ex_flag[(size_t)ci * v.ex_act + a]) {
             exact_cell_sequential(&v, c, lane, s_first, s_base);

@@ -419,14 +419,26 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
     const int4 *tab = v.act_tab + (size_t)ci * v.act_max;
     const int *list = v.retry_list + (size_t)ci * v.act_max;
     auto entry = [&](int i) { return tab[RETRY ? list[i] : i]; };
+    // cells without particles are passed by: from entry i, its record e, to the next that has some (i >= total: none)
+    auto pass_empty = [&](int &i, int4 &e) {
+        while (!RETRY && i < total && !((unsigned)e.z >> 24)) { // (32 entries at a time)
+            const int q = i + step * (1 + lane);
+            const unsigned some = __ballot_sync(0xffffffffu, q < total && ((unsigned)tab[q].z >> 24));
+            i += step * (some ? __ffs(some) : 32);
+            if (some || i < total) e = tab[i];
+        }
+    };
     if (a >= total) return;
+    int4 rec = entry(a); // cell, replica, coordinates (8 bits each) and count of the particles (capped), first slot
+    pass_empty(a, rec);
+    if (a >= total) return; // (the whole block)
     if (t == 0) {
         tc::mbar_init(&sm.full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    int4 rec = entry(a); // cell, replica, coordinates (8 bits each) and count of the particles (capped), first slot
-    int4 nxt = a + step < total ? entry(a + step) : make_int4(0, 0, 0, 0);
+    int an = a + step; // the next cell
+    int4 nxt = an < total ? entry(an) : make_int4(0, 0, 0, 0);
     const int kw = t - 32; // thread 32 + k: particle k
     if (w == 1) {
         prepare_stencil<typename SM::Stencil, AMAX, CCAP>(v, sm.st[0], rec, lane);
@@ -445,7 +457,6 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
         const FastK K = ONE_K ? ku : fast_consts(p.k);
         int mode = sm.st[which].skip; // 0 runs here, 1 not an FP32 cell, 2 handed over (capacity), 3 handed over (terms)
         const int na = sm.st[which].cnt[13];
-        const bool more = a + step < total;
         int s26 = 0;
         unsigned long long npairs = 0ull;
         if (mode == 0) {
@@ -809,6 +820,8 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
                 }
             }
         }
+        pass_empty(an, nxt); // (here its record has long been loaded)
+        const bool more = an < total;
         // (the list is read no more: every thread has passed the barrier after the task queue)
         if (w != 0) {
             if (w == 1 && more) {
@@ -880,8 +893,9 @@ __device__ __forceinline__ void phase_fast_body(const DevView &v, const FastK &k
         }
         if (!more) break;
         rec = nxt;
-        a += step;
-        if (a + step < total) nxt = entry(a + step);
+        a = an;
+        an += step;
+        if (an < total) nxt = entry(an);
         which ^= 1;
     }
     if (RETRY) { // the block comes back with the barrier's memory
