@@ -774,8 +774,8 @@ static bool same_pair_consts(const GBConsts &a, const GBConsts &b)
            a.f_half_chip == b.f_half_chip && a.f_big == b.f_big;
 }
 
-// The shape of the FP32 phase kernel: the class's own, or the light one when no
-// system's rule asks for more than 40 particles per cell, but one whose arrays
+// The shape of the FP32 phase kernel: the class's own, or the light or the sparse
+// one when no system's rule asks for more than 40 or 32 particles per cell, but one whose arrays
 // hold the neighbour cells' particles (cells are as wide as the box allows, so
 // they can be fuller than the class's liquid): a cell above them is run again by
 // the hand-over kernel, and the phase waits for it, 24 us, as long as the phase
@@ -803,11 +803,15 @@ static void choose_fast_shape(lcmc_ctx *c)
         for (int s = 0; s < FAST_SHAPES; s++)
             if (need > fast_shape_candidates(s)) above[s] += cells;
     }
-    int shape = c->fast.cls == 0 && c->need_amax <= 40 ? 0 : 1 + c->fast.cls;
+    int shape = c->fast.cls == 0 && c->need_amax <= 40 ? 1 : 2 + c->fast.cls;
+    // a gas: two warps per cell, ten blocks per SM, once four warps and six blocks would take a phase in more than
+    // one round (phases of a sweep, six -> ten blocks: a million rods at 0.05 3.78 -> 2.54 ms, 200,000 at 0.12 0.47 ->
+    // 0.34, 20,000 at 0.03, 1000 cells, 0.194 -> 0.131; 30,000 at 0.10, 512 cells, would take 0.145 instead of 0.133)
+    if (shape == 1 && c->need_amax <= FAST_SPARSE && act > 6 * c->sms) shape = 0;
     // (a batch keeps a shape that a few of its cells do not fit)
     while (shape < FAST_SHAPES - 1 && above[shape] * 20 > act) shape++;
     c->fast.shape = shape;
-    c->fast.wide = act <= c->sms;
+    c->fast.wide = shape > 0 && act <= c->sms;
     // blocks: the fewest per SM that take as many rounds over a phase's cells as the most that fit (fewer
     // neighbours, so each round ends sooner)
     if (c->fit == 0 || !c->fast.same_kernel(c->fit_of)) {

@@ -65,7 +65,7 @@ struct FastChoice {
     int cls = 0;        // capacity class
     bool spec21 = true; // mu = 2, nu = 1, sigma0 = 1 in every replica
     bool one_k = true;  // the same pair constants in every replica: they come with the launch
-    int shape = 1;      // block shape: 0 for at most 40 particles per cell, 1 + class by class
+    int shape = 2;      // block shape: 0 for cells of a gas, 1 for at most 40 particles, 2 + class by class
     bool wide = false;  // 512 threads per cell: at most a cell per SM
     // the same kernel (the class is only a capacity)
     bool same_kernel(const FastChoice &o) const
@@ -74,7 +74,8 @@ struct FastChoice {
     }
     bool operator==(const FastChoice &o) const { return cls == o.cls && same_kernel(o); }
 };
-constexpr int FAST_SHAPES = 4;
+constexpr int FAST_SHAPES = 5;
+constexpr int FAST_SPARSE = 32; // most particles of a cell of shape 0
 int fast_shape_candidates(int shape); // places of the static cells' particles
 int fast_variant_count();
 FastVariant fast_variant(int i);

@@ -1138,11 +1138,13 @@ __global__ void __launch_bounds__(NT) k_phase_rescue(const __grid_constant__ Dev
 namespace lcmc {
 
 // Capacity classes: (active particles, places of the static cells' particles, list entries).
-// "Light" is the 48-particle class for systems whose capacity rule asks for at most 40.
+// "Light" is the 48-particle class for systems whose capacity rule asks for at most 40, "sparse" for gases.
+#define FAST32 32, 336, 2048
 #define FAST40 40, 780, 2688
 #define FAST48 48, 832, 3456
 #define FAST56 56, 1040, 4096
 #define FAST64 64, 1440, 5376
+static_assert(sizeof(FastSmem<FAST32>) + 1024 <= 233472 / 10, "sparse: ten blocks per SM");
 static_assert(sizeof(FastSmem<FAST40>) + 1024 <= 233472 / 6, "light: six blocks per SM");
 static_assert(sizeof(FastSmem<FAST48>) + 1024 <= 233472 / 5, "48-class: five blocks per SM");
 static_assert(sizeof(FastSmem<FAST56>) + 1024 <= 233472 / 4, "56-class: four blocks per SM");
@@ -1155,7 +1157,7 @@ FastVariant fast_variant(int i) { return kVariants[i]; }
 static constexpr int shape_candidates(int, int ccap, int) { return ccap; }
 int fast_shape_candidates(int shape)
 {
-    constexpr int n[FAST_SHAPES] = {shape_candidates(FAST40), shape_candidates(FAST48), shape_candidates(FAST56),
+    constexpr int n[FAST_SHAPES] = {shape_candidates(FAST32), shape_candidates(FAST40), shape_candidates(FAST48), shape_candidates(FAST56),
                                     shape_candidates(FAST64)};
     return n[shape];
 }
@@ -1183,6 +1185,8 @@ struct FastLaunch {
 // 1.66), sixteen where it has not and a phase takes one cell's latency (32,768
 // rods NPT: 0.19 ms against 0.30 with four).  The light shape holds six blocks
 // per SM where the class's own 48-particle arrays leave five (1.48 against 1.60).
+// The sparse one takes two warps per cell: the cells of a gas have a few particles
+// with some hundred neighbours, and what counts is how many are in flight.
 // The kernel of a variant: shape, wide (a block per SM), specialisation (mu = 2,
 // nu = 1, sigma0 = 1; of that, whether all replicas have the same pair constants,
 // which then come as a kernel argument).  Twelve systems of 30,000 rods of three
@@ -1195,9 +1199,10 @@ static auto with_variant(const FastChoice &c, F f)
     (!c.spec21 ? f(FastLaunch<NT, MINB, __VA_ARGS__, false, false>())                                                  \
                : c.one_k ? f(FastLaunch<NT, MINB, __VA_ARGS__, true, true>()) : f(FastLaunch<NT, MINB, __VA_ARGS__, true, false>()))
 #define FAST_PICK(MINB, ...) (c.wide ? FAST_SPEC(512, 1, __VA_ARGS__) : FAST_SPEC(128, MINB, __VA_ARGS__))
-    if (c.shape == 0) return FAST_PICK(6, FAST40);
-    if (c.shape == 1) return FAST_PICK(5, FAST48);
-    if (c.shape == 2) return FAST_PICK(4, FAST56);
+    if (c.shape == 0) return FAST_SPEC(64, 10, FAST32);
+    if (c.shape == 1) return FAST_PICK(6, FAST40);
+    if (c.shape == 2) return FAST_PICK(5, FAST48);
+    if (c.shape == 3) return FAST_PICK(4, FAST56);
     return FAST_PICK(3, FAST64);
 #undef FAST_PICK
 #undef FAST_SPEC
