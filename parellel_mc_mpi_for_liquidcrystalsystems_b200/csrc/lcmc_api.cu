@@ -49,7 +49,7 @@ struct lcmc_ctx {
     unsigned long long *d_cell_pairs = nullptr, *d_cell_cands = nullptr;
     double *d_cell_abs = nullptr;
     int *d_cell_fp64 = nullptr;
-    int *d_p2c = nullptr, *d_resc_count = nullptr, *d_resc_list = nullptr;
+    int *d_p2c = nullptr, *d_resc_count = nullptr, *d_resc_next = nullptr, *d_resc_list = nullptr;
     int *d_retry_count = nullptr, *d_retry_list = nullptr;
     // FP64 colour phases (allocated when a replica first needs them)
     int *d_ex_p = nullptr;
@@ -532,6 +532,7 @@ static DevView view(const lcmc_ctx *c, int parity)
     v.cell_fp64 = c->d_cell_fp64;
     v.p2c = c->d_p2c;
     v.resc_count = c->d_resc_count;
+    v.resc_next = c->d_resc_next;
     v.retry_count = c->d_retry_count;
     v.retry_list = c->d_retry_list;
     v.nphase = c->nphase;
@@ -592,7 +593,7 @@ static void free_ctx(lcmc_ctx *c)
                     c->d_perm, c->d_scid, c->d_cell_count, c->d_cell_start, c->d_block_sums, c->d_flag, c->d_cell_e0,
                     c->d_cell_e1, c->d_cell_n0, c->d_cell_n1, c->d_cell_pairs, c->d_cell_cands, c->d_outcome,
                     c->d_pe0, c->d_pe1, c->d_phard, c->d_red, c->d_red_part, c->d_cell_abs, c->d_cell_fp64,
-                    c->d_rec_dE, c->d_rec_lu, c->d_p2c, c->d_resc_count, c->d_resc_list, c->d_retry_count, c->d_retry_list, c->d_ex_p, c->d_ex_r, c->d_ex_flag,
+                    c->d_rec_dE, c->d_rec_lu, c->d_p2c, c->d_resc_count, c->d_resc_next, c->d_resc_list, c->d_retry_count, c->d_retry_list, c->d_ex_p, c->d_ex_r, c->d_ex_flag,
                     c->d_ex_rows};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -1008,6 +1009,7 @@ extern "C" int lcmc_create_batch(const lcmc_params *params, int n, lcmc_ctx **ou
     ALLOC(c->d_cell_fp64, c->ctot);
     ALLOC(c->d_p2c, c->ctot);
     ALLOC(c->d_resc_count, c->nphase * c->ngroup);
+    ALLOC(c->d_resc_next, c->nphase * c->ngroup);
     ALLOC(c->d_resc_list, (size_t)c->nphase * c->ngroup * c->ctot);
     ALLOC(c->d_retry_count, c->nphase * c->ngroup);
     ALLOC(c->d_retry_list, (size_t)c->nphase * c->ngroup * c->act_max);
@@ -1045,6 +1047,7 @@ extern "C" int lcmc_create_batch(const lcmc_params *params, int n, lcmc_ctx **ou
         for (int i = 0; i < c->rep[r].nc_max * c->rep[r].nc_max * c->rep[r].nc_max; i++) p2c[c->rep[r].cell_off + i] = r;
     cudaMemcpy(c->d_p2c, p2c.data(), sizeof(int) * c->ctot, cudaMemcpyHostToDevice);
     cudaMemset(c->d_resc_count, 0, sizeof(int) * c->nphase * c->ngroup);
+    cudaMemset(c->d_resc_next, 0, sizeof(int) * c->nphase * c->ngroup);
     cudaMemset(c->d_retry_count, 0, sizeof(int) * c->nphase * c->ngroup);
     cudaMemset(c->d_stats, 0, sizeof(DevStats) * n);
     cudaMemset(c->d_outcome, 0, c->ntot);
@@ -1167,6 +1170,7 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
         vg.r_lo = c->grp_lo[g];
         vg.r_hi = c->grp_hi[g];
         vg.resc_count = c->d_resc_count + (size_t)g * c->nphase;
+        vg.resc_next = c->d_resc_next + (size_t)g * c->nphase;
         vg.retry_count = c->d_retry_count + (size_t)g * c->nphase;
         vg.retry_list = c->d_retry_list + (size_t)g * c->nphase * c->act_max;
         vg.resc_list = c->d_resc_list + (size_t)g * c->nphase * c->ctot;

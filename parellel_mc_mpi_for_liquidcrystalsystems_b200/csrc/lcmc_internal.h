@@ -176,6 +176,7 @@ struct DevView {
     int *p2c;                  // [ctot] replica of each cell slot
     int *resc_count;           // [nphase] cells the FP32 kernel handed over to the FP64 kernel, per colour phase
                                // (per group: a group's view points at its own nphase counts and lists)
+    int *resc_next;            // [nphase] of those, the next one a block of the hand-over kernel takes
     int *resc_list;            // [nphase x ctot] their codes: cell * 4 + mode (1 large term, 2 capacity)
     int *retry_count;          // [nphase] cells above the light or class kernel's own capacity, run again in FP32 with
     int *retry_list;           // the largest one: [nphase x act_max] indices into act_tab (per group likewise)

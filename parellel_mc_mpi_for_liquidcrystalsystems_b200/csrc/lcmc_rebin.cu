@@ -78,6 +78,7 @@ __global__ void k_sweep_setup(DevView v)
     __syncthreads();
     for (int i = threadIdx.x; i < v.nphase * v.ngroup; i += blockDim.x) {
         v.resc_count[i] = 0;
+        v.resc_next[i] = 0;
         v.retry_count[i] = 0;
     }
     if ((int)threadIdx.x < v.nphase) {
