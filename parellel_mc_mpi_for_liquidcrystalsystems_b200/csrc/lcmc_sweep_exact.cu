@@ -147,10 +147,14 @@ __device__ __forceinline__ void cell_stencil(const DevView &v, CellView &c, int 
 // run in ex_nb batches of cells.  A cell above a capacity (particles, stencil,
 // in-cutoff terms, terms after the own cell in one lane) is attempted by
 // k_exact_decide the sequential way (exact_cell_sequential).
+// The stencil's and the terms' capacity reach to cutoffs of 5 and 6 in a liquid: 8000
+// rods at 0.30 and a cutoff of 5, 125 in a cell, 101 -> 0.97 ms of phases a sweep
+// (96 chunks and 640 terms before; one warp per cell without records 88); the
+// arrays cost the terms kernel no resident block.
 // ---------------------------------------------------------------------------
 constexpr int EX_NA = 256;   // particles of a cell
-constexpr int EX_CH = 96;    // chunks of 32 stencil slots
-constexpr int EX_ENT = 640;  // in-cutoff terms of a particle
+constexpr int EX_CH = 128;   // chunks of 32 stencil slots
+constexpr int EX_ENT = 1024; // in-cutoff terms of a particle
 constexpr int EX_SUF = 12;   // static terms after the own cell, per lane
 constexpr int EX_J = 9;      // most chunks an own cell touches
 
@@ -456,7 +460,11 @@ __device__ __noinline__ void exact_cell_sequential(const DevView *__restrict__ v
 {
     const DevView &v = *vp;
     const Replica &p = v.rep[c.r];
-    const int cell = c.cell;
+    // (held in registers: the stores of the accepted states might change them, for all the compiler knows)
+    double *const px = v.px, *const py = v.py, *const pz = v.pz, *const ox = v.ox, *const oy = v.oy, *const oz = v.oz;
+    const double L[3] = {p.L[0], p.L[1], p.L[2]};
+    const GBConsts k = p.k;
+    const int cell = c.cell, ncell = c.ncell;
     const int cs = c.cs, ce = c.cs + c.na;
     double dE_sum = 0.0, dE_abs = 0.0;
     int nacc = 0, nhard = 0;
@@ -477,47 +485,47 @@ __device__ __noinline__ void exact_cell_sequential(const DevView *__restrict__ v
             nhard += code == 1;
             continue;
         }
-        const double ro[3] = {v.px[g], v.py[g], v.pz[g]}, eo[3] = {v.ox[g], v.oy[g], v.oz[g]};
+        const double ro[3] = {px[g], py[g], pz[g]}, eo[3] = {ox[g], oy[g], oz[g]};
         const double rn[3] = {v.tnx[g], v.tny[g], v.tnz[g]}, en[3] = {v.tux[g], v.tuy[g], v.tuz[g]};
         double po = 0.0, pn = 0.0;
         int np = 0;
-        for (int s = 0; s < c.ncell; s++) {
+        for (int s = 0; s < ncell; s++) {
             const int B = s_base[s], n_s = s_base[s + 1] - B;
             const int g0 = s_first[s];
             for (int q = B + ((lane - B) & 31); q < B + n_s; q += 32) {
                 const int j = g0 + (q - B);
                 if (j == g) continue;
-                const double rj[3] = {v.px[j], v.py[j], v.pz[j]}, ej[3] = {v.ox[j], v.oy[j], v.oz[j]};
+                const double rj[3] = {px[j], py[j], pz[j]}, ej[3] = {ox[j], oy[j], oz[j]};
                 double d[3];
-                double r2 = dist_fold(ro[0], ro[1], ro[2], rj[0], rj[1], rj[2], p.L, d);
-                if (r2 < p.k.rc2) {
-                    po += pair_exact(p.k, r2, d, eo, ej);
+                double r2 = dist_fold(ro[0], ro[1], ro[2], rj[0], rj[1], rj[2], L, d);
+                if (r2 < k.rc2) {
+                    po += pair_exact(k, r2, d, eo, ej);
                     np++;
                 }
-                r2 = dist_fold(rn[0], rn[1], rn[2], rj[0], rj[1], rj[2], p.L, d);
-                if (r2 < p.k.rc2) {
-                    pn += pair_exact(p.k, r2, d, en, ej);
+                r2 = dist_fold(rn[0], rn[1], rn[2], rj[0], rj[1], rj[2], L, d);
+                if (r2 < k.rc2) {
+                    pn += pair_exact(k, r2, d, en, ej);
                     np++;
                 }
             }
         }
         double Eo = warp_sum_butterfly(po);
         double En = warp_sum_butterfly(pn);
-        if (p.k.coll_on) {
-            Eo = Eo + colloid_rod(p.k, ro, eo, p.L);
-            En = En + colloid_rod(p.k, rn, en, p.L);
+        if (k.coll_on) {
+            Eo = Eo + colloid_rod(k, ro, eo, L);
+            En = En + colloid_rod(k, rn, en, L);
         }
         const double dE = En - Eo;
-        const bool acc = (dE <= 0.0) || (lu <= -p.k.beta * dE);
+        const bool acc = (dE <= 0.0) || (lu <= -k.beta * dE);
         npairs += (unsigned long long)np;
         if (acc) {
             if (lane == 0) {
-                v.px[g] = rn[0];
-                v.py[g] = rn[1];
-                v.pz[g] = rn[2];
-                v.ox[g] = en[0];
-                v.oy[g] = en[1];
-                v.oz[g] = en[2];
+                px[g] = rn[0];
+                py[g] = rn[1];
+                pz[g] = rn[2];
+                ox[g] = en[0];
+                oy[g] = en[1];
+                oz[g] = en[2];
             }
             dE_sum += dE;
             dE_abs += fabs(dE);
@@ -1172,6 +1180,10 @@ void exact_scratch_size(int ntot, long long *cap, long long *alloc, int *nb)
 void exact_init()
 {
     cudaFuncSetAttribute(k_exact_decide, cudaFuncAttributeMaxDynamicSharedMemorySize, EX_BYTES);
+    // the rest is L1, for the cells that are attempted sequentially (the default leaves it to blocks that a phase of at
+    // most a cell per SM does not have)
+    cudaFuncSetAttribute(k_exact_decide, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         (100 * (EX_BYTES + (int)sizeof(ExactShared) + 2048) + 233471) / 233472);
     cudaFuncSetAttribute(k_exact_decide_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, EX_PIPE_BYTES);
 }
 
