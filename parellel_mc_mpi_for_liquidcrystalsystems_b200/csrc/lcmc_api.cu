@@ -112,6 +112,7 @@ struct lcmc_ctx {
     bool checks_off = false; // no periodic energy checks (autotune trials)
     int grid_elem = 0, grid_exact = 0, grid_fast = 0, grid_energy = 0, grid_screen = 0;
     bool any_fast = false, any_exact = false, any_npt = false;
+    bool e_cells = true, e_particles = true; // total energies: systems summed by cells, by particles (either may be none)
     bool any_small = false; // a box may have fewer than four cells along an axis, or takes the per-particle energies
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -735,7 +736,7 @@ static int push_kernel_fields(lcmc_ctx *c)
 // kernels are launched all the time.
 static void box_launches(lcmc_ctx *c)
 {
-    c->any_exact = c->any_small = false;
+    c->any_exact = c->any_small = c->e_cells = c->e_particles = false;
     c->safe_sweeps = 1ll << 40;
     c->since_choice = 0;
     c->nrun = 8;
@@ -758,6 +759,12 @@ static void box_launches(lcmc_ctx *c)
         if (rp.kernel == 0 || small) n64 += rp.n;
         c->ex_need = std::max(c->ex_need, n64);
         c->any_small = c->any_small || small || !rp.vol_cells;
+        // total energy by cells from ENERGY_PER_CELL particles in each on (an NPT box may take any count up to nc_max)
+        long long cells = 1;
+        for (int a = 0; a < 3; a++)
+            cells *= rp.ensemble == 2 ? rp.nc_max : std::min(grid_dim_host(rp.L[a], rp.wmin, rp.fine), rp.nc_max);
+        c->e_cells = c->e_cells || rp.ensemble == 2 || (!small && rp.n >= ENERGY_PER_CELL * cells);
+        c->e_particles = c->e_particles || small || rp.n < ENERGY_PER_CELL * cells;
         // colours: 2 per axis, 3 on an odd count of the fine grid; an NPT box may take any count
         int ncol = rp.fine && rp.ensemble == 2 ? LCMC_MAX_COLOURS : 1;
         for (int a = 0; a < 3 && ncol < LCMC_MAX_COLOURS; a++) {
@@ -1150,7 +1157,10 @@ extern "C" int lcmc_set_kernel(lcmc_ctx *ctx, int kernel)
 // ---------------------------------------------------------------------------
 
 // Rebin into the other buffer: afterwards the current buffer is cur ^ 1.
-static void enqueue_rebin(lcmc_ctx *c, int parity) { launch_rebin(view(c, parity), c->stream, c->grid_elem); }
+static void enqueue_rebin(lcmc_ctx *c, int parity, bool trials)
+{
+    launch_rebin(view(c, parity), c->stream, c->grid_elem, trials);
+}
 
 // One sweep; the event records become event nodes of the captured graph and
 // time its parts on the device (lcmc_last_sweep_timing).
@@ -1159,7 +1169,7 @@ static void enqueue_sweep(lcmc_ctx *c, int parity)
     // cudaEventRecordExternal: captured as event-record nodes (timestamps), not
     // as internal dependencies
     cudaEventRecordWithFlags(c->ev[0], c->stream, cudaEventRecordExternal);
-    enqueue_rebin(c, parity);
+    enqueue_rebin(c, parity, true);
     cudaEventRecordWithFlags(c->ev[1], c->stream, cudaEventRecordExternal);
     DevView v = view(c, parity ^ 1);
     if (c->any_exact) launch_exact_offsets(v, c->stream);
@@ -1277,10 +1287,10 @@ static int check_flags(lcmc_ctx *c)
 // energy_check_interval): rebin, FP64 total energy, compare and reset.
 static void enqueue_energy_check(lcmc_ctx *c, int all)
 {
-    enqueue_rebin(c, c->cur);
+    enqueue_rebin(c, c->cur, false);
     c->cur ^= 1;
     DevView v = view(c, c->cur);
-    launch_total_energy(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_energy, true, c->any_small);
+    launch_total_energy(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_energy, true, c->e_cells, c->e_particles);
     launch_energy_check(v, c->stream, c->d_pe0, all);
 }
 
@@ -1645,10 +1655,10 @@ extern "C" int lcmc_last_sweep_timing(lcmc_ctx *ctx, double ms[4])
 // the FP64 kernel; resets the running energies.
 static int recompute_energy(lcmc_ctx *c, int replica_only, bool cells)
 {
-    enqueue_rebin(c, c->cur);
+    enqueue_rebin(c, c->cur, false);
     c->cur ^= 1;
     DevView v = view(c, c->cur);
-    launch_total_energy(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_energy, cells, c->any_small);
+    launch_total_energy(v, c->stream, c->d_pe0, c->d_pe1, c->d_phard, c->grid_energy, cells, c->e_cells, c->e_particles);
     launch_energy_reduce(v, c->stream, c->d_pe0, replica_only, cells);
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     CUDA_TRY(c, cudaGetLastError());

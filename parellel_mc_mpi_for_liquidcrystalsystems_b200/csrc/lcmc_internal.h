@@ -134,6 +134,11 @@ struct alignas(16) ActRec {
     int code, id, pad; // trial code (thard), particle id
 };
 
+// Particles per cell from which on the total energy is summed by cells: a block per
+// cell has little to do in a gas (200,000 rods, lcmc_total_energy by cells and by
+// particles: 3.8 to a cell 474 and 378 us, 7.5 to a cell 299 and 413).
+constexpr int ENERGY_PER_CELL = 5;
+
 // Launch view of the device buffers, passed by value to every kernel.
 // particles per chunk of the two-level reductions (sums over a replica)
 constexpr int LCMC_RED_CHUNK = 4096;

@@ -39,7 +39,7 @@ __device__ __forceinline__ void phase_begin()
 #endif
 
 // lcmc_rebin.cu
-void launch_rebin(const DevView &v, cudaStream_t s, int grid);
+void launch_rebin(const DevView &v, cudaStream_t s, int grid, bool trials); // trials: the sweep's trial moves too
 // per-cell results of the colour phases into the statistics and the running
 // energy (before the volume move); then the sweep counter and adaptive step
 void launch_sweep_stats(const DevView &v, cudaStream_t s);
@@ -53,7 +53,7 @@ void launch_phase_exact(const DevView &v, cudaStream_t s, int ci, int grid);
 void launch_volume_energies(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid,
                             bool per_particle);
 void launch_total_energy(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid, bool cells,
-                         bool per_particle);
+                         bool by_cells, bool per_particle);
 int energy_exact_blocks_per_sm(); // resident blocks of 128 threads per SM
 
 // lcmc_sweep_fast.cu (FP32)

@@ -216,7 +216,7 @@ __global__ void k_scatter(DevView v)
         v.perm[v.cell_start[v.cid[i]] + v.rank[i]] = i;
 }
 
-// Thread per cell: enters it in the table of its colour phase's active cells, so
+// Thread per cell, for a sweep: enters it in the table of its colour phase's active cells, so
 // that the phase kernels find a cell with one load (their order is the
 // enumeration of act_off: x fastest).  A cell without particles has its results
 // here: the phase kernels pass it by (a gas of 0.002, 362,000 cells, 87 % of them
@@ -224,9 +224,9 @@ __global__ void k_scatter(DevView v)
 // Warp per cell: order the cell's slots by particle id (ids are unique inside
 // a replica).  Writes the gather source of every destination slot to `rank`
 // (reused as the second permutation buffer).
-__global__ void k_sort_cells(DevView v)
+__global__ void k_sort_cells(DevView v, bool sweep)
 {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < v.ctot; c += gridDim.x * blockDim.x) {
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; sweep && c < v.ctot; c += gridDim.x * blockDim.x) {
         const int r = v.p2c[c];
         const Replica &p = v.rep[r];
         const int l = c - p.cell_off, nc0 = p.nc[0], nc1 = p.nc[1];
@@ -268,12 +268,22 @@ __global__ void k_sort_cells(DevView v)
     }
 }
 
-// Permute into the other buffer and build this sweep's trial move of every
-// particle (a particle is attempted once per sweep from its sweep-start state,
+// FP32 copy of a particle's state: (x, y, z, ux) and (uy, uz), the position relative to its own cell's origin.
+__device__ __forceinline__ void fp32_copy(const Replica &p, int cx, int cy, int cz, const double r[3], const double e[3],
+                                          float4 &c4, float2 &c2)
+{
+    c4.x = (float)fold_rel(r[0], p.shift[0] + (double)cx * p.w[0], 0.5 * p.w[0], p.L[0], 1.0 / p.L[0]);
+    c4.y = (float)fold_rel(r[1], p.shift[1] + (double)cy * p.w[1], 0.5 * p.w[1], p.L[1], 1.0 / p.L[1]);
+    c4.z = (float)fold_rel(r[2], p.shift[2] + (double)cz * p.w[2], 0.5 * p.w[2], p.L[2], 1.0 / p.L[2]);
+    unit_f32(e[0], e[1], e[2], c4.w, c2.x, c2.y);
+}
+
+// Permute into the other buffer and, for a sweep (trials), build the trial move of
+// every particle (a particle is attempted once per sweep from its sweep-start state,
 // so the trial is known now): new state, log of the Metropolis draw, trial code,
 // and for systems on the FP32 kernel the colloid-term change and the FP32 copies
 // of both states (the phase kernels then do no FP64 square root or division).
-__global__ void k_gather(DevView v)
+__global__ void k_gather(DevView v, bool trials)
 {
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < v.ntot; g += gridDim.x * blockDim.x) {
         int src = v.rank[g];
@@ -289,10 +299,20 @@ __global__ void k_gather(DevView v)
         v.qid[g] = id;
         v.scid[g] = v.cid[src];
         const Replica &p = v.rep[v.p2r[g]];
-        double rn[3], en[3], dsp[3], u;
-        const int ok = make_trial(p, (uint32_t)id, ro, eo, rn, en, dsp, &u);
         const int cl = v.cid[src] - p.cell_off;
         const int cx = cl % p.nc[0], cy = (cl / p.nc[0]) % p.nc[1], cz = cl / (p.nc[0] * p.nc[1]);
+        if (!trials) {
+            if (p.use_fast) {
+                float4 a;
+                float2 b;
+                fp32_copy(p, cx, cy, cz, ro, eo, a, b);
+                v.cl4[g] = a;
+                v.cl2[g] = b;
+            }
+            continue;
+        }
+        double rn[3], en[3], dsp[3], u;
+        const int ok = make_trial(p, (uint32_t)id, ro, eo, rn, en, dsp, &u);
         // 0 trial to evaluate, 1 colloid hard-core reject, 3 leaves its cell (rejected)
         const unsigned char code = !ok ? 1 : (leaves_cell(p, cx, cy, cz, ro, dsp) ? 3 : 0);
         v.tnx[g] = rn[0];
@@ -306,21 +326,18 @@ __global__ void k_gather(DevView v)
         if (!p.use_fast) continue;
         double dU = 0.0;
         if (code == 0 && p.k.coll_on) dU = colloid_rod(p.k, rn, en, p.L) - colloid_rod(p.k, ro, eo, p.L);
-        // FP32 copy relative to the particle's own cell origin
-        const double lx = fold_rel(ro[0], p.shift[0] + (double)cx * p.w[0], 0.5 * p.w[0], p.L[0], 1.0 / p.L[0]);
-        const double ly = fold_rel(ro[1], p.shift[1] + (double)cy * p.w[1], 0.5 * p.w[1], p.L[1], 1.0 / p.L[1]);
-        const double lz = fold_rel(ro[2], p.shift[2] + (double)cz * p.w[2], 0.5 * p.w[2], p.L[2], 1.0 / p.L[2]);
-        float ux, uy, uz;
-        unit_f32(eo[0], eo[1], eo[2], ux, uy, uz);
-        v.cl4[g] = make_float4((float)lx, (float)ly, (float)lz, ux);
-        v.cl2[g] = make_float2(uy, uz);
+        float4 c4;
+        float2 c2;
+        fp32_copy(p, cx, cy, cz, ro, eo, c4, c2);
+        v.cl4[g] = c4;
+        v.cl2[g] = c2;
         float bx, by, bz;
         unit_f32(en[0], en[1], en[2], bx, by, bz);
         const float dx = (float)dsp[0], dy = (float)dsp[1], dz = (float)dsp[2];
         ActRec ar;
-        ar.p0 = make_float4((float)lx, (float)lx + dx, (float)ly, (float)ly + dy);
-        ar.p1 = make_float4((float)lz, (float)lz + dz, ux, bx);
-        ar.p2 = make_float4(uy, by, uz, bz);
+        ar.p0 = make_float4(c4.x, c4.x + dx, c4.y, c4.y + dy);
+        ar.p1 = make_float4(c4.z, c4.z + dz, c4.w, bx);
+        ar.p2 = make_float4(c2.x, by, c2.y, bz);
         ar.tdU = dU;
         ar.tlu = log_unit(u);
         ar.reach = sqrtf(dx * dx + dy * dy + dz * dz);
@@ -433,7 +450,7 @@ __global__ void k_sweep_advance(DevView v)
 
 namespace lcmc {
 
-void launch_rebin(const DevView &v, cudaStream_t s, int grid)
+void launch_rebin(const DevView &v, cudaStream_t s, int grid, bool trials)
 {
     k_sweep_setup<<<1, 1024, 0, s>>>(v);
     cudaMemsetAsync(v.cell_count, 0, sizeof(int) * (size_t)v.ctot, s);
@@ -443,8 +460,8 @@ void launch_rebin(const DevView &v, cudaStream_t s, int grid)
     k_scan_sums<<<1, SCAN_BLOCK, 0, s>>>(v, tiles);
     k_scan_apply<<<tiles, SCAN_BLOCK, 0, s>>>(v);
     k_scatter<<<grid, 256, 0, s>>>(v);
-    k_sort_cells<<<grid, 256, 0, s>>>(v);
-    k_gather<<<grid, 256, 0, s>>>(v);
+    k_sort_cells<<<grid, 256, 0, s>>>(v, trials);
+    k_gather<<<grid, 256, 0, s>>>(v, trials);
 }
 
 void launch_sweep_stats(const DevView &v, cudaStream_t s)

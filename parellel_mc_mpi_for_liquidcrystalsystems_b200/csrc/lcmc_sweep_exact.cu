@@ -1237,13 +1237,15 @@ void launch_volume_energies(const DevView &v, cudaStream_t s, double *e0, double
     if (per_particle) k_energy_exact<true><<<grid, 128, 0, s>>>(v, e0, e1, hard, false);
 }
 
-// The total energy, likewise; cells = false: per particle for every system.
+// The total energy, likewise (by_cells: there may be systems the cell kernel
+// serves); cells = false: per particle for every system.
 // That is the order an uploaded configuration's energy is summed in: a start
 // with overlapping rods has terms of 1e20 and more, whose rounding stays in the
 // running energy after the overlaps have gone.
 void launch_total_energy(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid, bool cells,
-                         bool per_particle)
+                         bool by_cells, bool per_particle)
 {
+    cells = cells && by_cells;
     if (cells) k_cell_energy<2, false><<<cell_energy_grid<2>(), 128, 0, s>>>(v);
     if (!cells || per_particle) k_energy_exact<false><<<grid, 128, 0, s>>>(v, e0, e1, hard, !cells);
 }

@@ -58,7 +58,7 @@ template <int MODE>
 __device__ __forceinline__ bool cells_serve(const Replica &p)
 {
     const bool grid = p.nc[0] >= 4 && p.nc[1] >= 4 && p.nc[2] >= 4;
-    if (MODE == 2) return grid;
+    if (MODE == 2) return grid && p.n >= ENERGY_PER_CELL * (p.nc[0] * p.nc[1] * p.nc[2]);
     if (p.ensemble != 2) return false;
     if (MODE == 1) return p.da_kind == 2 && p.use_fast;
     if (p.da_on && !p.vol_stage1) return false; // screened out: no exact recompute
