@@ -456,9 +456,9 @@ __global__ void k_bias_act(float *Z, const float *bias, bf16 *Hb, bf16 *HbT, int
 
 // Second hidden layer and output, warp per row: Z2 += b2, A2 = silu(Z2),
 // y = A2 . w3 + b3; with a target also dy = 2 (y - t) / n_valid for rows <
-// n_valid, and the loss added up in *loss.
+// n_valid and the row's share of the loss.
 __global__ void k_act_out(float *Z2, const float *b2, const float *w3, const float *b3, float *A2, float *y,
-                          const float *target, float *dy, float *loss, int Bn, int Hn, int n_valid)
+                          const float *target, float *dy, float *row_loss, int Bn, int Hn, int n_valid)
 {
     const int lane = threadIdx.x & 31;
     for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < Bn; r += (gridDim.x * blockDim.x) >> 5) {
@@ -477,70 +477,87 @@ __global__ void k_act_out(float *Z2, const float *b2, const float *w3, const flo
             if (target) {
                 const float e = r < n_valid ? v - target[r] : 0.0f;
                 dy[r] = 2.0f * e / (float)n_valid;
-                atomicAdd(loss, e * e / (float)n_valid);
+                row_loss[r] = e * e / (float)n_valid;
             }
         }
     }
 }
 
-// The gradients of b1, w3, b3 and the loss are sums over the batch by atomics, in
-// the order in which the rows come to them, so their last bits differ from run to
-// run, and a training call's results with them: BF16 rounding of dZ turns a last
-// bit into 2^-9 of an element, and Adam divides a gradient by its size, so the
-// step of a weight whose gradient is nearly zero may turn.  Eight steps of 256
-// rows, 320 seeds, two runs of each: relative difference of the weights 1.2e-7 in
-// the median, 1.2e-5 in the 98th percentile, 1.3e-4 at most.  Sums in the rows'
-// order (a block per four columns) took 2.33 instead of 2.37 ms for such a call,
-// but are one more order beside these, and were taken back.
+// A layer's backward pass by columns: a block takes BK_COLS of the Hn columns and
+// every row.  The sums over the batch are the block's own (no atomics, nothing to
+// clear) and run in the rows' order, from shared memory, a thread per sum: 256
+// dependent additions take 0.6 us, less than one more launch (a call of 2048 rows
+// 2.33 ms, with sums by atomics 2.37).
+// A training call so gives the same bits every time.  By atomics two of its runs
+// differ: a last bit of a sum turns, through BF16 rounding of dZ, into 2^-9 of an
+// element, and Adam divides a gradient by its size, so the step of a weight whose
+// gradient is nearly zero may turn.  Relative difference of the weights, 160 seeds,
+// eight steps / sixteen steps of 256 rows: two runs by atomics 1e-7 / 6e-6 in the
+// median and above 2e-5 in 1 % / 27 % of the seeds; the rows' order against either
+// 2e-7 / 6e-6, 1 % / 24 %.
+constexpr int BK_COLS = 4, BK_THREADS = 256, BK_ROWS = BK_THREADS / BK_COLS;
 
-// dZ2 = (dy w3) * silu'(Z2), in BF16 (B x H and its transpose) and FP32; the
-// gradients of w3 and b3 added up
-__global__ void k_back_out(const float *dy, const float *w3, const float *Z2, const float *A2, float *gw3, float *gb3,
-                           bf16 *dZ2b, bf16 *dZ2bT, float *dZ2f, int Bn, int Hn)
+// dZ2 = (dy w3) * silu'(Z2) in BF16 (B x H and its transpose); gradients of w3
+// and b2, and (block 0) of b3 and the batch loss.
+__global__ void __launch_bounds__(BK_THREADS) k_back_out(const float *dy, const float *row_loss, const float *w3,
+                                                         const float *Z2, const float *A2, float *gw3, float *gb2,
+                                                         float *gb3, float *loss, bf16 *dZ2b, bf16 *dZ2bT, int Bn, int Hn)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Bn * Hn; i += gridDim.x * blockDim.x) {
-        const int b = i / Hn, h = i % Hn;
-        const float g = dy[b] * w3[h] * dsilu(Z2[i]);
-        const bf16 gb = __float2bfloat16(g);
-        dZ2b[i] = gb;
-        dZ2bT[(size_t)h * Bn + b] = gb;
-        dZ2f[i] = g;
-        atomicAdd(&gw3[h], dy[b] * A2[i]);
-        if (h == 0) atomicAdd(gb3, dy[b]);
-    }
-}
-
-// dZ1 = dH1 * silu'(Z1) -> dZ1^T (H x B) in BF16; the gradient of b1 added up
-__global__ void k_back_hidden(const float *dH, const float *Z, bf16 *dZbT, float *gbias, int Bn, int Hn)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Bn * Hn; i += gridDim.x * blockDim.x) {
-        const int b = i / Hn, h = i % Hn;
-        const float g = dH[i] * dsilu(Z[i]);
-        dZbT[(size_t)h * Bn + b] = __float2bfloat16(g);
-        atomicAdd(&gbias[h], g);
-    }
-}
-
-// Column sums in the rows' order: a block takes CS_COLS of the Hn columns, the
-// rows come into shared memory by all its threads, and a thread per column adds
-// them up (256 dependent additions take 0.6 us).
-constexpr int CS_COLS = 4, CS_THREADS = 256, CS_ROWS = CS_THREADS / CS_COLS;
-__global__ void __launch_bounds__(CS_THREADS) k_colsum(const float *X, float *out, int Bn, int Hn)
-{
-    __shared__ float term[CS_COLS][CS_THREADS];
-    const int c = threadIdx.x % CS_COLS, h = blockIdx.x * CS_COLS + c;
+    __shared__ float term[2 * BK_COLS + 2][BK_THREADS]; // per column: w3, b2; then b3 and the loss
+    const int c = threadIdx.x % BK_COLS, h = blockIdx.x * BK_COLS + c;
     float sum = 0.0f;
-    for (int b0 = 0; b0 < Bn; b0 += CS_THREADS) {
-        const int rows = min(CS_THREADS, Bn - b0);
+    for (int b0 = 0; b0 < Bn; b0 += BK_THREADS) {
+        const int rows = min(BK_THREADS, Bn - b0);
         __syncthreads();
-        for (int r = threadIdx.x / CS_COLS; r < rows; r += CS_ROWS) term[c][r] = X[(size_t)(b0 + r) * Hn + h];
+        for (int r = threadIdx.x / BK_COLS; r < rows; r += BK_ROWS) {
+            const int b = b0 + r;
+            const size_t i = (size_t)b * Hn + h;
+            const float d = dy[b], g = d * w3[h] * dsilu(Z2[i]);
+            const bf16 gb = __float2bfloat16(g);
+            dZ2b[i] = gb;
+            dZ2bT[(size_t)h * Bn + b] = gb;
+            term[c][r] = __fmul_rn(d, A2[i]);
+            term[BK_COLS + c][r] = g;
+            if (c == 0) {
+                term[2 * BK_COLS][r] = d;
+                term[2 * BK_COLS + 1][r] = row_loss[b];
+            }
+        }
         __syncthreads();
-        if (threadIdx.x < CS_COLS) {
+        if (threadIdx.x < 2 * BK_COLS + 2) {
 #pragma unroll 16
             for (int r = 0; r < rows; r++) sum += term[threadIdx.x][r];
         }
     }
-    if (threadIdx.x < CS_COLS) out[h] = sum;
+    const int t = threadIdx.x;
+    if (t < BK_COLS) gw3[h] = sum;
+    else if (t < 2 * BK_COLS) gb2[h] = sum;
+    else if (t < 2 * BK_COLS + 2 && blockIdx.x == 0) (t == 2 * BK_COLS ? gb3 : loss)[0] = sum;
+}
+
+// dZ1 = dH1 * silu'(Z1) -> dZ1^T (H x B) in BF16, and the gradient of b1
+__global__ void __launch_bounds__(BK_THREADS) k_back_hidden(const float *dH, const float *Z, bf16 *dZbT, float *gbias,
+                                                            int Bn, int Hn)
+{
+    __shared__ float term[BK_COLS][BK_THREADS];
+    const int c = threadIdx.x % BK_COLS, h = blockIdx.x * BK_COLS + c;
+    float sum = 0.0f;
+    for (int b0 = 0; b0 < Bn; b0 += BK_THREADS) {
+        const int rows = min(BK_THREADS, Bn - b0);
+        __syncthreads();
+        for (int r = threadIdx.x / BK_COLS; r < rows; r += BK_ROWS) {
+            const size_t i = (size_t)(b0 + r) * Hn + h;
+            const float g = dH[i] * dsilu(Z[i]);
+            dZbT[(size_t)h * Bn + b0 + r] = __float2bfloat16(g);
+            term[c][r] = g;
+        }
+        __syncthreads();
+        if (threadIdx.x < BK_COLS) {
+#pragma unroll 16
+            for (int r = 0; r < rows; r++) sum += term[threadIdx.x][r];
+        }
+    }
+    if (threadIdx.x < BK_COLS) gbias[h] = sum;
 }
 
 // rows pos[r] of the data set -> row r of X (16 bytes per thread and step)
@@ -626,7 +643,7 @@ struct lcmc_mlp {
     bf16 *W1b = nullptr, *W2b = nullptr, *W2bT = nullptr;
     // activations (bmax rows)
     bf16 *X = nullptr, *XT = nullptr, *H1 = nullptr, *H1T = nullptr, *dZ2 = nullptr, *dZ2T = nullptr, *dZ1T = nullptr;
-    float *Z1 = nullptr, *Z2 = nullptr, *A2 = nullptr, *y = nullptr, *t = nullptr, *dy = nullptr, *dZ2f = nullptr,
+    float *Z1 = nullptr, *Z2 = nullptr, *A2 = nullptr, *y = nullptr, *t = nullptr, *dy = nullptr, *row_loss = nullptr,
           *dH1 = nullptr, *loss = nullptr;
     int *err = nullptr;
     // host rows on their way to the device
@@ -656,7 +673,7 @@ extern "C" int lcmc_mlp_destroy(lcmc_mlp *m)
     if (!m) return LCMC_EINVAL;
     if (m->s) cudaStreamSynchronize(m->s);
     void *ptrs[] = {m->P, m->G, m->Mm, m->Vv, m->W1b, m->W2b, m->W2bT, m->X, m->XT, m->H1, m->H1T, m->dZ2,
-                    m->dZ2T, m->dZ1T, m->Z1, m->Z2, m->A2, m->y, m->t, m->dy, m->dZ2f, m->dH1, m->loss,
+                    m->dZ2T, m->dZ1T, m->Z1, m->Z2, m->A2, m->y, m->t, m->dy, m->row_loss, m->dH1, m->loss,
                     m->err, m->yall, m->rows, m->et, m->losses, m->pos};
     if (m->stage) cudaFreeHost(m->stage);
     for (cudaEvent_t ev : m->sent)
@@ -729,7 +746,7 @@ extern "C" int lcmc_mlp_create(int n_in, int hidden, int max_batch, uint64_t see
     MA(m->y, (size_t)B * 4);
     MA(m->t, (size_t)B * 4);
     MA(m->dy, (size_t)B * 4);
-    MA(m->dZ2f, (size_t)B * H * 4);
+    MA(m->row_loss, (size_t)B * 4);
     MA(m->dH1, (size_t)B * H * 4);
     MA(m->loss, 4);
     MA(m->err, 4);
@@ -782,14 +799,14 @@ extern "C" int lcmc_mlp_create(int n_in, int hidden, int max_batch, uint64_t see
 }
 
 // forward on B (a multiple of 128) rows of X -> activations A2, outputs y; with
-// targets t also dy, and the batch loss added to *loss
-static void mlp_forward_s(lcmc_mlp *m, const bf16 *X, int B, const float *t, float *loss, int n_valid, cudaStream_t s)
+// targets t also dy and the rows' losses
+static void mlp_forward_s(lcmc_mlp *m, const bf16 *X, int B, const float *t, int n_valid, cudaStream_t s)
 {
     const int H = m->hid, K1 = m->k1;
     gemm_tc(X, K1, m->W1b, K1, m->Z1, H, B, H, K1, 0, m->err, s);
     k_bias_act<<<(B * H + 255) / 256, 256, 0, s>>>(m->Z1, m->b1, m->H1, m->H1T, B, H);
     gemm_tc(m->H1, H, m->W2b, H, m->Z2, H, B, H, H, 0, m->err, s);
-    k_act_out<<<(B * 32 + 255) / 256, 256, 0, s>>>(m->Z2, m->b2, m->w3, m->b3, m->A2, m->y, t, m->dy, loss, B, H,
+    k_act_out<<<(B * 32 + 255) / 256, 256, 0, s>>>(m->Z2, m->b2, m->w3, m->b3, m->A2, m->y, t, m->dy, m->row_loss, B, H,
                                                    n_valid);
 }
 
@@ -803,7 +820,7 @@ int mlp_bmax(lcmc_mlp *m) { return m->bmax; }
 int mlp_n_in(lcmc_mlp *m) { return m->n_in; }
 const float *mlp_forward_device(lcmc_mlp *m, int B, cudaStream_t s)
 {
-    mlp_forward_s(m, m->X, B, nullptr, nullptr, B, s);
+    mlp_forward_s(m, m->X, B, nullptr, B, s);
     return m->y;
 }
 int *mlp_err(lcmc_mlp *m) { return m->err; }
@@ -957,7 +974,7 @@ extern "C" int lcmc_mlp_predict(lcmc_mlp *m, const float *x, int n, float *y)
             const int B = (nb + 127) / 128 * 128;
             e = send_rows(m, rc, x + (size_t)off * m->n_in, nullptr, nb, B, m->X);
             if (e != cudaSuccess) break;
-            mlp_forward_s(m, m->X, B, nullptr, nullptr, nb, m->s);
+            mlp_forward_s(m, m->X, B, nullptr, nb, m->s);
             e = cudaMemcpyAsync(m->yall + off, m->y, (size_t)nb * 4, cudaMemcpyDeviceToDevice, m->s);
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(y, m->yall, (size_t)n * 4, cudaMemcpyDeviceToHost, m->s);
@@ -976,20 +993,16 @@ static void mlp_backward(lcmc_mlp *m, const bf16 *X, const float *t, int n, floa
 {
     const int H = m->hid, K1 = m->k1;
     const int B = (n + 127) / 128 * 128;
+    mlp_forward_s(m, X, B, t, n, m->s);
     float *gW1 = m->G, *gb1 = gW1 + (size_t)H * K1, *gW2 = gb1 + H, *gb2 = gW2 + (size_t)H * H, *gw3 = gb2 + H,
           *gb3 = gw3 + H;
-    // (the sums by atomics start from zero; everything else is written)
-    cudaMemsetAsync(gb1, 0, (size_t)H * 4, m->s);
-    cudaMemsetAsync(gw3, 0, (size_t)(H + 1) * 4, m->s);
-    cudaMemsetAsync(loss, 0, 4, m->s);
-    mlp_forward_s(m, X, B, t, loss, n, m->s);
-    k_back_out<<<(B * H + 255) / 256, 256, 0, m->s>>>(m->dy, m->w3, m->Z2, m->A2, gw3, gb3, m->dZ2, m->dZ2T, m->dZ2f, B, H);
-    k_colsum<<<H / CS_COLS, CS_THREADS, 0, m->s>>>(m->dZ2f, gb2, B, H);
+    k_back_out<<<H / BK_COLS, BK_THREADS, 0, m->s>>>(m->dy, m->row_loss, m->w3, m->Z2, m->A2, gw3, gb2, gb3, loss, m->dZ2,
+                                                     m->dZ2T, B, H);
     // dW2 = dZ2^T H1: (H x B) . (H x B)^T
     gemm_tc(m->dZ2T, B, m->H1T, B, gW2, H, H, H, B, 0, m->err, m->s);
     // dH1 = dZ2 W2: (B x H) . (W2^T)^T
     gemm_tc(m->dZ2, H, m->W2bT, H, m->dH1, H, B, H, H, 0, m->err, m->s);
-    k_back_hidden<<<(B * H + 255) / 256, 256, 0, m->s>>>(m->dH1, m->Z1, m->dZ1T, gb1, B, H);
+    k_back_hidden<<<H / BK_COLS, BK_THREADS, 0, m->s>>>(m->dH1, m->Z1, m->dZ1T, gb1, B, H);
     // dW1 = dZ1^T X: (H x B) . (X^T)^T with X^T = K1 x B
     dim3 tg((K1 + 31) / 32, (B + 31) / 32), tb(32, 8);
     k_transpose_bf16<<<tg, tb, 0, m->s>>>(X, m->XT, B, K1);

@@ -1,6 +1,6 @@
 """The sums over a batch in the surrogate's backward pass (loss, gradients of b1,
-w3, b3 by atomics; b2 in the rows' order): each call's own, whatever the call
-before it left, for batches that fill their tile of 128 rows and that do not.
+b2, w3, b3): each call's own, whatever the call before it left, for batches that
+fill their tile of 128 rows and that do not.
 
 Loss and gradient of b3 are sums of n terms that the outputs give in FP32 exactly
 as the kernel forms them; any order of n - 1 additions is within (n - 1) u of the
