@@ -930,6 +930,11 @@ extern "C" int lcmc_create_batch(const lcmc_params *params, int n, lcmc_ctx **ou
         // cell grid capacity: NVT boxes keep their size; NPT boxes may grow (then cells stay wider)
         double Lmax = rp.ensemble == 2 ? 1.25 * L : L;
         rp.nc_max = grid_dim_host(Lmax, rp.wmin, rp.fine);
+        // the scan's limit, which also keeps a cell's coordinates below 256 (k_sort_cells packs them)
+        if (coff + (long long)rp.nc_max * rp.nc_max * rp.nc_max > 4096ll * 4096ll) {
+            free_ctx(c);
+            return set_err(nullptr, LCMC_EINVAL, "cell grid too large");
+        }
         rp.cell_off = coff;
         rp.sweep = 0ull;
         poff += rp.n;
@@ -1041,10 +1046,6 @@ extern "C" int lcmc_create_batch(const lcmc_params *params, int n, lcmc_ctx **ou
     ALLOC(c->d_feat_acc, (size_t)n * 512 * 7);
     ALLOC(c->d_feat_f, (size_t)n * LCMC_FEAT);
 #undef ALLOC
-    if ((c->ctot + 4095) / 4096 > 4096) {
-        free_ctx(c);
-        return set_err(nullptr, LCMC_EINVAL, "cell grid too large");
-    }
     std::vector<int> p2r(c->ntot);
     for (int r = 0; r < n; r++)
         for (int i = 0; i < c->rep[r].n; i++) p2r[c->rep[r].p_off + i] = r;

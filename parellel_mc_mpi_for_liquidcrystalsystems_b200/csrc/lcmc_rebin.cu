@@ -242,6 +242,7 @@ __global__ void k_sort_cells(DevView v, bool sweep)
         while (ci < p.ncol - 1 && p.perm[ci] != col) ci++;
         const int a = v.act_off[ci * (v.R + 1) + r] +
                       (jz * axis_colour_count(nc1, p.kc[1], by) + jy) * axis_colour_count(nc0, p.kc[0], bx) + jx;
+        // (a context's cells are at most 2^24, so an axis has at most 256: the coordinates fit in 8 bits)
         v.act_tab[(size_t)ci * v.act_max + a] =
             make_int4(c, r, (int)((unsigned)(x | y << 8 | z << 16) | (unsigned)min(n, 255) << 24), s);
         if (n == 0) {
