@@ -1236,7 +1236,7 @@ static int ensure_exact_scratch(lcmc_ctx *c)
     const long long act = c->act_max;
     long long cap, alloc;
     int nb;
-    exact_scratch_size(c->ex_need, &cap, &alloc, &nb);
+    exact_scratch_size(c->ex_need, EX_MOST, &cap, &alloc, &nb);
     // what a captured graph holds changes: the sizes, and the rows' address where they grow
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     invalidate_graphs(c);
@@ -1249,7 +1249,18 @@ static int ensure_exact_scratch(lcmc_ctx *c)
         c->d_ex_rows = nullptr;
         c->ex_alloc = 0;
         c->ex_have = 0;
-        CUDA_TRY(c, dalloc(&c->d_ex_rows, (size_t)c->ngroup * alloc * 32));
+        // no room for it: less, down to a sixty-fourth (more batches, more cells attempted sequentially)
+        cudaError_t e = dalloc(&c->d_ex_rows, (size_t)c->ngroup * alloc * 32);
+        for (long long most = EX_MOST / 2; e == cudaErrorMemoryAllocation && most >= EX_MOST / 64; most /= 2) {
+            cudaGetLastError();
+            exact_scratch_size(c->ex_need, most, &cap, &alloc, &nb);
+            e = dalloc(&c->d_ex_rows, (size_t)c->ngroup * alloc * 32);
+        }
+        if (e != cudaSuccess) {
+            c->d_ex_rows = nullptr;
+            cudaGetLastError();
+        }
+        CUDA_TRY(c, e);
         c->ex_alloc = alloc;
     }
     c->ex_act = (int)act;

@@ -47,7 +47,8 @@ void launch_sweep_advance(const DevView &v, cudaStream_t s);
 
 // lcmc_sweep_exact.cu (FP64, bit-identical to the CPU oracle)
 void exact_init(); // before the first FP64 colour phase
-void exact_scratch_size(int ntot, long long *cap, long long *alloc, int *nb);
+constexpr long long EX_MOST = 256ll << 20 >> 9; // rows (512 bytes) of a batch
+void exact_scratch_size(int ntot, long long most, long long *cap, long long *alloc, int *nb);
 void launch_exact_offsets(const DevView &v, cudaStream_t s); // after the rebin, before the colour phases
 void launch_phase_exact(const DevView &v, cudaStream_t s, int ci, int grid);
 void launch_volume_energies(const DevView &v, cudaStream_t s, double *e0, double *e1, int *hard, int grid,

@@ -13,6 +13,8 @@
 // canonical order the oracle reproduces.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "lcmc_gb.cuh"
 #include "lcmc_internal.h"
 #include "lcmc_launch.h"
@@ -1163,18 +1165,18 @@ __global__ void __launch_bounds__(128, LCMC_ENERGY_MIN_BLOCKS) k_energy_exact(De
 namespace lcmc {
 
 // Scratch rows (of 512 bytes) for ntot particles on the FP64 kernel: *cap rows
-// per batch and *nb batches per phase.  Most systems run in one batch; the
-// bound of 256 MB keeps the rows near the L2.  Active particles of a phase are
-// about an eighth of the system (all of it in a one-cell box); cells that the
-// batches do not reach are attempted sequentially.
-void exact_scratch_size(int ntot, long long *cap, long long *alloc, int *nb)
+// per batch, at most `most` (EX_MOST, 256 MB, less where there is no room), and
+// *nb batches per phase.  Most systems run in one batch.  Active particles of a
+// phase are about an eighth of the system (all of it in a one-cell box); cells
+// that the batches do not reach are attempted sequentially.
+void exact_scratch_size(int ntot, long long most, long long *cap, long long *alloc, int *nb)
 {
-    const long long most = 256ll << 20 >> 9;
     const long long all = (long long)ntot * ex_rows_per_particle(EX_NA);
     *cap = all < most ? all : most;
     *alloc = *cap + (long long)EX_NA * ex_rows_per_particle(EX_NA);
     const long long typical = (long long)ntot * ex_rows_per_particle(64) / 4;
     *nb = all <= most ? 1 : (int)((typical + most - 1) / most) + 1;
+    if (most < EX_MOST) *nb = std::min(*nb, 16);
 }
 
 void exact_init()
