@@ -457,8 +457,8 @@ __global__ void __launch_bounds__(128) k_exact_terms(const __grid_constant__ Dev
 // the lanes split the stencil slots, evaluate the terms where they are found
 // and combine the lane sums (the canonical order again).  For cells above a
 // capacity of the two-kernel path.
-__device__ __noinline__ void exact_cell_sequential(const DevView *__restrict__ vp, const CellView &c, int lane,
-                                                   const int *s_first, const int *s_base)
+__device__ __forceinline__ void exact_cell_sequential(const DevView *__restrict__ vp, const CellView &c, int lane,
+                                                      const int *s_first, const int *s_base)
 {
     const DevView &v = *vp;
     const Replica &p = v.rep[c.r];
@@ -554,6 +554,28 @@ __device__ __noinline__ void exact_cell_sequential(const DevView *__restrict__ v
         v.cell_cands[cell] = cands;
     }
     __syncwarp();
+}
+
+// The cells of a block that were left to the sequential attempts, after its others
+// (called among them, its registers were spilled from the decisions: a gas of 20,000
+// rods 0.60 -> 0.64 ms of phases a sweep).  Warp 0.
+__device__ __noinline__ void exact_cells_left(const DevView *__restrict__ vp, const ExactBatch eb, int ci, int a1, int *s_first,
+                                              int *s_base)
+{
+    const DevView &v = *vp;
+    const int *off = v.act_off + ci * (v.R + 1);
+    const int lane = threadIdx.x & 31;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    for (int a = eb.lo + blockIdx.x; a < a1; a += gridDim.x) {
+        if (a < eb.hi && !v.ex_flag[(size_t)ci * v.ex_act + a]) continue;
+        CellView c;
+        active_cell(v, off, ci, a, c);
+        if (v.rep[c.r].use_fast || c.na == 0) continue;
+        cell_stencil(v, c, lane, s_first, s_base);
+        exact_cell_sequential(vp, c, lane, s_first, s_base);
+        __syncwarp();
+    }
 }
 
 // The attempts of one cell (J chunks of own-cell slots), D = 3 at a time: attempt
@@ -778,6 +800,7 @@ __global__ void __launch_bounds__(EX_WARPS * 32) k_exact_decide(const __grid_con
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     unsigned phase = 0u; // bit h: parity of full[h]'s next completion
+    bool left = false;   // a cell to be attempted sequentially
     const int *off = v.act_off + ci * (v.R + 1);
     const long long *er = v.ex_r + (size_t)ci * (v.ex_act + 1);
     const ExactBatch eb = exact_batch(v, off, er, b);
@@ -794,7 +817,7 @@ __global__ void __launch_bounds__(EX_WARPS * 32) k_exact_decide(const __grid_con
         const CellView c = sh.c;
         if (v.rep[c.r].use_fast || c.na == 0) continue; // (an empty cell has its results from the rebin)
         if (a >= eb.hi || v.ex_flag[(size_t)ci * v.ex_act + a]) {
-            if (threadIdx.x < 32) exact_cell_sequential(&v, c, lane, sh.first, sh.base);
+            left = true;
             continue;
         }
         const double2 *rows = v.ex_rows + (size_t)(er[a] - eb.row0) * 32;
@@ -808,6 +831,7 @@ __global__ void __launch_bounds__(EX_WARPS * 32) k_exact_decide(const __grid_con
         }
         if (!ok) return; // (uniform)
     }
+    if (left) exact_cells_left(&v, eb, ci, a1, sh.first, sh.base);
 }
 
 __device__ __forceinline__ void cp_row_async(void *dst, const void *src)
@@ -971,6 +995,7 @@ __global__ void __launch_bounds__(32) k_exact_decide_warp(const __grid_constant_
     phase_begin();
     __shared__ int s_first[27], s_base[28];
     const int lane = threadIdx.x;
+    bool left = false; // a cell to be attempted sequentially
     const int *off = v.act_off + ci * (v.R + 1);
     const long long *er = v.ex_r + (size_t)ci * (v.ex_act + 1);
     const ExactBatch eb = exact_batch(v, off, er, b);
@@ -981,7 +1006,7 @@ __global__ void __launch_bounds__(32) k_exact_decide_warp(const __grid_constant_
         if (v.rep[c.r].use_fast || c.na == 0) continue; // (an empty cell has its results from the rebin)
         cell_stencil(v, c, lane, s_first, s_base);
         if (a >= eb.hi || v.ex_flag[(size_t)ci * v.ex_act + a]) {
-            exact_cell_sequential(&v, c, lane, s_first, s_base);
+            left = true;
             continue;
         }
         const double2 *rows = v.ex_rows + (size_t)(er[a] - eb.row0) * 32;
@@ -993,6 +1018,7 @@ __global__ void __launch_bounds__(32) k_exact_decide_warp(const __grid_constant_
         default: exact_decide_cell_warp<EX_J>(v, c, lane, q13, rows, ex_buf); break;
         }
     }
+    if (left) exact_cells_left(&v, eb, ci, a1, s_first, s_base);
 }
 
 // Total energy (tot_ene, MCnptColloid.c:1598-1622) in FP64, warp per particle:
@@ -1197,7 +1223,9 @@ void launch_phase_exact(const DevView &v, cudaStream_t s, int ci, int grid)
     for (int b = 0; b < v.ex_nb; b++) {
         launch_phase(k_exact_terms, gt, 128, 0, s, v, ci, b);
         // up to a cell per SM the patterns' warps are idle ones: 1000 particles (one active cell or eight) 0.655 ->
-        // 0.48 ms of phases per sweep, 8192 (27) 0.51 -> 0.465; 65,536 (343) would take 1.72 instead of 1.50
+        // 0.48 ms of phases per sweep, 8192 (27) 0.51 -> 0.465; 65,536 (343) would take 1.72 instead of 1.50.  What is
+        // compared is the most active cells the context was made for, ex_act: cells of its FP32 systems and of NPT
+        // boxes at 1.25 times their edge count too, so a few FP64 boxes among them take a warp per cell
         if (v.ex_act <= EX_SMS) launch_phase(k_exact_decide, gd, EX_WARPS * 32, EX_BYTES, s, v, ci, b);
         else launch_phase(k_exact_decide_warp, gd, 32, EX_PIPE_BYTES, s, v, ci, b);
     }
