@@ -422,8 +422,8 @@ def npt_da(lcmc, torch, sweeps, train_sweeps):
         "sweeps_per_s_ratio": {"learned": pl["ms_per_sweep"] / le["ms_per_sweep"],
                                "fp32_screen": pl["ms_per_sweep"] / sc["ms_per_sweep"]},
         "ess_note": "tau_int by Sokal's automatic window (c=5); with tau of a few hundred sweeps the ESS of one "
-                    "arm has a relative error of tens of percent, except that the fp32_screen arm repeats the "
-                    "plain arm's decisions (p2_series_equals_plain), so its ratio is exactly the sweep-rate ratio",
+                    "arm has a relative error of tens of percent; where the fp32_screen arm repeats the plain arm's "
+                    "decisions (p2_series_equals_plain), its ratio is exactly the sweep-rate ratio",
         "seconds_total": time.perf_counter() - t_start}
 
 

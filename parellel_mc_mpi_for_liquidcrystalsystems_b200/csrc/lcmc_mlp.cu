@@ -12,6 +12,7 @@
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -633,6 +634,151 @@ __global__ void k_adam(float *w, const float *g, float *m, float *v, int n, floa
 // ---------------------------------------------------------------------------
 using namespace lcmc;
 
+// Host rows on their way to the device: rounding and its threads (send_rows has the rest).
+
+// float -> BF16, round to nearest even, NaN to 0x7fff as __float2bfloat16 does
+static inline uint16_t bf16_bits(float f)
+{
+    uint32_t u;
+    memcpy(&u, &f, 4);
+    if ((u & 0x7fffffffu) > 0x7f800000u) return 0x7fff;
+    return (uint16_t)((u + 0x7fffu + ((u >> 16) & 1u)) >> 16);
+}
+
+static void convert_row(const float *x, int n_in, int k1, uint16_t *dst)
+{
+    int i = 0;
+#ifdef __SSE2__
+    const __m128i one = _mm_set1_epi32(1), bias = _mm_set1_epi32(0x7fff);
+    for (; i + 8 <= n_in; i += 8) {
+        const __m128 f0 = _mm_loadu_ps(x + i), f1 = _mm_loadu_ps(x + i + 4);
+        const __m128i u0 = _mm_castps_si128(f0), u1 = _mm_castps_si128(f1);
+        const __m128i v0 = _mm_add_epi32(_mm_add_epi32(u0, bias), _mm_and_si128(_mm_srli_epi32(u0, 16), one));
+        const __m128i v1 = _mm_add_epi32(_mm_add_epi32(u1, bias), _mm_and_si128(_mm_srli_epi32(u1, 16), one));
+        _mm_storeu_si128((__m128i *)(dst + i), _mm_packs_epi32(_mm_srai_epi32(v0, 16), _mm_srai_epi32(v1, 16)));
+        if (_mm_movemask_ps(_mm_cmpunord_ps(f0, f1))) // a NaN among them
+            for (int k = 0; k < 8; k++) dst[i + k] = bf16_bits(x[i + k]);
+    }
+#endif
+    for (; i < n_in; i++) dst[i] = bf16_bits(x[i]);
+    for (; i < k1; i++) dst[i] = 0;
+}
+
+// Host threads that round rows for a network: they come with its first large call,
+// sleep between calls and end with it.  A part is done when its rows are: the
+// caller takes rows like every thread, and a thread that is not scheduled in time
+// (other threads of the process may hold the cores) finds nothing left to do.
+// When every thread had to report, and to end with the call, the first prediction
+// of 600 rows after other host work took 4.5 ms, now 1.0 (a quiet host 1.1, now 0.9);
+// predictions of 4096 rows 2.15 -> 1.85 ms, 2048 rows of training 2.2-2.9 -> 2.13.
+class RowConverter {
+public:
+    ~RowConverter()
+    {
+        if (threads_.empty()) return;
+        if (getpid() != pid_) { // a child process: the threads are the parent's
+            for (auto &t : threads_) t.detach();
+            return;
+        }
+        {
+            std::lock_guard<std::mutex> l(mu_);
+            stop_.store(true);
+        }
+        cv_.notify_all();
+        for (auto &t : threads_) t.join();
+    }
+    // Before the parts of a call of that many values: threads in proportion (waking one takes as long as rounding a
+    // few hundred KB), so that small calls are the caller's alone.
+    void begin(size_t values)
+    {
+        want_ = (int)std::min<size_t>(values >> 19, 12);
+        if (want_ <= 1) return;
+        const int hw = (int)std::thread::hardware_concurrency();
+        want_ = std::min(want_, hw > 0 ? hw : 1);
+        if (threads_.empty()) pid_ = getpid();
+        else if (getpid() != pid_) want_ = 1;
+        try {
+            threads_.reserve(16);
+            while ((int)threads_.size() < want_ - 1) threads_.emplace_back([this] { work(); });
+        } catch (...) { // fewer threads then
+        }
+        active_.store(true);
+    }
+    // After a call's last part: the threads may sleep.
+    void end() { active_.store(false); }
+    bool alone() const { return want_ <= 1; }
+    // rows idx[r] (idx null: r) of x -> rows r of dst
+    void run(const float *x, const int *idx, int n, int n_in, int k1, uint16_t *dst)
+    {
+        const uint64_t gen = ++part_;
+        next_.store(gen << 32 | 0xffffffffu); // closed: no thread takes a row by the last part's count
+        x_ = x, idx_ = idx, n_in_ = n_in, k1_ = k1, dst_ = dst;
+        n_.store(n);
+        done_.store(0);
+        next_.store(gen << 32);
+        if (!alone()) {
+            {
+                std::lock_guard<std::mutex> l(mu_);
+                gen_.store(gen);
+            }
+            if (want_ > (int)threads_.size()) cv_.notify_all(); // (one call of the system for all of them)
+            else
+                for (int i = 1; i < want_; i++) cv_.notify_one();
+        }
+        rows(gen);
+        while (done_.load() < n) std::this_thread::yield(); // (rows that a thread has taken)
+    }
+
+private:
+    // rows of part `gen` until none is left
+    void rows(uint64_t gen)
+    {
+        constexpr int STEP = 8;
+        for (uint64_t v = next_.load(); v >> 32 == (gen & 0xffffffffu);) {
+            const uint32_t r0 = (uint32_t)v;
+            const int n = n_.load();
+            if (r0 >= (uint32_t)n) return;
+            if (!next_.compare_exchange_weak(v, v + STEP)) continue; // (taken: the part's description holds until it is done)
+            const int r1 = std::min(n, (int)r0 + STEP);
+            for (int r = (int)r0; r < r1; r++)
+                convert_row(x_ + (size_t)(idx_ ? idx_[r] : r) * n_in_, n_in_, k1_, dst_ + (size_t)r * k1_);
+            done_.fetch_add(r1 - (int)r0);
+            v = next_.load();
+        }
+    }
+    void work()
+    {
+        uint64_t seen = 0;
+        for (;;) {
+            // the next part of a call follows within 10 to 100 us (a training step's launches lie between two
+            // batches): look for it a while before sleeping
+            for (int i = 0; i < 2048 && active_.load() && gen_.load() == seen && !stop_.load(); i++)
+                std::this_thread::yield();
+            if (gen_.load() == seen) {
+                std::unique_lock<std::mutex> l(mu_);
+                cv_.wait(l, [&] { return stop_.load() || gen_.load() != seen; });
+            }
+            if (stop_.load()) return;
+            seen = gen_.load();
+            rows(seen);
+        }
+    }
+    std::vector<std::thread> threads_;
+    std::mutex mu_;
+    std::condition_variable cv_;
+    std::atomic<uint64_t> next_{0}; // part (32 bits), its next row
+    std::atomic<uint64_t> gen_{0};  // the part the threads are told of
+    std::atomic<int> n_{0}, done_{0};
+    std::atomic<bool> stop_{false}, active_{false};
+    uint64_t part_ = 0;
+    int want_ = 1;
+    pid_t pid_ = 0;
+    const float *x_ = nullptr;
+    const int *idx_ = nullptr;
+    int n_in_ = 0, k1_ = 0;
+    uint16_t *dst_ = nullptr;
+};
+
 struct lcmc_mlp {
     int n_in = 0, k1 = 0, hid = 0, bmax = 0;
     cudaStream_t s = nullptr;
@@ -641,7 +787,7 @@ struct lcmc_mlp {
     float *P = nullptr, *G = nullptr, *Mm = nullptr, *Vv = nullptr; // parameter / grad / moment blocks
     size_t np = 0;
     bf16 *W1b = nullptr, *W2b = nullptr, *W2bT = nullptr;
-    // activations (bmax rows)
+    char *base = nullptr; // of the weights above and the activations (bmax rows)
     bf16 *X = nullptr, *XT = nullptr, *H1 = nullptr, *H1T = nullptr, *dZ2 = nullptr, *dZ2T = nullptr, *dZ1T = nullptr;
     float *Z1 = nullptr, *Z2 = nullptr, *A2 = nullptr, *y = nullptr, *t = nullptr, *dy = nullptr, *row_loss = nullptr,
           *dH1 = nullptr, *loss = nullptr;
@@ -651,6 +797,7 @@ struct lcmc_mlp {
     uint16_t *stage = nullptr; // pinned, SLOTS x STAGE_ROWS rows of k1 BF16 values each
     cudaEvent_t sent[SLOTS] = {nullptr, nullptr};
     int slot = 0;
+    RowConverter rc;
     // training: the rows (BF16), an epoch's targets and places of its rows, its losses (grown as needed)
     bf16 *rows = nullptr;
     float *et = nullptr, *losses = nullptr;
@@ -672,9 +819,7 @@ extern "C" int lcmc_mlp_destroy(lcmc_mlp *m)
 {
     if (!m) return LCMC_EINVAL;
     if (m->s) cudaStreamSynchronize(m->s);
-    void *ptrs[] = {m->P, m->G, m->Mm, m->Vv, m->W1b, m->W2b, m->W2bT, m->X, m->XT, m->H1, m->H1T, m->dZ2,
-                    m->dZ2T, m->dZ1T, m->Z1, m->Z2, m->A2, m->y, m->t, m->dy, m->row_loss, m->dH1, m->loss,
-                    m->err, m->yall, m->rows, m->et, m->losses, m->pos};
+    void *ptrs[] = {m->base, m->yall, m->rows, m->et, m->losses, m->pos};
     if (m->stage) cudaFreeHost(m->stage);
     for (cudaEvent_t ev : m->sent)
         if (ev) cudaEventDestroy(ev);
@@ -719,38 +864,30 @@ extern "C" int lcmc_mlp_create(int n_in, int hidden, int max_batch, uint64_t see
         lcmc_mlp_destroy(m);
         return LCMC_ECUDA;
     }
-#define MA(ptr, bytes)                                                                                                \
-    do {                                                                                                              \
-        if ((e = cudaMalloc((void **)&(ptr), (bytes))) != cudaSuccess) {                                              \
-            lcmc_mlp_destroy(m);                                                                                      \
-            return LCMC_ENOMEM;                                                                                       \
-        }                                                                                                             \
-    } while (0)
-    MA(m->P, m->np * 4);
-    MA(m->G, m->np * 4);
-    MA(m->Mm, m->np * 4);
-    MA(m->Vv, m->np * 4);
-    MA(m->W1b, (size_t)H * K1 * 2);
-    MA(m->W2b, (size_t)H * H * 2);
-    MA(m->W2bT, (size_t)H * H * 2);
-    MA(m->X, (size_t)B * K1 * 2);
-    MA(m->XT, (size_t)B * K1 * 2);
-    MA(m->H1, (size_t)B * H * 2);
-    MA(m->H1T, (size_t)B * H * 2);
-    MA(m->dZ2, (size_t)B * H * 2);
-    MA(m->dZ2T, (size_t)B * H * 2);
-    MA(m->dZ1T, (size_t)B * H * 2);
-    MA(m->Z1, (size_t)B * H * 4);
-    MA(m->Z2, (size_t)B * H * 4);
-    MA(m->A2, (size_t)B * H * 4);
-    MA(m->y, (size_t)B * 4);
-    MA(m->t, (size_t)B * 4);
-    MA(m->dy, (size_t)B * 4);
-    MA(m->row_loss, (size_t)B * 4);
-    MA(m->dH1, (size_t)B * H * 4);
-    MA(m->loss, 4);
-    MA(m->err, 4);
-#undef MA
+    // one allocation: a dozen MB, where each of its own would take as long as all of it
+    const std::pair<void **, size_t> bufs[] = {
+        {(void **)&m->P, m->np * 4}, {(void **)&m->G, m->np * 4}, {(void **)&m->Mm, m->np * 4},
+        {(void **)&m->Vv, m->np * 4}, {(void **)&m->W1b, (size_t)H * K1 * 2}, {(void **)&m->W2b, (size_t)H * H * 2},
+        {(void **)&m->W2bT, (size_t)H * H * 2}, {(void **)&m->X, (size_t)B * K1 * 2},
+        {(void **)&m->XT, (size_t)B * K1 * 2}, {(void **)&m->H1, (size_t)B * H * 2},
+        {(void **)&m->H1T, (size_t)B * H * 2}, {(void **)&m->dZ2, (size_t)B * H * 2},
+        {(void **)&m->dZ2T, (size_t)B * H * 2}, {(void **)&m->dZ1T, (size_t)B * H * 2},
+        {(void **)&m->Z1, (size_t)B * H * 4}, {(void **)&m->Z2, (size_t)B * H * 4},
+        {(void **)&m->A2, (size_t)B * H * 4}, {(void **)&m->y, (size_t)B * 4}, {(void **)&m->t, (size_t)B * 4},
+        {(void **)&m->dy, (size_t)B * 4}, {(void **)&m->row_loss, (size_t)B * 4},
+        {(void **)&m->dH1, (size_t)B * H * 4}, {(void **)&m->loss, 4}, {(void **)&m->err, 4}};
+    size_t total = 0;
+    for (const auto &b : bufs) total += (b.second + 255) / 256 * 256;
+    if (cudaMalloc((void **)&m->base, total) != cudaSuccess) {
+        cudaGetLastError();
+        lcmc_mlp_destroy(m);
+        return LCMC_ENOMEM;
+    }
+    size_t at = 0;
+    for (const auto &b : bufs) {
+        *b.first = m->base + at;
+        at += (b.second + 255) / 256 * 256;
+    }
     e = cudaMallocHost((void **)&m->stage, (size_t)lcmc_mlp::SLOTS * lcmc_mlp::STAGE_ROWS * K1 * 2);
     for (cudaEvent_t &ev : m->sent)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
@@ -832,113 +969,11 @@ int *mlp_err(lcmc_mlp *m) { return m->err; }
 // staging, and that was nearly all of a call.  Here host threads round them to
 // BF16, which the network takes, into pinned buffers whose copies run while the
 // next rows are converted: half the bytes on the link.  Predictions of 4096 rows
-// 8.2 -> 2.2 ms, an epoch of 2048 rows in batches of 256 10.6 -> 2.2 ms; bound by
-// the threads' reads of the FP32 rows (67 MB in 4096 of them).
+// 8.2 -> 1.85 ms, an epoch of 2048 rows in batches of 256 10.6 -> 2.1 ms; bound by
+// the threads' reads of the FP32 rows (67 MB in 4096 of them).  That is for rows
+// used again and again; the first call of a new network on new rows 8.8 -> 2.6 ms
+// (4096 rows) on a quiet host, 9.2 -> 3.6 where other threads still hold the cores.
 // ---------------------------------------------------------------------------
-
-// float -> BF16, round to nearest even, NaN to 0x7fff as __float2bfloat16 does
-static inline uint16_t bf16_bits(float f)
-{
-    uint32_t u;
-    memcpy(&u, &f, 4);
-    if ((u & 0x7fffffffu) > 0x7f800000u) return 0x7fff;
-    return (uint16_t)((u + 0x7fffu + ((u >> 16) & 1u)) >> 16);
-}
-
-static void convert_row(const float *x, int n_in, int k1, uint16_t *dst)
-{
-    int i = 0;
-#ifdef __SSE2__
-    const __m128i one = _mm_set1_epi32(1), bias = _mm_set1_epi32(0x7fff);
-    for (; i + 8 <= n_in; i += 8) {
-        const __m128 f0 = _mm_loadu_ps(x + i), f1 = _mm_loadu_ps(x + i + 4);
-        const __m128i u0 = _mm_castps_si128(f0), u1 = _mm_castps_si128(f1);
-        const __m128i v0 = _mm_add_epi32(_mm_add_epi32(u0, bias), _mm_and_si128(_mm_srli_epi32(u0, 16), one));
-        const __m128i v1 = _mm_add_epi32(_mm_add_epi32(u1, bias), _mm_and_si128(_mm_srli_epi32(u1, 16), one));
-        _mm_storeu_si128((__m128i *)(dst + i), _mm_packs_epi32(_mm_srai_epi32(v0, 16), _mm_srai_epi32(v1, 16)));
-        if (_mm_movemask_ps(_mm_cmpunord_ps(f0, f1))) // a NaN among them
-            for (int k = 0; k < 8; k++) dst[i + k] = bf16_bits(x[i + k]);
-    }
-#endif
-    for (; i < n_in; i++) dst[i] = bf16_bits(x[i]);
-    for (; i < k1; i++) dst[i] = 0;
-}
-
-// The threads of one call: rows [0, n) of a batch split among them.  They live
-// from the first batch to the end of the call.
-class RowConverter {
-public:
-    RowConverter(size_t values)
-    {
-        // one thread for small calls (starting a thread takes as long as converting a few hundred KB)
-        const unsigned hw = std::thread::hardware_concurrency();
-        const int want = (int)std::min<size_t>(values >> 19, std::min(hw ? hw : 1u, 12u));
-        try {
-            threads_.reserve(want > 1 ? want - 1 : 0);
-            for (int i = 1; i < want; i++) threads_.emplace_back([this] { work(); });
-        } catch (...) { // fewer threads then
-        }
-    }
-    ~RowConverter()
-    {
-        {
-            std::lock_guard<std::mutex> l(mu_);
-            stop_.store(true);
-        }
-        cv_.notify_all();
-        for (auto &t : threads_) t.join();
-    }
-    bool alone() const { return threads_.empty(); }
-    // rows idx[r] (idx null: r) of x -> rows r of dst
-    void run(const float *x, const int *idx, int n, int n_in, int k1, uint16_t *dst)
-    {
-        x_ = x, idx_ = idx, n_ = n, n_in_ = n_in, k1_ = k1, dst_ = dst;
-        next_.store(0);
-        busy_.store((int)threads_.size());
-        {
-            std::lock_guard<std::mutex> l(mu_);
-            gen_.fetch_add(1);
-        }
-        cv_.notify_all();
-        rows();
-        while (busy_.load() > 0) std::this_thread::yield(); // (the last rows of other threads)
-    }
-
-private:
-    void rows()
-    {
-        constexpr int STEP = 8;
-        for (int r0; (r0 = next_.fetch_add(STEP)) < n_;)
-            for (int r = r0; r < std::min(n_, r0 + STEP); r++)
-                convert_row(x_ + (size_t)(idx_ ? idx_[r] : r) * n_in_, n_in_, k1_, dst_ + (size_t)r * k1_);
-    }
-    void work()
-    {
-        long long seen = 0;
-        for (;;) {
-            // the next part follows within some 10 us: look for it before sleeping
-            for (int i = 0; i < 64 && gen_.load() == seen && !stop_.load(); i++) std::this_thread::yield();
-            if (gen_.load() == seen) {
-                std::unique_lock<std::mutex> l(mu_);
-                cv_.wait(l, [&] { return stop_.load() || gen_.load() != seen; });
-            }
-            if (stop_.load()) return;
-            seen = gen_.load();
-            rows();
-            busy_.fetch_sub(1);
-        }
-    }
-    std::vector<std::thread> threads_;
-    std::mutex mu_;
-    std::condition_variable cv_;
-    std::atomic<int> next_{0}, busy_{0};
-    std::atomic<long long> gen_{0};
-    std::atomic<bool> stop_{false};
-    const float *x_ = nullptr;
-    const int *idx_ = nullptr;
-    int n_ = 0, n_in_ = 0, k1_ = 0;
-    uint16_t *dst_ = nullptr;
-};
 
 // Below 256 rows a single thread converts: its parts are small, so that only the
 // last one's copy is left when it is done (96 rows: 245 us a call with one part, 209
@@ -947,17 +982,17 @@ constexpr int SMALL_PART = 32;
 
 // Rows idx[0 .. n) (idx null: the first n) of the caller's features to rows [0, B)
 // of dst on the network's stream, zeros beyond n.
-static cudaError_t send_rows(lcmc_mlp *m, RowConverter &rc, const float *x, const int *idx, int n, int B, bf16 *dst)
+static cudaError_t send_rows(lcmc_mlp *m, const float *x, const int *idx, int n, int B, bf16 *dst)
 {
     cudaError_t e;
     const size_t row = (size_t)m->k1 * 2;
-    const int step = rc.alone() ? SMALL_PART : lcmc_mlp::STAGE_ROWS;
+    const int step = m->rc.alone() ? SMALL_PART : lcmc_mlp::STAGE_ROWS;
     for (int off = 0; off < n; off += step) {
         const int i = m->slot, c = std::min(step, n - off);
         m->slot = (i + 1) % lcmc_mlp::SLOTS;
         if ((e = cudaEventSynchronize(m->sent[i])) != cudaSuccess) return e; // its last copy has left
         uint16_t *stage = m->stage + (size_t)i * lcmc_mlp::STAGE_ROWS * m->k1;
-        rc.run(idx ? x : x + (size_t)off * m->n_in, idx ? idx + off : nullptr, c, m->n_in, m->k1, stage);
+        m->rc.run(idx ? x : x + (size_t)off * m->n_in, idx ? idx + off : nullptr, c, m->n_in, m->k1, stage);
         e = cudaMemcpyAsync(dst + (size_t)off * m->k1, stage, (size_t)c * row, cudaMemcpyHostToDevice, m->s);
         if (e != cudaSuccess) return e;
         if ((e = cudaEventRecord(m->sent[i], m->s)) != cudaSuccess) return e;
@@ -974,15 +1009,16 @@ extern "C" int lcmc_mlp_predict(lcmc_mlp *m, const float *x, int n, float *y)
         // outputs of several batches gather on the device: one copy back, after the last rows
         const bool gather = n > m->bmax;
         if (gather && (e = grow(&m->yall, &m->yall_n, (size_t)(n + 127) / 128 * 128)) != cudaSuccess) return mlp_fail(m, "predict", e);
-        RowConverter rc((size_t)n * m->n_in);
+        m->rc.begin((size_t)n * m->n_in);
         for (int off = 0; off < n && e == cudaSuccess; off += m->bmax) {
             const int nb = n - off < m->bmax ? n - off : m->bmax;
             const int B = (nb + 127) / 128 * 128;
-            e = send_rows(m, rc, x + (size_t)off * m->n_in, nullptr, nb, B, m->X);
+            e = send_rows(m, x + (size_t)off * m->n_in, nullptr, nb, B, m->X);
             if (e != cudaSuccess) break;
             mlp_forward_s(m, m->X, B, nullptr, nb, m->s);
             if (gather) e = cudaMemcpyAsync(m->yall + off, m->y, (size_t)nb * 4, cudaMemcpyDeviceToDevice, m->s);
         }
+        m->rc.end();
         if (e == cudaSuccess) e = cudaMemcpyAsync(y, gather ? m->yall : m->y, (size_t)n * 4, cudaMemcpyDeviceToHost, m->s);
     }
     const cudaError_t es = cudaStreamSynchronize(m->s);
@@ -1034,10 +1070,9 @@ extern "C" int lcmc_mlp_gradients(lcmc_mlp *m, const float *x, const float *t, i
     if (!m || !x || !t || !grad || n <= 0 || n > m->bmax) return LCMC_EINVAL;
     const int B = (n + 127) / 128 * 128;
     cudaError_t e;
-    {
-        RowConverter rc((size_t)n * m->n_in);
-        e = send_rows(m, rc, x, nullptr, n, B, m->X);
-    }
+    m->rc.begin((size_t)n * m->n_in);
+    e = send_rows(m, x, nullptr, n, B, m->X);
+    m->rc.end();
     if (e != cudaSuccess) return mlp_fail(m, "gradients", e);
     cudaMemsetAsync(m->t, 0, (size_t)B * 4, m->s);
     cudaMemcpyAsync(m->t, t, (size_t)n * 4, cudaMemcpyHostToDevice, m->s);
@@ -1096,7 +1131,7 @@ extern "C" int lcmc_mlp_train(lcmc_mlp *m, const float *x, const float *t, int n
         cudaGetLastError();
         keep = false;
     }
-    RowConverter rc((size_t)n * m->n_in);
+    m->rc.begin((size_t)n * m->n_in);
     for (int ep = 0; ep < epochs && e == cudaSuccess && nb > 0; ep++) {
         for (int i = n - 1; i > 0; i--) { // shuffle
             U4 o = draw(key, (uint32_t)i, (uint64_t)ep, 0x301u);
@@ -1121,7 +1156,7 @@ extern "C" int lcmc_mlp_train(lcmc_mlp *m, const float *x, const float *t, int n
                 if (B > batch)
                     e = cudaMemsetAsync(m->X + (size_t)batch * K1, 0, (size_t)(B - batch) * K1 * 2, m->s);
             } else {
-                e = send_rows(m, rc, x, idx.data() + off, batch, B, m->X);
+                e = send_rows(m, x, idx.data() + off, batch, B, m->X);
                 if (e == cudaSuccess && keep)
                     e = cudaMemcpyAsync(m->rows + (size_t)off * K1, m->X, (size_t)batch * K1 * 2,
                                         cudaMemcpyDeviceToDevice, m->s);
@@ -1131,8 +1166,10 @@ extern "C" int lcmc_mlp_train(lcmc_mlp *m, const float *x, const float *t, int n
             mlp_update(m, lr);
         }
         if (ep == 0 && keep && e == cudaSuccess && used < n) // rows that no batch of the first epoch took
-            e = send_rows(m, rc, x, idx.data() + used, n - used, n - used, m->rows + (size_t)used * K1);
+            e = send_rows(m, x, idx.data() + used, n - used, n - used, m->rows + (size_t)used * K1);
+        if (keep) m->rc.end(); // (later epochs send none)
     }
+    m->rc.end();
     if (e == cudaSuccess && nb > 0)
         e = cudaMemcpyAsync(losses.data(), m->losses, (size_t)nb * 4, cudaMemcpyDeviceToHost, m->s);
     const cudaError_t es = cudaStreamSynchronize(m->s);

@@ -84,19 +84,6 @@
 
 namespace lcmc {
 
-__device__ __forceinline__ int find_replica_f(const int *off, int R, int a)
-{
-    int lo = 0, hi = R;
-    while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (off[mid] <= a) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
-__device__ __forceinline__ int tri(int p, int q) { return (q * (q - 1)) / 2 + p; } // p < q
-
 // FP64 pair term for a pair the FP32 term cannot carry: pair_energy64's
 // form for mu = 2, nu = 1, sigma0 = 1, else the reference-order pair_exact.
 template <bool SPEC21>
@@ -113,8 +100,8 @@ struct BigPair {
 
 // Both states of one static pair (active particle at slot gk, its trial
 // state, candidate at slot gj) in FP64 from the master arrays, on the one-fold
-// minimum image, the cutoff decided in FP64.  Not inlined: the rare path keeps
-// its registers out of the hot loop's allocation.
+// minimum image, the cutoff decided in FP64.  (For fixup_big, which is not
+// inlined: the rare path keeps its registers out of the hot loop's allocation.)
 template <bool SPEC21>
 __device__ __forceinline__ BigPair big_pair64(const double *__restrict__ px, const double *__restrict__ py,
                                            const double *__restrict__ pz, const double *__restrict__ ox,

@@ -43,3 +43,20 @@ def test_gas_shape_agrees(n, L, kw):
     assert np.array_equal(out, want) and st["accepted"] == sb["accepted"] and st["energy"] == sb["energy"]
     for x, y in zip(a, b):
         assert np.array_equal(x, y)
+
+
+def test_cells_above_the_arrays_run_in_fp32():
+    """41 to 48 rods in the cells of a slab, more than the light shape's arrays hold: none is left to FP64, so the
+    hand-over kernel ran them in FP32."""
+    L = 36.0
+    pos = slab(L, 0.45, 1.15, 3.05)
+    n = len(pos[0])
+    with lcmc.GBSystem(lcmc.default_params(num_particles=n, system_density=n / L**3, gb_kappa=3.0, gb_kappa_prime=5.0,
+                                           gb_mu_exponent=2.0, gb_nu_exponent=1.0, cutoff_radius=4.0, max_displacement=0.02,
+                                           max_rotation=0.02, precision_mode=1, rng_seed=5)) as s:
+        s.upload(*pos, np.zeros(n), np.zeros(n), np.ones(n), np.full(3, L), energy=0.0)
+        s.sweep(2)
+        st = s.stats()
+    cells = np.floor(np.array(pos) / (L / 8)).astype(int)
+    assert np.bincount(cells[0] + 8 * (cells[1] + 8 * cells[2])).max() > 40
+    assert st["kernel"] == 1 and st["fp64_cells"] == 0 and st["attempted"] == 2 * n
