@@ -272,9 +272,9 @@ def kernel_traffic():
     k_phase_fast launch on this workload and where the figure comes from: a
     fixed ncu capture (ncu cannot run inside the timed process), so it is
     the same in every run and is refreshed when the kernel changes."""
-    return 47.222980e6 + 1.815793e6, ("fixed, from ncu (dram__bytes_read.sum + dram__bytes_write.sum) over 17 "
-                                      "k_phase_fast launches of this workload, 22-24 sweeps from the lattice start "
-                                      "(47.2 MB read + 1.8 MB written per launch); not measured in this run")
+    return 47.73e6 + 1.72e6, ("fixed, from ncu (dram__bytes_read.sum + dram__bytes_write.sum) over 18 k_phase_fast "
+                              "launches of this workload, 20-22 sweeps from the lattice start (47.7 MB read + 1.7 MB "
+                              "written per launch); not measured in this run")
 
 
 # ---------------------------------------------------------------------------

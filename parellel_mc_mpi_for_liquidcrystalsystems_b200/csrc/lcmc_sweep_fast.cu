@@ -24,7 +24,7 @@
 // What bounds it: one cell's attempt is a chain of short stages (staging, reach
 // tests, pair terms, decisions, write-back) with a block barrier between them,
 // so an SM needs several cells in flight, and how many is set by the shared
-// memory of one (36-74 KB); with six blocks of four warps the schedulers issue
+// memory of one (36-74 KB, 21 KB for the cells of a gas); with six blocks of four warps the schedulers issue
 // in 58 % of the cycles (the pair terms take 37 % of the instructions, the
 // MUFU pipe is at 29 %, DRAM at 3 %).  Stages of a cell:
 //   1 copies   the 26 static cells' FP32 states (float4 x,y,z,ux and float2
@@ -54,7 +54,7 @@
 // the capacity class: a system's moves do not depend on how it is batched.
 // One B200, 1,048,576 rods at rho* = 0.32 (5832 cells per phase), all eight
 // phases: 1.97 ms before the tests went to matrix instructions and the terms to
-// packed operations, 1.51 ms now; 262,144 rods at 0.28: 0.57 -> 0.46 ms; a grid
+// packed operations, 1.49 ms now; 262,144 rods at 0.28: 0.57 -> 0.46 ms; a grid
 // of at most one cell per SM (wide blocks): 0.32 -> 0.19 ms (32,768 rods NPT).
 //
 // FP64 for overlaps: FP32 rounding of a pair term is relative to the term,
